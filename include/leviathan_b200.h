@@ -315,10 +315,7 @@ int lev_set_grid_wait(LevEngine *h, uint64_t limit_ns, uint32_t extra_arrivals);
 int lev_num_pair_variants(void);
 int lev_pair_variant_info(int32_t v, int32_t *unroll, int32_t *min_blocks,
                           int32_t *deep);
-/* Threads per row of pair variant v (1, or 4: the row's SELL entries split
- * over four lanes, for low-degree networks; the coupling sum is formed in
- * CSR order from the four lanes' terms, bitwise as with one lane).  The
- * autotuner searches this dimension with the others, per degree class. */
+/* Threads per row of pair variant v (1). */
 int lev_pair_variant_lanes(int32_t v, int32_t *lanes);
 int lev_pair_info(const LevEngine *h, int32_t c, int32_t *eligible, int32_t *enabled,
                   int32_t *pair_variant, float *pair_ms, float *step_ms);

@@ -85,28 +85,38 @@ static const StepVariant kVariants[] = {
 constexpr int kNumVariants = sizeof(kVariants) / sizeof(kVariants[0]);
 
 // Two-steps-per-launch variants (lev_pair.cuh): pair_kernel<MATH, U, MINB,
-// DEEP> (DEEP: two-stage software pipeline).  Measured on B200: fewer
-// resident CTAs with more loads in flight per lane win at large networks
-// (the L1 keeps the tile's ring lines and col/delay words between the two
-// walks); more CTAs win at the small networks of a sweep.
-// LANES: threads per row (1: pair_kernel, 256-thread CTAs; 4: pair4_kernel,
-// 1024-thread CTAs for low-degree rows).
+// DEEP> (DEEP: two-stage software pipeline).  Measured on B200 (us per pair
+// launch, reduce included; 1M: N = 10^6, k = 32; 1M8: N = 10^6, k = 8; 100k:
+// N = 10^5, k = 20; sweep: 128 networks, 29 M edges):
+//          (8,3,0) (6,3,1) (6,3,0) (4,4,1) (4,4,0) (8,2,1) (12,2,0)
+//   1M       257     264     270     309     302     289     265
+//   1M8      133     126     126     125     124     179     137
+//   100k    27.5    28.0    25.9    28.5    25.9    29.5    27.5
+//   sweep    262     265     261     270     265     319     287
+// Long rows want many entries in flight per lane, short rows and networks of
+// less than one wave more resident CTAs.
 struct PairVariant {
-  int U, MINB, DEEP, LANES;
+  int U, MINB, DEEP;
   StepFn fn[2];  // [math mode]
 };
 #define LEV_PAIR_VARIANT(U, M, D) \
-  { U, M, D, 1, { pair_kernel<0, U, M, D>, pair_kernel<1, U, M, D> } }
-#define LEV_PAIR4_VARIANT(U, M) \
-  { U, M, 0, 4, { pair4_kernel<0, U, M>, pair4_kernel<1, U, M> } }
+  { U, M, D, { pair_kernel<0, U, M, D>, pair_kernel<1, U, M, D> } }
 static const PairVariant kPairVariants[] = {
-    LEV_PAIR_VARIANT(8, 2, 1), LEV_PAIR_VARIANT(6, 3, 1), LEV_PAIR_VARIANT(8, 3, 0),
-    LEV_PAIR_VARIANT(4, 4, 1), LEV_PAIR_VARIANT(10, 2, 1), LEV_PAIR4_VARIANT(2, 1),
-    LEV_PAIR4_VARIANT(4, 1),
+    LEV_PAIR_VARIANT(8, 3, 0), LEV_PAIR_VARIANT(6, 3, 1), LEV_PAIR_VARIANT(6, 3, 0),
+    LEV_PAIR_VARIANT(4, 4, 1), LEV_PAIR_VARIANT(4, 4, 0), LEV_PAIR_VARIANT(8, 2, 1),
+    LEV_PAIR_VARIANT(12, 2, 0),
 };
 #undef LEV_PAIR_VARIANT
-#undef LEV_PAIR4_VARIANT
 constexpr int kNumPairVariants = sizeof(kPairVariants) / sizeof(kPairVariants[0]);
+
+// Pair variant of an engine that has not been tuned, by its tiles and mean
+// slice length, one for all its classes so that they run merged: up to one
+// wave of (4,4,0) -- 592 tiles -- or short rows, (4,4,0); up to 26 entries per
+// row (6,3,0); above, (8,3,0).  The lines follow the table above.
+inline int default_pair_variant(int ntiles, double mean_slice_len) {
+  if (ntiles <= 592 || mean_slice_len <= 14.0) return 4;
+  return mean_slice_len <= 26.0 ? 2 : 0;
+}
 
 // Networks of a batch are grouped by the mean SELL slice length (the
 // per-lane edge count): each class has its own tile list and variant.
@@ -576,9 +586,8 @@ int launch_pair_tc(LevEngine *h, const TileClass &tc, StepArgs a, int phase,
         tc.pair_variant < 0
             ? reinterpret_cast<const void *>(kVariants[tc.variant].fn[mode])
             : reinterpret_cast<const void *>(kPairVariants[tc.pair_variant].fn[mode]);
-    const int lanes = tc.pair_variant < 0 ? 1 : kPairVariants[tc.pair_variant].LANES;
     void *args[] = {&a};
-    LEV_TRY_CUDA(cudaLaunchKernel(fn, dim3(tc.ntiles), dim3(lanes * kTile), args, 0, s));
+    LEV_TRY_CUDA(cudaLaunchKernel(fn, dim3(tc.ntiles), dim3(kTile), args, 0, s));
   } else {
     const int blocks = (tc.ntiles + kFinishTiles - 1) / kFinishTiles;
     if (mode)
@@ -1510,12 +1519,16 @@ int create_impl(LevEngine **out, int num_nets, const int32_t *Ns,
     }
     {
       // remembered choices of earlier engines with a similar class
+      double len_sum = 0.0;
+      for (int c = 0; c < kNumClasses; ++c)
+        len_sum += h->classes[c].mean_len * h->classes[c].ntiles;
+      const int pv = default_pair_variant(h->total_tiles, len_sum / std::max(h->total_tiles, 1));
       std::lock_guard<std::mutex> lk(g_tune_mu);
       for (int c = 0; c < kNumClasses; ++c) {
         auto it = g_tune_cache.find(tune_key(h->classes[c], c));
         h->classes[c].variant = (it != g_tune_cache.end()) ? it->second : 0;
         auto ip = g_pair_cache.find(tune_key(h->classes[c], c));
-        h->classes[c].pair_variant = (ip != g_pair_cache.end()) ? ip->second : 0;
+        h->classes[c].pair_variant = (ip != g_pair_cache.end()) ? ip->second : pv;
       }
     }
 
@@ -2355,7 +2368,7 @@ int lev_pair_variant_info(int32_t v, int32_t *unroll, int32_t *min_blocks,
 
 int lev_pair_variant_lanes(int32_t v, int32_t *lanes) {
   if (v < 0 || v >= kNumPairVariants || !lanes) return fail(LEV_ERR_ARG, "bad pair variant");
-  *lanes = kPairVariants[v].LANES;
+  *lanes = 1;
   return LEV_OK;
 }
 
@@ -2613,6 +2626,54 @@ int lev_autotune(LevEngine *h, float dt, int32_t trial_steps,
     std::lock_guard<std::mutex> lk(g_tune_mu);
     g_tune_cache[tune_key(tc, c)] = best_v;
     if (h->pair_ok) g_pair_cache[tune_key(tc, c)] = tc.pair_variant;
+  }
+  // classes that chose different pair variants run as one chain of launches
+  // each; with one variant for all they run merged (merged_pairs).  Time both
+  // and keep the faster.
+  {
+    TileClass merged;
+    int busy = 0;
+    bool pairs = rc == LEV_OK && h->pair_ok;
+    float apart = 0.0f;
+    int own[kNumClasses];
+    for (int c = 0; c < kNumClasses; ++c) {
+      own[c] = h->classes[c].pair_variant;
+      if (h->classes[c].ntiles == 0) continue;
+      ++busy;
+      pairs = pairs && own[c] >= 0;
+      apart += h->classes[c].pair_ms;
+    }
+    if (pairs && busy > 1 && !merged_pairs(h, &merged)) {
+      int best_v = -1;
+      for (int v = 0; v < kNumPairVariants && rc == LEV_OK; ++v) {
+        bool used = false;  // the choice of some class
+        for (int c = 0; c < kNumClasses; ++c)
+          used = used || (h->classes[c].ntiles > 0 && own[c] == v);
+        if (!used) continue;
+        for (int c = 0; c < kNumClasses; ++c) h->classes[c].pair_variant = v;
+        merged_pairs(h, &merged);
+        float ms = 0.0f;
+        for (int round = 0; round < 2 && rc == LEV_OK; ++round) {  // warm-up, timed
+          cudaEventRecord(e0, h->stream);
+          for (int i = 0; i < 2 * trial_steps && rc == LEV_OK; ++i) {
+            a.reverse = i & 1;
+            rc = launch_pair_tc(h, merged, a, i & 1);
+          }
+          cudaEventRecord(e1, h->stream);
+          if (rc == LEV_OK && cudaEventSynchronize(e1) != cudaSuccess)
+            rc = fail(LEV_ERR_CUDA, "autotune: merged trial failed");
+        }
+        if (rc != LEV_OK) break;
+        cudaEventElapsedTime(&ms, e0, e1);
+        ms /= 2.0f * trial_steps;
+        if (ms < apart) {
+          apart = ms;
+          best_v = v;
+        }
+      }
+      for (int c = 0; c < kNumClasses; ++c)
+        if (h->classes[c].ntiles > 0) h->classes[c].pair_variant = best_v >= 0 ? best_v : own[c];
+    }
   }
   // small and mid-sized single networks: per-step graph replay, the
   // cluster-resident kernel or the grid-resident kernel (each rows-per-CTA
@@ -4166,12 +4227,12 @@ int lev_part_step_end(LevEngine *h, float dt, const void *partials_all_dev,
 }
 
 // The single degree class of a partition engine that takes two steps per
-// launch with a one-lane pair variant, or -1.
+// launch, or -1.
 static int part_pair_class(const LevEngine *h) {
   if (!pairs_all(h)) return -1;
   for (int c = 0; c < kNumClasses; ++c) {
     const TileClass &tc = h->classes[c];
-    if (tc.ntiles > 0) return kPairVariants[tc.pair_variant].LANES == 1 ? c : -1;
+    if (tc.ntiles > 0) return c;
   }
   return -1;
 }

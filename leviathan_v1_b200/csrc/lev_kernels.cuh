@@ -186,9 +186,44 @@ __device__ __forceinline__ float div_two_pi(float x) {
   return __fmaf_rn(rem, kInvTwoPi, q0);
 }
 
-__device__ __forceinline__ float wrap_pm_pi(float diff) {
-  // symmetric wrap to [-pi, pi): leviathan_kernel.cu:105 and :146
+// Symmetric wrap to [-pi, pi) (leviathan_kernel.cu:105 and :146) of any input.
+__device__ __forceinline__ float wrap_pm_pi_any(float diff) {
   return diff - floorf(div_two_pi(diff) + 0.5f) * kTwoPi;
+}
+
+// The same wrap for |diff| <= kWrapNear, where the floor is -1, 0 or 1: the
+// quotient, its rounding and the floor never decrease with diff, so the floor
+// steps at one float each, and diff -+ 2pi is the multiply-add of the general
+// form with a factor of one.  Differences of two phases in [0, 2pi] always
+// qualify.  Two compares and a predicated add take the place of the division
+// (three multiply-adds), the add and the floor, which runs in the quarter-rate
+// unit.  lev_selftest_wraps() checks all 2^32 inputs.
+constexpr float kWrapNear = 9.0f;              // below 3 pi - the next step is past it
+constexpr float kWrapUp = 0x1.921fb4p+1f;      // first float whose floor is 1
+constexpr float kWrapDown = -0x1.921fb6p+1f;   // first float whose floor is 0
+__device__ __forceinline__ float wrap_pm_pi_near(float diff) {
+  const float step = copysignf(kTwoPi, diff);
+  return (diff >= kWrapUp || diff < kWrapDown) ? diff - step : diff;
+}
+
+__device__ __forceinline__ float wrap_pm_pi(float diff) {
+  return fabsf(diff) <= kWrapNear ? wrap_pm_pi_near(diff) : wrap_pm_pi_any(diff);
+}
+
+// U phase differences wrapped in place: one range test for the group, the
+// general wrap only when a lane holds a value out of range (or a NaN).
+template <int U>
+__device__ __forceinline__ void wrap_pm_pi_group(float (&diff)[U]) {
+  bool far = false;
+#pragma unroll
+  for (int u = 0; u < U; ++u) far |= !(fabsf(diff[u]) <= kWrapNear);
+  if (far) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) diff[u] = wrap_pm_pi_any(diff[u]);
+  } else {
+#pragma unroll
+    for (int u = 0; u < U; ++u) diff[u] = wrap_pm_pi_near(diff[u]);
+  }
 }
 
 __device__ __forceinline__ float wrap_0_2pi(float x) {
@@ -235,6 +270,39 @@ __device__ __forceinline__ float ld_ring(const float *p) { return __ldg(p); }
 // slot then spans 32 sectors).  slots * Np < 2^32 is checked at creation.
 __host__ __device__ __forceinline__ unsigned ring_pos(int slot, unsigned col, int Np) {
   return ((unsigned)(slot >> 2) * (unsigned)Np + col) * 4u + (unsigned)(slot & 3);
+}
+
+// ring_pos of a packed edge word (col << 8 | delay) read from slot
+// (base - delay) mod bsi: the unsigned minimum of the slot with and without
+// bsi added is the one in range, and the node's and the slot's parts of the
+// index are merged bitwise.
+__device__ __forceinline__ unsigned ring_pos_word(uint32_t word, int base, int bsi, int Np) {
+  const unsigned s0 = (unsigned)(base - (int)(word & 255u));
+  const unsigned slot = min(s0, s0 + (unsigned)bsi);
+  return (slot >> 2) * ((unsigned)Np * 4u) + (((word >> 6) & ~3u) | (slot & 3u));
+}
+
+// One edge (csr_physics_kernel, leviathan_kernel.cu:146-164) from its wrapped
+// phase difference: sin of the difference and the new weight.  The caller adds
+// w * sin to the row's sum in CSR order and stores the weight, both under the
+// predicate that the entry is one of the row's, so that a walk over the padded
+// slice has no branch per entry.
+struct EdgeParams {
+  float dt, eta, lam, hebb;  // hebb = 1 - gamma |eps| of the row
+  float w_min, w_max;
+};
+template <int MATH>
+__device__ __forceinline__ float edge_update(const EdgeParams &e, float diff, float w,
+                                             float *sin_diff) {
+  float cos_diff;
+  lev_sincos<MATH>(diff, sin_diff, &cos_diff);
+  // dt * (eta cos (1 - gamma |eps|) - lam w), the products fused as nvcc fuses
+  // them in the reference; written out, because which product of the
+  // difference is fused is otherwise the compiler's choice per kernel
+  const float dw = __fmaf_rn(__fmul_rn(e.eta, cos_diff), e.hebb, -__fmul_rn(e.lam, w));
+  w = __fmaf_rn(e.dt, dw, w);
+  if (!isfinite(w)) w = e.w_min;
+  return fmaxf(e.w_min, fminf(e.w_max, w));
 }
 
 // Slots allocated per node: bsi rounded up to whole groups of four.
