@@ -81,7 +81,7 @@ struct AdjGridFwdArgs {
 template <int MATH, int R, int U>
 __device__ __forceinline__ void adj_grid_fwd_body(const AdjGridFwdArgs &a, const int cta,
                                                   const unsigned G, unsigned char *smem) {
-  constexpr int LPR = kGridLPR;
+  constexpr int LPR = kSplitLPR;
   constexpr int nslices = R / 32;
   __shared__ float s_g;
   __shared__ int s_ok;
@@ -420,7 +420,7 @@ struct AdjGridBwdArgs {
 template <int MATH, int R, int U>
 __device__ __forceinline__ void adj_grid_bwd_body(const AdjGridBwdArgs &a, const int cta,
                                                   const unsigned G, unsigned char *smem) {
-  constexpr int LPR = kGridLPR;
+  constexpr int LPR = kSplitLPR;
   constexpr int nslices = R / 32;
   __shared__ float s_red[32];
   __shared__ float s_lg;
@@ -668,14 +668,14 @@ __device__ __forceinline__ void adj_grid_bwd_body(const AdjGridBwdArgs &a, const
 }
 
 template <int MATH, int R, int U>
-__global__ void __launch_bounds__(kGridLPR * R, 256 / R)
+__global__ void __launch_bounds__(kSplitLPR * R, 256 / R)
     adj_grid_fwd_kernel(const AdjGridFwdArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
   adj_grid_fwd_body<MATH, R, U>(a, blockIdx.x, gridDim.x, smem);
 }
 
 template <int MATH, int R, int U>
-__global__ void __launch_bounds__(kGridLPR * R, R == 64 ? 2 : 1)
+__global__ void __launch_bounds__(kSplitLPR * R, R == 64 ? 2 : 1)
     adj_grid_bwd_kernel(const AdjGridBwdArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
   adj_grid_bwd_body<MATH, R, U>(a, blockIdx.x, gridDim.x, smem);
@@ -687,7 +687,7 @@ __global__ void __launch_bounds__(kGridLPR * R, R == 64 ? 2 : 1)
 // other, so the two latency-bound step chains overlap.  Every CTA of both
 // groups is resident at once (cooperative launch).
 template <int MATH, int R, int UF, int UB>
-__global__ void __launch_bounds__(kGridLPR * R, 256 / R)
+__global__ void __launch_bounds__(kSplitLPR * R, 256 / R)
     adj_grid_pair_kernel(const AdjGridFwdArgs f, const AdjGridBwdArgs b, const int gf) {
   extern __shared__ __align__(16) unsigned char smem[];
   if ((int)blockIdx.x < gf)

@@ -29,6 +29,8 @@
 
 #include <cooperative_groups.h>
 
+#include "lev_split.cuh"
+
 namespace lev {
 
 constexpr int kClusterMax = 16;     // CTAs per cluster (non-portable size)
@@ -88,6 +90,7 @@ struct ClusterArgs {
   float *omega_hat;
   float *ring;
   float *r_hist;  // [n] (row rpos + k), or null
+  HubMonitor *hubs;  // observes hub phases after every step, or null (cluster_split_kernel)
   int r_cap;
   int n_steps;
   int R;          // rows per CTA (a power of two, 32 .. 1024)
@@ -336,43 +339,96 @@ __global__ void __launch_bounds__(MAXR, 1) cluster_kernel(const ClusterArgs a) {
   cluster.sync();
 }
 
-// The cluster-resident step with four lanes per row (CTA = 4R threads, R up
-// to 128, lanes 4r .. 4r+3 on row r).  The row's first lane runs the node work and forms the
-// coupling sum in CSR order from the per-edge terms the row's lanes computed
-// (shuffled, same expression); the warp-level trees of the block sums read
-// the rows' values from shared memory in row order.  Bitwise the results of
-// cluster_kernel and step_kernel.  Shared memory as cluster_kernel plus
-// ord float [2][R] after omh.
-template <int MATH, int U>
-__global__ void __launch_bounds__(4 * 128, 1) cluster_split_kernel(const ClusterArgs a) {
+// ---------------------------------------------------------------------------
+// The cluster-resident step with four lanes per row (CTA = 4R threads, R up to
+// 128; rows and entries to lanes as in lev_split.cuh).  Bitwise the results of
+// cluster_kernel and step_kernel.
+//
+// A step is one latency chain (N = 1000: 16 CTAs of 64 rows, two warps per SM
+// sub-core), so the chain is kept short: the row's state stays in registers,
+// alike in its four lanes; a warp writes its part of the slice sums into every
+// CTA of the cluster and arrives; after the wait every warp reduces them from
+// its own shared memory.  The only synchronisation of a step is the cluster
+// barrier.
+// ---------------------------------------------------------------------------
+constexpr int kSplitLPR = 4;  // lanes per row
+constexpr int kSplitSlicesMax = kClusterMax * 128 / 32;  // 64: at most 8 blocks of 256 nodes
+
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t local, int rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ float ld_cluster(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr));
+  return v;
+}
+__device__ __forceinline__ void st_cluster(uint32_t addr, float2 v) {
+  asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(addr), "f"(v.x), "f"(v.y)
+               : "memory");
+}
+
+// (sum cos, sum sin) from the warps' parts [slices][4] of up to 64 slices
+// (zero past the network), by one warp, in every lane: lane l closes slice l's
+// tree, three shuffle levels close the 256-node blocks (block_tree8), and two
+// more add the at most eight blocks in the order of final_reduce_r_kernel
+// (leviathan_kernel.cu:242-263: lane b holds block b, the first two levels add
+// zeros).
+__device__ __forceinline__ float2 split_sums(const float2 *parts, int nslices, int lane) {
+  const unsigned mask = 0xffffffffu;
+  float c[2] = {0.0f, 0.0f}, s[2] = {0.0f, 0.0f};
+#pragma unroll
+  for (int grp = 0; grp < 2; ++grp) {
+    if (32 * grp >= nslices) break;  // uniform
+    const float4 *p = reinterpret_cast<const float4 *>(parts + 4 * (32 * grp + lane));
+    const float4 a = p[0], b = p[1];
+    float vc = __fadd_rn(__fadd_rn((a.x + b.x) + (a.z + b.z), 0.0f), 0.0f);
+    float vs = __fadd_rn(__fadd_rn((a.y + b.y) + (a.w + b.w), 0.0f), 0.0f);
+#pragma unroll
+    for (int off = 4; off > 0; off /= 2) {
+      vc += __shfl_down_sync(mask, vc, off);
+      vs += __shfl_down_sync(mask, vs, off);
+    }
+    c[grp] = __fadd_rn(0.0f, vc);  // lanes 0, 8, 16, 24: blocks 4 grp + 0 .. 3
+    s[grp] = __fadd_rn(0.0f, vs);
+  }
+  float sc = c[0] + c[1], ss = s[0] + s[1];
+#pragma unroll
+  for (int off = 16; off >= 8; off /= 2) {
+    sc += __shfl_down_sync(mask, sc, off);
+    ss += __shfl_down_sync(mask, ss, off);
+  }
+  return make_float2(__shfl_sync(mask, sc, 0), __shfl_sync(mask, ss, 0));
+}
+
+// shared memory (bytes, from the dynamic base):
+//   parts  float2 [2][kSplitSlicesMax * 4]   every CTA's copy of the warps' parts
+//   sloff, sllen  int [R/32]
+//   ring   float  [bsi][R]
+//   cd     uint32 [edge_cap], w float [edge_cap]   (order of lev_split.cuh)
+template <int MATH>
+__global__ void __launch_bounds__(kSplitLPR * 128, 1) cluster_split_kernel(const ClusterArgs a) {
   namespace cg = cooperative_groups;
-  constexpr int LPR = 4;
   cg::cluster_group cluster = cg::this_cluster();
   extern __shared__ __align__(16) unsigned char smem[];
 
   const NetDesc nd = *a.net;
   const int rank = (int)cluster.block_rank();
+  const int C = (int)cluster.num_blocks();
   const int R = a.R;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int q = tid & (LPR - 1);
-  const int rloc = tid / LPR;
-  const int lead = lane & ~(LPR - 1);
-  const unsigned mask = 0xffffffffu;
+  const SplitLane sl = split_lane<kSplitLPR>(tid);
   const int N = nd.N, bsi = nd.bsi, Np = nd.Np;
   const int row0 = rank * R;
-  const int row = row0 + rloc;
+  const int row = row0 + sl.rloc;
   const bool live = row < N;
   const int nslices = R / 32;
 
-  float2 *wsum = reinterpret_cast<float2 *>(smem);
-  int *sloff = reinterpret_cast<int *>(wsum + 2 * kClusterWarpsMax);
+  float2 *parts = reinterpret_cast<float2 *>(smem);
+  int *sloff = reinterpret_cast<int *>(parts + 2 * 4 * kSplitSlicesMax);
   int *sllen = sloff + nslices;
-  float *s_th = reinterpret_cast<float *>(sllen + nslices);
-  float *s_thh = s_th + R;
-  float *s_om = s_thh + R;
-  float *s_omh = s_om + R;
-  float *s_ord = s_omh + R;
-  float *s_ring = s_ord + 2 * R;
+  float *s_ring = reinterpret_cast<float *>(sllen + nslices);
   uint32_t *s_cd = reinterpret_cast<uint32_t *>(s_ring + (size_t)bsi * R);
   float *s_w = reinterpret_cast<float *>(s_cd + a.edge_cap);
 
@@ -380,191 +436,115 @@ __global__ void __launch_bounds__(4 * 128, 1) cluster_split_kernel(const Cluster
   const long long sl0 = nd.slice_base + row0 / 32;
   const int my_slices = max(0, min(nslices, (N - row0 + 31) / 32));
   const long long ebase = my_slices ? a.sl_off[sl0] : 0;
-  long long eend = ebase;
   for (int s = tid; s < nslices; s += blockDim.x) {
-    if (s < my_slices) {
-      sloff[s] = (int)(a.sl_off[sl0 + s] - ebase);
-      sllen[s] = a.sl_len[sl0 + s];
-    } else {
-      sloff[s] = 0;
-      sllen[s] = 0;
-    }
+    sloff[s] = s < my_slices ? (int)(a.sl_off[sl0 + s] - ebase) : 0;
+    sllen[s] = s < my_slices ? a.sl_len[sl0 + s] : 0;
   }
-  if (my_slices) eend = a.sl_off[sl0 + my_slices - 1] + 32LL * a.sl_len[sl0 + my_slices - 1];
-  const int nent = (int)(eend - ebase);
-  for (int k = tid; k < nent; k += blockDim.x) {
-    s_cd[k] = a.sl_cd[ebase + k];
-    s_w[k] = a.sl_w[ebase + k];
-  }
+  for (int k = tid; k < 2 * 4 * kSplitSlicesMax; k += blockDim.x)
+    parts[k] = make_float2(0.0f, 0.0f);
+  __syncthreads();
+  split_for_entries<kSplitLPR>(sloff, sllen, my_slices, [&](int at, int e) {
+    s_cd[at] = a.sl_cd[ebase + e];
+    s_w[at] = a.sl_w[ebase + e];
+  });
   int deg = 0;
+  float th = 0.0f, thh = 0.0f, om = 0.0f, omh = 0.0f;  // alike in the row's four lanes
   if (live) {
     const long long gi = nd.node_off + row;
-    if (q == 0) {
-      s_th[rloc] = a.theta[gi];
-      s_thh[rloc] = a.theta_hat[gi];
-      s_om[rloc] = a.omega[gi];
-      s_omh[rloc] = a.omega_hat[gi];
-    }
+    th = a.theta[gi];
+    thh = a.theta_hat[gi];
+    om = a.omega[gi];
+    omh = a.omega_hat[gi];
     const int *rp = a.row_ptr + nd.rp_off + row;
     deg = rp[1] - rp[0];
+    for (int s = sl.q; s < bsi; s += kSplitLPR)
+      s_ring[(size_t)s * R + sl.rloc] = a.ring[nd.ring_off + ring_pos(s, row, Np)];
   }
-  for (int s = q; s < bsi; s += LPR)
-    if (live) s_ring[(size_t)s * R + rloc] = a.ring[nd.ring_off + ring_pos(s, row, Np)];
-  NetState ns = *a.st;
+  const NetState ns = *a.st;
   int cur = ns.cur, rbuf = ns.rbuf;
   float g = ns.g, r = ns.r;
-  const int nblocks = (N + kTile - 1) / kTile;
-  if (rank == 0)
-    for (int k = tid; k < 2 * kClusterWarpsMax; k += blockDim.x) wsum[k] = make_float2(0.0f, 0.0f);
+  const int all_slices = 8 * nd.ntiles;
   const float dt = a.dt;
-  const float eta = nd.eta, gamma = nd.gamma, lam = nd.lam;
-  const float w_min = nd.w_min, w_max = nd.w_max;
-  // the warp's 8 rows share one SELL slice
-  const int wslice = (warp * (32 / LPR)) / 32;
-  const bool slice_live = row0 + wslice * 32 < N;
+  const float inv_N = 1.0f / (float)N;
+  const int len = sllen[sl.ws], base = sloff[sl.ws];
+  const uint32_t ring_addr = (uint32_t)__cvta_generic_to_shared(s_ring);
+  // lane l's copy of this warp's part in CTA l
+  const uint32_t part_addr = cluster_addr(
+      (uint32_t)__cvta_generic_to_shared(parts + 4 * (row0 / 32) + warp), lane < C ? lane : 0);
+  // the last warp of CTA 0 feeds an attached hub monitor
+  const bool observe = a.hubs && rank == 0 && warp == (int)(blockDim.x >> 5) - 1;
+  HubWarp hub;
+  if (observe) hub.open(a.hubs);
+  auto phase = [&](int j, int slot) {
+    const uint32_t at = ring_addr + 4u * (unsigned)(slot * R + (j & (R - 1)));
+    return ld_cluster(cluster_addr(at, j >> a.lgR));
+  };
+  // r and g after `steps` steps of this launch, alike in every thread
+  auto close_step = [&](int steps) {
+    const float2 sums =
+        split_sums(parts + ((steps - 1) & 1) * 4 * kSplitSlicesMax, all_slices, lane);
+    r = order_parameter(sums.x, sums.y, inv_N);
+    if (nd.ctrl) g = gain_controller(g, r, dt, nd);
+    if (rank == 0 && tid == 0 && a.r_hist) {
+      const int k = ns.rpos + steps - 1;
+      if (k < a.r_cap) a.r_hist[k] = r;
+    }
+  };
   cluster.sync();
 
-  float2 *wsum0 = cluster.map_shared_rank(wsum, 0);
-  __shared__ float s_g;
   for (int step = 0; step < a.n_steps; ++step) {
     // with zero delays: step-1's barrier before the gathers
     if (step > 0 && !a.early) cluster_wait();
-    // ---- predictor (row's first lane) --------------------------------------
-    float th = 0.0f, eps = 0.0f;
-    if (live && q == 0) {
-      th = s_th[rloc];
-      const float thh = s_thh[rloc];
-      const float wh = s_omh[rloc];
-      float diff = th - thh;
-      diff = wrap_pm_pi(diff);
-      eps = sinf(diff);
-      s_thh[rloc] = thh + dt * wh;
-      s_omh[rloc] = wh + nd.kappa_w * dt * eps;
-    }
-    th = __shfl_sync(mask, th, lead);
-    eps = __shfl_sync(mask, eps, lead);
-    const float my_eps = fabsf(eps);
-    // ---- edges: lane q takes entries q, q+4, ...; the sum in CSR order -----
-    float local_sum = 0.0f;
-    if (slice_live) {
-      const int len = sllen[wslice];
-      const int base = sloff[wslice] + (rloc & 31);
-      for (int kb = 0; kb < len; kb += LPR * U) {
-        uint32_t p[U];
-        float wv[U], dj[U], sn[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          const int k = kb + LPR * u + q;
-          const bool in = k < deg;
-          p[u] = in ? s_cd[base + 32 * k] : 0u;
-          wv[u] = in ? s_w[base + 32 * k] : 0.0f;
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          int slot = cur - (int)(p[u] & 255u);
-          slot += (slot < 0) ? bsi : 0;
-          const int j = (int)(p[u] >> 8);
-          const int owner = j >> a.lgR;
-          const int loc = j & (R - 1);
-          const float *src = (owner == rank) ? s_ring : cluster.map_shared_rank(s_ring, owner);
-          dj[u] = src[(size_t)slot * R + loc];
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          const int k = kb + LPR * u + q;
-          sn[u] = 0.0f;
-          if (k < deg) {
-            const float delayed_j = dj[u];
-            float diff = delayed_j - th;
-            diff = wrap_pm_pi(diff);
-            float w = wv[u];
-            float sin_diff, cos_diff;
-            lev_sincos<MATH>(diff, &sin_diff, &cos_diff);
-            sn[u] = sin_diff;
-            float dw = dt * (eta * cos_diff * (1.0f - gamma * my_eps) - lam * w);
-            w += dw;
-            if (!isfinite(w)) w = w_min;
-            w = fmaxf(w_min, fminf(w_max, w));
-            s_w[base + 32 * k] = w;
-          }
-        }
-#pragma unroll
-        for (int e = 0; e < LPR * U; ++e) {
-          const int srcl = lead + (e % LPR);
-          const float w = __shfl_sync(mask, wv[e / LPR], srcl);
-          const float sin_diff = __shfl_sync(mask, sn[e / LPR], srcl);
-          if (kb + e < deg) local_sum += w * sin_diff;  // the expression of cluster_kernel
-        }
-      }
-    }
-    // ---- r and gain of the previous step (warp 0 of every CTA) -------------
+    // ---- predictor ----------------------------------------------------------
+    const float eps = sinf(wrap_pm_pi(th - thh));
+    thh = thh + dt * omh;
+    omh = omh + nd.kappa_w * dt * eps;
+    // ---- edges ----------------------------------------------------------------
+    const EdgeParams ep = {dt, nd.eta, nd.lam, __fmaf_rn(-nd.gamma, fabsf(eps), 1.0f),
+                           nd.w_min, nd.w_max};
+    const float local_sum =
+        split_walk<MATH, kSplitLPR>(s_cd + base, s_w + base, len, deg, sl, th, ep, [&](uint32_t word) {
+          const unsigned s0 = (unsigned)(cur - (int)(word & 255u));
+          return phase((int)(word >> 8), (int)min(s0, s0 + (unsigned)bsi));
+        });
+    // ---- r and gain of the previous step --------------------------------------
+    float hub_phase = 0.0f;
     if (step > 0) {
       if (a.early) cluster_wait();
-      if (warp == 0) {
-        const float2 sums =
-            cluster_sums(wsum0 + ((step - 1) & 1) * kClusterWarpsMax, nblocks, lane);
-        if (lane == 0) {
-          float inv_N = 1.0f / (float)N;
-          r = sqrtf(sums.x * sums.x + sums.y * sums.y) * inv_N;
-          if (nd.ctrl) g = gain_controller(g, r, dt, nd);
-          s_g = g;
-          if (rank == 0 && a.r_hist) {
-            const int k = ns.rpos + step - 1;
-            if (k < a.r_cap) a.r_hist[k] = r;
-          }
-        }
-      }
-      __syncthreads();
-      g = s_g;
+      if (observe) hub_phase = phase(hub.node, cur);
+      close_step(step);
     }
-    // ---- integrate (row's first lane) --------------------------------------
+    // ---- integrate --------------------------------------------------------------
     int nxt = cur + 1;
     if (nxt == bsi) nxt = 0;
-    if (q == 0) {
-      float my_cos = 0.0f, my_sin = 0.0f;
-      if (live) {
-        float inc = dt * (s_om[rloc] + g * local_sum - nd.alpha * eps);
-        float x = th + inc;
-        x = wrap_0_2pi(x);
-        if (!isfinite(x)) x = 0.0f;
-        s_th[rloc] = x;
-        s_ring[(size_t)nxt * R + rloc] = x;
-        lev_sincos<MATH>(x, &my_sin, &my_cos);
-      }
-      s_ord[rloc] = my_cos;
-      s_ord[R + rloc] = my_sin;
+    float my_cos = 0.0f, my_sin = 0.0f;
+    if (live) {
+      float inc = dt * (om + g * local_sum - nd.alpha * eps);
+      float x = th + inc;
+      x = wrap_0_2pi(x);
+      if (!isfinite(x)) x = 0.0f;
+      th = x;
+      if (sl.q == 0) s_ring[(size_t)nxt * R + sl.rloc] = x;
+      lev_sincos<MATH>(x, &my_sin, &my_cos);
     }
-    __syncthreads();
-    // ---- warp sums in row order to CTA 0 (leviathan_kernel.cu:198-214) ----
-    if (tid < R) {
-      float c = s_ord[tid], sn = s_ord[R + tid];
-#pragma unroll
-      for (int off = 16; off > 0; off /= 2) {
-        c += __shfl_down_sync(mask, c, off);
-        sn += __shfl_down_sync(mask, sn, off);
-      }
-      if (lane == 0)
-        wsum0[(step & 1) * kClusterWarpsMax + row0 / 32 + warp] = make_float2(c, sn);
-    }
+    // ---- this warp's part of the slice sums (leviathan_kernel.cu:198-214), to
+    // every CTA ------------------------------------------------------------------
+    float2 part = split_warp_sum<kSplitLPR>(my_cos, my_sin);
+    part.x = __shfl_sync(0xffffffffu, part.x, 0);
+    part.y = __shfl_sync(0xffffffffu, part.y, 0);
+    if (lane < C)
+      st_cluster(part_addr + (step & 1) * (unsigned)(sizeof(float2) * 4 * kSplitSlicesMax), part);
+    __syncwarp();
     cur = nxt;
     rbuf = (rbuf + 1 == nd.max_delay + 1) ? 0 : rbuf + 1;
     cluster_arrive();
+    if (observe && step > 0) hub.observe(hub_phase);
   }
-  if (a.n_steps > 0) cluster_wait();
   // ---- r of the last step, then write the state back ------------------------
   if (a.n_steps > 0) {
-    const float2 sums =
-        cluster_sums(wsum0 + ((a.n_steps - 1) & 1) * kClusterWarpsMax, nblocks, lane);
-    const float sum_cos = __shfl_sync(mask, sums.x, 0);
-    const float sum_sin = __shfl_sync(mask, sums.y, 0);
-    float inv_N = 1.0f / (float)N;
-    r = sqrtf(sum_cos * sum_cos + sum_sin * sum_sin) * inv_N;
-    if (nd.ctrl) g = gain_controller(g, r, dt, nd);
+    cluster_wait();
+    close_step(a.n_steps);
     if (rank == 0 && tid == 0) {
-      if (a.r_hist) {
-        const int k = ns.rpos + a.n_steps - 1;
-        if (k < a.r_cap) a.r_hist[k] = r;
-      }
       NetState o = ns;
       o.g = g;
       o.r = r;
@@ -575,18 +555,23 @@ __global__ void __launch_bounds__(4 * 128, 1) cluster_split_kernel(const Cluster
       o.ticket = 0u;
       *a.st = o;
     }
+    if (observe) {
+      hub.observe(phase(hub.node, cur));
+      hub.close(a.n_steps);
+    }
   }
   if (live) {
     const long long gi = nd.node_off + row;
-    if (q == 0) {
-      a.theta[gi] = s_th[rloc];
-      a.theta_hat[gi] = s_thh[rloc];
-      a.omega_hat[gi] = s_omh[rloc];
+    if (sl.q == 0) {
+      a.theta[gi] = th;
+      a.theta_hat[gi] = thh;
+      a.omega_hat[gi] = omh;
     }
-    for (int s = q; s < bsi; s += LPR)
-      a.ring[nd.ring_off + ring_pos(s, row, Np)] = s_ring[(size_t)s * R + rloc];
+    for (int s = sl.q; s < bsi; s += kSplitLPR)
+      a.ring[nd.ring_off + ring_pos(s, row, Np)] = s_ring[(size_t)s * R + sl.rloc];
   }
-  for (int k = tid; k < nent; k += blockDim.x) a.sl_w[ebase + k] = s_w[k];
+  split_for_entries<kSplitLPR>(sloff, sllen, my_slices,
+                    [&](int at, int e) { a.sl_w[ebase + e] = s_w[at]; });
   // no CTA may leave while a peer can still read its shared memory
   cluster.sync();
 }

@@ -241,9 +241,11 @@ struct LevEngine {
   bool grid_R_ok[3] = {false, false, false};  // R = 64, 128, 256
   int grid_cap[3] = {0, 0, 0};                // SELL entries per CTA
   size_t grid_smem_R[3] = {0, 0, 0};
-  int grid_nwarps = 0;
-  float2 *d_gwsum = nullptr;  // [2][grid_nwarps]
-  unsigned *d_gbar = nullptr;
+  int grid_max_tiles = 0;     // tiles of the largest network
+  int grid_map_off[3] = {0, 0, 0};            // first entry of each choice in d_gmap
+  int2 *d_gmap = nullptr;     // batches: (network, CTA) per CTA
+  float2 *d_gwsum = nullptr;  // published sums, 32 per 256-node block
+  unsigned *d_gbar = nullptr; // arrival counters
   int *h_gerr = nullptr, *d_gerr = nullptr;  // barrier timeout flag (mapped)
   GridWait grid_wait = {kGridWaitNs, 0u, 0u};  // bound of the barrier waits
 
@@ -413,10 +415,11 @@ void free_engine(LevEngine *h) {
   dfree(h->d_class_nets);
   dfree(h->d_rhist);
   dfree(h->d_gwsum);
+  dfree(h->d_gmap);
   dfree(h->d_gbar);
   if (h->spec_block) cudaFreeAsync(h->spec_block, h->stream);
   if (h->slab) cudaFreeAsync(h->slab, h->stream);  // back to the engine pool
-  if (h->h_gerr) cudaFreeHost(h->h_gerr);
+  if (h->h_gerr) mapped_free(reinterpret_cast<float *>(h->h_gerr));
   mapped_free(h->h_rmap);
   if (h->h_rstage) cudaFreeHost(h->h_rstage);
   for (int c = 0; c < kNumClasses; ++c) {
@@ -783,7 +786,7 @@ int get_graph(LevEngine *h, int len, float dt, cudaGraphExec_t *out) {
 using ClusterFn = void (*)(ClusterArgs);
 ClusterFn cluster_fn(int R, int math_mode) {
   const bool acc = math_mode == LEV_MATH_ACCURATE;
-  if (R <= 128) return acc ? cluster_split_kernel<1, 8> : cluster_split_kernel<0, 8>;
+  if (R <= 128) return acc ? cluster_split_kernel<1> : cluster_split_kernel<0>;
   if (R <= 256) return acc ? cluster_kernel<1, 256, 24> : cluster_kernel<0, 256, 24>;
   return acc ? cluster_kernel<1, kClusterRowsMax, 8> : cluster_kernel<0, kClusterRowsMax, 8>;
 }
@@ -807,6 +810,7 @@ int launch_cluster(LevEngine *h, float dt, int len) {
   ca.omega_hat = h->d_omega_hat;
   ca.ring = h->d_ring;
   ca.r_hist = h->d_rhist;
+  ca.hubs = h->hubs ? h->hubs->d_mon : nullptr;
   ca.r_cap = h->block_len;
   ca.n_steps = len;
   ca.R = h->cluster_R;
@@ -831,10 +835,28 @@ int launch_cluster(LevEngine *h, float dt, int len) {
   return LEV_OK;
 }
 
+// Lets launches of a kernel use up to `bytes` of dynamic shared memory.  The
+// attribute belongs to the function, not to a launch, and every engine of the
+// process shares it, so it only ever grows: a smaller engine created later
+// must not take the room of one that still steps.
+bool allow_smem(const void *fn, size_t bytes) {
+  static std::mutex mu;
+  static std::map<std::pair<int, const void *>, size_t> allowed;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return false;
+  std::lock_guard<std::mutex> lk(mu);
+  size_t &cur = allowed[std::make_pair(dev, fn)];
+  if (bytes <= cur) return true;
+  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) !=
+      cudaSuccess)
+    return false;
+  cur = bytes;
+  return true;
+}
+
 // Small single networks: choose rows per CTA and check that the cluster
 // kernel can run (shared memory, cluster size, occupancy).
-void setup_cluster(LevEngine *h, const std::vector<long long> &sl_off,
-                   const std::vector<int> &sl_len) {
+void setup_cluster(LevEngine *h, const std::vector<int> &sl_len) {
   h->cluster_ok = false;
   if (h->num_nets != 1) return;
   const NetDesc &d = h->h_nets[0];
@@ -854,16 +876,16 @@ void setup_cluster(LevEngine *h, const std::vector<long long> &sl_off,
         e += 32LL * sl_len[d.slice_base + s];
       cap = std::max(cap, e);
     }
-    const size_t smem = sizeof(float2) * 2 * kClusterWarpsMax + sizeof(int) * 2 * (R / 32) +
-                        sizeof(float) * (R <= 128 ? 6 : 4) * R +
+    const size_t node = R <= 128 ? sizeof(float2) * 2 * 4 * kSplitSlicesMax
+                                 : sizeof(float2) * 2 * kClusterWarpsMax + sizeof(float) * 4 * R;
+    const size_t smem = node + sizeof(int) * 2 * (R / 32) +
                         sizeof(float) * (size_t)d.bsi * R + 8 * (size_t)cap;
     if (smem + 1024 > (size_t)max_smem) continue;
     bool ok = true;
     for (int m = 0; m < 2 && ok; ++m) {
       const void *fn = reinterpret_cast<const void *>(
           cluster_fn(R, m ? LEV_MATH_ACCURATE : LEV_MATH_REFERENCE));
-      ok = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) ==
-               cudaSuccess &&
+      ok = allow_smem(fn, smem) &&
            cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
                cudaSuccess;
       if (ok) {
@@ -897,26 +919,37 @@ void setup_cluster(LevEngine *h, const std::vector<long long> &sl_off,
   }
 }
 
-// Grid kernel for R rows per CTA (64, 128, 256), four lanes per row.
+// Grid kernel for R rows per CTA (64, 128, 256).
 using GridFn = void (*)(GridArgs);
 constexpr int kGridRs[3] = {64, 128, 256};
 GridFn grid_fn(int R, int math_mode) {
   const bool acc = math_mode == LEV_MATH_ACCURATE;
-  if (R == 64) return acc ? grid_kernel<1, 64, 8> : grid_kernel<0, 64, 8>;
-  if (R == 128) return acc ? grid_kernel<1, 128, 8> : grid_kernel<0, 128, 8>;
-  return acc ? grid_kernel<1, 256, 8> : grid_kernel<0, 256, 8>;
+  if (R == 64) return acc ? grid_kernel<1, 64> : grid_kernel<0, 64>;
+  if (R == 128) return acc ? grid_kernel<1, 128> : grid_kernel<0, 128>;
+  return acc ? grid_kernel<1, 256> : grid_kernel<0, 256>;
 }
 inline int grid_r_index(int R) { return R == 64 ? 0 : (R == 128 ? 1 : 2); }
+
+// CTAs of R rows over all networks.
+long long grid_ctas(const LevEngine *h, int R) {
+  long long c = 0;
+  for (const NetDesc &d : h->h_nets) c += (d.N + R - 1) / R;
+  return c;
+}
 
 // One cooperative launch of the grid-resident kernel: `len` steps, r history
 // rows 0..len-1 in d_rhist.
 int launch_grid(LevEngine *h, float dt, int len) {
   reset_rpos_kernel<<<1, 128, 0, h->stream>>>(h->d_st, h->num_nets);
-  LEV_TRY_CUDA(cudaMemsetAsync(h->d_gbar, 0, sizeof(unsigned), h->stream));
+  LEV_TRY_CUDA(cudaMemsetAsync(h->d_gbar, 0,
+                               sizeof(unsigned) * kGridBarPitch * (size_t)h->num_nets, h->stream));
+  LEV_TRY_CUDA(cudaMemsetAsync(h->d_gwsum, 0xff,  // no sum published (kNoSum)
+                               sizeof(float2) * 32 * (size_t)h->total_tiles, h->stream));
   const int R = h->grid_R, ri = grid_r_index(R);
   GridArgs ga;
-  ga.net = h->d_nets;
+  ga.nets = h->d_nets;
   ga.st = h->d_st;
+  ga.map = h->num_nets > 1 ? h->d_gmap + h->grid_map_off[ri] : nullptr;
   ga.row_ptr = h->d_row_ptr;
   ga.sl_off = h->d_sl_off;
   ga.sl_len = h->d_sl_len;
@@ -929,18 +962,20 @@ int launch_grid(LevEngine *h, float dt, int len) {
   ga.ring = h->d_ring;
   ga.wsum = h->d_gwsum;
   ga.bar = h->d_gbar;
+  ga.hubs = h->hubs ? h->hubs->d_mon : nullptr;
   ga.early = h->pair_ok ? 1 : 0;  // no delay is 0
   ga.err = h->d_gerr;
   ga.wait = h->grid_wait;
   ga.r_hist = h->d_rhist;
   ga.r_cap = h->block_len;
+  ga.num_nets = h->num_nets;
   ga.n_steps = len;
-  ga.nwarps = h->grid_nwarps;
   ga.edge_cap = h->grid_cap[ri];
+  ga.sum_cap = R < 256 ? 8 * h->grid_max_tiles : 0;
   ga.dt = dt;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((h->h_nets[0].N + R - 1) / R);
-  cfg.blockDim = dim3(kGridLPR * R);
+  cfg.gridDim = dim3((unsigned)grid_ctas(h, R));
+  cfg.blockDim = dim3(kGridThreads);
   cfg.dynamicSmemBytes = h->grid_smem_R[ri];
   cfg.stream = h->stream;
   cudaLaunchAttribute attr[1];
@@ -952,14 +987,13 @@ int launch_grid(LevEngine *h, float dt, int len) {
   return LEV_OK;
 }
 
-// Mid-sized single networks: for each rows-per-CTA choice, check that every
-// CTA of the grid kernel can be resident at once (shared memory, occupancy,
-// cooperative launch).  Allocates the warp sums, barrier and error flag.
-int setup_grid(LevEngine *h, const std::vector<long long> &sl_off,
-               const std::vector<int> &sl_len) {
+// Mid-sized single networks, and batches of as many rows in all: for each
+// rows-per-CTA choice, check that every CTA of the grid kernel can be resident
+// at once (shared memory, occupancy, cooperative launch).  Allocates the slice
+// sums, barriers, CTA map and error flag.
+int setup_grid(LevEngine *h, const std::vector<int> &sl_len) {
   h->grid_ok = false;
-  if (h->num_nets != 1) return LEV_OK;
-  const NetDesc &d = h->h_nets[0];
+  if (h->part) return LEV_OK;
   int dev = 0, max_smem = 0, coop = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) !=
@@ -970,20 +1004,24 @@ int setup_grid(LevEngine *h, const std::vector<long long> &sl_off,
     return LEV_OK;
   }
   if (!coop) return LEV_OK;
-  const int nblocks = (d.N + kTile - 1) / kTile;
-  const int nwarps = 8 * nblocks;
+  for (const NetDesc &d : h->h_nets) h->grid_max_tiles = std::max(h->grid_max_tiles, d.ntiles);
   for (int ri = 0; ri < 3; ++ri) {
     const int R = kGridRs[ri];
-    const int C = (d.N + R - 1) / R;
-    if (C < 2) continue;  // one CTA: the cluster path or graph replay
+    const long long C = grid_ctas(h, R);
+    // one CTA: the cluster path or graph replay; more threads than the device
+    // holds: the per-step launches
+    if (C < 2 || C * kGridThreads > 2048LL * sms) continue;
     long long cap = 0;
-    for (int c = 0; c < C; ++c) {
-      long long e = 0;
-      for (int s = c * R / 32; s < std::min<long long>((c + 1) * R / 32, (d.N + 31) / 32); ++s)
-        e += 32LL * sl_len[d.slice_base + s];
-      cap = std::max(cap, e);
+    for (const NetDesc &d : h->h_nets) {
+      const long long ns = (d.N + 31) / 32;
+      for (long long s0 = 0; s0 < ns; s0 += R / 32) {
+        long long e = 0;
+        for (long long s = s0; s < std::min<long long>(s0 + R / 32, ns); ++s)
+          e += 32LL * sl_len[d.slice_base + s];
+        cap = std::max(cap, e);
+      }
     }
-    const size_t smem = sizeof(float2) * nwarps + sizeof(float) * 6 * R +
+    const size_t smem = (R < 256 ? sizeof(float2) * 8 * (size_t)h->grid_max_tiles : 0) +
                         sizeof(int) * 2 * (R / 32) + 8 * (size_t)cap;
     if (smem + 1024 > (size_t)max_smem) continue;
     bool ok = true;
@@ -991,9 +1029,8 @@ int setup_grid(LevEngine *h, const std::vector<long long> &sl_off,
       const void *fn = reinterpret_cast<const void *>(
           grid_fn(R, m ? LEV_MATH_ACCURATE : LEV_MATH_REFERENCE));
       int per_sm = 0;
-      ok = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) ==
-               cudaSuccess &&
-           cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kGridLPR * R, smem) ==
+      ok = allow_smem(fn, smem) &&
+           cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kGridThreads, smem) ==
                cudaSuccess &&
            (long long)per_sm * sms >= C;
     }
@@ -1006,13 +1043,31 @@ int setup_grid(LevEngine *h, const std::vector<long long> &sl_off,
     h->grid_ok = true;
   }
   if (!h->grid_ok) return LEV_OK;
-  h->grid_nwarps = nwarps;
-  int rc = dev_alloc(h, &h->d_gwsum, 2 * (size_t)nwarps);
-  if (rc == LEV_OK) rc = dev_alloc(h, &h->d_gbar, 1);
+  const size_t nsum = 32 * (size_t)h->total_tiles;
+  const size_t nbar = kGridBarPitch * (size_t)h->num_nets;
+  int rc = dev_alloc(h, &h->d_gwsum, nsum);
+  if (rc == LEV_OK) rc = dev_alloc(h, &h->d_gbar, nbar);
   if (rc != LEV_OK) return rc;
-  LEV_TRY_CUDA(cudaMemset(h->d_gwsum, 0, sizeof(float2) * 2 * (size_t)nwarps));
-  LEV_TRY_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&h->h_gerr), sizeof(int),
-                             cudaHostAllocMapped));
+  if (h->num_nets > 1) {
+    // CTAs of a network side by side, the largest networks first
+    std::vector<int> order(h->num_nets);
+    for (int n = 0; n < h->num_nets; ++n) order[n] = n;
+    std::stable_sort(order.begin(), order.end(),
+                     [&](int x, int y) { return h->h_nets[x].N > h->h_nets[y].N; });
+    std::vector<int2> map;
+    for (int ri = 0; ri < 3; ++ri) {
+      h->grid_map_off[ri] = (int)map.size();
+      if (!h->grid_R_ok[ri]) continue;
+      for (int n : order)
+        for (int c = 0; c * kGridRs[ri] < h->h_nets[n].N; ++c) map.push_back(make_int2(n, c));
+    }
+    rc = dev_alloc(h, &h->d_gmap, map.size());
+    if (rc != LEV_OK) return rc;
+    LEV_TRY_CUDA(cudaMemcpy(h->d_gmap, map.data(), sizeof(int2) * map.size(),
+                            cudaMemcpyHostToDevice));
+  }
+  h->h_gerr = reinterpret_cast<int *>(mapped_alloc(1));
+  if (!h->h_gerr) return fail(LEV_ERR_NOMEM, "mapped host memory: allocation failed");
   *h->h_gerr = 0;
   LEV_TRY_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void **>(&h->d_gerr), h->h_gerr, 0));
   return LEV_OK;
@@ -1039,10 +1094,10 @@ int enqueue_steps(LevEngine *h, float dt, int n, float *stage) {
   int done = 0;
   while (done < n) {
     const int len = std::min(h->block_len, n - done);
-    if (h->cluster_ok && h->use_cluster && !h->hubs) {
+    if (h->cluster_ok && h->use_cluster && (!h->hubs || h->cluster_R <= 128)) {
       int rc = launch_cluster(h, dt, len);
       if (rc != LEV_OK) return rc;
-    } else if (h->grid_ok && h->use_grid && !h->hubs) {
+    } else if (h->grid_ok && h->use_grid) {
       int rc = launch_grid(h, dt, len);
       if (rc != LEV_OK) return rc;
     } else {
@@ -1546,8 +1601,8 @@ int create_impl(LevEngine **out, int num_nets, const int32_t *Ns,
     t0 = std::chrono::steady_clock::now();
     if (lrc == LEV_OK) lrc = prepare_step_kernels();
     if (lrc == LEV_OK) {
-      setup_cluster(h, h_sl_off, h_sl_len);
-      lrc = setup_grid(h, h_sl_off, h_sl_len);
+      setup_cluster(h, h_sl_len);
+      lrc = setup_grid(h, h_sl_len);
     }
     if (lrc == LEV_OK) {
       int nbusy = 0;
@@ -3210,7 +3265,7 @@ void adj_free(LevAdjoint *a) {
   }
   if (a->ev_start) cudaEventDestroy(a->ev_start);
   if (a->rstream) cudaStreamDestroy(a->rstream);
-  if (a->h_gerr) cudaFreeHost(a->h_gerr);
+  if (a->h_gerr) mapped_free(reinterpret_cast<float *>(a->h_gerr));
   delete a;
 }
 
@@ -3355,13 +3410,10 @@ int adj_setup_grid(LevAdjoint *a, const std::vector<long long> &sl_off,
       const void *ff = reinterpret_cast<const void *>(adj_grid_fwd_fn(R, mm));
       const void *bf = reinterpret_cast<const void *>(adj_grid_bwd_fn(R, mm));
       int pf = 0, pb = 0;
-      ok = cudaFuncSetAttribute(ff, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fsm) ==
+      ok = allow_smem(ff, fsm) && allow_smem(bf, bsm) &&
+           cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pf, ff, kSplitLPR * R, fsm) ==
                cudaSuccess &&
-           cudaFuncSetAttribute(bf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bsm) ==
-               cudaSuccess &&
-           cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pf, ff, kGridLPR * R, fsm) ==
-               cudaSuccess &&
-           cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pb, bf, kGridLPR * R, bsm) ==
+           cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pb, bf, kSplitLPR * R, bsm) ==
                cudaSuccess &&
            (long long)pf * sms >= C && (long long)pb * sms >= C;
     }
@@ -3374,9 +3426,8 @@ int adj_setup_grid(LevAdjoint *a, const std::vector<long long> &sl_off,
           adj_grid_pair_fn(R, m ? LEV_MATH_ACCURATE : LEV_MATH_REFERENCE));
       const size_t psm = std::max(fsm, bsm);
       int per_sm = 0;
-      pok = cudaFuncSetAttribute(pf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psm) ==
-                cudaSuccess &&
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pf, kGridLPR * R, psm) ==
+      pok = allow_smem(pf, psm) &&
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pf, kSplitLPR * R, psm) ==
                 cudaSuccess &&
             (long long)per_sm * sms >= 2LL * C;
     }
@@ -3398,8 +3449,8 @@ int adj_setup_grid(LevAdjoint *a, const std::vector<long long> &sl_off,
   if (rc == LEV_OK) rc = adj_alloc(a, &a->g_bar, 2);
   if (rc != LEV_OK) return rc;
   LEV_TRY_CUDA(cudaMemset(a->g_wsum, 0, sizeof(float2) * 2 * (size_t)nwarps));
-  LEV_TRY_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&a->h_gerr), sizeof(int),
-                             cudaHostAllocMapped));
+  a->h_gerr = reinterpret_cast<int *>(mapped_alloc(1));
+  if (!a->h_gerr) return fail(LEV_ERR_NOMEM, "mapped host memory: allocation failed");
   *a->h_gerr = 0;
   LEV_TRY_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void **>(&a->d_gerr), a->h_gerr, 0));
   return LEV_OK;
@@ -3466,7 +3517,7 @@ int adj_grid_launch_fwd(LevAdjoint *a, AdjGridFwdArgs f, int n, cudaStream_t s) 
   adj_grid_fill_fwd(a, f, n);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((a->h_nets[0].N + R - 1) / R);
-  cfg.blockDim = dim3(kGridLPR * R);
+  cfg.blockDim = dim3(kSplitLPR * R);
   cfg.dynamicSmemBytes = a->gf_smem[ri];
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
@@ -3511,7 +3562,7 @@ int adj_grid_launch_bwd(LevAdjoint *a, AdjGridBwdArgs b, cudaStream_t s) {
   adj_grid_fill_bwd(a, b);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((a->h_nets[0].N + R - 1) / R);
-  cfg.blockDim = dim3(kGridLPR * R);
+  cfg.blockDim = dim3(kSplitLPR * R);
   cfg.dynamicSmemBytes = a->gb_smem[ri];
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
@@ -3538,7 +3589,7 @@ int adj_grid_launch_pair(LevAdjoint *a, AdjGridFwdArgs f, int n, AdjGridBwdArgs 
   b.bar = a->g_bar + 1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * C);
-  cfg.blockDim = dim3(kGridLPR * R);
+  cfg.blockDim = dim3(kSplitLPR * R);
   cfg.dynamicSmemBytes = std::max(a->gf_smem[ri], a->gb_smem[ri]);
   cfg.stream = s;
   cudaLaunchAttribute attr[1];

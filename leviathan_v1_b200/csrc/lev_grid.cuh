@@ -1,45 +1,36 @@
-// lev_grid.cuh -- grid-resident engine for mid-sized single networks.
+// lev_grid.cuh -- grid-resident engine for mid-sized networks and batches.
 // Included once, from lev_engine.cu.
 //
-// A single network whose CTAs all fit on the device at once (one cooperative
-// launch, co-residency guaranteed by the launch) is stepped n times in ONE
-// launch:
-//   * CTA b owns rows [b*R, b*R + R), four lanes per row (4R threads); its
-//     SELL-32 slices (col|delay, weights) and its rows' node state stay in
-//     shared memory for the whole launch;
+// Networks whose CTAs all fit on the device at once (one cooperative launch,
+// co-residency guaranteed by the launch) are stepped n times in ONE launch: a
+// single network, or a batch, whose networks step independently of one
+// another:
+//   * CTA b of a network owns its rows [b*R, b*R + R), R = 64, 128 or 256, with
+//     four, two or one lanes per row (lev_split.cuh); its SELL-32 slices
+//     (col|delay, weights) stay in shared memory and its rows' node state in
+//     registers for the whole launch;
 //   * the delay ring stays in global memory, which at these sizes is
 //     L2-resident: each step writes theta(t+1) of the CTA's rows to ring slot
 //     t+1 through L2, and every gather reads through L2 (ld.global.cg), so no
 //     SM reads a stale L1 line of a slot another SM rewrote;
-//   * one grid barrier per step (an arrival counter in global memory): a CTA
-//     arrives after step t's ring write and warp sums and waits for barrier
-//     t before step t+1's integrate, which needs g(t+1) and overwrites ring
-//     slot t+2 = t-max_delay (mod max_delay+2), read by step t.  With zero
-//     delays step t+1's gathers read slot t+1 and the wait comes before
-//     them.  Without, they read slots <= t, ordered by barrier t-1, so the
-//     wait for barrier t comes after the predictor and the edge work of step
-//     t+1, which hide the barrier's latency;
-//   * each warp's shuffle-tree (sum cos, sum sin) of its 32 rows goes to a
-//     double-buffered array of warp sums; after the barrier every CTA stages
-//     them in shared memory (cp.async, in flight during the next step's edge
-//     work), forms the reference's 256-node block sums from eight warp sums
-//     (block_tree8) and reduces the blocks in the order of
-//     leviathan_kernel.cu:242-263.  All CTAs so compute the same r and gain,
-//     which the next step needs only at its integrate.
+//   * every CTA publishes its part of (sum cos, sum sin) of a step, and every
+//     CTA adds all parts in the order of leviathan_kernel.cu:198-263, so all
+//     CTAs of a network compute the same r and gain (see grid_kernel);
+//   * an arrival counter per network orders the ring's phases;
+//   * an attached hub monitor is fed by the network's CTA 0.
 // Arithmetic and summation order are those of step_kernel: results are
 // bitwise the same as stepping with step_kernel.
 //
-// The barrier's wait is bounded (GridWait, 2 s by default): on a timeout
+// Every wait is bounded (GridWait, 2 s by default): on a timeout
 // the CTA writes 1 to the error flag (mapped host memory), leaves the step
 // loop and writes nothing back; the host reports the error.
 
 #pragma once
 
-#include "lev_kernels.cuh"
+#include "lev_split.cuh"
 
 namespace lev {
 
-constexpr int kGridLPR = 4;                               // lanes per row
 constexpr unsigned long long kGridWaitNs = 2000000000ull;  // default wait limit
 
 // Bound of every grid-barrier wait of a launch.  `extra` is 0 in normal use;
@@ -53,8 +44,9 @@ struct GridWait {
 };
 
 struct GridArgs {
-  const NetDesc *net;
+  const NetDesc *nets;
   NetState *st;
+  const int2 *map;  // per CTA (network, CTA within the network); null: one network
   const int *row_ptr;
   const long long *sl_off;
   const int *sl_len;
@@ -65,16 +57,18 @@ struct GridArgs {
   const float *omega;
   float *omega_hat;
   float *ring;
-  float2 *wsum;      // [2][nwarps]: warp sums of the network's 32-row groups
-  unsigned *bar;     // arrival counter, zero at launch
+  float2 *wsum;      // per network [4][8 * tiles] sums, at 32 * part_off; kNoSum at launch
+  unsigned *bar;     // per network arrival counter, zero at launch, kGridBarPitch apart
+  HubMonitor *hubs;  // observes hub phases after every step of hubs->net, or null
   int early;         // no delay is 0: wait for barrier t after step t+1's edges
   int *err;          // error flag (mapped host memory)
   GridWait wait;     // bound of the barrier waits
-  float *r_hist;     // [n] (row rpos + k), or null
+  float *r_hist;     // [r_cap][num_nets] (row rpos + k), or null
   int r_cap;
+  int num_nets;
   int n_steps;
-  int nwarps;        // 8 * 256-node blocks, rounded up to even
   int edge_cap;      // SELL entries per CTA the shared memory was sized for
+  int sum_cap;       // sums staged per CTA the shared memory was sized for (R < 256)
   float dt;
 };
 
@@ -128,42 +122,189 @@ __device__ __forceinline__ bool grid_wait(unsigned *bar, unsigned target, int *e
   return *reinterpret_cast<volatile int *>(s_ok) != 0;
 }
 
+// Waits like grid_wait, but one lane only; returns false after a timeout.
+__device__ __forceinline__ bool grid_poll(unsigned *bar, unsigned target, const GridWait &gw) {
+  const unsigned long long t0 = global_ns();
+  while (ld_acquire_gpu(bar) < target + gw.extra)
+    if (global_ns() - t0 > gw.ns) return false;
+  return true;
+}
+
+// A sum that has not been published yet: a NaN pattern that no published sum
+// has (grid_publish changes it into another NaN).
+constexpr unsigned kNoSum = 0xffffffffu;
+
+__device__ __forceinline__ uint4 ld_relaxed_gpu4(const void *p) {
+  uint4 v;
+  asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint2 ld_relaxed_gpu2(const void *p) {
+  uint2 v;
+  asm volatile("ld.relaxed.gpu.global.v2.u32 {%0, %1}, [%2];"
+               : "=r"(v.x), "=r"(v.y) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void grid_publish(float2 *p, float2 v) {
+  unsigned x = __float_as_uint(v.x), y = __float_as_uint(v.y);
+  if (x == kNoSum) x = 0x7fffffffu;
+  if (y == kNoSum) y = 0x7fffffffu;
+  asm volatile("st.relaxed.gpu.global.v2.u32 [%0], {%1, %2};" ::"l"(p), "r"(x), "r"(y) : "memory");
+}
+__device__ __forceinline__ void grid_unpublish(float2 *p) {
+  asm volatile("st.relaxed.gpu.global.v2.u32 [%0], {%1, %1};" ::"l"(p), "r"(kNoSum) : "memory");
+}
+
+// Waits, at most gw.ns, until all sums of a step are published and adds them
+// up, one warp; returns false, in every lane, after a timeout.
+//   BLOCKS: `n` sums of whole 256-node blocks; lane l takes blocks l, l+32, ...
+//           and adds them in the order of leviathan_kernel.cu:242-263.
+//   else:   `n` sums of 32-row slices (an even number), read as 16-byte pairs
+//           in memory order, staged in s_sum (zeros up to 8 per block) and
+//           formed into blocks with the reference's second-level tree
+//           (:216-233) first.
+template <bool BLOCKS>
+__device__ __forceinline__ bool grid_sums(const float2 *buf, int n, int nblocks, int lane,
+                                          const GridWait &gw, float2 *s_sum, float2 *out) {
+  const unsigned mask = 0xffffffffu;
+  const unsigned long long t0 = global_ns();
+  float sum_cos = 0.0f, sum_sin = 0.0f;
+  constexpr int K = 8;  // loads in flight per lane
+  const int items = BLOCKS ? n : n / 2;
+  for (int base = 0; base < items; base += 32 * K) {
+    uint4 v[K];
+    for (;;) {
+      bool ready = gw.extra == 0;
+#pragma unroll
+      for (int j = 0; j < K; ++j) {
+        const int i = base + 32 * j + lane;
+        v[j] = make_uint4(0u, 0u, 0u, 0u);
+        if (i < items) {
+          if (BLOCKS) {
+            const uint2 t = ld_relaxed_gpu2(buf + i);
+            v[j].x = t.x;
+            v[j].y = t.y;
+          } else {
+            v[j] = ld_relaxed_gpu4(buf + 2 * i);
+          }
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < K; ++j) {
+        ready = ready && v[j].x != kNoSum && v[j].y != kNoSum;
+        if (!BLOCKS) ready = ready && v[j].z != kNoSum && v[j].w != kNoSum;
+      }
+      if (__all_sync(mask, ready)) break;
+      if (__any_sync(mask, global_ns() - t0 > gw.ns)) return false;
+    }
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+      const int i = base + 32 * j + lane;
+      if (i >= items) continue;
+      if (BLOCKS) {
+        sum_cos += __uint_as_float(v[j].x);
+        sum_sin += __uint_as_float(v[j].y);
+      } else {
+        reinterpret_cast<uint4 *>(s_sum)[i] = v[j];
+      }
+    }
+  }
+  if (!BLOCKS) {
+    __syncwarp();
+    for (int b = lane; b < nblocks; b += 32) {
+      float vc[8], vs[8];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float4 t = reinterpret_cast<const float4 *>(s_sum)[4 * b + i];
+        vc[2 * i] = t.x;
+        vs[2 * i] = t.y;
+        vc[2 * i + 1] = t.z;
+        vs[2 * i + 1] = t.w;
+      }
+      sum_cos += block_tree8(vc);
+      sum_sin += block_tree8(vs);
+    }
+    __syncwarp();
+  }
+#pragma unroll
+  for (int off = 16; off > 0; off /= 2) {
+    sum_cos += __shfl_down_sync(mask, sum_cos, off);
+    sum_sin += __shfl_down_sync(mask, sum_sin, off);
+  }
+  *out = make_float2(sum_cos, sum_sin);
+  return true;
+}
+
+constexpr int kGridBarPitch = 32;  // arrival counters of two networks share no 128-byte line
+constexpr int kGridThreads = 256 + 32;  // eight warps on rows, one for the other CTAs
+
+// Barrier of a CTA whose warps run different code.
+__device__ __forceinline__ void cta_barrier() {
+  asm volatile("bar.sync 1, %0;" ::"n"(kGridThreads) : "memory");
+}
+
 // shared memory layout (bytes, from the dynamic base):
-//   s_ws   float2 [nwarps]    staged warp sums of the previous step
-//   th, thh, om, omh  float [R]
-//   ord    float  [2R]        the rows' (cos, sin) in row order
+//   sums   float2 [8 * blocks of the largest network]  (R < 256)
 //   sloff, sllen  int [R/32]
-//   cd     uint32 [edge_cap]
+//   cd     uint32 [edge_cap]  (order of lev_split.cuh)
 //   w      float  [edge_cap]
-// R: rows per CTA (64, 128 or 256); U: edges per lane in flight together.
-template <int MATH, int R, int U>
-__global__ void __launch_bounds__(kGridLPR * R, 256 / R) grid_kernel(const GridArgs a) {
-  constexpr int LPR = kGridLPR;
+// R: rows per CTA, 64, 128 or 256, with LPR = 256 / R lanes per row.
+//
+// What bounds a step is a chain of L2 round trips (about 600 cycles each).
+// With the CTA's first warp doing both its rows' edges and the exchange, at N =
+// 10^4 (R = 64) a step took 6,990 cycles: edges 2,070, waiting for the counter
+// 960, reading the sums 2,130, integrate 620, and 1,190 in the release fence
+// of the arrival, one after the other.  So a ninth warp does the exchange while
+// the others walk their edges, and the sums carry their own "published" mark:
+// they go out without waiting for the fence, which only the ring phases need
+// and which is paid while the sums travel.
+//
+// Order of one step s, edge warps | ninth warp:
+//   predictor, edges            | wait for the sums of s-1; r, g of step s
+//   ------------------------ barrier A: g ------------------------
+//   integrate, ring slot s+1    | wait for every CTA's arrival s-1 (its phases)
+//   ------------------------ barrier B: warp parts ---------------
+//   (step s+1)                  | publish the sums of s, clear those of s-2;
+//                               | fence, arrive
+// Gathers of step s+1 read slots <= s (no zero delay), whose phases were
+// ordered by arrival s-1 before barrier B of step s.  The integrate of step s
+// overwrites the slot that the gathers of step s-1 read last; those CTAs have
+// published the sums of s-1, which follow from the gathered values.  Sums of
+// s live in buffer s mod 4; a CTA clears its part of buffer (s+2) mod 4, the
+// sums of s-2, once all sums of s-1 have shown that nobody still reads them,
+// and its arrival s orders the clearing before anybody looks for the sums of
+// s+2 there.  With zero delays step s gathers slot s, and the wait for arrival
+// s-1 comes before the edges.
+template <int MATH, int R>
+__global__ void __launch_bounds__(kGridThreads, 3) grid_kernel(const GridArgs a) {
+  constexpr int LPR = 256 / R;
   constexpr int nslices = R / 32;
+  constexpr bool kBlocks = R == 256;  // a CTA closes its 256-node block itself
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ float s_g;
   __shared__ int s_ok;
+  __shared__ float2 s_part[8];
 
-  const NetDesc nd = *a.net;
-  const int cta = blockIdx.x;
+  const int2 me = a.map ? a.map[blockIdx.x] : make_int2(0, (int)blockIdx.x);
+  const NetDesc nd = a.nets[me.x];
+  const int cta = me.y;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int q = tid & (LPR - 1);
-  const int rloc = tid / LPR;
-  const int lead = lane & ~(LPR - 1);
-  const unsigned mask = 0xffffffffu;
+  const bool exchange = warp == 8;
+  const SplitLane sl = split_lane<LPR>(tid & 255);
   const int N = nd.N, bsi = nd.bsi, Np = nd.Np;
   const int row0 = cta * R;
-  const int row = row0 + rloc;
-  const bool live = row < N;
-  const int nwarps = a.nwarps;
+  const int row = row0 + sl.rloc;
+  const bool live = !exchange && row < N;
+  const unsigned G = (unsigned)((N + R - 1) / R);
+  const int nblocks = nd.ntiles;
+  unsigned *bar = a.bar + kGridBarPitch * me.x;
+  float2 *wsum = a.wsum + 32 * (long long)nd.part_off;  // four buffers of 8 * nblocks
+  // sums published per step: blocks, or slices up to the last whole block
+  const int nsum = kBlocks ? nblocks : min(8 * nblocks, (int)G * nslices);
 
-  float2 *s_ws = reinterpret_cast<float2 *>(smem);
-  float *s_th = reinterpret_cast<float *>(s_ws + nwarps);
-  float *s_thh = s_th + R;
-  float *s_om = s_thh + R;
-  float *s_omh = s_om + R;
-  float *s_ord = s_omh + R;
-  int *sloff = reinterpret_cast<int *>(s_ord + 2 * R);
+  float2 *s_sum = reinterpret_cast<float2 *>(smem);
+  int *sloff = reinterpret_cast<int *>(s_sum + a.sum_cap);
   int *sllen = sloff + nslices;
   uint32_t *s_cd = reinterpret_cast<uint32_t *>(sllen + nslices);
   float *s_w = reinterpret_cast<float *>(s_cd + a.edge_cap);
@@ -172,222 +313,181 @@ __global__ void __launch_bounds__(kGridLPR * R, 256 / R) grid_kernel(const GridA
   const long long sl0 = nd.slice_base + row0 / 32;
   const int my_slices = max(0, min(nslices, (N - row0 + 31) / 32));
   const long long ebase = my_slices ? a.sl_off[sl0] : 0;
-  long long eend = ebase;
   for (int s = tid; s < nslices; s += blockDim.x) {
-    if (s < my_slices) {
-      sloff[s] = (int)(a.sl_off[sl0 + s] - ebase);
-      sllen[s] = a.sl_len[sl0 + s];
-    } else {
-      sloff[s] = 0;
-      sllen[s] = 0;
-    }
+    sloff[s] = s < my_slices ? (int)(a.sl_off[sl0 + s] - ebase) : 0;
+    sllen[s] = s < my_slices ? a.sl_len[sl0 + s] : 0;
   }
-  if (my_slices) eend = a.sl_off[sl0 + my_slices - 1] + 32LL * a.sl_len[sl0 + my_slices - 1];
-  const int nent = (int)(eend - ebase);
-  for (int k = tid; k < nent; k += blockDim.x) {
-    s_cd[k] = a.sl_cd[ebase + k];
-    s_w[k] = a.sl_w[ebase + k];
-  }
+  for (int k = tid; k < a.sum_cap; k += blockDim.x) s_sum[k] = make_float2(0.0f, 0.0f);
+  if (tid == 0) s_ok = 1;
+  __syncthreads();
+  split_for_entries<LPR>(sloff, sllen, my_slices, [&](int at, int e) {
+    s_cd[at] = a.sl_cd[ebase + e];
+    s_w[at] = a.sl_w[ebase + e];
+  });
+  const long long gi = nd.node_off + row;
   int deg = 0;
+  float th = 0.0f, thh = 0.0f, om = 0.0f, omh = 0.0f;  // alike in the row's lanes
   if (live) {
-    const long long gi = nd.node_off + row;
-    if (q == 0) {
-      s_th[rloc] = a.theta[gi];
-      s_thh[rloc] = a.theta_hat[gi];
-      s_om[rloc] = a.omega[gi];
-      s_omh[rloc] = a.omega_hat[gi];
-    }
+    th = a.theta[gi];
+    thh = a.theta_hat[gi];
+    om = a.omega[gi];
+    omh = a.omega_hat[gi];
     const int *rp = a.row_ptr + nd.rp_off + row;
     deg = rp[1] - rp[0];
   }
-  const NetState ns = *a.st;
-  int cur = ns.cur, rbuf = ns.rbuf;
-  float g = ns.g, r = ns.r;
-  const int nblocks = (N + kTile - 1) / kTile;
-  const float *ring = a.ring + nd.ring_off;
-  float *ring_w = a.ring + nd.ring_off;
+  const NetState ns = a.st[me.x];
+  int cur = ns.cur;
+  float g = ns.g;
+  float *ring = a.ring + nd.ring_off;
   const float dt = a.dt;
-  const float eta = nd.eta, gamma = nd.gamma, lam = nd.lam;
-  const float w_min = nd.w_min, w_max = nd.w_max;
-  // the warp's 8 rows share one SELL slice
-  const int wslice = (warp * (32 / LPR)) / 32;
-  const bool slice_live = row0 + wslice * 32 < N;
-  if (tid == 0) s_ok = 1;
   __syncthreads();
 
-  const unsigned G = gridDim.x;
-  // warp sums of step s into shared memory (warp 0), after barrier s
-  auto stage_sums = [&](int s) {
-    if (warp == 0) {
-      const float2 *src = a.wsum + (s & 1) * nwarps;
-      for (int c = lane; c < nwarps / 2; c += 32) cp_async_cg16(s_ws + 2 * c, src + 2 * c);
-      cp_async_commit();
-    }
-  };
-  int step = 0;
-  bool ok = true;
-  for (; step < a.n_steps; ++step) {
-    // with zero delays: barrier step-1 before the gathers; the warp sums are
-    // in flight during the predictor and the edge work
-    if (step > 0 && !a.early) {
-      if (!(ok = grid_wait(a.bar, (unsigned)step * G, a.err, &s_ok, a.wait))) break;
-      stage_sums(step - 1);
-    }
-    // ---- predictor (row's first lane) --------------------------------------
-    float th = 0.0f, eps = 0.0f;
-    if (live && q == 0) {
-      th = s_th[rloc];
-      const float thh = s_thh[rloc];
-      const float wh = s_omh[rloc];
-      float diff = th - thh;
-      diff = wrap_pm_pi(diff);
-      eps = sinf(diff);
-      s_thh[rloc] = thh + dt * wh;
-      s_omh[rloc] = wh + nd.kappa_w * dt * eps;
-    }
-    th = __shfl_sync(mask, th, lead);
-    eps = __shfl_sync(mask, eps, lead);
-    const float my_eps = fabsf(eps);
-    // ---- edges: lane q takes entries q, q+4, ...; the sum in CSR order -----
-    float local_sum = 0.0f;
-    if (slice_live) {
-      const int len = sllen[wslice];
-      const int base = sloff[wslice] + (rloc & 31);
-      for (int kb = 0; kb < len; kb += LPR * U) {
-        uint32_t p[U];
-        float wv[U], dj[U], sn[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          const int k = kb + LPR * u + q;
-          const bool in = k < deg;
-          p[u] = in ? s_cd[base + 32 * k] : 0u;
-          wv[u] = in ? s_w[base + 32 * k] : 0.0f;
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          int slot = cur - (int)(p[u] & 255u);
-          slot += (slot < 0) ? bsi : 0;
-          dj[u] = __ldcg(ring + ring_pos(slot, p[u] >> 8, Np));
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          const int k = kb + LPR * u + q;
-          sn[u] = 0.0f;
-          if (k < deg) {
-            const float delayed_j = dj[u];
-            float diff = delayed_j - th;
-            diff = wrap_pm_pi(diff);
-            float w = wv[u];
-            float sin_diff, cos_diff;
-            lev_sincos<MATH>(diff, &sin_diff, &cos_diff);
-            sn[u] = sin_diff;
-            float dw = dt * (eta * cos_diff * (1.0f - gamma * my_eps) - lam * w);
-            w += dw;
-            if (!isfinite(w)) w = w_min;
-            w = fmaxf(w_min, fminf(w_max, w));
-            s_w[base + 32 * k] = w;
-          }
-        }
-#pragma unroll
-        for (int e = 0; e < LPR * U; ++e) {
-          const int srcl = lead + (e % LPR);
-          const float w = __shfl_sync(mask, wv[e / LPR], srcl);
-          const float sin_diff = __shfl_sync(mask, sn[e / LPR], srcl);
-          if (kb + e < deg) local_sum += w * sin_diff;  // the expression of cluster_kernel
-        }
+  if (!exchange) {
+    const int len = sllen[sl.ws], base = sloff[sl.ws];
+    for (int step = 0; step < a.n_steps; ++step) {
+      if (step > 0 && !a.early) cta_barrier();
+      // ---- predictor ----------------------------------------------------------
+      const float eps = sinf(wrap_pm_pi(th - thh));
+      thh = thh + dt * omh;
+      omh = omh + nd.kappa_w * dt * eps;
+      // ---- edges ----------------------------------------------------------------
+      const EdgeParams ep = {dt, nd.eta, nd.lam, __fmaf_rn(-nd.gamma, fabsf(eps), 1.0f),
+                             nd.w_min, nd.w_max};
+      const float local_sum =
+          split_walk<MATH, LPR>(s_cd + base, s_w + base, len, deg, sl, th, ep, [&](uint32_t word) {
+            return __ldcg(ring + ring_pos_word(word, cur, bsi, Np));
+          });
+      if (step > 0) {
+        cta_barrier();  // A
+        if (*reinterpret_cast<volatile int *>(&s_ok) == 0) break;
+        g = s_g;
       }
-    }
-    // ---- r and gain of the previous step (warp 0, from the staged sums) ----
-    if (step > 0) {
-      if (a.early) {
-        if (!(ok = grid_wait(a.bar, (unsigned)step * G, a.err, &s_ok, a.wait))) break;
-        stage_sums(step - 1);
-      }
-      if (warp == 0) {
-        cp_async_wait_all();
-        __syncwarp();
-        const float2 sums = cluster_sums(s_ws, nblocks, lane);
-        if (lane == 0) {
-          float inv_N = 1.0f / (float)N;
-          r = sqrtf(sums.x * sums.x + sums.y * sums.y) * inv_N;
-          if (nd.ctrl) g = gain_controller(g, r, dt, nd);
-          s_g = g;
-          if (cta == 0 && a.r_hist) {
-            const int k = ns.rpos + step - 1;
-            if (k < a.r_cap) a.r_hist[k] = r;
-          }
-        }
-      }
-      __syncthreads();
-      g = s_g;
-    }
-    // ---- integrate (row's first lane) --------------------------------------
-    int nxt = cur + 1;
-    if (nxt == bsi) nxt = 0;
-    if (q == 0) {
+      // ---- integrate --------------------------------------------------------------
+      int nxt = cur + 1;
+      if (nxt == bsi) nxt = 0;
       float my_cos = 0.0f, my_sin = 0.0f;
       if (live) {
-        float inc = dt * (s_om[rloc] + g * local_sum - nd.alpha * eps);
+        float inc = dt * (om + g * local_sum - nd.alpha * eps);
         float x = th + inc;
         x = wrap_0_2pi(x);
         if (!isfinite(x)) x = 0.0f;
-        s_th[rloc] = x;
-        __stcg(ring_w + ring_pos(nxt, row, Np), x);
+        th = x;
+        if (sl.q == 0) __stcg(ring + ring_pos(nxt, row, Np), x);
         lev_sincos<MATH>(x, &my_sin, &my_cos);
       }
-      s_ord[rloc] = my_cos;
-      s_ord[R + rloc] = my_sin;
+      const float2 part = split_warp_sum<LPR>(my_cos, my_sin);
+      if (lane == 0) s_part[warp] = part;
+      cur = nxt;
+      cta_barrier();  // B
     }
-    __syncthreads();
-    // ---- warp sums in row order (leviathan_kernel.cu:198-214) --------------
-    if (tid < R) {
-      float c = s_ord[tid], sn = s_ord[R + tid];
-#pragma unroll
-      for (int off = 16; off > 0; off /= 2) {
-        c += __shfl_down_sync(mask, c, off);
-        sn += __shfl_down_sync(mask, sn, off);
-      }
-      if (lane == 0) __stcg(a.wsum + (step & 1) * nwarps + row0 / 32 + warp, make_float2(c, sn));
-    }
-    cur = nxt;
-    rbuf = (rbuf + 1 == nd.max_delay + 1) ? 0 : rbuf + 1;
-    grid_arrive(a.bar);
-  }
-  // CTA 0 needs every warp sum of the last step
-  if (ok && a.n_steps > 0 && cta == 0) ok = grid_wait(a.bar, (unsigned)a.n_steps * G, a.err, &s_ok, a.wait);
-  if (!ok) return;  // barrier timeout: the host reports it
-  // ---- r of the last step (CTA 0), then write the state back ---------------
-  if (a.n_steps > 0 && cta == 0 && warp == 0) {
-    const float2 *src = a.wsum + ((a.n_steps - 1) & 1) * nwarps;
-    for (int k = lane; k < nwarps; k += 32) s_ws[k] = __ldcg(src + k);
-    __syncwarp();
-    const float2 sums = cluster_sums(s_ws, nblocks, lane);
-    if (lane == 0) {
-      float inv_N = 1.0f / (float)N;
-      r = sqrtf(sums.x * sums.x + sums.y * sums.y) * inv_N;
+  } else {
+    const float inv_N = 1.0f / (float)N;
+    float r = ns.r;
+    // CTA 0 feeds an attached hub monitor
+    const bool observe = a.hubs && a.hubs->net == me.x && cta == 0;
+    HubWarp hub;
+    if (observe) hub.open(a.hubs);
+    // r and g after `steps` steps of this launch (lane 0); false after a timeout
+    auto close_step = [&](int steps) -> bool {
+      float2 sums;
+      if (!grid_sums<kBlocks>(wsum + ((steps - 1) & 3) * 8 * nblocks, nsum, nblocks, lane, a.wait,
+                              s_sum, &sums))
+        return false;
+      r = order_parameter(sums.x, sums.y, inv_N);
       if (nd.ctrl) g = gain_controller(g, r, dt, nd);
-      if (a.r_hist) {
-        const int k = ns.rpos + a.n_steps - 1;
-        if (k < a.r_cap) a.r_hist[k] = r;
+      if (lane == 0) {
+        s_g = g;
+        if (cta == 0 && a.r_hist) {
+          const int k = ns.rpos + steps - 1;
+          if (k < a.r_cap) a.r_hist[(long long)k * a.num_nets + me.x] = r;
+        }
       }
-      NetState o = ns;
-      o.g = g;
-      o.r = r;
-      o.cur = cur;
-      o.rbuf = rbuf;
-      o.t = ns.t + a.n_steps;
-      o.rpos = ns.rpos + a.n_steps;
-      o.ticket = 0u;
-      *a.st = o;
+      return true;
+    };
+    // every CTA's phases of the first `steps` steps are in the ring
+    auto phases_of = [&](int steps) -> bool {
+      const bool ok = lane != 0 || grid_poll(bar, (unsigned)steps * G, a.wait);
+      return __all_sync(0xffffffffu, ok);
+    };
+    auto fail = [&]() {
+      if (lane == 0) {
+        *reinterpret_cast<volatile int *>(a.err) = 1;
+        *reinterpret_cast<volatile int *>(&s_ok) = 0;
+      }
+      __syncwarp();
+    };
+    bool ok = true;
+    for (int step = 0; step < a.n_steps; ++step) {
+      float hub_phase = 0.0f;
+      if (step > 0) {
+        if (!a.early) {
+          ok = ok && phases_of(step);
+          cta_barrier();
+        }
+        ok = ok && close_step(step);
+        if (!ok) fail();
+        cta_barrier();  // A
+        if (!ok) break;
+        // a timeout here shows at the next barrier A
+        if (a.early) ok = phases_of(step);
+        if (observe && ok) hub_phase = __ldcg(ring + ring_pos(cur, hub.node, Np));
+      }
+      cur = (cur + 1 == bsi) ? 0 : cur + 1;
+      cta_barrier();  // B
+      const int first = kBlocks ? cta : row0 / 32;
+      const bool mine = lane < (kBlocks ? 1 : nslices) && first + lane < nsum;
+      if (mine) {
+        float2 v;
+        if (kBlocks) {
+          float vc[8], vs[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            vc[i] = s_part[i].x;
+            vs[i] = s_part[i].y;
+          }
+          v = make_float2(block_tree8(vc), block_tree8(vs));
+        } else {
+          v = split_slice_sum<LPR>(s_part + LPR * lane);
+        }
+        grid_publish(wsum + (step & 3) * 8 * nblocks + first + lane, v);
+        grid_unpublish(wsum + ((step + 2) & 3) * 8 * nblocks + first + lane);
+      }
+      __syncwarp();
+      if (lane == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+      if (observe && ok && step > 0) hub.observe(hub_phase);
+    }
+    if (!ok) fail();
+    // CTA 0 closes the last step
+    if (ok && a.n_steps > 0 && cta == 0) {
+      ok = close_step(a.n_steps) && phases_of(a.n_steps);
+      if (!ok) fail();
+      if (ok && observe) {
+        hub.observe(__ldcg(ring + ring_pos(cur, hub.node, Np)));
+        hub.close(a.n_steps);
+      }
+      if (ok && lane == 0) {
+        NetState o = ns;
+        o.g = g;
+        o.r = r;
+        o.cur = cur;
+        o.rbuf = (int)((ns.rbuf + (long long)a.n_steps) % (nd.max_delay + 1));
+        o.t = ns.t + a.n_steps;
+        o.rpos = ns.rpos + a.n_steps;
+        o.ticket = 0u;
+        a.st[me.x] = o;
+      }
     }
   }
-  if (live && q == 0) {
-    const long long gi = nd.node_off + row;
-    a.theta[gi] = s_th[rloc];
-    a.theta_hat[gi] = s_thh[rloc];
-    a.omega_hat[gi] = s_omh[rloc];
+  __syncthreads();
+  if (*reinterpret_cast<volatile int *>(&s_ok) == 0) return;  // timeout: the host reports it
+  // ---- write the state back -------------------------------------------------
+  if (live && sl.q == 0) {
+    a.theta[gi] = th;
+    a.theta_hat[gi] = thh;
+    a.omega_hat[gi] = omh;
   }
-  for (int k = tid; k < nent; k += blockDim.x) a.sl_w[ebase + k] = s_w[k];
+  split_for_entries<LPR>(sloff, sllen, my_slices,
+                         [&](int at, int e) { a.sl_w[ebase + e] = s_w[at]; });
 }
 
 }  // namespace lev
