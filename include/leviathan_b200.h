@@ -269,12 +269,12 @@ int lev_cluster_info(const LevEngine *h, int32_t *eligible, int32_t *enabled,
                      int32_t *ctas, int32_t *rows_per_cta, int64_t *smem_bytes);
 int lev_set_cluster_mode(LevEngine *h, int32_t enabled);
 
-/* Grid-resident path (no reference counterpart): a single network whose CTAs
- * (64, 128 or 256 rows each, four lanes per row, its edges and node state in
+/* Grid-resident path (no reference counterpart): a network, or a batch, whose
+ * CTAs (64, 128 or 256 rows each, four, two or one lanes per row, its edges in
  * shared memory) can all be resident at once is stepped by lev_step_n /
  * lev_step_n_async with one cooperative launch per block of steps; the delay
- * ring stays in global memory (L2) and one grid barrier orders each step.
- * The barrier wait is bounded; a timeout makes lev_step_n / lev_sync return
+ * ring stays in global memory (L2) and the CTAs of a network exchange their
+ * sums and arrivals every step.  The waits are bounded; a timeout makes lev_step_n / lev_sync return
  * LEV_ERR_CUDA and disables the path.  Results are bitwise those of the
  * per-step kernel.  The cluster path takes precedence when both are enabled.
  * lev_grid_info: enabled = eligible and allowed (the path step blocks use;

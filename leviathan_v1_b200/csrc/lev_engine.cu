@@ -243,7 +243,8 @@ struct LevEngine {
   size_t grid_smem_R[3] = {0, 0, 0};
   int grid_max_tiles = 0;     // tiles of the largest network
   int grid_map_off[3] = {0, 0, 0};            // first entry of each choice in d_gmap
-  int2 *d_gmap = nullptr;     // batches: (network, CTA) per CTA
+  std::vector<int2> h_gmap;   // batches: (network, CTA) per CTA
+  int2 *d_gmap = nullptr;
   float2 *d_gwsum = nullptr;  // published sums, 32 per 256-node block
   unsigned *d_gbar = nullptr; // arrival counters
   int *h_gerr = nullptr, *d_gerr = nullptr;  // barrier timeout flag (mapped)
@@ -414,9 +415,6 @@ void free_engine(LevEngine *h) {
   dfree(h->d_omh_spec);
   dfree(h->d_class_nets);
   dfree(h->d_rhist);
-  dfree(h->d_gwsum);
-  dfree(h->d_gmap);
-  dfree(h->d_gbar);
   if (h->spec_block) cudaFreeAsync(h->spec_block, h->stream);
   if (h->slab) cudaFreeAsync(h->slab, h->stream);  // back to the engine pool
   if (h->h_gerr) mapped_free(reinterpret_cast<float *>(h->h_gerr));
@@ -911,10 +909,10 @@ void setup_cluster(LevEngine *h, const std::vector<int> &sl_len) {
     h->cluster_C = C;
     h->cluster_edge_cap = (int)cap;
     h->cluster_smem = smem;
-    // measured on B200: faster than per-step graph replay up to 256 rows per
-    // CTA (N = 4096 on 16 CTAs), slower at 1024; lev_autotune times both
-    // and decides per engine
-    h->use_cluster = R <= 256;
+    // up to 128 rows per CTA (N = 2048 on 16 CTAs) the cluster kernel beats the
+    // grid-resident one (N = 1000: 2.0 against 2.5 us per step), above it does
+    // not (N = 4096, k = 32: 8.1 against 2.7); lev_autotune times both
+    h->use_cluster = R <= 128;
     return;
   }
 }
@@ -989,8 +987,8 @@ int launch_grid(LevEngine *h, float dt, int len) {
 
 // Mid-sized single networks, and batches of as many rows in all: for each
 // rows-per-CTA choice, check that every CTA of the grid kernel can be resident
-// at once (shared memory, occupancy, cooperative launch).  Allocates the slice
-// sums, barriers, CTA map and error flag.
+// at once (shared memory, occupancy, cooperative launch), and lay out the CTA
+// map of a batch.  The device arrays are part of the engine's slab.
 int setup_grid(LevEngine *h, const std::vector<int> &sl_len) {
   h->grid_ok = false;
   if (h->part) return LEV_OK;
@@ -1005,6 +1003,14 @@ int setup_grid(LevEngine *h, const std::vector<int> &sl_len) {
   }
   if (!coop) return LEV_OK;
   for (const NetDesc &d : h->h_nets) h->grid_max_tiles = std::max(h->grid_max_tiles, d.ntiles);
+  double mean_len = 0.0;  // of the network with the longest rows
+  for (const NetDesc &d : h->h_nets) {
+    const long long ns = (d.N + 31) / 32;
+    double sum = 0.0;
+    for (long long s = 0; s < ns; ++s) sum += sl_len[d.slice_base + s];
+    if (ns) mean_len = std::max(mean_len, sum / (double)ns);
+  }
+  bool R_set = false;  // the rows-per-CTA choice below is made
   for (int ri = 0; ri < 3; ++ri) {
     const int R = kGridRs[ri];
     const long long C = grid_ctas(h, R);
@@ -1039,32 +1045,30 @@ int setup_grid(LevEngine *h, const std::vector<int> &sl_len) {
     h->grid_R_ok[ri] = true;
     h->grid_cap[ri] = (int)cap;
     h->grid_smem_R[ri] = smem;
-    if (!h->grid_ok) h->grid_R = R;  // the smallest: the most SMs
     h->grid_ok = true;
+    // The choice of an engine that has not been tuned: long rows (more than 26
+    // entries) want many lanes per row, the smallest R; short ones the smallest
+    // R with little more than one CTA per SM, else the largest.  Measured, us
+    // per step at R = 64 / 128 / 256: N = 10^4, k = 20 2.53 / 2.70 / 3.95;
+    // 1.4*10^4 2.83 / 2.68 / 3.89; 2.8*10^4 4.01 / 3.99 / 3.84; k = 32 4.50 /
+    // 4.70 / 6.93; 5*10^4, k = 8 - / 5.19 / 3.30.
+    if (R_set) continue;
+    h->grid_R = R;
+    R_set = mean_len > 26.0 || 4 * C <= 5LL * sms;
   }
   if (!h->grid_ok) return LEV_OK;
-  const size_t nsum = 32 * (size_t)h->total_tiles;
-  const size_t nbar = kGridBarPitch * (size_t)h->num_nets;
-  int rc = dev_alloc(h, &h->d_gwsum, nsum);
-  if (rc == LEV_OK) rc = dev_alloc(h, &h->d_gbar, nbar);
-  if (rc != LEV_OK) return rc;
   if (h->num_nets > 1) {
     // CTAs of a network side by side, the largest networks first
     std::vector<int> order(h->num_nets);
     for (int n = 0; n < h->num_nets; ++n) order[n] = n;
     std::stable_sort(order.begin(), order.end(),
                      [&](int x, int y) { return h->h_nets[x].N > h->h_nets[y].N; });
-    std::vector<int2> map;
     for (int ri = 0; ri < 3; ++ri) {
-      h->grid_map_off[ri] = (int)map.size();
+      h->grid_map_off[ri] = (int)h->h_gmap.size();
       if (!h->grid_R_ok[ri]) continue;
       for (int n : order)
-        for (int c = 0; c * kGridRs[ri] < h->h_nets[n].N; ++c) map.push_back(make_int2(n, c));
+        for (int c = 0; c * kGridRs[ri] < h->h_nets[n].N; ++c) h->h_gmap.push_back(make_int2(n, c));
     }
-    rc = dev_alloc(h, &h->d_gmap, map.size());
-    if (rc != LEV_OK) return rc;
-    LEV_TRY_CUDA(cudaMemcpy(h->d_gmap, map.data(), sizeof(int2) * map.size(),
-                            cudaMemcpyHostToDevice));
   }
   h->h_gerr = reinterpret_cast<int *>(mapped_alloc(1));
   if (!h->h_gerr) return fail(LEV_ERR_NOMEM, "mapped host memory: allocation failed");
@@ -1659,6 +1663,9 @@ int create_impl(LevEngine **out, int num_nets, const int32_t *Ns,
         {(void **)&h->d_rhist, sizeof(float) * h->block_len * num_nets},
         {(void **)&h->d_class_nets, sizeof(int) * num_nets},
         {(void **)&h->d_pend, sizeof(float2) * node_off},
+        {(void **)&h->d_gwsum, h->grid_ok ? sizeof(float2) * 32 * (size_t)tiles : 0},
+        {(void **)&h->d_gbar, h->grid_ok ? sizeof(unsigned) * kGridBarPitch * (size_t)num_nets : 0},
+        {(void **)&h->d_gmap, sizeof(int2) * h->h_gmap.size()},
     };
     size_t total = 0;
     for (const Part &q : parts) total += (q.bytes + 255) / 256 * 256;
@@ -1717,6 +1724,7 @@ int create_impl(LevEngine **out, int num_nets, const int32_t *Ns,
         {h->d_sl_off, h_sl_off.data(), sizeof(long long) * slices},
         {h->d_sl_len, h_sl_len.data(), sizeof(int) * slices},
         {t_sn, slice_net.data(), sizeof(int) * slices},
+        {h->d_gmap, h->h_gmap.data(), sizeof(int2) * h->h_gmap.size()},
     };
     if (e == cudaSuccess) e = cudaMemsetAsync(t_err, 0, sizeof(unsigned), h->stream);
     for (const auto &c : small)

@@ -11,8 +11,11 @@
 //     registers for the whole launch;
 //   * the delay ring stays in global memory, which at these sizes is
 //     L2-resident: each step writes theta(t+1) of the CTA's rows to ring slot
-//     t+1 through L2, and every gather reads through L2 (ld.global.cg), so no
-//     SM reads a stale L1 line of a slot another SM rewrote;
+//     t+1 through L2.  Gathers may hit L1: a CTA acquires the arrivals of every
+//     step (ld.acquire.gpu, which drops the SM's L1 lines) before it gathers
+//     phases of that step, so no line outlives a rewrite of its slot.  Within a
+//     step a 32-byte sector (two nodes, four slots) serves three gathers of a
+//     tile; through L2 only, N = 10^5, k = 20 took 8.4 us per step against 7.6;
 //   * every CTA publishes its part of (sum cos, sum sin) of a step, and every
 //     CTA adds all parts in the order of leviathan_kernel.cu:198-263, so all
 //     CTAs of a network compute the same r and gain (see grid_kernel);
@@ -355,7 +358,7 @@ __global__ void __launch_bounds__(kGridThreads, 3) grid_kernel(const GridArgs a)
                              nd.w_min, nd.w_max};
       const float local_sum =
           split_walk<MATH, LPR>(s_cd + base, s_w + base, len, deg, sl, th, ep, [&](uint32_t word) {
-            return __ldcg(ring + ring_pos_word(word, cur, bsi, Np));
+            return __ldca(ring + ring_pos_word(word, cur, bsi, Np));
           });
       if (step > 0) {
         cta_barrier();  // A
