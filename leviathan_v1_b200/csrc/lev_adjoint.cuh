@@ -31,11 +31,15 @@
 //     lam_thh(s) = lam_thh(s+1) - lam_diff;  lam_omh(s) = lam_omh(s+1) + dt lam_thh(s+1)
 //   lam_g(s)   = lam_g(s+1) dg(s+1)/dg(s) + sum_i lam_th'_i dt S_i
 // The wraps have derivative 1; a clamped weight or gain passes nothing;
-// |eps| has derivative sign(eps).  The adjoint ring has max_delay+2 slots so
-// the slot finalised at the start of a launch is never one scattered into by
-// the same launch (reads of time s+1, writes of times s-max_delay..s).
+// |eps| has derivative sign(eps).  The adjoint ring has max_delay+3 slots: the
+// slot finalised by a reverse step (time s+1) is not one that the same step
+// scatters into (times s-max_delay..s), nor one that the step reversed next
+// does, so the grid-resident reverse orders its clearing one step later.
 
 namespace lev {
+
+// Slots of the adjoint ring.
+__host__ __device__ __forceinline__ int adj_slots(int max_delay) { return max_delay + 3; }
 
 struct AdjFwdArgs {
   const NetDesc *nets;  // adjoint copies: bsi = C + max_delay + 2
@@ -524,7 +528,7 @@ __global__ void __launch_bounds__(kTile, MINB) adj_bwd_kernel(const AdjBwdArgs a
   const long long gi = nd.node_off + row;
   const float dt = a.dt;
   const int Np = nd.Np;
-  const int bsa = nd.max_delay + 2;
+  const int bsa = adj_slots(nd.max_delay);
   const int hs = (int)(a.s - a.seg_start) + nd.max_delay;  // history slot of theta(s)
   const float *H = a.H + nd.ring_off;
   float *AR = a.adj_ring + nd.aux_off;
@@ -701,7 +705,7 @@ __global__ void __launch_bounds__(kTile, 4) adj_bwd_split_kernel(const AdjBwdArg
   const long long gi = nd.node_off + row;
   const float dt = a.dt;
   const int Np = nd.Np;
-  const int bsa = nd.max_delay + 2;
+  const int bsa = adj_slots(nd.max_delay);
   const int hs = (int)(a.s - a.seg_start) + nd.max_delay;  // history slot of theta(s)
   const float *H = a.H + nd.ring_off;
   float *AR = a.adj_ring + nd.aux_off;
@@ -895,7 +899,7 @@ __global__ void adj_finalize_kernel(const NetDesc *nets, int num_nets,
   const int n = blockIdx.y;
   if (n >= num_nets) return;
   const NetDesc nd = nets[n];
-  const int bsa = nd.max_delay + 2;
+  const int bsa = adj_slots(nd.max_delay);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nd.N;
        i += gridDim.x * blockDim.x) {
     float v = lam_th[nd.node_off + i];

@@ -3240,7 +3240,7 @@ struct LevAdjoint {
   size_t gf_smem[3] = {0, 0, 0}, gb_smem[3] = {0, 0, 0};
   bool gp_ok[3] = {false, false, false};  // paired recompute + reverse launch fits
   bool use_pair = true;
-  int g_nwarps = 0, g_gpad = 0;
+  int g_gpad = 0;
   float2 *g_wsum = nullptr;
   float *g_lgp = nullptr;
   unsigned *g_bar = nullptr;
@@ -3355,26 +3355,16 @@ int adj_ckpt(LevAdjoint *a, int seg, bool save, cudaStream_t s = nullptr,
 
 using AdjGridFwdFn = void (*)(AdjGridFwdArgs);
 using AdjGridBwdFn = void (*)(AdjGridBwdArgs);
-AdjGridFwdFn adj_grid_fwd_fn(int R, int math_mode) {
-  const bool acc = math_mode == LEV_MATH_ACCURATE;
-  if (R == 64) return acc ? adj_grid_fwd_kernel<1, 64, 8> : adj_grid_fwd_kernel<0, 64, 8>;
-  if (R == 128) return acc ? adj_grid_fwd_kernel<1, 128, 8> : adj_grid_fwd_kernel<0, 128, 8>;
-  return acc ? adj_grid_fwd_kernel<1, 256, 8> : adj_grid_fwd_kernel<0, 256, 8>;
-}
 using AdjGridPairFn = void (*)(AdjGridFwdArgs, AdjGridBwdArgs, int);
-AdjGridPairFn adj_grid_pair_fn(int R, int math_mode) {
-  const bool acc = math_mode == LEV_MATH_ACCURATE;
-  if (R == 64) return acc ? adj_grid_pair_kernel<1, 64, 8, 4> : adj_grid_pair_kernel<0, 64, 8, 4>;
-  if (R == 128)
-    return acc ? adj_grid_pair_kernel<1, 128, 8, 4> : adj_grid_pair_kernel<0, 128, 8, 4>;
-  return acc ? adj_grid_pair_kernel<1, 256, 8, 4> : adj_grid_pair_kernel<0, 256, 8, 4>;
-}
-AdjGridBwdFn adj_grid_bwd_fn(int R, int math_mode) {
-  const bool acc = math_mode == LEV_MATH_ACCURATE;
-  if (R == 64) return acc ? adj_grid_bwd_kernel<1, 64, 8> : adj_grid_bwd_kernel<0, 64, 8>;
-  if (R == 128) return acc ? adj_grid_bwd_kernel<1, 128, 8> : adj_grid_bwd_kernel<0, 128, 8>;
-  return acc ? adj_grid_bwd_kernel<1, 256, 4> : adj_grid_bwd_kernel<0, 256, 4>;
-}
+#define LEV_BY_ROWS(kernel)                                 \
+  const bool acc = math_mode == LEV_MATH_ACCURATE;          \
+  if (R == 64) return acc ? kernel<1, 64> : kernel<0, 64>;  \
+  if (R == 128) return acc ? kernel<1, 128> : kernel<0, 128>; \
+  return acc ? kernel<1, 256> : kernel<0, 256>;
+AdjGridFwdFn adj_grid_fwd_fn(int R, int math_mode) { LEV_BY_ROWS(adj_grid_fwd_kernel) }
+AdjGridPairFn adj_grid_pair_fn(int R, int math_mode) { LEV_BY_ROWS(adj_grid_pair_kernel) }
+AdjGridBwdFn adj_grid_bwd_fn(int R, int math_mode) { LEV_BY_ROWS(adj_grid_bwd_kernel) }
+#undef LEV_BY_ROWS
 
 // Grid-resident segments for a single network: per rows-per-CTA choice, the
 // shared memory of both kernels and whether every CTA can be resident at once.
@@ -3393,8 +3383,8 @@ int adj_setup_grid(LevAdjoint *a, const std::vector<long long> &sl_off,
     return LEV_OK;
   }
   if (!coop) return LEV_OK;
-  const int nwarps = 8 * ((d.N + kTile - 1) / kTile);
   int max_gpad = 0;
+  bool R_set = false;
   for (int ri = 0; ri < 3; ++ri) {
     const int R = kGridRs[ri];
     const int C = (d.N + R - 1) / R;
@@ -3407,10 +3397,9 @@ int adj_setup_grid(LevAdjoint *a, const std::vector<long long> &sl_off,
         e += 32LL * sl_len[d.slice_base + s];
       cap = std::max(cap, e);
     }
-    const size_t fsm = sizeof(float2) * nwarps + sizeof(float) * 6 * R +
+    const size_t fsm = (R < 256 ? sizeof(float2) * 8 * (size_t)d.ntiles : 0) +
                        sizeof(int) * 2 * (R / 32) + 8 * (size_t)cap;
-    const size_t bsm = sizeof(float) * (4 * R + gpad) + sizeof(int) * 2 * (R / 32) +
-                       8 * (size_t)cap;
+    const size_t bsm = sizeof(int) * 2 * (R / 32) + 16 * (size_t)cap;
     if (std::max(fsm, bsm) + 1024 > (size_t)max_smem) continue;
     bool ok = true;
     for (int m = 0; m < 2 && ok; ++m) {
@@ -3419,9 +3408,9 @@ int adj_setup_grid(LevAdjoint *a, const std::vector<long long> &sl_off,
       const void *bf = reinterpret_cast<const void *>(adj_grid_bwd_fn(R, mm));
       int pf = 0, pb = 0;
       ok = allow_smem(ff, fsm) && allow_smem(bf, bsm) &&
-           cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pf, ff, kSplitLPR * R, fsm) ==
+           cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pf, ff, kGridThreads, fsm) ==
                cudaSuccess &&
-           cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pb, bf, kSplitLPR * R, bsm) ==
+           cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pb, bf, kGridThreads, bsm) ==
                cudaSuccess &&
            (long long)pf * sms >= C && (long long)pb * sms >= C;
     }
@@ -3435,7 +3424,7 @@ int adj_setup_grid(LevAdjoint *a, const std::vector<long long> &sl_off,
       const size_t psm = std::max(fsm, bsm);
       int per_sm = 0;
       pok = allow_smem(pf, psm) &&
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pf, kSplitLPR * R, psm) ==
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pf, kGridThreads, psm) ==
                 cudaSuccess &&
             (long long)per_sm * sms >= 2LL * C;
     }
@@ -3446,17 +3435,21 @@ int adj_setup_grid(LevAdjoint *a, const std::vector<long long> &sl_off,
     a->gf_smem[ri] = fsm;
     a->gb_smem[ri] = bsm;
     max_gpad = std::max(max_gpad, gpad);
-    if (!a->grid_ok) a->grid_R = R;  // the smallest: the most SMs
+    // the smallest with little more than one CTA per SM, else the largest
+    if (!R_set) {
+      a->grid_R = R;
+      R_set = 4 * C <= 5 * sms;
+    }
     a->grid_ok = true;
   }
   if (!a->grid_ok) return LEV_OK;
-  a->g_nwarps = nwarps;
+  // arrival counters, published sums and parts: one block, so that a launch
+  // clears what it uses with two fills
   a->g_gpad = max_gpad;
-  int rc = adj_alloc(a, &a->g_wsum, 2LL * nwarps);
-  if (rc == LEV_OK) rc = adj_alloc(a, &a->g_lgp, 2LL * max_gpad);
-  if (rc == LEV_OK) rc = adj_alloc(a, &a->g_bar, 2);
+  int rc = adj_alloc(a, &a->g_bar, 2 * kGridBarPitch);
+  if (rc == LEV_OK) rc = adj_alloc(a, &a->g_wsum, 32LL * d.ntiles + 2LL * max_gpad);
   if (rc != LEV_OK) return rc;
-  LEV_TRY_CUDA(cudaMemset(a->g_wsum, 0, sizeof(float2) * 2 * (size_t)nwarps));
+  a->g_lgp = reinterpret_cast<float *>(a->g_wsum + 32LL * d.ntiles);
   a->h_gerr = reinterpret_cast<int *>(mapped_alloc(1));
   if (!a->h_gerr) return fail(LEV_ERR_NOMEM, "mapped host memory: allocation failed");
   *a->h_gerr = 0;
@@ -3511,9 +3504,19 @@ void adj_grid_fill_fwd(LevAdjoint *a, AdjGridFwdArgs &f, int n) {
   f.wait = a->grid_wait;
   f.SL = a->SL;
   f.early = e->pair_ok ? 1 : 0;  // no delay is 0
-  f.nwarps = a->g_nwarps;
+  f.sum_cap = a->grid_R < 256 ? 8 * a->h_nets[0].ntiles : 0;
   f.edge_cap = a->g_cap[ri];
   f.n_steps = n;
+}
+
+// No arrivals, nothing published.
+cudaError_t adj_grid_clear(LevAdjoint *a, cudaStream_t s) {
+  cudaError_t e = cudaMemsetAsync(a->g_bar, 0, sizeof(unsigned) * 2 * kGridBarPitch, s);
+  if (e == cudaSuccess)
+    e = cudaMemsetAsync(a->g_wsum, 0xff,
+                        sizeof(float2) * (32 * (size_t)a->h_nets[0].ntiles +
+                                          2 * (size_t)a->g_gpad), s);
+  return e;
 }
 
 // One cooperative launch of the grid-resident forward over `n` steps (the
@@ -3521,11 +3524,11 @@ void adj_grid_fill_fwd(LevAdjoint *a, AdjGridFwdArgs &f, int n) {
 int adj_grid_launch_fwd(LevAdjoint *a, AdjGridFwdArgs f, int n, cudaStream_t s) {
   LevEngine *e = a->e;
   const int R = a->grid_R, ri = grid_r_index(R);
-  LEV_TRY_CUDA(cudaMemsetAsync(a->g_bar, 0, sizeof(unsigned), s));
+  LEV_TRY_CUDA(adj_grid_clear(a, s));
   adj_grid_fill_fwd(a, f, n);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((a->h_nets[0].N + R - 1) / R);
-  cfg.blockDim = dim3(kSplitLPR * R);
+  cfg.blockDim = dim3(kGridThreads);
   cfg.dynamicSmemBytes = a->gf_smem[ri];
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
@@ -3554,7 +3557,8 @@ void adj_grid_fill_bwd(LevAdjoint *a, AdjGridBwdArgs &b) {
   b.lam_g = a->lam_g;
   b.grad_omega = a->grad_omega_acc;
   b.lgp = a->g_lgp;
-  b.bar = a->g_bar;
+  b.gpad = a->g_gpad;
+  b.bar = a->g_bar + kGridBarPitch;
   b.err = a->d_gerr;
   b.wait = a->grid_wait;
   b.early = e->pair_ok ? 1 : 0;  // no delay is 0
@@ -3566,11 +3570,11 @@ void adj_grid_fill_bwd(LevAdjoint *a, AdjGridBwdArgs &b) {
 int adj_grid_launch_bwd(LevAdjoint *a, AdjGridBwdArgs b, cudaStream_t s) {
   LevEngine *e = a->e;
   const int R = a->grid_R, ri = grid_r_index(R);
-  LEV_TRY_CUDA(cudaMemsetAsync(a->g_bar, 0, sizeof(unsigned), s));
+  LEV_TRY_CUDA(adj_grid_clear(a, s));
   adj_grid_fill_bwd(a, b);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((a->h_nets[0].N + R - 1) / R);
-  cfg.blockDim = dim3(kSplitLPR * R);
+  cfg.blockDim = dim3(kGridThreads);
   cfg.dynamicSmemBytes = a->gb_smem[ri];
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
@@ -3590,14 +3594,12 @@ int adj_grid_launch_pair(LevAdjoint *a, AdjGridFwdArgs f, int n, AdjGridBwdArgs 
   LevEngine *e = a->e;
   const int R = a->grid_R, ri = grid_r_index(R);
   const int C = (a->h_nets[0].N + R - 1) / R;
-  LEV_TRY_CUDA(cudaMemsetAsync(a->g_bar, 0, 2 * sizeof(unsigned), s));
+  LEV_TRY_CUDA(adj_grid_clear(a, s));
   adj_grid_fill_fwd(a, f, n);
   adj_grid_fill_bwd(a, b);
-  f.bar = a->g_bar;
-  b.bar = a->g_bar + 1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * C);
-  cfg.blockDim = dim3(kSplitLPR * R);
+  cfg.blockDim = dim3(kGridThreads);
   cfg.dynamicSmemBytes = std::max(a->gf_smem[ri], a->gb_smem[ri]);
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
@@ -3637,7 +3639,7 @@ int lev_adj_create(LevAdjoint **out, LevEngine *e, int32_t segment,
     d.ring_off = a->ring_floats;
     d.aux_off = a->aux_floats;
     a->ring_floats += (long long)d.bsi * d.Np;
-    a->aux_floats += (long long)(d.max_delay + 2) * d.Np;
+    a->aux_floats += (long long)adj_slots(d.max_delay) * d.Np;
     ck_off[n] = a->ckr_floats;
     a->ckr_floats += (long long)(d.max_delay + 1) * d.N;
     if ((unsigned long long)d.bsi * (unsigned long long)d.Np >= (1ull << 32)) {

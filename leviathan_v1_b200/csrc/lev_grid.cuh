@@ -247,6 +247,31 @@ __device__ __forceinline__ void cta_barrier() {
   asm volatile("bar.sync 1, %0;" ::"n"(kGridThreads) : "memory");
 }
 
+// One warp publishes its CTA's sums of step `step` from the warps' parts and
+// clears those of step-2 for step+2.
+template <int R>
+__device__ __forceinline__ void grid_publish_part(float2 *wsum, int step, int nblocks, int nsum,
+                                                  int cta, int lane, const float2 *s_part) {
+  constexpr int LPR = 256 / R;
+  constexpr int count = R == 256 ? 1 : R / 32;
+  const int at = cta * count + lane;
+  if (lane >= count || at >= nsum) return;
+  float2 v;
+  if (R == 256) {
+    float vc[8], vs[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      vc[i] = s_part[i].x;
+      vs[i] = s_part[i].y;
+    }
+    v = make_float2(block_tree8(vc), block_tree8(vs));
+  } else {
+    v = split_slice_sum<LPR>(s_part + LPR * lane);
+  }
+  grid_publish(wsum + (step & 3) * 8 * nblocks + at, v);
+  grid_unpublish(wsum + ((step + 2) & 3) * 8 * nblocks + at);
+}
+
 // shared memory layout (bytes, from the dynamic base):
 //   sums   float2 [8 * blocks of the largest network]  (R < 256)
 //   sloff, sllen  int [R/32]
@@ -437,24 +462,7 @@ __global__ void __launch_bounds__(kGridThreads, 3) grid_kernel(const GridArgs a)
       }
       cur = (cur + 1 == bsi) ? 0 : cur + 1;
       cta_barrier();  // B
-      const int first = kBlocks ? cta : row0 / 32;
-      const bool mine = lane < (kBlocks ? 1 : nslices) && first + lane < nsum;
-      if (mine) {
-        float2 v;
-        if (kBlocks) {
-          float vc[8], vs[8];
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            vc[i] = s_part[i].x;
-            vs[i] = s_part[i].y;
-          }
-          v = make_float2(block_tree8(vc), block_tree8(vs));
-        } else {
-          v = split_slice_sum<LPR>(s_part + LPR * lane);
-        }
-        grid_publish(wsum + (step & 3) * 8 * nblocks + first + lane, v);
-        grid_unpublish(wsum + ((step + 2) & 3) * 8 * nblocks + first + lane);
-      }
+      grid_publish_part<R>(wsum, step, nblocks, nsum, cta, lane, s_part);
       __syncwarp();
       if (lane == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
       if (observe && ok && step > 0) hub.observe(hub_phase);

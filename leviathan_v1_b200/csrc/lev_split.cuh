@@ -72,13 +72,14 @@ __device__ __forceinline__ void split_for_entries(const int *sloff, const int *s
 
 // The row's walk (csr_physics_kernel, leviathan_kernel.cu:126-165) over cd /
 // w, the slice's entries in shared memory; gather(word) returns the delayed
-// phase.  Returns the row's coupling sum in all its lanes.  Entries past the
+// phase and keep(k, weight) sees the new weight of the row's entry k.  Returns
+// the row's coupling sum in all its lanes.  Entries past the
 // row's degree enter the sum as 0 * sin(0 - th): a zero, or a NaN in a row
 // whose phase is not finite and whose step sets it to 0 whatever the sum.
-template <int MATH, int LPR, int U, class Gather>
+template <int MATH, int LPR, int U, class Gather, class Keep>
 __device__ __forceinline__ float split_walk_u(const uint32_t *cd, float *w, int len, int deg,
                                               const SplitLane &sl, float th,
-                                              const EdgeParams &ep, Gather gather) {
+                                              const EdgeParams &ep, Gather gather, Keep keep) {
   const unsigned mask = 0xffffffffu;
   const int lq = (sl.l + sl.q) & 31;
   float local_sum = 0.0f;
@@ -101,7 +102,10 @@ __device__ __forceinline__ float split_walk_u(const uint32_t *cd, float *w, int 
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const float wn = edge_update<MATH>(ep, dj[u], wv[u], &dj[u]);
-      if (k0 + u < deg) w[at + 32 * u] = wn;
+      if (k0 + u < deg) {
+        w[at + 32 * u] = wn;
+        keep(k0 + u, wn);
+      }
     }
 #pragma unroll
     for (int ph = 0; ph < LPR; ++ph) {
@@ -113,20 +117,26 @@ __device__ __forceinline__ float split_walk_u(const uint32_t *cd, float *w, int 
   return local_sum;
 }
 
+template <int MATH, int LPR, class Gather, class Keep>
+__device__ __forceinline__ float split_walk(const uint32_t *cd, float *w, int len, int deg,
+                                            const SplitLane &sl, float th, const EdgeParams &ep,
+                                            Gather gather, Keep keep) {
+  switch (split_unroll<LPR>(len)) {  // warp-uniform
+    case 1: return split_walk_u<MATH, LPR, 1>(cd, w, len, deg, sl, th, ep, gather, keep);
+    case 2: return split_walk_u<MATH, LPR, 2>(cd, w, len, deg, sl, th, ep, gather, keep);
+    case 3: return split_walk_u<MATH, LPR, 3>(cd, w, len, deg, sl, th, ep, gather, keep);
+    case 4: return split_walk_u<MATH, LPR, 4>(cd, w, len, deg, sl, th, ep, gather, keep);
+    case 5: return split_walk_u<MATH, LPR, 5>(cd, w, len, deg, sl, th, ep, gather, keep);
+    case 6: return split_walk_u<MATH, LPR, 6>(cd, w, len, deg, sl, th, ep, gather, keep);
+    case 7: return split_walk_u<MATH, LPR, 7>(cd, w, len, deg, sl, th, ep, gather, keep);
+    default: return split_walk_u<MATH, LPR, 8>(cd, w, len, deg, sl, th, ep, gather, keep);
+  }
+}
 template <int MATH, int LPR, class Gather>
 __device__ __forceinline__ float split_walk(const uint32_t *cd, float *w, int len, int deg,
                                             const SplitLane &sl, float th, const EdgeParams &ep,
                                             Gather gather) {
-  switch (split_unroll<LPR>(len)) {  // warp-uniform
-    case 1: return split_walk_u<MATH, LPR, 1>(cd, w, len, deg, sl, th, ep, gather);
-    case 2: return split_walk_u<MATH, LPR, 2>(cd, w, len, deg, sl, th, ep, gather);
-    case 3: return split_walk_u<MATH, LPR, 3>(cd, w, len, deg, sl, th, ep, gather);
-    case 4: return split_walk_u<MATH, LPR, 4>(cd, w, len, deg, sl, th, ep, gather);
-    case 5: return split_walk_u<MATH, LPR, 5>(cd, w, len, deg, sl, th, ep, gather);
-    case 6: return split_walk_u<MATH, LPR, 6>(cd, w, len, deg, sl, th, ep, gather);
-    case 7: return split_walk_u<MATH, LPR, 7>(cd, w, len, deg, sl, th, ep, gather);
-    default: return split_walk_u<MATH, LPR, 8>(cd, w, len, deg, sl, th, ep, gather);
-  }
+  return split_walk<MATH, LPR>(cd, w, len, deg, sl, th, ep, gather, [](int, float) {});
 }
 
 // The warp's part of the 32-row tree: rows 16 down to LPR apart; lane 0 holds
