@@ -480,8 +480,7 @@ __device__ __forceinline__ void adj_grid_bwd_body(const AdjGridBwdArgs &a, const
       const float eps = sinf(diff);
       float sn1, cs1;
       sincosf(th1, &sn1, &cs1);
-      const float ae = fabsf(eps);
-      const float hebb = 1.0f - gamma * ae;
+      const EdgeParams ep = {dt, eta, lam, __fmaf_rn(-gamma, fabsf(eps), 1.0f), w_min, w_max};
       const float *w_s = a.w_hist + (long long)kk * a.SL + ebase + eoff + sl.l;
       float S_i = 0.0f, labs = 0.0f;
       for (int kb = 0; kb < len; kb += LPR * U) {
@@ -496,21 +495,23 @@ __device__ __forceinline__ void adj_grid_bwd_body(const AdjGridBwdArgs &a, const
         }
 #pragma unroll
         for (int u = 0; u < U; ++u)
-          dj[u] = __ldg(H + (long long)(hs - (int)(p[u] & 255u)) * Np + (p[u] >> 8)) - th;
-        wrap_pm_pi_group(dj);
+          dj[u] = (kb + LPR * u + sl.q < deg)
+                      ? __ldg(H + ((unsigned)(hs - (int)(p[u] & 255u)) * (unsigned)Np + (p[u] >> 8))) - th
+                      : 0.0f;
+        float sn[U], cs[U];
+        wrap_sincos_group<MATH>(dj, sn, cs);
 #pragma unroll
         for (int u = 0; u < U; ++u) {
           const int e = kb + LPR * u + sl.q;
+          const float w = wv[u];
+          S_i += w * sn[u];
+          const float w_pre = edge_weight_free(ep, cs[u], w);
+          const float lw = (e < deg) ? s_lw[at0 + 32 * e] : 0.0f;
+          const float m = (w_pre >= w_min && w_pre <= w_max) ? lw : 0.0f;
+          labs += m * cs[u];
           if (e < deg) {
-            const float w = wv[u];
-            float sn, cs;
-            lev_sincos<MATH>(dj[u], &sn, &cs);
-            S_i += w * sn;
-            const float w_pre = w + dt * (eta * cs * hebb - lam * w);
-            const float m = (w_pre >= w_min && w_pre <= w_max) ? s_lw[at0 + 32 * e] : 0.0f;
-            labs -= m * dt * eta * gamma * cs;
             s_lw[at0 + 32 * e] = m;
-            s_sa[at0 + 32 * e] = make_float2(sn, w * cs);
+            s_sa[at0 + 32 * e] = make_float2(sn[u], w * cs[u]);
           }
         }
       }
@@ -548,19 +549,18 @@ __device__ __forceinline__ void adj_grid_bwd_body(const AdjGridBwdArgs &a, const
       cta_barrier();  // B
       // ---- scatter ------------------------------------------------------------------
       const float lam_S = lt1 * dt * tr.x;
-      const float hq = dt * eta * hebb;
+      const float hq = dt * eta * ep.hebb;
       float lsum = 0.0f;
-      for (int e = sl.q; e < len; e += LPR) {
-        if (e < deg) {
-          const uint32_t p = s_cd[at0 + 32 * e];
-          const float m = s_lw[at0 + 32 * e];
-          const float2 sa = s_sa[at0 + 32 * e];
-          s_lw[at0 + 32 * e] = m * decay + lam_S * sa.x;
-          const float lD = lam_S * sa.y - m * hq * sa.x;
-          const unsigned s0 = (unsigned)(as_s - (int)(p & 255u));
-          atomicAdd(AR + (min(s0, s0 + (unsigned)bsa) * (unsigned)Np + (p >> 8)), lD);
-          lsum -= lD;
-        }
+#pragma unroll 4
+      for (int e = sl.q; e < deg; e += LPR) {
+        const uint32_t p = s_cd[at0 + 32 * e];
+        const float m = s_lw[at0 + 32 * e];
+        const float2 sa = s_sa[at0 + 32 * e];
+        s_lw[at0 + 32 * e] = m * decay + lam_S * sa.x;
+        const float lD = lam_S * sa.y - m * hq * sa.x;
+        const unsigned s0 = (unsigned)(as_s - (int)(p & 255u));
+        atomicAdd(AR + (min(s0, s0 + (unsigned)bsa) * (unsigned)Np + (p >> 8)), lD);
+        lsum -= lD;
       }
 #pragma unroll
       for (int off = 1; off < LPR; off *= 2) lsum += __shfl_xor_sync(mask, lsum, off);
@@ -573,7 +573,8 @@ __device__ __forceinline__ void adj_grid_bwd_body(const AdjGridBwdArgs &a, const
         }
         // (D) predictor
         const float sgn = (eps > 0.0f) ? 1.0f : ((eps < 0.0f) ? -1.0f : 0.0f);
-        const float leps = -lt1 * dt * nd.alpha + labs * sgn + lomh * nd.kappa_w * dt;
+        const float leps = -lt1 * dt * nd.alpha - dt * eta * gamma * labs * sgn +
+                           lomh * nd.kappa_w * dt;
         const float ldiff = leps * cosf(diff);
         lt = lt1 + lsum + ldiff;
         const float lthh1 = lthh;

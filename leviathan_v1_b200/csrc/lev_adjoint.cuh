@@ -113,9 +113,8 @@ __global__ void __launch_bounds__(kTile, 5) adj_fwd_kernel(const AdjFwdArgs a) {
     const int *rp = a.row_ptr + nd.rp_off + row;
     deg = rp[1] - rp[0];
   }
-  const float my_eps = fabsf(eps);
-  const float eta = nd.eta, gamma = nd.gamma, lam = nd.lam;
-  const float w_min = nd.w_min, w_max = nd.w_max;
+  const EdgeParams ep = {dt, nd.eta, nd.lam, __fmaf_rn(-nd.gamma, fabsf(eps), 1.0f),
+                         nd.w_min, nd.w_max};
   float local_sum = 0.0f;
   const int slice_row0 = row0 + 32 * warp;
   if (slice_row0 < N) {
@@ -137,9 +136,8 @@ __global__ void __launch_bounds__(kTile, 5) adj_fwd_kernel(const AdjFwdArgs a) {
       float dj[U];
 #pragma unroll
       for (int u = 0; u < U; ++u) {
-        int slot = cur - (int)(p[u] & 255u);
-        slot += (slot < 0) ? bsi : 0;
-        dj[u] = ld_ring(ring + ((unsigned)slot * (unsigned)Np + (p[u] >> 8)));
+        const unsigned s0 = (unsigned)(cur - (int)(p[u] & 255u));
+        dj[u] = ld_ring(ring + (min(s0, s0 + (unsigned)bsi) * (unsigned)Np + (p[u] >> 8)));
       }
       uint32_t pn[U];
       float wn[U];
@@ -149,23 +147,22 @@ __global__ void __launch_bounds__(kTile, 5) adj_fwd_kernel(const AdjFwdArgs a) {
         pn[u] = in ? __ldg(a.sl_cd + base + 32 * (k0 + U + u)) : 0u;
         wn[u] = in ? a.w_in[base + 32 * (k0 + U + u)] : 0.0f;
       }
+      if (a.dj_rec) {
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (k0 + u < deg) a.dj_rec[base + 32 * (k0 + u)] = dj[u];
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) dj[u] -= th;
+      float sn[U], cs[U];
+      wrap_sincos_group<MATH>(dj, sn, cs);
 #pragma unroll
       for (int u = 0; u < U; ++u) {
-        if (k0 + u < deg) {
-          const float delayed_j = dj[u];
-          float diff = delayed_j - th;
-          diff = wrap_pm_pi(diff);
-          float w = wv[u];
-          float sin_diff, cos_diff;
-          lev_sincos<MATH>(diff, &sin_diff, &cos_diff);
-          local_sum += w * sin_diff;
-          float dw = dt * (eta * cos_diff * (1.0f - gamma * my_eps) - lam * w);
-          w += dw;
-          if (!isfinite(w)) w = w_min;
-          w = fmaxf(w_min, fminf(w_max, w));
-          a.w_out[base + 32 * (k0 + u)] = w;
-          if (a.dj_rec) a.dj_rec[base + 32 * (k0 + u)] = delayed_j;
-        }
+        const bool in = k0 + u < deg;
+        const float sum = __fmaf_rn(wv[u], sn[u], local_sum);
+        local_sum = in ? sum : local_sum;
+        const float w = edge_weight(ep, cs[u], wv[u]);
+        if (in) a.w_out[base + 32 * (k0 + u)] = w;
       }
 #pragma unroll
       for (int u = 0; u < U; ++u) {
@@ -581,10 +578,10 @@ __global__ void __launch_bounds__(kTile, MINB) adj_bwd_kernel(const AdjBwdArgs a
     const int *rp = a.row_ptr + nd.rp_off + row;
     deg = rp[1] - rp[0];
   }
-  const float ae = fabsf(eps);
-  const float eta = nd.eta, gamma = nd.gamma, lam = nd.lam;
-  const float w_min = nd.w_min, w_max = nd.w_max;
-  const float decay = 1.0f - dt * lam;
+  const EdgeParams ep = {dt, nd.eta, nd.lam, __fmaf_rn(-nd.gamma, fabsf(eps), 1.0f),
+                         nd.w_min, nd.w_max};
+  const float decay = 1.0f - dt * nd.lam;
+  const float hq = dt * nd.eta * ep.hebb;
   float S_i = 0.0f, lth = lt1, labs = 0.0f;
   const int slice_row0 = row0 + 32 * warp;
   if (slice_row0 < N) {
@@ -604,39 +601,36 @@ __global__ void __launch_bounds__(kTile, MINB) adj_bwd_kernel(const AdjBwdArgs a
         p[u] = in ? __ldg(a.sl_cd + base + 32 * (k0 + u)) : 0u;
         wv[u] = in ? a.w_s[base + 32 * (k0 + u)] : 0.0f;
         lw[u] = in ? a.lam_w[base + 32 * (k0 + u)] : 0.0f;
-        if (a.dj_s) dj[u] = in ? __ldcs(a.dj_s + base + 32 * (k0 + u)) : 0.0f;
+        if (a.dj_s) dj[u] = in ? __ldcs(a.dj_s + base + 32 * (k0 + u)) : th;
       }
       if (!a.dj_s) {
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-          const int d = (int)(p[u] & 255u);
-          dj[u] = H[(long long)(hs - d) * Np + (p[u] >> 8)];
-        }
+        for (int u = 0; u < U; ++u)
+          dj[u] = (k0 + u < deg) ? H[(unsigned)(hs - (int)(p[u] & 255u)) * (unsigned)Np + (p[u] >> 8)]
+                                 : th;
       }
 #pragma unroll
+      for (int u = 0; u < U; ++u) dj[u] -= th;
+      float sn[U], cs[U];
+      wrap_sincos_group<MATH>(dj, sn, cs);
+#pragma unroll
       for (int u = 0; u < U; ++u) {
+        const float w = wv[u];
+        const float w_pre = edge_weight_free(ep, cs[u], w);
+        const float m = (w_pre >= ep.w_min && w_pre <= ep.w_max) ? lw[u] : 0.0f;
+        const float lD = lam_S * (w * cs[u]) - m * hq * sn[u];
         if (k0 + u < deg) {
-          const int j = (int)(p[u] >> 8), d = (int)(p[u] & 255u);
-          const float delayed_j = dj[u];
-          float dlt = delayed_j - th;
-          dlt = wrap_pm_pi(dlt);
-          const float w = wv[u];
-          float sn, cs;
-          lev_sincos<MATH>(dlt, &sn, &cs);
-          S_i += w * sn;
-          const float w_pre = w + dt * (eta * cs * (1.0f - gamma * ae) - lam * w);
-          const float c = (w_pre >= w_min && w_pre <= w_max) ? 1.0f : 0.0f;
-          const float lwn = lw[u];
-          a.lam_w[base + 32 * (k0 + u)] = lwn * c * decay + lam_S * sn;
-          const float lD = lam_S * w * cs - lwn * c * dt * eta * sn * (1.0f - gamma * ae);
-          labs -= lwn * c * dt * eta * gamma * cs;
-          const int slot = (as_s - d < 0) ? as_s - d + bsa : as_s - d;
-          atomicAdd(AR + (long long)slot * Np + j, lD);
+          S_i += w * sn[u];
+          labs += m * cs[u];
           lth -= lD;
+          a.lam_w[base + 32 * (k0 + u)] = m * decay + lam_S * sn[u];
+          const unsigned s0 = (unsigned)(as_s - (int)(p[u] & 255u));
+          atomicAdd(AR + (min(s0, s0 + (unsigned)bsa) * (unsigned)Np + (p[u] >> 8)), lD);
         }
       }
     }
   }
+  labs *= -dt * nd.eta * nd.gamma;
   if (live) {
     // (D) predictor
     const float sgn = (eps > 0.0f) ? 1.0f : ((eps < 0.0f) ? -1.0f : 0.0f);

@@ -3384,7 +3384,6 @@ int adj_setup_grid(LevAdjoint *a, const std::vector<long long> &sl_off,
   }
   if (!coop) return LEV_OK;
   int max_gpad = 0;
-  bool R_set = false;
   for (int ri = 0; ri < 3; ++ri) {
     const int R = kGridRs[ri];
     const int C = (d.N + R - 1) / R;
@@ -3435,11 +3434,11 @@ int adj_setup_grid(LevAdjoint *a, const std::vector<long long> &sl_off,
     a->gf_smem[ri] = fsm;
     a->gb_smem[ri] = bsm;
     max_gpad = std::max(max_gpad, gpad);
-    // the smallest with little more than one CTA per SM, else the largest
-    if (!R_set) {
-      a->grid_R = R;
-      R_set = 4 * C <= 5 * sms;
-    }
+    // the smallest: the steps wait on instructions, and more lanes per row are
+    // more warps (us per 100 steps forward / backward, k = 20: N = 2*10^4 R = 64
+    // 518 / 1,391, R = 128 587 / 1,439; 5*10^4 R = 128 778 / 2,230, R = 256 918 /
+    // 2,822)
+    if (!a->grid_ok) a->grid_R = R;
     a->grid_ok = true;
   }
   if (!a->grid_ok) return LEV_OK;
@@ -4042,17 +4041,17 @@ int lev_adj_backward(LevAdjoint *a, const float *dLdr, const float *dLdtheta,
         b.grad_ra = a->res_gra;
         b.grad_rb = a->res_grb;
       }
-      // measured on B200: grids of many waves (batch-64 reservoir) run best
-      // at 5 CTAs/SM with 6 edges in flight per lane (fwd+bwd 1.75-1.77 s;
-      // 4 CTAs/SM with 4 edges 2.00 s, 6 with 4 1.77 s, 7 or 8 spill: 2.00 s);
-      // a grid of one partial wave (N = 10^4) with four lanes per row
+      // measured on B200, batch 16 x N = 2*10^4, 50 steps (fwd+bwd, ms): 4 CTAs/SM
+      // with 6 edges in flight per lane 11.5; (edges, CTAs) = (4, 5) 11.9, (6, 5)
+      // 12.8 (spills), (4, 4) 12.4, (8, 3) 12.4, (3, 6) 12.3, (4, 6) 12.5.
+      // A grid of one partial wave (N = 10^4): four lanes per row
       if (e->total_tiles <= 148) {
         const int g4 = e->total_tiles * 4;
         if (mode) adj_bwd_split_kernel<1, 4, 2><<<g4, kTile, 0, s>>>(b);
         else adj_bwd_split_kernel<0, 4, 2><<<g4, kTile, 0, s>>>(b);
       } else if (e->total_tiles > 3 * 148 * 2) {
-        if (mode) adj_bwd_kernel<1, 6, 5><<<e->total_tiles, kTile, 0, s>>>(b);
-        else adj_bwd_kernel<0, 6, 5><<<e->total_tiles, kTile, 0, s>>>(b);
+        if (mode) adj_bwd_kernel<1, 6, 4><<<e->total_tiles, kTile, 0, s>>>(b);
+        else adj_bwd_kernel<0, 6, 4><<<e->total_tiles, kTile, 0, s>>>(b);
       } else {
         if (mode) adj_bwd_kernel<1, 8, 3><<<e->total_tiles, kTile, 0, s>>>(b);
         else adj_bwd_kernel<0, 8, 3><<<e->total_tiles, kTile, 0, s>>>(b);

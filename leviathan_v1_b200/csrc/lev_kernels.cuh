@@ -210,22 +210,6 @@ __device__ __forceinline__ float wrap_pm_pi(float diff) {
   return fabsf(diff) <= kWrapNear ? wrap_pm_pi_near(diff) : wrap_pm_pi_any(diff);
 }
 
-// U phase differences wrapped in place: one range test for the group, the
-// general wrap only when a lane holds a value out of range (or a NaN).
-template <int U>
-__device__ __forceinline__ void wrap_pm_pi_group(float (&diff)[U]) {
-  bool far = false;
-#pragma unroll
-  for (int u = 0; u < U; ++u) far |= !(fabsf(diff[u]) <= kWrapNear);
-  if (far) {
-#pragma unroll
-    for (int u = 0; u < U; ++u) diff[u] = wrap_pm_pi_any(diff[u]);
-  } else {
-#pragma unroll
-    for (int u = 0; u < U; ++u) diff[u] = wrap_pm_pi_near(diff[u]);
-  }
-}
-
 __device__ __forceinline__ float wrap_0_2pi(float x) {
   // wrap to [0, 2pi): leviathan_kernel.cu:188
   return x - floorf(div_two_pi(x)) * kTwoPi;
@@ -238,6 +222,25 @@ __device__ __forceinline__ void lev_sincos(float x, float *s, float *c) {
   } else {
     sincosf(x, s, c);
   }
+}
+
+// U phase differences wrapped in place (wrap_pm_pi) and their sines and
+// cosines: one range test for the group, the general wrap only when a lane
+// holds a value out of range (or a NaN).
+template <int MATH, int U>
+__device__ __forceinline__ void wrap_sincos_group(float (&diff)[U], float (&sn)[U], float (&cs)[U]) {
+  bool far = false;
+#pragma unroll
+  for (int u = 0; u < U; ++u) far |= !(fabsf(diff[u]) <= kWrapNear);
+  if (far) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) diff[u] = wrap_pm_pi_any(diff[u]);
+  } else {
+#pragma unroll
+    for (int u = 0; u < U; ++u) diff[u] = wrap_pm_pi_near(diff[u]);
+  }
+#pragma unroll
+  for (int u = 0; u < U; ++u) lev_sincos<MATH>(diff[u], &sn[u], &cs[u]);
 }
 
 // Host gain controller of leviathan_step (leviathan_kernel.cu:431-435),
@@ -282,25 +285,23 @@ __device__ __forceinline__ unsigned ring_pos_word(uint32_t word, int base, int b
   return (slot >> 2) * ((unsigned)Np * 4u) + (((word >> 6) & ~3u) | (slot & 3u));
 }
 
-// One edge (csr_physics_kernel, leviathan_kernel.cu:146-164) from its wrapped
-// phase difference: sin of the difference and the new weight.  The caller adds
-// w * sin to the row's sum in CSR order and stores the weight, both under the
-// predicate that the entry is one of the row's, so that a walk over the padded
-// slice has no branch per entry.
+// The weight update of one edge (csr_physics_kernel, leviathan_kernel.cu:
+// 155-164).  A walk adds w * sin to the row's sum in CSR order and stores the new
+// weight, both under the predicate that the entry is one of the row's, so that
+// a walk over the padded slice has no branch per entry.
 struct EdgeParams {
   float dt, eta, lam, hebb;  // hebb = 1 - gamma |eps| of the row
   float w_min, w_max;
 };
-template <int MATH>
-__device__ __forceinline__ float edge_update(const EdgeParams &e, float diff, float w,
-                                             float *sin_diff) {
-  float cos_diff;
-  lev_sincos<MATH>(diff, sin_diff, &cos_diff);
-  // dt * (eta cos (1 - gamma |eps|) - lam w), the products fused as nvcc fuses
-  // them in the reference; written out, because which product of the
-  // difference is fused is otherwise the compiler's choice per kernel
+// w + dt * (eta cos (1 - gamma |eps|) - lam w), the products fused as nvcc fuses
+// them in the reference; written out, because which product of the difference
+// is fused is otherwise the compiler's choice per kernel.
+__device__ __forceinline__ float edge_weight_free(const EdgeParams &e, float cos_diff, float w) {
   const float dw = __fmaf_rn(__fmul_rn(e.eta, cos_diff), e.hebb, -__fmul_rn(e.lam, w));
-  w = __fmaf_rn(e.dt, dw, w);
+  return __fmaf_rn(e.dt, dw, w);
+}
+__device__ __forceinline__ float edge_weight(const EdgeParams &e, float cos_diff, float w) {
+  w = edge_weight_free(e, cos_diff, w);
   if (!isfinite(w)) w = e.w_min;
   return fmaxf(e.w_min, fminf(e.w_max, w));
 }

@@ -194,13 +194,13 @@ __device__ __forceinline__ float row_walk(const uint32_t *__restrict__ cdp,
   auto compute = [&](int k0, float (&g)[U], const float (&wv)[U]) {
 #pragma unroll
     for (int u = 0; u < U; ++u) g[u] -= th;
-    wrap_pm_pi_group(g);
+    float sn[U], cs[U];
+    wrap_sincos_group<MATH>(g, sn, cs);
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      float sin_diff;
-      const float w = edge_update<MATH>(ep, g[u], wv[u], &sin_diff);
+      const float w = edge_weight(ep, cs[u], wv[u]);
       const bool in = k0 + u < deg;
-      const float sum = __fmaf_rn(wv[u], sin_diff, local_sum);
+      const float sum = __fmaf_rn(wv[u], sn[u], local_sum);
       local_sum = in ? sum : local_sum;
       if (in) {
         if (SECOND)

@@ -98,10 +98,11 @@ __device__ __forceinline__ float split_walk_u(const uint32_t *cd, float *w, int 
     for (int u = 0; u < U; ++u) dj[u] = (k0 + u < deg) ? gather(p[u]) : 0.0f;
 #pragma unroll
     for (int u = 0; u < U; ++u) dj[u] -= th;
-    wrap_pm_pi_group(dj);
+    float sn[U], cs[U];
+    wrap_sincos_group<MATH>(dj, sn, cs);
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const float wn = edge_update<MATH>(ep, dj[u], wv[u], &dj[u]);
+      const float wn = edge_weight(ep, cs[u], wv[u]);
       if (k0 + u < deg) {
         w[at + 32 * u] = wn;
         keep(k0 + u, wn);
@@ -110,7 +111,7 @@ __device__ __forceinline__ float split_walk_u(const uint32_t *cd, float *w, int 
 #pragma unroll
     for (int ph = 0; ph < LPR; ++ph) {
 #pragma unroll
-      for (int u = 0; u < U; ++u) local_sum = __fmaf_rn(wv[u], dj[u], local_sum);
+      for (int u = 0; u < U; ++u) local_sum = __fmaf_rn(wv[u], sn[u], local_sum);
       if (LPR > 1) local_sum = __shfl_sync(mask, local_sum, sl.lead + ph);
     }
   }
