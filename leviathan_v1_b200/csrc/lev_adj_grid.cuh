@@ -40,6 +40,7 @@ struct AdjGridFwdArgs {
   const float *omega;
   float *omega_hat;
   float *ring;
+  const float *ring_src;  // ck_mode 1 and 3: the ring window of the initial state
   const float *drive;  // drive of step k at drive + k*N, or null
   const float *win;    // reservoir drive u_i = win_i * xin[k], or null
   const float *xin;
@@ -55,7 +56,10 @@ struct AdjGridFwdArgs {
   // last max_delay+1 ring slots as [m][N], g): ck_mode 1 writes it from the
   // initial state (forward pass); 2 takes the initial state from it and
   // refills ring slots 0..max_delay, the unwrapped segment ring (backward
-  // recompute), then w0_out (if not null) receives the initial weights
+  // recompute); 3 writes it from the initial state and the ring window of
+  // ring_src and goes on in the unwrapped ring `ring` (last segment of a forward
+  // pass, which may be ring_src itself).  In 2 and 3 w0_out (if not null)
+  // receives the initial weights
   int ck_mode;
   float *ck_theta, *ck_thh, *ck_omh, *ck_w, *ck_ring, *ck_g;
   float *w0_out;
@@ -110,13 +114,15 @@ __device__ __forceinline__ void adj_grid_fwd_body(const AdjGridFwdArgs &a, const
   if (tid == 0) s_ok = 1;
   __syncthreads();
   const bool restore = a.ck_mode == 2;
+  const bool save = (a.ck_mode & 1) != 0;
+  const bool unwrap = a.ck_mode >= 2;  // the segment runs in an unwrapped ring
   const float *w_src = restore ? a.ck_w : a.w_in;
   split_for_entries<LPR>(sloff, sllen, my_slices, [&](int at, int e) {
     s_cd[at] = a.sl_cd[ebase + e];
     const float w = w_src[ebase + e];
     s_w[at] = w;
-    if (a.ck_mode == 1) a.ck_w[ebase + e] = w;
-    if (restore && a.w0_out) a.w0_out[ebase + e] = w;
+    if (save) a.ck_w[ebase + e] = w;
+    if (unwrap && a.w0_out) a.w0_out[ebase + e] = w;
   });
   const long long gi = nd.node_off + row;
   int deg = 0;
@@ -126,7 +132,7 @@ __device__ __forceinline__ void adj_grid_fwd_body(const AdjGridFwdArgs &a, const
     thh = restore ? a.ck_thh[gi] : a.theta_hat[gi];
     omh = restore ? a.ck_omh[gi] : a.omega_hat[gi];
     om = a.omega[gi];
-    if (a.ck_mode == 1 && sl.q == 0) {
+    if (save && sl.q == 0) {
       a.ck_theta[gi] = th;
       a.ck_thh[gi] = thh;
       a.ck_omh[gi] = omh;
@@ -148,24 +154,26 @@ __device__ __forceinline__ void adj_grid_fwd_body(const AdjGridFwdArgs &a, const
     ns = *a.st;
   }
   float *ring = a.ring + nd.ring_off;
-  if (a.ck_mode == 1) {
+  if (save) {
     // ring window: theta(t - m) -> ck_ring[m][N], m = 0..max_delay
+    const float *src = a.ring_src + nd.ring_off;
     if (live)
       for (int m = sl.q; m <= nd.max_delay; m += LPR) {
         int slot = ns.cur - m;
         slot += (slot < 0) ? bsi : 0;
-        a.ck_ring[(long long)m * N + row] = ring[(long long)slot * Np + row];
+        a.ck_ring[(long long)m * N + row] = src[(long long)slot * Np + row];
       }
     if (cta == 0 && tid == 0) a.ck_g[0] = ns.g;
   }
-  int cur = ns.cur;
+  int cur = unwrap ? nd.max_delay : ns.cur;
   float g = ns.g;
   const float dt = a.dt;
   __syncthreads();
-  // restored segment: theta(s0 - m) -> ring slot max_delay - m of every row,
+  // unwrapped segment: theta(s0 - m) -> ring slot max_delay - m of every row
+  // (from the checkpoint, so that the ring may be the one it was taken from),
   // read by every CTA's first gathers: all arrive once before step 0
   unsigned base = 0;
-  if (restore) {
+  if (unwrap) {
     if (live)
       for (int m = sl.q; m <= nd.max_delay; m += LPR)
         __stcg(ring + (long long)(nd.max_delay - m) * Np + row, a.ck_ring[(long long)m * N + row]);

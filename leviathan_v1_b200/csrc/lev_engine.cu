@@ -478,10 +478,21 @@ int check_params(const LevParams &p) {
 
 int launch_fill(LevEngine *h, int n) {
   const NetDesc &nd = h->h_nets[n];
-  const long long total = (long long)nd.bsi * nd.N;
-  int blocks = (int)std::min<long long>((total + 255) / 256, 148LL * 16);
-  ring_fill_kernel<<<blocks, 256, 0, h->stream>>>(
-      h->d_theta + nd.node_off, h->d_ring + nd.ring_off, nd.N, nd.Np, nd.bsi, 0, 1);
+  const int groups = ring_slots(nd.bsi) / 4;
+  const int bx = std::min((nd.N + 255) / 256, 148 * 16);
+  // a few groups per thread where the nodes alone fill the device
+  const int by = std::max(1, std::min(groups, 148 * 16 / bx));
+  ring_fill_kernel<<<dim3(bx, by), 256, 0, h->stream>>>(
+      h->d_theta + nd.node_off, h->d_ring + nd.ring_off, nd.N, nd.Np, nd.bsi, 0);
+  LEV_TRY_CUDA(cudaGetLastError());
+  return LEV_OK;
+}
+
+// ... of every network.
+int launch_fill_all(LevEngine *h) {
+  const int by = std::max(1, 148 * 8 / h->total_tiles);
+  ring_fill_tiles_kernel<<<dim3(h->total_tiles, by), kTile, 0, h->stream>>>(
+      h->d_nets, h->d_tiles, h->d_theta, h->d_ring, 1);
   LEV_TRY_CUDA(cudaGetLastError());
   return LEV_OK;
 }
@@ -1307,10 +1318,9 @@ int fill_ext_columns(LevEngine *h, int n_ext, const float *theta_ext) {
   cudaError_t e = cudaMemcpyAsync(d_tmp, theta_ext, sizeof(float) * n_ext,
                                   cudaMemcpyHostToDevice, h->stream);
   if (e == cudaSuccess) {
-    const long long total = (long long)nd.bsi * n_ext;
-    int blocks = (int)std::min<long long>((total + 255) / 256, 148LL * 16);
+    const int blocks = std::min((n_ext + 255) / 256, 148 * 16);
     ring_fill_kernel<<<blocks, 256, 0, h->stream>>>(
-        d_tmp, h->d_ring + nd.ring_off, n_ext, nd.Np, nd.bsi, nd.N, 1);
+        d_tmp, h->d_ring + nd.ring_off, n_ext, nd.Np, nd.bsi, nd.N);
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
@@ -1759,8 +1769,8 @@ int create_impl(LevEngine **out, int num_nets, const int32_t *Ns,
         return cleanup_fail(LEV_ERR_CUDA, std::string("SELL packing: ") + cudaGetErrorString(e));
     }
   }
-  for (int n = 0; n < num_nets; ++n) {
-    int r2 = launch_fill(h, n);
+  {
+    int r2 = launch_fill_all(h);
     if (r2 != LEV_OK) return cleanup_fail(r2, g_last_error);
   }
   h->create_ms[6] = lap();
@@ -2037,7 +2047,7 @@ int lev_set_theta(LevEngine *h, const float *theta_in) {
   if (!h || !theta_in) return fail(LEV_ERR_ARG, "null argument");
   DeviceScope ds(h->device);
   int rc = upload_nodes(h, h->d_theta, theta_in, 0, h->total_nodes);
-  for (int n = 0; n < h->num_nets && rc == LEV_OK; ++n) rc = launch_fill(h, n);
+  if (rc == LEV_OK) rc = launch_fill_all(h);
   if (rc != LEV_OK) return rc;
   LEV_TRY_CUDA(cudaStreamSynchronize(h->stream));
   return LEV_OK;
@@ -2057,19 +2067,35 @@ int lev_set_theta_net(LevEngine *h, int32_t net, const float *theta_in) {
   return LEV_OK;
 }
 
-// Weights between the caller's CSR order and the engine's SELL-32 layout,
-// through a temporary device buffer in CSR order (mode 1: CSR -> SELL,
-// mode 2: SELL -> CSR).
-static int convert_weights(LevEngine *h, float *d_csr, int mode) {
-  for (int n = 0; n < h->num_nets; ++n) {
-    const NetDesc &d = h->h_nets[n];
-    if (h->net_E[n] == 0) continue;
-    int blocks = (int)std::min<long long>((d.N + 255) / 256, 148LL * 16);
-    sell_convert_kernel<<<blocks, 256, 0, h->stream>>>(
-        mode, h->d_row_ptr + d.rp_off, d.N, d.N, d.slice_base, h->d_sl_off,
-        nullptr, nullptr, d_csr + d.edge_off, h->d_sl_cd, h->d_sl_w,
-        d.max_delay, nullptr);
+// A temporary device buffer for the weights in the caller's CSR order, from
+// the engine pool: freed blocks of the construction serve it, where a driver
+// allocation and its free cost 0.1 ms on a quiet device and up to 20 ms
+// otherwise.
+struct CsrTemp {
+  LevEngine *h;
+  float *p = nullptr;
+  explicit CsrTemp(LevEngine *e) : h(e) {}
+  int alloc() {
+    cudaMemPool_t pool = nullptr;
+    cudaError_t e = engine_pool(h->device, &pool);
+    if (e == cudaSuccess)
+      e = cudaMallocFromPoolAsync(reinterpret_cast<void **>(&p), sizeof(float) * h->total_edges,
+                                  pool, h->stream);
+    if (e == cudaSuccess) return LEV_OK;
+    cudaGetLastError();
+    p = nullptr;
+    return fail(LEV_ERR_NOMEM, "device allocation of " +
+                                   std::to_string(sizeof(float) * h->total_edges) +
+                                   " bytes failed: " + cudaGetErrorString(e));
   }
+  ~CsrTemp() {
+    if (p) cudaFreeAsync(p, h->stream);
+  }
+};
+
+static int convert_weights(LevEngine *h, float *d_csr, int to_csr) {
+  sell_weights_kernel<<<h->total_tiles, kTile, 0, h->stream>>>(
+      to_csr, h->d_nets, h->d_tiles, h->d_row_ptr, h->d_sl_off, h->d_sl_len, d_csr, h->d_sl_w);
   LEV_TRY_CUDA(cudaGetLastError());
   return LEV_OK;
 }
@@ -2079,11 +2105,10 @@ int lev_get_weights(LevEngine *h, float *w_out) {
     return fail(LEV_ERR_ARG, "null argument");
   DeviceScope ds(h->device);
   if (h->total_edges == 0) return LEV_OK;
-  float *tmp = nullptr;
-  LEV_TRY_CUDA(cudaMalloc(&tmp, sizeof(float) * h->total_edges));
-  int rc = convert_weights(h, tmp, 2);
-  if (rc == LEV_OK) rc = copy_nodes(h, w_out, tmp, 0, h->total_edges);
-  cudaFree(tmp);
+  CsrTemp tmp(h);
+  int rc = tmp.alloc();
+  if (rc == LEV_OK) rc = convert_weights(h, tmp.p, 1);
+  if (rc == LEV_OK) rc = copy_nodes(h, w_out, tmp.p, 0, h->total_edges);
   return rc;
 }
 
@@ -2093,12 +2118,11 @@ int lev_reset_weights(LevEngine *h, const float *w_in) {
     return fail(LEV_ERR_ARG, "null argument");
   DeviceScope ds(h->device);
   if (h->total_edges == 0) return LEV_OK;
-  float *tmp = nullptr;
-  LEV_TRY_CUDA(cudaMalloc(&tmp, sizeof(float) * h->total_edges));
-  int rc = upload_nodes(h, tmp, w_in, 0, h->total_edges);
-  if (rc == LEV_OK) rc = convert_weights(h, tmp, 1);
+  CsrTemp tmp(h);
+  int rc = tmp.alloc();
+  if (rc == LEV_OK) rc = upload_nodes(h, tmp.p, w_in, 0, h->total_edges);
+  if (rc == LEV_OK) rc = convert_weights(h, tmp.p, 0);
   cudaError_t ce = cudaStreamSynchronize(h->stream);
-  cudaFree(tmp);
   if (rc != LEV_OK) return rc;
   if (ce != cudaSuccess)
     return fail(LEV_ERR_CUDA, std::string("reset_weights: ") + cudaGetErrorString(ce));
@@ -3223,6 +3247,9 @@ struct LevAdjoint {
   size_t bytes = 0;
   int last_T = 0;
   float last_dt = 0.0f;
+  // the last segment's records, left by the forward pass: made by which
+  // kernels (0: none), in which record set, under which math mode
+  int rec_path = 0, rec_set = 0, rec_mode = 0;
   const float *drive = nullptr;
   // reservoir (fused drive win * x and cos/sin readout), all device pointers
   const float *res_win = nullptr, *res_x = nullptr, *res_ra = nullptr,
@@ -3318,6 +3345,19 @@ int adj_launch_fwd(LevAdjoint *a, const AdjFwdArgs &f, cudaStream_t s = nullptr)
   return LEV_OK;
 }
 
+// The ring part of checkpoint `seg` (modes of adj_ring_ckpt_kernel).
+void adj_ring_ckpt(LevAdjoint *a, int seg, int mode, float *ring, float *segment,
+                   cudaStream_t s) {
+  LevEngine *e = a->e;
+  int md = 0;
+  for (const NetDesc &d : a->h_nets) md = std::max(md, d.max_delay);
+  // few tiles: the slots are spread over blocks as well
+  const int by = std::max(1, std::min(md + 1, 148 * 8 / std::max(e->total_tiles, 1)));
+  adj_ring_ckpt_kernel<<<dim3(e->total_tiles, by), kTile, 0, s>>>(
+      mode, a->d_nets, e->d_tiles, a->d_st, ring, segment,
+      a->ck_ring + (size_t)seg * a->ckr_floats, a->d_ck_off);
+}
+
 // Checkpoint `seg` of the working state: save (forward pass) or restore into
 // the working state and the extended ring `ring` (backward recompute).
 int adj_ckpt(LevAdjoint *a, int seg, bool save, cudaStream_t s = nullptr,
@@ -3335,20 +3375,9 @@ int adj_ckpt(LevAdjoint *a, int seg, bool save, cudaStream_t s = nullptr,
   LEV_TRY_CUDA(cp(a->ck_omh + (size_t)seg * a->TN, a->omega_hat, nb));
   LEV_TRY_CUDA(cp(a->ck_w + (size_t)seg * a->SL, a->w,
                   sizeof(float) * std::max<long long>(a->SL, 1)));
-  dim3 grid(64, a->NN);
-  if (save) {
-    adj_state_kernel<<<1, 128, 0, s>>>(1, a->d_nets, a->d_st,
-                                       a->ck_g + (size_t)seg * a->NN, nullptr, a->NN);
-    adj_ring_ckpt_kernel<<<grid, 256, 0, s>>>(0, a->d_nets, a->d_st, ring,
-                                              a->ck_ring + (size_t)seg * a->ckr_floats,
-                                              a->d_ck_off, a->NN);
-  } else {
-    adj_ring_ckpt_kernel<<<grid, 256, 0, s>>>(1, a->d_nets, a->d_st, ring,
-                                              a->ck_ring + (size_t)seg * a->ckr_floats,
-                                              a->d_ck_off, a->NN);
-    adj_state_kernel<<<1, 128, 0, s>>>(2, a->d_nets, a->d_st,
-                                       a->ck_g + (size_t)seg * a->NN, nullptr, a->NN);
-  }
+  adj_ring_ckpt(a, seg, save ? 0 : 1, save ? ring : nullptr, save ? nullptr : ring, s);
+  adj_state_kernel<<<1, 128, 0, s>>>(save ? 1 : 2, a->d_nets, a->d_st,
+                                     a->ck_g + (size_t)seg * a->NN, nullptr, a->NN);
   LEV_TRY_CUDA(cudaGetLastError());
   return LEV_OK;
 }
@@ -3754,6 +3783,25 @@ int lev_adj_bytes(const LevAdjoint *a, size_t *bytes) {
   return LEV_OK;
 }
 
+// Record set of segment `seg` of a run of `nseg` segments, per path.
+enum { kRecNone = 0, kRecSteps = 1, kRecGrid = 2 };
+static bool adj_paired(const LevAdjoint *a, int nseg) {
+  return a->ring2 != nullptr && a->use_pair && a->gp_ok[grid_r_index(a->grid_R)] && nseg > 1;
+}
+static int adj_record_set(const LevAdjoint *a, int path, int seg, int nseg) {
+  if (path == kRecGrid) return adj_paired(a, nseg) ? (seg & 1) : 0;
+  return (a->rstream != nullptr && nseg > 1) ? (seg & 1) : 0;
+}
+static bool adj_recorded(const LevAdjoint *a, int path, int nseg) {
+  return a->rec_path == path && a->rec_mode == a->e->math_mode &&
+         a->rec_set == adj_record_set(a, path, nseg - 1, nseg);
+}
+
+// The forward pass keeps, beside the checkpoints, the records of its last
+// segment (weights, theta_hat, trace, phases in an unwrapped ring): the backward
+// pass starts with that segment and need not recompute it.  Recording costs a
+// forward step little (the stores of the new weights go to the record instead);
+// it saves one of the recomputed segments.
 int lev_adj_forward(LevAdjoint *a, float dt, int32_t T, const float *omega,
                     const float *w0_csr, const float *K, const float *drive,
                     float *r_out, float *theta_out) {
@@ -3766,25 +3814,18 @@ int lev_adj_forward(LevAdjoint *a, float dt, int32_t T, const float *omega,
   DeviceScope ds(e->device);
   cudaStream_t s = e->stream;
   const size_t nb = sizeof(float) * a->TN;
+  const int nseg = (T + a->C - 1) / a->C;
+  a->rec_path = kRecNone;
   LEV_TRY_CUDA(cudaMemcpyAsync(a->theta, a->theta0, nb, cudaMemcpyDeviceToDevice, s));
   LEV_TRY_CUDA(cudaMemcpyAsync(a->theta_hat, a->theta_hat0, nb, cudaMemcpyDeviceToDevice, s));
   LEV_TRY_CUDA(cudaMemcpyAsync(a->omega, omega, nb, cudaMemcpyDeviceToDevice, s));
   // omega_hat starts as omega (leviathan_kernel.cu:350)
   LEV_TRY_CUDA(cudaMemcpyAsync(a->omega_hat, omega, nb, cudaMemcpyDeviceToDevice, s));
-  LEV_TRY_CUDA(cudaMemsetAsync(a->w, 0, sizeof(float) * std::max<long long>(a->SL, 1), s));
-  for (int n = 0; n < a->NN; ++n) {
-    const NetDesc &d = a->h_nets[n];
-    if (e->net_E[n] == 0) continue;
-    int blocks = (int)std::min<long long>((d.N + 255) / 256, 148LL * 16);
-    sell_convert_kernel<<<blocks, 256, 0, s>>>(
-        1, e->d_row_ptr + d.rp_off, d.N, d.N, d.slice_base, e->d_sl_off, nullptr,
-        nullptr, const_cast<float *>(w0_csr) + d.edge_off, e->d_sl_cd, a->w,
-        d.max_delay, nullptr);
-    const long long total = (long long)d.bsi * d.N;
-    int fb = (int)std::min<long long>((total + 255) / 256, 148LL * 16);
-    ring_fill_kernel<<<fb, 256, 0, s>>>(a->theta0 + d.node_off, a->ring + d.ring_off,
-                                       d.N, d.Np, d.bsi, 0, 0);  // slot-major
-  }
+  sell_weights_kernel<<<e->total_tiles, kTile, 0, s>>>(
+      0, e->d_nets, e->d_tiles, e->d_row_ptr, e->d_sl_off, e->d_sl_len,
+      const_cast<float *>(w0_csr), a->w);
+  ring_fill_tiles_kernel<<<dim3(e->total_tiles, std::max(1, 148 * 8 / e->total_tiles)), kTile, 0,
+                           s>>>(a->d_nets, e->d_tiles, a->theta0, a->ring, 0);
   adj_state_kernel<<<1, 128, 0, s>>>(0, a->d_nets, a->d_st, nullptr, K, a->NN);
   LEV_TRY_CUDA(cudaGetLastError());
   if (adj_grid_on(a)) {
@@ -3794,10 +3835,23 @@ int lev_adj_forward(LevAdjoint *a, float dt, int32_t T, const float *omega,
       const int n = std::min(a->C, T - t0);
       AdjGridFwdArgs g;
       std::memset(&g, 0, sizeof(g));
-      adj_grid_ckpt_args(a, t0 / a->C, 1, g);
+      const int seg = t0 / a->C;
+      const bool last = seg == nseg - 1;
+      adj_grid_ckpt_args(a, seg, last ? 3 : 1, g);
       g.w_in = a->w;
       g.w_out = a->w;
       g.ring = a->ring;
+      g.ring_src = a->ring;
+      if (last) {
+        const int k = adj_record_set(a, kRecGrid, seg, nseg);
+        float *wh = k ? a->w_hist2 : a->w_hist;
+        g.ring = k ? a->ring2 : a->ring;
+        g.w0_out = wh;
+        g.w_rec = wh + a->SL;
+        g.w_out = wh + (size_t)n * a->SL;
+        g.thh_rec = k ? a->thh_hist2 : a->thh_hist;
+        g.trace = k ? a->trace2 : a->trace;
+      }
       g.drive = drive ? drive + (size_t)t0 * a->TN : nullptr;
       if (a->res_win) {
         g.win = a->res_win;
@@ -3815,14 +3869,41 @@ int lev_adj_forward(LevAdjoint *a, float dt, int32_t T, const float *omega,
     a->last_T = T;
     a->last_dt = dt;
     a->drive = drive;
+    a->rec_path = kRecGrid;
+    a->rec_set = adj_record_set(a, kRecGrid, nseg - 1, nseg);
+    a->rec_mode = e->math_mode;
     return LEV_OK;
   }
   AdjFwdArgs f = adj_fwd_args(a, dt);
   f.drive = nullptr;
+  const int last0 = (nseg - 1) * a->C;  // first step of the last segment
+  const int rec = adj_record_set(a, kRecSteps, nseg - 1, nseg);
+  float *rec_w = rec ? a->w_hist2 : a->w_hist, *rec_ring = rec ? a->ring2 : a->ring;
+  float *rec_dj = rec ? a->dj_hist2 : a->dj_hist, *rec_thh = rec ? a->thh_hist2 : a->thh_hist;
+  float4 *rec_trace = rec ? a->trace2 : a->trace;
   for (int t = 0; t < T; ++t) {
     if (t % a->C == 0) {
       int rc = adj_ckpt(a, t / a->C, true);
       if (rc != LEV_OK) return rc;
+    }
+    if (t == last0) {
+      // from here on in the record set: the ring window unwrapped, as after a
+      // restore
+      adj_ring_ckpt(a, nseg - 1, 1, nullptr, rec_ring, s);
+      adj_state_kernel<<<1, 128, 0, s>>>(2, a->d_nets, a->d_st,
+                                         a->ck_g + (size_t)(nseg - 1) * a->NN, nullptr, a->NN);
+      LEV_TRY_CUDA(cudaMemcpyAsync(rec_w, a->w,
+                                   sizeof(float) * std::max<long long>(a->SL, 1),
+                                   cudaMemcpyDeviceToDevice, s));
+      f.ring = rec_ring;
+    }
+    if (t >= last0) {
+      const int k = t - last0;
+      f.w_in = rec_w + (size_t)k * a->SL;
+      f.w_out = rec_w + (size_t)(k + 1) * a->SL;
+      f.thh_rec = rec_thh + (size_t)k * a->TN;
+      f.dj_rec = rec_dj ? rec_dj + (size_t)k * a->SL : nullptr;
+      f.trace = rec_trace + (size_t)k * a->NN;
     }
     f.drive = drive ? drive + (size_t)t * a->TN : nullptr;
     f.r_out = r_out + (size_t)t * a->NN;
@@ -3844,6 +3925,9 @@ int lev_adj_forward(LevAdjoint *a, float dt, int32_t T, const float *omega,
   a->last_T = T;
   a->last_dt = dt;
   a->drive = drive;
+  a->rec_path = kRecSteps;
+  a->rec_set = rec;
+  a->rec_mode = e->math_mode;
   return LEV_OK;
 }
 
@@ -3878,7 +3962,9 @@ int lev_adj_backward(LevAdjoint *a, const float *dLdr, const float *dLdtheta,
     // share one paired launch when both groups fit on the device; otherwise
     // each segment is recomputed, then reversed, in launches of their own.
     const bool two = a->ring2 != nullptr;
-    const bool paired = two && a->use_pair && a->gp_ok[grid_r_index(a->grid_R)] && nseg > 1;
+    const bool paired = adj_paired(a, nseg);
+    const bool recorded = adj_recorded(a, kRecGrid, nseg);
+    a->rec_path = kRecNone;  // the sets are reused below
     float *rings[2] = {a->ring, two ? a->ring2 : a->ring};
     float *whs[2] = {a->w_hist, two ? a->w_hist2 : a->w_hist};
     float *ths[2] = {a->thh_hist, two ? a->thh_hist2 : a->thh_hist};
@@ -3928,8 +4014,10 @@ int lev_adj_backward(LevAdjoint *a, const float *dLdr, const float *dLdtheta,
     AdjGridBwdArgs b;
     int rc = LEV_OK;
     if (paired) {
-      rc = prep_fwd(nseg - 1, g);
-      if (rc == LEV_OK) rc = adj_grid_launch_fwd(a, g, seg_len(nseg - 1), s);
+      if (!recorded) {
+        rc = prep_fwd(nseg - 1, g);
+        if (rc == LEV_OK) rc = adj_grid_launch_fwd(a, g, seg_len(nseg - 1), s);
+      }
       for (int seg = nseg - 1; seg >= 0 && rc == LEV_OK; --seg) {
         prep_bwd(seg, b);
         if (seg > 0) {
@@ -3941,8 +4029,10 @@ int lev_adj_backward(LevAdjoint *a, const float *dLdr, const float *dLdtheta,
       }
     } else {
       for (int seg = nseg - 1; seg >= 0 && rc == LEV_OK; --seg) {
-        rc = prep_fwd(seg, g);
-        if (rc == LEV_OK) rc = adj_grid_launch_fwd(a, g, seg_len(seg), s);
+        if (!recorded || seg < nseg - 1) {
+          rc = prep_fwd(seg, g);
+          if (rc == LEV_OK) rc = adj_grid_launch_fwd(a, g, seg_len(seg), s);
+        }
         prep_bwd(seg, b);
         if (rc == LEV_OK) rc = adj_grid_launch_bwd(a, b, s);
       }
@@ -3992,7 +4082,13 @@ int lev_adj_backward(LevAdjoint *a, const float *dLdr, const float *dLdtheta,
     return LEV_OK;
   };
   bool rev_recorded[2] = {false, false};
-  int rc = recompute(nseg - 1);
+  const bool recorded = adj_recorded(a, kRecSteps, nseg);
+  a->rec_path = kRecNone;  // the sets are reused below
+  int rc = LEV_OK;
+  if (!recorded)
+    rc = recompute(nseg - 1);
+  else if (overlap)
+    LEV_TRY_CUDA(cudaEventRecord(a->ev_rec[(nseg - 1) & 1], rs));
   if (rc != LEV_OK) return rc;
   for (int seg = nseg - 1; seg >= 0; --seg) {
     const int buf = seg & 1;
@@ -4081,16 +4177,9 @@ int lev_adj_backward(LevAdjoint *a, const float *dLdr, const float *dLdtheta,
     LEV_TRY_CUDA(cudaMemcpyAsync(grad_omega, a->grad_omega_acc, nb, cudaMemcpyDeviceToDevice, s));
     add_kernel<<<148, 256, 0, s>>>(grad_omega, a->lam_omh, a->TN);
   }
-  if (grad_w0_csr) {
-    for (int n = 0; n < a->NN; ++n) {
-      const NetDesc &d = a->h_nets[n];
-      if (e->net_E[n] == 0) continue;
-      int blocks = (int)std::min<long long>((d.N + 255) / 256, 148LL * 16);
-      sell_convert_kernel<<<blocks, 256, 0, s>>>(
-          2, e->d_row_ptr + d.rp_off, d.N, d.N, d.slice_base, e->d_sl_off, nullptr, nullptr,
-          grad_w0_csr + d.edge_off, e->d_sl_cd, a->lam_w, d.max_delay, nullptr);
-    }
-  }
+  if (grad_w0_csr)
+    sell_weights_kernel<<<e->total_tiles, kTile, 0, s>>>(
+        1, e->d_nets, e->d_tiles, e->d_row_ptr, e->d_sl_off, e->d_sl_len, grad_w0_csr, a->lam_w);
   if (grad_K)
     LEV_TRY_CUDA(cudaMemcpyAsync(grad_K, a->lam_g, sizeof(float) * a->NN,
                                  cudaMemcpyDeviceToDevice, s));
@@ -4148,6 +4237,7 @@ int lev_adj_set_grid_mode(LevAdjoint *a, int32_t enabled, int32_t rows_per_cta) 
 int lev_adj_set_reservoir(LevAdjoint *a, const float *win, const float *x,
                           const float *ra, const float *rb, float *y_out) {
   if (!a) return fail(LEV_ERR_ARG, "null handle");
+  a->rec_path = kRecNone;  // records of a run with other inputs
   if ((win == nullptr) != (x == nullptr))
     return fail(LEV_ERR_ARG, "win and x must be given together");
   if ((ra == nullptr) != (rb == nullptr))

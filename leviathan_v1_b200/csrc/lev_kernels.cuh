@@ -549,61 +549,83 @@ __global__ void __launch_bounds__(kTile, MINB) step_kernel(const StepArgs a) {
 // ---------------------------------------------------------------------------
 
 // Every ring slot of nodes col0 .. col0+N-1 := theta (init_buffer_kernel,
-// leviathan_kernel.cu:79-90).  pairs 1: the engine's ring (ring_pos);
-// pairs 0: a slot-major ring [bsi][Np] (the adjoint's own rings).
-__global__ void ring_fill_kernel(const float *__restrict__ theta,
-                                 float *__restrict__ ring, int N, int Np,
-                                 int bsi, int col0, int pairs) {
-  const long long total = (long long)bsi * N;
-  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-       k < total; k += (long long)gridDim.x * blockDim.x) {
-    const int s = (int)(k / N);
-    const int i = (int)(k - (long long)s * N);
-    if (pairs)
-      ring[ring_pos(s, (unsigned)(col0 + i), Np)] = theta[i];
-    else
-      ring[(long long)s * Np + col0 + i] = theta[i];
+// leviathan_kernel.cu:79-90), the engine's ring (ring_pos): a thread writes one
+// node's groups of four slots, 16 bytes each.  N = 10^6, 66 slots: 266 us with a
+// division per element and 4-byte stores, 45 us so.
+__global__ void ring_fill_kernel(const float *__restrict__ theta, float *__restrict__ ring, int N,
+                                 int Np, int bsi, int col0) {
+  const int groups = ring_slots(bsi) / 4;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
+    const float x = theta[i];
+    float4 *at = reinterpret_cast<float4 *>(ring) + (col0 + i);
+    for (int m = blockIdx.y; m < groups; m += gridDim.y)
+      at[(long long)m * Np] = make_float4(x, x, x, x);
   }
 }
 
-// CSR -> SELL-32 for one network: entry k of row i goes to
-// sl_off[slice_base + i/32] + 32k + i%32.  One thread per row.
-// mode 0: pack (col, delay) into sl_cd and copy weights, validating
-//         col in [0,ncols) and delay <= max_delay (bits 1, 2 of *err); bit 4
-//         reports a zero delay (ncols = N, or N plus the halo columns of a
-//         partition, lev_part.cuh);
-// mode 1: weights only, CSR -> SELL;   mode 2: weights only, SELL -> CSR.
-__global__ void sell_convert_kernel(int mode, const int *__restrict__ row_ptr,
-                                    int N, int ncols, long long slice_base,
-                                    const long long *__restrict__ sl_off,
-                                    const int *__restrict__ col,
-                                    const uint8_t *__restrict__ delays,
-                                    float *__restrict__ w_csr,
-                                    uint32_t *__restrict__ sl_cd,
-                                    float *__restrict__ sl_w, int max_delay,
-                                    unsigned *__restrict__ err) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N;
-       i += gridDim.x * blockDim.x) {
-    const int e0 = row_ptr[i], e1 = row_ptr[i + 1];
-    const long long base = sl_off[slice_base + (i >> 5)] + (i & 31);
-    unsigned bad = 0u;
-    for (int e = e0; e < e1; ++e) {
-      const long long idx = base + 32LL * (e - e0);
-      if (mode == 0) {
-        const int c = col[e];
-        const int d = delays[e];
-        if (c < 0 || c >= ncols) bad |= 1u;
-        if (d > max_delay) bad |= 2u;
-        if (d == 0) bad |= 4u;  // not an error: rules out two steps per launch
-        sl_cd[idx] = ((uint32_t)c << 8) | (uint32_t)d;
-        sl_w[idx] = w_csr[e];
-      } else if (mode == 1) {
-        sl_w[idx] = w_csr[e];
-      } else {
-        w_csr[e] = sl_w[idx];
+// The same for every network, one block row per 256-row tile: grouped 1 the
+// engine's ring, 0 slot-major rings [bsi][Np] (the adjoint's).
+__global__ void ring_fill_tiles_kernel(const NetDesc *__restrict__ nets,
+                                       const int2 *__restrict__ tiles,
+                                       const float *__restrict__ theta, float *__restrict__ ring,
+                                       int grouped) {
+  const int2 tile = tiles[blockIdx.x];
+  const NetDesc &nd = nets[tile.x];
+  const int row = tile.y + threadIdx.x;
+  if (row >= nd.N) return;
+  const float x = theta[nd.node_off + row];
+  if (grouped) {
+    float4 *at = reinterpret_cast<float4 *>(ring + nd.ring_off) + row;
+    for (int m = blockIdx.y; m < ring_slots(nd.bsi) / 4; m += gridDim.y)
+      at[(long long)m * nd.Np] = make_float4(x, x, x, x);
+  } else {
+    float *at = ring + nd.ring_off + row;
+    for (int s = blockIdx.y; s < nd.bsi; s += gridDim.y) at[(long long)s * nd.Np] = x;
+  }
+}
+
+// Weights between the caller's CSR order and SELL-32, every network in one
+// launch: one warp per slice (CTA = one 256-row tile), entry k of row i at
+// sl_off[slice] + 32k + i%32.  To SELL: lane l walks row l, so the stores are
+// whole 128-byte lines (padding zeroed) and a row's CSR line is read from L1
+// after its first entry.  To CSR: the slice's entries are contiguous there, so
+// the warp takes 32 at a time and each lane looks its row up in the slice's 33
+// offsets.
+__global__ void __launch_bounds__(kTile) sell_weights_kernel(
+    int to_csr, const NetDesc *__restrict__ nets, const int2 *__restrict__ tiles,
+    const int *__restrict__ row_ptr, const long long *__restrict__ sl_off,
+    const int *__restrict__ sl_len, float *__restrict__ w_csr, float *__restrict__ sl_w) {
+  const unsigned mask = 0xffffffffu;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int2 tile = tiles[blockIdx.x];
+  const NetDesc &nd = nets[tile.x];
+  const int N = nd.N;
+  const int row0 = tile.y + 32 * warp;
+  if (row0 >= N) return;
+  const long long s = nd.slice_base + (row0 >> 5);
+  const int *rp = row_ptr + nd.rp_off;
+  const int e0 = rp[min(row0 + lane, N)];
+  float *csr = w_csr + nd.edge_off;
+  const long long off = sl_off[s];
+  if (to_csr) {
+    const int first = __shfl_sync(mask, e0, 0);
+    const int end = rp[min(row0 + 32, N)];
+    for (int base = first; base < end; base += 32) {
+      const int e = base + lane;
+      int r = 0;  // the last row of the slice that starts at or before e
+#pragma unroll
+      for (int step = 16; step > 0; step /= 2) {
+        const int v = __shfl_sync(mask, e0, r + step);
+        if (v <= e) r += step;
       }
+      const int start = __shfl_sync(mask, e0, r);
+      if (e < end) csr[e] = sl_w[off + 32LL * (e - start) + r];
     }
-    if (bad) atomicOr(err, bad);
+  } else {
+    const int deg = (row0 + lane < N) ? rp[row0 + lane + 1] - e0 : 0;
+    const int len = sl_len[s];
+    for (int k = 0; k < len; ++k)
+      sl_w[off + 32LL * k + lane] = (k < deg) ? csr[e0 + k] : 0.0f;
   }
 }
 
@@ -613,7 +635,7 @@ __global__ void sell_convert_kernel(int mode, const int *__restrict__ row_ptr,
 // one contiguous 128-byte store per warp; entries past the row's degree are
 // padding (node 0, delay 0, weight 0: read, never used).  The CSR arrays
 // (concatenated over networks, as the caller passed them) were copied to the
-// device as they are.  Validation as sell_convert_kernel: bit 1 a column
+// device as they are.  Validation (bits of *err): bit 1 a column
 // outside [0, ncols) (ncols = N, plus the halo columns of a partition for
 // network 0), bit 2 a delay above max_delay, bit 4 a zero delay (not an
 // error: it rules out two steps per launch).
