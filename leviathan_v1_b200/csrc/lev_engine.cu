@@ -585,6 +585,22 @@ bool pairs_active(const LevEngine *h) {
   return false;
 }
 
+// Launch by programmatic dependent launch (see wait_dependency): the next
+// kernel of the chain is set up and its CTAs read what does not change while
+// this one drains.
+cudaError_t launch_after(const void *fn, int blocks, int threads, void **args, cudaStream_t s) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(threads);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelExC(&cfg, fn, args);
+}
+
 // phase 0: pair_kernel (or a first step_kernel for a class without a pair
 // variant); phase 1: finish_kernel (or a second step_kernel).
 int launch_pair_tc(LevEngine *h, const TileClass &tc, StepArgs a, int phase,
@@ -599,18 +615,24 @@ int launch_pair_tc(LevEngine *h, const TileClass &tc, StepArgs a, int phase,
             ? reinterpret_cast<const void *>(kVariants[tc.variant].fn[mode])
             : reinterpret_cast<const void *>(kPairVariants[tc.pair_variant].fn[mode]);
     void *args[] = {&a};
-    LEV_TRY_CUDA(cudaLaunchKernel(fn, dim3(tc.ntiles), dim3(kTile), args, 0, s));
+    if (tc.pair_variant < 0) {
+      LEV_TRY_CUDA(cudaLaunchKernel(fn, dim3(tc.ntiles), dim3(kTile), args, 0, s));
+    } else {
+      LEV_TRY_CUDA(launch_after(fn, tc.ntiles, kTile, args, s));
+    }
   } else {
     const int blocks = (tc.ntiles + kFinishTiles - 1) / kFinishTiles;
-    if (mode)
-      finish_kernel<1><<<blocks, kTile, 0, s>>>(a, tc.ntiles);
-    else
-      finish_kernel<0><<<blocks, kTile, 0, s>>>(a, tc.ntiles);
-    LEV_TRY_CUDA(cudaGetLastError());
+    int ntiles = tc.ntiles;
+    void *args[] = {&a, &ntiles};
+    LEV_TRY_CUDA(launch_after(mode ? reinterpret_cast<const void *>(finish_kernel<1>)
+                                   : reinterpret_cast<const void *>(finish_kernel<0>),
+                              blocks, kTile, args, s));
   }
   if (tc.pair_variant >= 0) {  // r and g of the class's networks
-    reduce_kernel<<<tc.nnets, kReduceThreads, 0, s>>>(a, h->d_class_nets + tc.net_off);
-    LEV_TRY_CUDA(cudaGetLastError());
+    const int *nets = h->d_class_nets + tc.net_off;
+    void *args[] = {&a, &nets};
+    LEV_TRY_CUDA(launch_after(reinterpret_cast<const void *>(reduce_kernel), tc.nnets,
+                              kReduceThreads, args, s));
   }
   return LEV_OK;
 }

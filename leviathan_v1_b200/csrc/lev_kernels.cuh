@@ -258,6 +258,16 @@ __device__ __forceinline__ float gain_controller(float g, float r, float dt,
   return fmaxf(nd.g_min, fminf(nd.g_max, gn));
 }
 
+// Programmatic dependent launch: a kernel launched with it may start while the
+// one before it still runs and waits, before it reads anything that one writes,
+// until that one has completed (and, by the same wait there, all before it).
+__device__ __forceinline__ void launch_dependents() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void wait_dependency() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // Ring gather: read-only (non-coherent) path.  The slot written by the same
 // launch is never read by it (see the ring note at the top).
 __device__ __forceinline__ float ld_ring(const float *p) { return __ldg(p); }

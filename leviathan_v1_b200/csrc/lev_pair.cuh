@@ -86,6 +86,8 @@ __global__ void __launch_bounds__(kReduceThreads) reduce_kernel(const StepArgs a
   const int net = nets[blockIdx.x];
   const NetDesc nd = a.nets[net];
   NetState *ns = a.st + net;
+  launch_dependents();
+  wait_dependency();
   // network state read up front, off the partial-sum critical path
   NetState st;
   if (tid == 0) st = *ns;
@@ -272,6 +274,8 @@ __global__ void __launch_bounds__(kTile, MINB) pair_kernel(const StepArgs a) {
   const float dt = a.dt;
   const int bsi = nd.bsi;
   const int Np = nd.Np;
+  launch_dependents();
+  wait_dependency();
   const int cur = ns->cur;
   const int nxt = nxt_slot(cur, bsi);
   const float g = ns->g;
@@ -375,6 +379,8 @@ __global__ void __launch_bounds__(kTile) finish_kernel(const StepArgs a, int nti
     tile[q] = make_int2(-1, 0);
     if (t < ntiles) tile[q] = a.tiles[a.reverse ? ntiles - 1 - t : t];
   }
+  launch_dependents();
+  wait_dependency();
 #pragma unroll
   for (int q = 0; q < kFinishTiles; ++q) {
     my_cos[q] = my_sin[q] = 0.0f;
