@@ -1912,12 +1912,40 @@ int lev_net_shape(const LevEngine *h, int32_t net, int32_t *N, int64_t *E,
   return LEV_OK;
 }
 
+// The r of a single step arrives in mapped host memory a few microseconds
+// before the stream counts as drained: the host puts a mark there, launches,
+// and spins until every network's r has replaced it.  The stream is asked now
+// and then, so that a failed launch ends the wait, and so does an r that has
+// the mark's bits.
+constexpr uint32_t kNoR = 0xffffffffu;
+static void mark_r(LevEngine *h) {
+  volatile uint32_t *p = reinterpret_cast<volatile uint32_t *>(h->h_rmap);
+  for (int n = 0; n < h->num_nets; ++n) p[n] = kNoR;
+}
+static int wait_r(LevEngine *h) {
+  volatile uint32_t *p = reinterpret_cast<volatile uint32_t *>(h->h_rmap);
+  unsigned spins = 0;
+  for (int n = 0; n < h->num_nets; ++n) {
+    while (p[n] == kNoR) {
+      if ((++spins & 4095u) == 0u) {
+        const cudaError_t e = cudaStreamQuery(h->stream);
+        if (e == cudaSuccess) return LEV_OK;
+        if (e != cudaErrorNotReady)
+          return fail(LEV_ERR_CUDA, std::string("step: ") + cudaGetErrorString(e));
+      }
+    }
+  }
+  std::atomic_thread_fence(std::memory_order_acquire);
+  return LEV_OK;
+}
+
 int lev_step(LevEngine *h, float dt, float *r_out) {
   if (!h) return fail(LEV_ERR_ARG, "null handle");
   if (h->part) return fail(LEV_ERR_STATE, "partition engine: step with lev_part_step_begin / lev_part_step_end");
   if (!std::isfinite(dt)) return fail(LEV_ERR_ARG, "dt is not finite");
   DeviceScope ds(h->device);
   StepArgs a = make_args(h, dt, nullptr, 0, h->d_rmap);
+  mark_r(h);
   int rc = LEV_OK;
   uint32_t dbits;
   std::memcpy(&dbits, &dt, 4);
@@ -1977,7 +2005,8 @@ int lev_step(LevEngine *h, float dt, float *r_out) {
     rc = launch_step(h, a);
     if (rc != LEV_OK) return rc;
   }
-  LEV_TRY_CUDA(cudaStreamSynchronize(h->stream));
+  rc = wait_r(h);
+  if (rc != LEV_OK) return rc;
   if (r_out) {
     const volatile float *src = h->h_rmap;
     for (int n = 0; n < h->num_nets; ++n) r_out[n] = src[n];

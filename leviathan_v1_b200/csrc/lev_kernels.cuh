@@ -543,7 +543,10 @@ __global__ void __launch_bounds__(kTile, MINB) step_kernel(const StepArgs a) {
       ns->rbuf = rb;
       ns->t = ns->t + 1;
       ns->ticket = 0u;
-      if (a.r_host) a.r_host[tile.x] = r;
+      if (a.r_host) {
+        *reinterpret_cast<volatile float *>(a.r_host + tile.x) = r;
+        __threadfence_system();  // the host spins on it
+      }
       if (a.r_hist) {
         const int k = ns->rpos;
         if (k < a.r_cap) a.r_hist[(long long)k * a.num_nets + tile.x] = r;

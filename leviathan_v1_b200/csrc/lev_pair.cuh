@@ -126,7 +126,10 @@ __global__ void __launch_bounds__(kReduceThreads) reduce_kernel(const StepArgs a
       const int rb = st.rbuf + 1;
       st.rbuf = (rb == nd.max_delay + 1) ? 0 : rb;
       st.t = st.t + 1;
-      if (a.r_host) a.r_host[net] = r;
+      if (a.r_host) {
+        *reinterpret_cast<volatile float *>(a.r_host + net) = r;
+        __threadfence_system();  // the host spins on it
+      }
       if (a.r_hist) {
         if (st.rpos < a.r_cap) a.r_hist[(long long)st.rpos * a.num_nets + net] = r;
         st.rpos = st.rpos + 1;
