@@ -585,10 +585,16 @@ bool pairs_active(const LevEngine *h) {
   return false;
 }
 
-// Launch by programmatic dependent launch (see wait_dependency): the next
-// kernel of the chain is set up and its CTAs read what does not change while
-// this one drains.
-cudaError_t launch_after(const void *fn, int blocks, int threads, void **args, cudaStream_t s) {
+// Launch by programmatic dependent launch (see wait_dependency) when `early`: the
+// next kernel of the chain is set up and its CTAs read what does not change
+// while this one drains.  With more than one wave of pair CTAs (444 tiles) that
+// is faster (us per step, without / with: N = 10^6 133.1 / 131.3, 5*10^5 68.0 /
+// 66.4, 2*10^5 18.8 / 17.7, 1.2*10^5 20.8 / 20.7), and so it is where launches
+// are most of the step (10^4 9.4 / 8.6, 2.8*10^4 9.7 / 8.2); between, the whole
+// chain comes to wait on the SMs beside the first kernel (1.1*10^5 13.0 / 15.0,
+// 6*10^4 10.9 / 13.8).
+cudaError_t launch_after(const void *fn, int blocks, int threads, void **args, bool early,
+                         cudaStream_t s) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(blocks);
   cfg.blockDim = dim3(threads);
@@ -597,7 +603,7 @@ cudaError_t launch_after(const void *fn, int blocks, int threads, void **args, c
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = early ? 1 : 0;
   return cudaLaunchKernelExC(&cfg, fn, args);
 }
 
@@ -609,6 +615,7 @@ int launch_pair_tc(LevEngine *h, const TileClass &tc, StepArgs a, int phase,
   if (!s) s = h->stream;
   a.tiles = h->d_tiles + tc.tile_off;
   const int mode = (h->math_mode == LEV_MATH_ACCURATE) ? 1 : 0;
+  const bool early = tc.ntiles > 444 || tc.ntiles <= 111;
   if (tc.pair_variant < 0 || phase == 0) {
     const void *fn =
         tc.pair_variant < 0
@@ -618,7 +625,7 @@ int launch_pair_tc(LevEngine *h, const TileClass &tc, StepArgs a, int phase,
     if (tc.pair_variant < 0) {
       LEV_TRY_CUDA(cudaLaunchKernel(fn, dim3(tc.ntiles), dim3(kTile), args, 0, s));
     } else {
-      LEV_TRY_CUDA(launch_after(fn, tc.ntiles, kTile, args, s));
+      LEV_TRY_CUDA(launch_after(fn, tc.ntiles, kTile, args, early, s));
     }
   } else {
     const int blocks = (tc.ntiles + kFinishTiles - 1) / kFinishTiles;
@@ -626,13 +633,13 @@ int launch_pair_tc(LevEngine *h, const TileClass &tc, StepArgs a, int phase,
     void *args[] = {&a, &ntiles};
     LEV_TRY_CUDA(launch_after(mode ? reinterpret_cast<const void *>(finish_kernel<1>)
                                    : reinterpret_cast<const void *>(finish_kernel<0>),
-                              blocks, kTile, args, s));
+                              blocks, kTile, args, early, s));
   }
   if (tc.pair_variant >= 0) {  // r and g of the class's networks
     const int *nets = h->d_class_nets + tc.net_off;
     void *args[] = {&a, &nets};
     LEV_TRY_CUDA(launch_after(reinterpret_cast<const void *>(reduce_kernel), tc.nnets,
-                              kReduceThreads, args, s));
+                              kReduceThreads, args, early, s));
   }
   return LEV_OK;
 }
