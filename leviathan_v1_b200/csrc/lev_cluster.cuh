@@ -97,6 +97,8 @@ struct ClusterArgs {
   int lgR;        // log2(R)
   int edge_cap;   // SELL entries per CTA the shared memory was sized for
   int early;      // no delay is 0: wait for step t's barrier after step t+1's edges
+  int *err;       // error flag (mapped host memory) (cluster_split_kernel)
+  GridWait wait;  // bound of the waits (cluster_split_kernel)
   float dt;
 };
 
@@ -340,16 +342,33 @@ __global__ void __launch_bounds__(MAXR, 1) cluster_kernel(const ClusterArgs a) {
 }
 
 // ---------------------------------------------------------------------------
-// The cluster-resident step with four lanes per row (CTA = 4R threads, R up to
-// 128; rows and entries to lanes as in lev_split.cuh).  Bitwise the results of
-// cluster_kernel and step_kernel.
+// The cluster-resident step with four lanes per row (R up to 128; rows and
+// entries to lanes as in lev_split.cuh) and a warp for the other CTAs.  Bitwise
+// the results of cluster_kernel and step_kernel.
 //
 // A step is one latency chain (N = 1000: 16 CTAs of 64 rows, two warps per SM
-// sub-core), so the chain is kept short: the row's state stays in registers,
-// alike in its four lanes; a warp writes its part of the slice sums into every
-// CTA of the cluster and arrives; after the wait every warp reduces them from
-// its own shared memory.  The only synchronisation of a step is the cluster
-// barrier.
+// sub-core).  With every thread in the cluster barrier, 710 of a step's 3,800
+// cycles went into the arrival, whose release waits for the remote stores of
+// the sums, and 600 into the reduction.  So the exchange has a warp of its own,
+// as in grid_kernel: it sends its CTA's slice sums to every CTA with st.async,
+// which signals the receiver's mbarrier as the data lands and needs no answer,
+// waits on its own mbarrier for those of all CTAs and reduces them, while the
+// edge warps walk the next step's edges.
+//
+// Order of one step s (barriers A and B are the CTA's):
+//   edge warps               | exchange warp
+//   predictor, edges         | wait for all slice sums of s-1; r, g of step s
+//   ------------------------ barrier A: g (before the edges with zero delays)
+//   integrate, ring slot s+1 |
+//   ------------------------ barrier B: warp parts
+//   (step s+1)               | send the slice sums of s to every CTA
+// With the sums goes an arrival with release semantics, which orders the CTA's
+// phases of step s: gathers of step s+1 read slots <= s, and every CTA's arrival
+// of step s-1 was among those that barrier A of step s waited for.  The integrate of step s
+// overwrites the slot that the gathers of step s-1 read last; the CTAs that did
+// have sent the sums of s-1, which follow from the gathered values.  Sums of s
+// go to buffer s mod 2: whoever sends them has received all sums of s-1, whose
+// senders had done with those of s-2.
 // ---------------------------------------------------------------------------
 constexpr int kSplitLPR = 4;  // lanes per row
 constexpr int kSplitSlicesMax = kClusterMax * 128 / 32;  // 64: at most 8 blocks of 256 nodes
@@ -364,27 +383,49 @@ __device__ __forceinline__ float ld_cluster(uint32_t addr) {
   asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr));
   return v;
 }
-__device__ __forceinline__ void st_cluster(uint32_t addr, float2 v) {
-  asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(addr), "f"(v.x), "f"(v.y)
+// 8 bytes to another CTA's shared memory, counted by the mbarrier `bar` there.
+__device__ __forceinline__ void st_cluster_async(uint32_t addr, float2 v, uint32_t bar) {
+  asm volatile(
+      "st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [%0], {%1, %2}, [%3];" ::"r"(
+          addr), "r"(__float_as_uint(v.x)), "r"(__float_as_uint(v.y)), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void mbar_init(uint32_t bar, unsigned count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
+}
+// An arrival at an mbarrier of the cluster that orders this CTA's writes before it.
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar)
                : "memory");
 }
+// This phase's arrival, and the bytes it waits for.
+__device__ __forceinline__ void mbar_expect(uint32_t bar, unsigned bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.release.cta.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
+               "r"(bytes) : "memory");
+}
+__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, unsigned parity) {
+  unsigned done;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+  return done != 0;
+}
 
-// (sum cos, sum sin) from the warps' parts [slices][4] of up to 64 slices
-// (zero past the network), by one warp, in every lane: lane l closes slice l's
-// tree, three shuffle levels close the 256-node blocks (block_tree8), and two
-// more add the at most eight blocks in the order of final_reduce_r_kernel
-// (leviathan_kernel.cu:242-263: lane b holds block b, the first two levels add
-// zeros).
-__device__ __forceinline__ float2 split_sums(const float2 *parts, int nslices, int lane) {
+// (sum cos, sum sin) from up to 64 slice sums (zero past the network), by one
+// warp, in every lane: three shuffle levels close the 256-node blocks
+// (block_tree8), and two more add the at most eight blocks in the order of
+// final_reduce_r_kernel (leviathan_kernel.cu:242-263: lane b holds block b, the
+// first two levels add zeros).
+__device__ __forceinline__ float2 split_sums(const float2 *sums, int nslices, int lane) {
   const unsigned mask = 0xffffffffu;
   float c[2] = {0.0f, 0.0f}, s[2] = {0.0f, 0.0f};
 #pragma unroll
   for (int grp = 0; grp < 2; ++grp) {
     if (32 * grp >= nslices) break;  // uniform
-    const float4 *p = reinterpret_cast<const float4 *>(parts + 4 * (32 * grp + lane));
-    const float4 a = p[0], b = p[1];
-    float vc = __fadd_rn(__fadd_rn((a.x + b.x) + (a.z + b.z), 0.0f), 0.0f);
-    float vs = __fadd_rn(__fadd_rn((a.y + b.y) + (a.w + b.w), 0.0f), 0.0f);
+    const float2 a = sums[32 * grp + lane];
+    float vc = __fadd_rn(__fadd_rn(a.x, 0.0f), 0.0f);
+    float vs = __fadd_rn(__fadd_rn(a.y, 0.0f), 0.0f);
 #pragma unroll
     for (int off = 4; off > 0; off /= 2) {
       vc += __shfl_down_sync(mask, vc, off);
@@ -403,30 +444,40 @@ __device__ __forceinline__ float2 split_sums(const float2 *parts, int nslices, i
 }
 
 // shared memory (bytes, from the dynamic base):
-//   parts  float2 [2][kSplitSlicesMax * 4]   every CTA's copy of the warps' parts
+//   sums   float2 [2][kSplitSlicesMax]   every CTA's copy of the slice sums
 //   sloff, sllen  int [R/32]
 //   ring   float  [bsi][R]
 //   cd     uint32 [edge_cap], w float [edge_cap]   (order of lev_split.cuh)
+// The wait is bounded (GridWait): on a timeout the CTA writes 1 to the error
+// flag (mapped host memory), leaves the step loop and writes nothing back.
 template <int MATH>
-__global__ void __launch_bounds__(kSplitLPR * 128, 1) cluster_split_kernel(const ClusterArgs a) {
+__global__ void __launch_bounds__(kSplitLPR * 128 + 32, 1)
+    cluster_split_kernel(const ClusterArgs a) {
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
   extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ __align__(8) unsigned long long s_mbar[2];
+  __shared__ float2 s_part[kSplitLPR * 128 / 32];
+  __shared__ float s_g;
+  __shared__ int s_ok;
 
   const NetDesc nd = *a.net;
   const int rank = (int)cluster.block_rank();
   const int C = (int)cluster.num_blocks();
   const int R = a.R;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const SplitLane sl = split_lane<kSplitLPR>(tid);
+  const int nthreads = blockDim.x;  // 4R + 32
+  const bool edges = tid < kSplitLPR * R;
+  const SplitLane sl = split_lane<kSplitLPR>(edges ? tid : lane);
   const int N = nd.N, bsi = nd.bsi, Np = nd.Np;
   const int row0 = rank * R;
   const int row = row0 + sl.rloc;
-  const bool live = row < N;
+  const bool live = edges && row < N;
   const int nslices = R / 32;
+  auto cta_sync = [&]() { asm volatile("bar.sync 1, %0;" ::"r"(nthreads) : "memory"); };
 
-  float2 *parts = reinterpret_cast<float2 *>(smem);
-  int *sloff = reinterpret_cast<int *>(parts + 2 * 4 * kSplitSlicesMax);
+  float2 *s_sums = reinterpret_cast<float2 *>(smem);
+  int *sloff = reinterpret_cast<int *>(s_sums + 2 * kSplitSlicesMax);
   int *sllen = sloff + nslices;
   float *s_ring = reinterpret_cast<float *>(sllen + nslices);
   uint32_t *s_cd = reinterpret_cast<uint32_t *>(s_ring + (size_t)bsi * R);
@@ -436,12 +487,18 @@ __global__ void __launch_bounds__(kSplitLPR * 128, 1) cluster_split_kernel(const
   const long long sl0 = nd.slice_base + row0 / 32;
   const int my_slices = max(0, min(nslices, (N - row0 + 31) / 32));
   const long long ebase = my_slices ? a.sl_off[sl0] : 0;
-  for (int s = tid; s < nslices; s += blockDim.x) {
+  for (int s = tid; s < nslices; s += nthreads) {
     sloff[s] = s < my_slices ? (int)(a.sl_off[sl0 + s] - ebase) : 0;
     sllen[s] = s < my_slices ? a.sl_len[sl0 + s] : 0;
   }
-  for (int k = tid; k < 2 * 4 * kSplitSlicesMax; k += blockDim.x)
-    parts[k] = make_float2(0.0f, 0.0f);
+  for (int k = tid; k < 2 * kSplitSlicesMax; k += nthreads) s_sums[k] = make_float2(0.0f, 0.0f);
+  const uint32_t mbar = (uint32_t)__cvta_generic_to_shared(s_mbar);
+  if (tid == 0) {
+    s_ok = 1;
+    mbar_init(mbar, (unsigned)C + 1u);  // every CTA, and this one's expected bytes
+    mbar_init(mbar + 8, (unsigned)C + 1u);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
   __syncthreads();
   split_for_entries<kSplitLPR>(sloff, sllen, my_slices, [&](int at, int e) {
     s_cd[at] = a.sl_cd[ebase + e];
@@ -461,117 +518,164 @@ __global__ void __launch_bounds__(kSplitLPR * 128, 1) cluster_split_kernel(const
       s_ring[(size_t)s * R + sl.rloc] = a.ring[nd.ring_off + ring_pos(s, row, Np)];
   }
   const NetState ns = *a.st;
-  int cur = ns.cur, rbuf = ns.rbuf;
-  float g = ns.g, r = ns.r;
-  const int all_slices = 8 * nd.ntiles;
+  int cur = ns.cur;
+  float g = ns.g;
   const float dt = a.dt;
-  const float inv_N = 1.0f / (float)N;
-  const int len = sllen[sl.ws], base = sloff[sl.ws];
   const uint32_t ring_addr = (uint32_t)__cvta_generic_to_shared(s_ring);
-  // lane l's copy of this warp's part in CTA l
-  const uint32_t part_addr = cluster_addr(
-      (uint32_t)__cvta_generic_to_shared(parts + 4 * (row0 / 32) + warp), lane < C ? lane : 0);
-  // the last warp of CTA 0 feeds an attached hub monitor
-  const bool observe = a.hubs && rank == 0 && warp == (int)(blockDim.x >> 5) - 1;
-  HubWarp hub;
-  if (observe) hub.open(a.hubs);
   auto phase = [&](int j, int slot) {
     const uint32_t at = ring_addr + 4u * (unsigned)(slot * R + (j & (R - 1)));
     return ld_cluster(cluster_addr(at, j >> a.lgR));
   };
-  // r and g after `steps` steps of this launch, alike in every thread
-  auto close_step = [&](int steps) {
-    const float2 sums =
-        split_sums(parts + ((steps - 1) & 1) * 4 * kSplitSlicesMax, all_slices, lane);
-    r = order_parameter(sums.x, sums.y, inv_N);
-    if (nd.ctrl) g = gain_controller(g, r, dt, nd);
-    if (rank == 0 && tid == 0 && a.r_hist) {
-      const int k = ns.rpos + steps - 1;
-      if (k < a.r_cap) a.r_hist[k] = r;
-    }
-  };
   cluster.sync();
 
-  for (int step = 0; step < a.n_steps; ++step) {
-    // with zero delays: step-1's barrier before the gathers
-    if (step > 0 && !a.early) cluster_wait();
-    // ---- predictor ----------------------------------------------------------
-    const float eps = sinf(wrap_pm_pi(th - thh));
-    thh = thh + dt * omh;
-    omh = omh + nd.kappa_w * dt * eps;
-    // ---- edges ----------------------------------------------------------------
-    const EdgeParams ep = {dt, nd.eta, nd.lam, __fmaf_rn(-nd.gamma, fabsf(eps), 1.0f),
-                           nd.w_min, nd.w_max};
-    const float local_sum =
-        split_walk<MATH, kSplitLPR>(s_cd + base, s_w + base, len, deg, sl, th, ep, [&](uint32_t word) {
-          const unsigned s0 = (unsigned)(cur - (int)(word & 255u));
-          return phase((int)(word >> 8), (int)min(s0, s0 + (unsigned)bsi));
-        });
-    // ---- r and gain of the previous step --------------------------------------
-    float hub_phase = 0.0f;
-    if (step > 0) {
-      if (a.early) cluster_wait();
-      if (observe) hub_phase = phase(hub.node, cur);
-      close_step(step);
+  if (edges) {
+    const int len = sllen[sl.ws], base = sloff[sl.ws];
+    for (int step = 0; step < a.n_steps; ++step) {
+      if (step > 0 && !a.early) {
+        cta_sync();  // A, before the gathers of slot `step`
+        if (*reinterpret_cast<volatile int *>(&s_ok) == 0) break;
+      }
+      // ---- predictor ----------------------------------------------------------
+      const float eps = sinf(wrap_pm_pi(th - thh));
+      thh = thh + dt * omh;
+      omh = omh + nd.kappa_w * dt * eps;
+      // ---- edges ----------------------------------------------------------------
+      const EdgeParams ep = {dt, nd.eta, nd.lam, __fmaf_rn(-nd.gamma, fabsf(eps), 1.0f),
+                             nd.w_min, nd.w_max};
+      const float local_sum =
+          split_walk<MATH, kSplitLPR>(s_cd + base, s_w + base, len, deg, sl, th, ep,
+                                      [&](uint32_t word) {
+            const unsigned s0 = (unsigned)(cur - (int)(word & 255u));
+            return phase((int)(word >> 8), (int)min(s0, s0 + (unsigned)bsi));
+          });
+      if (step > 0) {
+        if (a.early) {
+          cta_sync();  // A
+          if (*reinterpret_cast<volatile int *>(&s_ok) == 0) break;
+        }
+        g = s_g;
+      }
+      // ---- integrate --------------------------------------------------------------
+      int nxt = cur + 1;
+      if (nxt == bsi) nxt = 0;
+      float my_cos = 0.0f, my_sin = 0.0f;
+      if (live) {
+        float inc = dt * (om + g * local_sum - nd.alpha * eps);
+        float x = th + inc;
+        x = wrap_0_2pi(x);
+        if (!isfinite(x)) x = 0.0f;
+        th = x;
+        if (sl.q == 0) s_ring[(size_t)nxt * R + sl.rloc] = x;
+        lev_sincos<MATH>(x, &my_sin, &my_cos);
+      }
+      // ---- this warp's part of the slice sums (leviathan_kernel.cu:198-214) -------
+      const float2 part = split_warp_sum<kSplitLPR>(my_cos, my_sin);
+      if (lane == 0) s_part[warp] = part;
+      cur = nxt;
+      cta_sync();  // B
     }
-    // ---- integrate --------------------------------------------------------------
-    int nxt = cur + 1;
-    if (nxt == bsi) nxt = 0;
-    float my_cos = 0.0f, my_sin = 0.0f;
+  } else {
+    const float inv_N = 1.0f / (float)N;
+    const int all_slices = 8 * nd.ntiles;
+    const unsigned bytes = (unsigned)(C * nslices) * 8u;
+    float r = ns.r;
+    // lane c sends to CTA c
+    const int to = lane < C ? lane : 0;
+    const uint32_t sums_to = cluster_addr(
+        (uint32_t)__cvta_generic_to_shared(s_sums + row0 / 32), to);
+    const uint32_t mbar_to = cluster_addr(mbar, to);
+    // CTA 0 feeds an attached hub monitor
+    const bool observe = a.hubs && rank == 0;
+    HubWarp hub;
+    if (observe) hub.open(a.hubs);
+    // r and g after `steps` steps of this launch, alike in every lane; false
+    // after a timeout
+    auto close_step = [&](int steps) -> bool {
+      const int b = (steps - 1) & 1;
+      const unsigned parity = (unsigned)((steps - 1) >> 1) & 1u;
+      const unsigned long long t0 = global_ns();
+      while (a.wait.extra || !__all_sync(0xffffffffu, mbar_try_wait(mbar + 8 * b, parity)))
+        if (__any_sync(0xffffffffu, global_ns() - t0 > a.wait.ns)) return false;
+      const float2 sums = split_sums(s_sums + b * kSplitSlicesMax, all_slices, lane);
+      r = order_parameter(sums.x, sums.y, inv_N);
+      if (nd.ctrl) g = gain_controller(g, r, dt, nd);
+      if (lane == 0) {
+        s_g = g;
+        if (rank == 0 && a.r_hist) {
+          const int k = ns.rpos + steps - 1;
+          if (k < a.r_cap) a.r_hist[k] = r;
+        }
+      }
+      return true;
+    };
+    auto give_up = [&]() {
+      if (lane == 0) {
+        *reinterpret_cast<volatile int *>(a.err) = 1;
+        *reinterpret_cast<volatile int *>(&s_ok) = 0;
+      }
+      __syncwarp();
+    };
+    bool ok = true;
+    for (int step = 0; step < a.n_steps; ++step) {
+      float hub_phase = 0.0f;
+      if (step > 0) {
+        ok = close_step(step);
+        if (!ok) give_up();
+        cta_sync();  // A
+        if (!ok) break;
+        if (observe) hub_phase = phase(hub.node, cur);
+      }
+      if (lane == 0) mbar_expect(mbar + 8 * (step & 1), bytes);
+      cur = (cur + 1 == bsi) ? 0 : cur + 1;
+      cta_sync();  // B
+      if (lane < C) mbar_arrive_cluster(mbar_to + 8u * (unsigned)(step & 1));
+      for (int s = 0; s < nslices; ++s) {
+        const float2 v = split_slice_sum<kSplitLPR>(s_part + kSplitLPR * s);
+        if (lane < C)
+          st_cluster_async(sums_to + 8u * (unsigned)((step & 1) * kSplitSlicesMax + s), v,
+                           mbar_to + 8u * (unsigned)(step & 1));
+      }
+      __syncwarp();
+      if (observe && step > 0) hub.observe(hub_phase);
+    }
+    // the last step: every CTA waits for its sums (they land in its memory)
+    if (ok && a.n_steps > 0) {
+      ok = close_step(a.n_steps);
+      if (!ok) give_up();
+      if (ok && rank == 0) {
+        if (lane == 0) {
+          NetState o = ns;
+          o.g = g;
+          o.r = r;
+          o.cur = cur;
+          o.rbuf = (int)((ns.rbuf + (long long)a.n_steps) % (nd.max_delay + 1));
+          o.t = ns.t + a.n_steps;
+          o.rpos = ns.rpos + a.n_steps;
+          o.ticket = 0u;
+          *a.st = o;
+        }
+        if (observe) {
+          hub.observe(phase(hub.node, cur));
+          hub.close(a.n_steps);
+        }
+      }
+    }
+  }
+  __syncthreads();
+  if (*reinterpret_cast<volatile int *>(&s_ok) != 0) {
     if (live) {
-      float inc = dt * (om + g * local_sum - nd.alpha * eps);
-      float x = th + inc;
-      x = wrap_0_2pi(x);
-      if (!isfinite(x)) x = 0.0f;
-      th = x;
-      if (sl.q == 0) s_ring[(size_t)nxt * R + sl.rloc] = x;
-      lev_sincos<MATH>(x, &my_sin, &my_cos);
+      const long long gi = nd.node_off + row;
+      if (sl.q == 0) {
+        a.theta[gi] = th;
+        a.theta_hat[gi] = thh;
+        a.omega_hat[gi] = omh;
+      }
+      for (int s = sl.q; s < bsi; s += kSplitLPR)
+        a.ring[nd.ring_off + ring_pos(s, row, Np)] = s_ring[(size_t)s * R + sl.rloc];
     }
-    // ---- this warp's part of the slice sums (leviathan_kernel.cu:198-214), to
-    // every CTA ------------------------------------------------------------------
-    float2 part = split_warp_sum<kSplitLPR>(my_cos, my_sin);
-    part.x = __shfl_sync(0xffffffffu, part.x, 0);
-    part.y = __shfl_sync(0xffffffffu, part.y, 0);
-    if (lane < C)
-      st_cluster(part_addr + (step & 1) * (unsigned)(sizeof(float2) * 4 * kSplitSlicesMax), part);
-    __syncwarp();
-    cur = nxt;
-    rbuf = (rbuf + 1 == nd.max_delay + 1) ? 0 : rbuf + 1;
-    cluster_arrive();
-    if (observe && step > 0) hub.observe(hub_phase);
+    split_for_entries<kSplitLPR>(sloff, sllen, my_slices,
+                                 [&](int at, int e) { a.sl_w[ebase + e] = s_w[at]; });
   }
-  // ---- r of the last step, then write the state back ------------------------
-  if (a.n_steps > 0) {
-    cluster_wait();
-    close_step(a.n_steps);
-    if (rank == 0 && tid == 0) {
-      NetState o = ns;
-      o.g = g;
-      o.r = r;
-      o.cur = cur;
-      o.rbuf = rbuf;
-      o.t = ns.t + a.n_steps;
-      o.rpos = ns.rpos + a.n_steps;
-      o.ticket = 0u;
-      *a.st = o;
-    }
-    if (observe) {
-      hub.observe(phase(hub.node, cur));
-      hub.close(a.n_steps);
-    }
-  }
-  if (live) {
-    const long long gi = nd.node_off + row;
-    if (sl.q == 0) {
-      a.theta[gi] = th;
-      a.theta_hat[gi] = thh;
-      a.omega_hat[gi] = omh;
-    }
-    for (int s = sl.q; s < bsi; s += kSplitLPR)
-      a.ring[nd.ring_off + ring_pos(s, row, Np)] = s_ring[(size_t)s * R + sl.rloc];
-  }
-  split_for_entries<kSplitLPR>(sloff, sllen, my_slices,
-                    [&](int at, int e) { a.sl_w[ebase + e] = s_w[at]; });
   // no CTA may leave while a peer can still read its shared memory
   cluster.sync();
 }

@@ -218,8 +218,9 @@ struct LevEngine {
   float *d_rmap = nullptr;
 
   // r history of step blocks
-  int block_len = 256;
-  float *d_rhist = nullptr;   // [block_len][num_nets]
+  int block_len = 256;        // steps per graph
+  int rhist_rows = 256;       // rows of d_rhist; steps per launch of the resident kernels
+  float *d_rhist = nullptr;   // [rhist_rows][num_nets]
   float *h_rstage = nullptr;  // pinned staging for lev_step_n
   size_t h_rstage_len = 0;
 
@@ -828,7 +829,7 @@ ClusterFn cluster_fn(int R, int math_mode) {
   if (R <= 256) return acc ? cluster_kernel<1, 256, 24> : cluster_kernel<0, 256, 24>;
   return acc ? cluster_kernel<1, kClusterRowsMax, 8> : cluster_kernel<0, kClusterRowsMax, 8>;
 }
-inline int cluster_threads(int R) { return R <= 128 ? 4 * R : R; }
+inline int cluster_threads(int R) { return R <= 128 ? 4 * R + 32 : R; }
 
 // One launch of the cluster-resident kernel: `len` steps, r history rows
 // 0..len-1 in d_rhist.
@@ -849,13 +850,15 @@ int launch_cluster(LevEngine *h, float dt, int len) {
   ca.ring = h->d_ring;
   ca.r_hist = h->d_rhist;
   ca.hubs = h->hubs ? h->hubs->d_mon : nullptr;
-  ca.r_cap = h->block_len;
+  ca.r_cap = h->rhist_rows;
   ca.n_steps = len;
   ca.R = h->cluster_R;
   ca.lgR = 0;
   while ((1 << ca.lgR) < h->cluster_R) ++ca.lgR;
   ca.edge_cap = h->cluster_edge_cap;
   ca.early = h->pair_ok ? 1 : 0;  // no delay is 0
+  ca.err = h->d_gerr;
+  ca.wait = h->grid_wait;
   ca.dt = dt;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(h->cluster_C);
@@ -914,7 +917,7 @@ void setup_cluster(LevEngine *h, const std::vector<int> &sl_len) {
         e += 32LL * sl_len[d.slice_base + s];
       cap = std::max(cap, e);
     }
-    const size_t node = R <= 128 ? sizeof(float2) * 2 * 4 * kSplitSlicesMax
+    const size_t node = R <= 128 ? sizeof(float2) * 2 * kSplitSlicesMax
                                  : sizeof(float2) * 2 * kClusterWarpsMax + sizeof(float) * 4 * R;
     const size_t smem = node + sizeof(int) * 2 * (R / 32) +
                         sizeof(float) * (size_t)d.bsi * R + 8 * (size_t)cap;
@@ -1005,7 +1008,7 @@ int launch_grid(LevEngine *h, float dt, int len) {
   ga.err = h->d_gerr;
   ga.wait = h->grid_wait;
   ga.r_hist = h->d_rhist;
-  ga.r_cap = h->block_len;
+  ga.r_cap = h->rhist_rows;
   ga.num_nets = h->num_nets;
   ga.n_steps = len;
   ga.edge_cap = h->grid_cap[ri];
@@ -1022,6 +1025,18 @@ int launch_grid(LevEngine *h, float dt, int len) {
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   LEV_TRY_CUDA(cudaLaunchKernelEx(&cfg, grid_fn(R, h->math_mode), ga));
+  return LEV_OK;
+}
+
+// The error flag of the resident kernels' waits, and their r history.
+int setup_wait_flag(LevEngine *h) {
+  if (!h->cluster_ok && !h->grid_ok) return LEV_OK;
+  // a launch loads and stores the whole state (N = 1000: 15 us): long blocks
+  h->rhist_rows = 2048;
+  h->h_gerr = reinterpret_cast<int *>(mapped_alloc(1));
+  if (!h->h_gerr) return fail(LEV_ERR_NOMEM, "mapped host memory: allocation failed");
+  *h->h_gerr = 0;
+  LEV_TRY_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void **>(&h->d_gerr), h->h_gerr, 0));
   return LEV_OK;
 }
 
@@ -1110,21 +1125,18 @@ int setup_grid(LevEngine *h, const std::vector<int> &sl_len) {
         for (int c = 0; c * kGridRs[ri] < h->h_nets[n].N; ++c) h->h_gmap.push_back(make_int2(n, c));
     }
   }
-  h->h_gerr = reinterpret_cast<int *>(mapped_alloc(1));
-  if (!h->h_gerr) return fail(LEV_ERR_NOMEM, "mapped host memory: allocation failed");
-  *h->h_gerr = 0;
-  LEV_TRY_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void **>(&h->d_gerr), h->h_gerr, 0));
   return LEV_OK;
 }
 
-// After the stream has drained: a grid barrier that timed out leaves the
-// engine state undefined; report it once and stop using the grid path.
+// After the stream has drained: a wait that timed out leaves the engine state
+// undefined; report it once and stop using the resident paths.
 int check_grid_error(LevEngine *h) {
   if (h->h_gerr && *reinterpret_cast<volatile int *>(h->h_gerr)) {
     *h->h_gerr = 0;
     h->grid_ok = false;
+    h->cluster_ok = false;
     return fail(LEV_ERR_CUDA,
-                "grid-resident step block: a grid barrier wait timed out; the engine state "
+                "resident step block: a wait for the other CTAs timed out; the engine state "
                 "is undefined");
   }
   return LEV_OK;
@@ -1137,11 +1149,13 @@ int enqueue_steps(LevEngine *h, float dt, int n, float *stage) {
   spec_drop(h);
   int done = 0;
   while (done < n) {
-    const int len = std::min(h->block_len, n - done);
-    if (h->cluster_ok && h->use_cluster && (!h->hubs || h->cluster_R <= 128)) {
+    const bool cluster = h->cluster_ok && h->use_cluster && (!h->hubs || h->cluster_R <= 128);
+    const bool grid = !cluster && h->grid_ok && h->use_grid;
+    const int len = std::min(cluster || grid ? h->rhist_rows : h->block_len, n - done);
+    if (cluster) {
       int rc = launch_cluster(h, dt, len);
       if (rc != LEV_OK) return rc;
-    } else if (h->grid_ok && h->use_grid) {
+    } else if (grid) {
       int rc = launch_grid(h, dt, len);
       if (rc != LEV_OK) return rc;
     } else {
@@ -1646,6 +1660,7 @@ int create_impl(LevEngine **out, int num_nets, const int32_t *Ns,
     if (lrc == LEV_OK) {
       setup_cluster(h, h_sl_len);
       lrc = setup_grid(h, h_sl_len);
+      if (lrc == LEV_OK) lrc = setup_wait_flag(h);
     }
     if (lrc == LEV_OK) {
       int nbusy = 0;
@@ -1699,7 +1714,7 @@ int create_impl(LevEngine **out, int num_nets, const int32_t *Ns,
         {(void **)&h->d_omega_hat, sizeof(float) * node_off},
         {(void **)&h->d_ring, sizeof(float) * ring_off},
         {(void **)&h->d_part, sizeof(float2) * std::max(tiles, 1)},
-        {(void **)&h->d_rhist, sizeof(float) * h->block_len * num_nets},
+        {(void **)&h->d_rhist, sizeof(float) * h->rhist_rows * num_nets},
         {(void **)&h->d_class_nets, sizeof(int) * num_nets},
         {(void **)&h->d_pend, sizeof(float2) * node_off},
         {(void **)&h->d_gwsum, h->grid_ok ? sizeof(float2) * 32 * (size_t)tiles : 0},

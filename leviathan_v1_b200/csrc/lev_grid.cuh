@@ -34,18 +34,6 @@
 
 namespace lev {
 
-constexpr unsigned long long kGridWaitNs = 2000000000ull;  // default wait limit
-
-// Bound of every grid-barrier wait of a launch.  `extra` is 0 in normal use;
-// a positive value makes each wait expect that many arrivals more than the
-// grid makes, so the first wait runs out after `ns` -- the timeout path can
-// then be exercised by a test without faulting or hanging the GPU.
-struct GridWait {
-  unsigned long long ns;  // limit of one wait, globaltimer nanoseconds
-  unsigned extra;
-  unsigned pad;
-};
-
 struct GridArgs {
   const NetDesc *nets;
   NetState *st;
@@ -79,12 +67,6 @@ __device__ __forceinline__ unsigned ld_acquire_gpu(const unsigned *p) {
   unsigned v;
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
-}
-
-__device__ __forceinline__ unsigned long long global_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
 }
 
 // Grid barrier, split in two.  Arrive: every thread of the CTA calls it

@@ -27,6 +27,24 @@
 
 namespace lev {
 
+constexpr unsigned long long kGridWaitNs = 2000000000ull;  // default wait limit
+
+// Bound of every wait on other CTAs of a launch.  `extra` is 0 in normal use;
+// a positive value makes each wait expect that many arrivals more than the
+// grid makes, so the first wait runs out after `ns` -- the timeout path can
+// then be exercised by a test without faulting or hanging the GPU.
+struct GridWait {
+  unsigned long long ns;  // limit of one wait, globaltimer nanoseconds
+  unsigned extra;
+  unsigned pad;
+};
+
+__device__ __forceinline__ unsigned long long global_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
+
 // Entries per lane and chunk for slices of `len` entries per row: as few
 // chunks as entries of at most 8 per lane allow, of equal size (an empty
 // entry costs the instructions of a full one).
