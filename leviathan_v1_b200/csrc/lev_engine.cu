@@ -242,6 +242,7 @@ struct LevEngine {
   bool grid_R_ok[3] = {false, false, false};  // R = 64, 128, 256
   int grid_cap[3] = {0, 0, 0};                // SELL entries per CTA
   size_t grid_smem_R[3] = {0, 0, 0};
+  bool grid_order[3] = {false, false, false};  // with an order warp
   int grid_max_tiles = 0;     // tiles of the largest network
   int grid_map_off[3] = {0, 0, 0};            // first entry of each choice in d_gmap
   std::vector<int2> h_gmap;   // batches: (network, CTA) per CTA
@@ -963,11 +964,16 @@ void setup_cluster(LevEngine *h, const std::vector<int> &sl_len) {
 // Grid kernel for R rows per CTA (64, 128, 256).
 using GridFn = void (*)(GridArgs);
 constexpr int kGridRs[3] = {64, 128, 256};
-GridFn grid_fn(int R, int math_mode) {
+template <bool ORDER>
+GridFn grid_fn_of(int R, int math_mode) {
   const bool acc = math_mode == LEV_MATH_ACCURATE;
-  if (R == 64) return acc ? grid_kernel<1, 64> : grid_kernel<0, 64>;
-  if (R == 128) return acc ? grid_kernel<1, 128> : grid_kernel<0, 128>;
-  return acc ? grid_kernel<1, 256> : grid_kernel<0, 256>;
+  if (R == 64) return acc ? grid_kernel<1, 64, ORDER> : grid_kernel<0, 64, ORDER>;
+  return acc ? grid_kernel<1, 128, ORDER> : grid_kernel<0, 128, ORDER>;
+}
+GridFn grid_fn(int R, int math_mode, bool order) {
+  if (R == 256)
+    return math_mode == LEV_MATH_ACCURATE ? grid_kernel<1, 256, false> : grid_kernel<0, 256, false>;
+  return order ? grid_fn_of<true>(R, math_mode) : grid_fn_of<false>(R, math_mode);
 }
 inline int grid_r_index(int R) { return R == 64 ? 0 : (R == 128 ? 1 : 2); }
 
@@ -1016,7 +1022,7 @@ int launch_grid(LevEngine *h, float dt, int len) {
   ga.dt = dt;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid_ctas(h, R));
-  cfg.blockDim = dim3(kGridThreads);
+  cfg.blockDim = dim3(grid_threads(h->grid_order[ri]));
   cfg.dynamicSmemBytes = h->grid_smem_R[ri];
   cfg.stream = h->stream;
   cudaLaunchAttribute attr[1];
@@ -1024,7 +1030,7 @@ int launch_grid(LevEngine *h, float dt, int len) {
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  LEV_TRY_CUDA(cudaLaunchKernelEx(&cfg, grid_fn(R, h->math_mode), ga));
+  LEV_TRY_CUDA(cudaLaunchKernelEx(&cfg, grid_fn(R, h->math_mode, h->grid_order[ri]), ga));
   return LEV_OK;
 }
 
@@ -1085,15 +1091,23 @@ int setup_grid(LevEngine *h, const std::vector<int> &sl_len) {
     const size_t smem = (R < 256 ? sizeof(float2) * 8 * (size_t)h->grid_max_tiles : 0) +
                         sizeof(int) * 2 * (R / 32) + 8 * (size_t)cap;
     if (smem + 1024 > (size_t)max_smem) continue;
-    bool ok = true;
-    for (int m = 0; m < 2 && ok; ++m) {
-      const void *fn = reinterpret_cast<const void *>(
-          grid_fn(R, m ? LEV_MATH_ACCURATE : LEV_MATH_REFERENCE));
-      int per_sm = 0;
-      ok = allow_smem(fn, smem) &&
-           cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kGridThreads, smem) ==
-               cudaSuccess &&
-           (long long)per_sm * sms >= C;
+    // With an order warp if every CTA is then resident, else without; with one
+    // lane per row (R = 256) never: us per step with / without at N = 5*10^4,
+    // k = 8 4.50 / 3.27, at N = 7.5*10^4, k = 32 8.75 / 8.16, and for R = 64,
+    // 128 at N = 6,000, k = 20 2.11 / 2.37, at N = 18,900 2.85 / 3.17.
+    bool ok = false;
+    for (int order = R < 256 ? 1 : 0; order >= 0 && !ok; --order) {
+      ok = true;
+      for (int m = 0; m < 2 && ok; ++m) {
+        const void *fn = reinterpret_cast<const void *>(
+            grid_fn(R, m ? LEV_MATH_ACCURATE : LEV_MATH_REFERENCE, order != 0));
+        int per_sm = 0;
+        ok = allow_smem(fn, smem) &&
+             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, grid_threads(order != 0),
+                                                           smem) == cudaSuccess &&
+             (long long)per_sm * sms >= C;
+      }
+      h->grid_order[ri] = order != 0;
     }
     cudaGetLastError();  // clear a refused attribute, if any
     if (!ok) continue;

@@ -210,12 +210,19 @@ __device__ __forceinline__ bool grid_sums(const float2 *buf, int n, int nblocks,
   return true;
 }
 
+constexpr unsigned kSumsSleep = 400;  // ns, of a sums warp before its first poll
 constexpr int kGridBarPitch = 32;  // arrival counters of two networks share no 128-byte line
 constexpr int kGridThreads = 256 + 32;  // eight warps on rows, one for the other CTAs
 
+// Threads of grid_kernel: with an order warp, two for the other CTAs.
+__host__ __device__ constexpr int grid_threads(bool order_warp) {
+  return order_warp ? 256 + 64 : kGridThreads;
+}
+
 // Barrier of a CTA whose warps run different code.
+template <int THREADS = kGridThreads>
 __device__ __forceinline__ void cta_barrier() {
-  asm volatile("bar.sync 1, %0;" ::"n"(kGridThreads) : "memory");
+  asm volatile("bar.sync 1, %0;" ::"n"(THREADS) : "memory");
 }
 
 // One warp publishes its CTA's sums of step `step` from the warps' parts and
@@ -254,30 +261,45 @@ __device__ __forceinline__ void grid_publish_part(float2 *wsum, int step, int nb
 // With the CTA's first warp doing both its rows' edges and the exchange, at N =
 // 10^4 (R = 64) a step took 6,990 cycles: edges 2,070, waiting for the counter
 // 960, reading the sums 2,130, integrate 620, and 1,190 in the release fence
-// of the arrival, one after the other.  So a ninth warp does the exchange while
-// the others walk their edges, and the sums carry their own "published" mark:
-// they go out without waiting for the fence, which only the ring phases need
-// and which is paid while the sums travel.
+// of the arrival, one after the other.  So the exchange has warps of its own,
+// and the sums carry their own "published" mark: they go out without waiting
+// for the fence, which only the ring phases need.  The sums warp publishes and
+// collects the sums, the order warp pays the fence, arrives and waits for the
+// others' arrivals.  With R = 256 and in grids of more than two CTAs per SM
+// (ORDER = false) one warp does both, in that order: there the rows' gathers
+// bound the step, and 72 registers keep three CTAs per SM.
 //
-// Order of one step s, edge warps | ninth warp:
-//   predictor, edges            | wait for the sums of s-1; r, g of step s
-//   ------------------------ barrier A: g ------------------------
-//   integrate, ring slot s+1    | wait for every CTA's arrival s-1 (its phases)
-//   ------------------------ barrier B: warp parts ---------------
-//   (step s+1)                  | publish the sums of s, clear those of s-2;
-//                               | fence, arrive
-// Gathers of step s+1 read slots <= s (no zero delay), whose phases were
-// ordered by arrival s-1 before barrier B of step s.  The integrate of step s
-// overwrites the slot that the gathers of step s-1 read last; those CTAs have
-// published the sums of s-1, which follow from the gathered values.  Sums of
-// s live in buffer s mod 4; a CTA clears its part of buffer (s+2) mod 4, the
-// sums of s-2, once all sums of s-1 have shown that nobody still reads them,
-// and its arrival s orders the clearing before anybody looks for the sums of
-// s+2 there.  With zero delays step s gathers slot s, and the wait for arrival
-// s-1 comes before the edges.
-template <int MATH, int R>
-__global__ void __launch_bounds__(kGridThreads, 3) grid_kernel(const GridArgs a) {
+// Order of one step s:
+//   edge warps            | sums warp                 | order warp
+//   predictor, edges      | wait for the sums of s-1; | fence and arrive for s-1
+//                         | r, g of step s            |
+//   ------------------------------- barrier A: g ----------------------------
+//   integrate, slot s+1   |                           | wait for every arrival s-1
+//   ------------------------------- barrier B: warp parts -------------------
+//   (step s+1)            | publish the sums of s,    | fence, arrive for s
+//                         | clear those of s-2        |
+// Gathers of step s+1 read slots <= s (no zero delay), whose phases arrivals
+// s-1 ordered before barrier B of step s.  The integrate of step s overwrites
+// the slot that the gathers of step s-1 read last; those CTAs have published
+// the sums of s-1, which follow from the gathered values.  Sums of s live in
+// buffer s mod 4; a CTA clears its part of buffer (s+2) mod 4, the sums of s-2,
+// once all sums of s-1 have shown that nobody still reads them, and its arrival
+// s+1 orders the clearing before anybody looks for the sums of s+2 there (in
+// step s+3).  With zero delays step s gathers slot s, and the wait for arrivals
+// s-1 comes before the edges (barrier C).
+//
+// Every wait for arrivals comes late, when they have mostly come: polling from
+// the arrival on holds up the arrivals themselves, and every acquire drops the
+// L1 lines the gathers live on.  The sums warp sleeps before its first poll for
+// the same reason.  Measured per step (us), edges and exchange in one warp / one
+// exchange warp / two: N = 6,000, k = 20 (R = 64) - / 2.37 / 2.11; N = 10^4 (64)
+// 3.5 / 2.62 / 2.46; N = 18,900 (128) - / 3.17 / 2.85; N = 10^5 (256) - / 7.6 /
+// 8.8 (two steps per launch: 13.1).
+template <int MATH, int R, bool ORDER>
+__global__ void __launch_bounds__(grid_threads(ORDER), ORDER ? 2 : 3)
+    grid_kernel(const GridArgs a) {
   constexpr int LPR = 256 / R;
+  constexpr int kThreads = grid_threads(ORDER);
   constexpr int nslices = R / 32;
   constexpr bool kBlocks = R == 256;  // a CTA closes its 256-node block itself
   extern __shared__ __align__(16) unsigned char smem[];
@@ -289,12 +311,12 @@ __global__ void __launch_bounds__(kGridThreads, 3) grid_kernel(const GridArgs a)
   const NetDesc nd = a.nets[me.x];
   const int cta = me.y;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const bool exchange = warp == 8;
+  const bool edges = warp < 8;
   const SplitLane sl = split_lane<LPR>(tid & 255);
   const int N = nd.N, bsi = nd.bsi, Np = nd.Np;
   const int row0 = cta * R;
   const int row = row0 + sl.rloc;
-  const bool live = !exchange && row < N;
+  const bool live = edges && row < N;
   const unsigned G = (unsigned)((N + R - 1) / R);
   const int nblocks = nd.ntiles;
   unsigned *bar = a.bar + kGridBarPitch * me.x;
@@ -341,24 +363,52 @@ __global__ void __launch_bounds__(kGridThreads, 3) grid_kernel(const GridArgs a)
   const float dt = a.dt;
   __syncthreads();
 
-  if (!exchange) {
+  // a timeout of one of the exchange warps: all warps read the flag after
+  // barrier A, and it is only written between B and A
+  auto stopped = [&]() { return *reinterpret_cast<volatile int *>(&s_ok) == 0; };
+  auto give_up = [&]() {
+    if (lane == 0) {
+      *reinterpret_cast<volatile int *>(a.err) = 1;
+      *reinterpret_cast<volatile int *>(&s_ok) = 0;
+    }
+    __syncwarp();
+  };
+  // the phases of the first `steps` steps of every CTA are in the ring
+  auto phases_of = [&](int steps) -> bool {
+    const bool ok = lane != 0 || grid_poll(bar, (unsigned)steps * G, a.wait);
+    return __all_sync(0xffffffffu, ok);
+  };
+  auto arrive = [&]() {
+    if (lane == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+  };
+  if (edges) {
     const int len = sllen[sl.ws], base = sloff[sl.ws];
     for (int step = 0; step < a.n_steps; ++step) {
-      if (step > 0 && !a.early) cta_barrier();
-      // ---- predictor ----------------------------------------------------------
-      const float eps = sinf(wrap_pm_pi(th - thh));
-      thh = thh + dt * omh;
-      omh = omh + nd.kappa_w * dt * eps;
-      // ---- edges ----------------------------------------------------------------
-      const EdgeParams ep = {dt, nd.eta, nd.lam, __fmaf_rn(-nd.gamma, fabsf(eps), 1.0f),
-                             nd.w_min, nd.w_max};
-      const float local_sum =
-          split_walk<MATH, LPR>(s_cd + base, s_w + base, len, deg, sl, th, ep, [&](uint32_t word) {
-            return __ldca(ring + ring_pos_word(word, cur, bsi, Np));
-          });
+      if (step > 0 && !a.early) cta_barrier<kThreads>();  // C
+      // ---- predictor; edges -------------------------------------------------------
+      float eps = 0.0f;
+      auto predictor = [&]() -> EdgeParams {
+        eps = sinf(wrap_pm_pi(th - thh));
+        thh = thh + dt * omh;
+        omh = omh + nd.kappa_w * dt * eps;
+        return {dt, nd.eta, nd.lam, __fmaf_rn(-nd.gamma, fabsf(eps), 1.0f), nd.w_min, nd.w_max};
+      };
+      auto gather = [&](uint32_t word) {
+        return __ldca(ring + ring_pos_word(word, cur, bsi, Np));
+      };
+      float local_sum;
+      if constexpr (ORDER) {
+        // the edges are on the step's critical path: the predictor runs while
+        // the first gathers are in flight
+        local_sum = split_walk<MATH, LPR>(s_cd + base, s_w + base, len, deg, sl, th, predictor,
+                                          gather);
+      } else {
+        const EdgeParams ep = predictor();
+        local_sum = split_walk<MATH, LPR>(s_cd + base, s_w + base, len, deg, sl, th, ep, gather);
+      }
       if (step > 0) {
-        cta_barrier();  // A
-        if (*reinterpret_cast<volatile int *>(&s_ok) == 0) break;
+        cta_barrier<kThreads>();  // A
+        if (stopped()) break;
         g = s_g;
       }
       // ---- integrate --------------------------------------------------------------
@@ -377,22 +427,25 @@ __global__ void __launch_bounds__(kGridThreads, 3) grid_kernel(const GridArgs a)
       const float2 part = split_warp_sum<LPR>(my_cos, my_sin);
       if (lane == 0) s_part[warp] = part;
       cur = nxt;
-      cta_barrier();  // B
+      cta_barrier<kThreads>();  // B
     }
   } else {
+    // what the two exchange warps do; one warp does both where there is no
+    // order warp
+    const bool sums = warp == 8, order = warp == 9 || !ORDER;
     const float inv_N = 1.0f / (float)N;
     float r = ns.r;
     // CTA 0 feeds an attached hub monitor
-    const bool observe = a.hubs && a.hubs->net == me.x && cta == 0;
+    const bool observe = order && a.hubs && a.hubs->net == me.x && cta == 0;
     HubWarp hub;
     if (observe) hub.open(a.hubs);
     // r and g after `steps` steps of this launch (lane 0); false after a timeout
     auto close_step = [&](int steps) -> bool {
-      float2 sums;
+      float2 s;
       if (!grid_sums<kBlocks>(wsum + ((steps - 1) & 3) * 8 * nblocks, nsum, nblocks, lane, a.wait,
-                              s_sum, &sums))
+                              s_sum, &s))
         return false;
-      r = order_parameter(sums.x, sums.y, inv_N);
+      r = order_parameter(s.x, s.y, inv_N);
       if (nd.ctrl) g = gain_controller(g, r, dt, nd);
       if (lane == 0) {
         s_g = g;
@@ -403,60 +456,58 @@ __global__ void __launch_bounds__(kGridThreads, 3) grid_kernel(const GridArgs a)
       }
       return true;
     };
-    // every CTA's phases of the first `steps` steps are in the ring
-    auto phases_of = [&](int steps) -> bool {
-      const bool ok = lane != 0 || grid_poll(bar, (unsigned)steps * G, a.wait);
-      return __all_sync(0xffffffffu, ok);
-    };
-    auto fail = [&]() {
-      if (lane == 0) {
-        *reinterpret_cast<volatile int *>(a.err) = 1;
-        *reinterpret_cast<volatile int *>(&s_ok) = 0;
-      }
-      __syncwarp();
-    };
-    bool ok = true;
+    bool ok = true, go_on = true;
+    float hub_phase = 0.0f;
     for (int step = 0; step < a.n_steps; ++step) {
-      float hub_phase = 0.0f;
       if (step > 0) {
         if (!a.early) {
-          ok = ok && phases_of(step);
-          cta_barrier();
+          if (order && !phases_of(step)) give_up();
+          cta_barrier<kThreads>();  // C
         }
-        ok = ok && close_step(step);
-        if (!ok) fail();
-        cta_barrier();  // A
-        if (!ok) break;
-        // a timeout here shows at the next barrier A
-        if (a.early) ok = phases_of(step);
-        if (observe && ok) hub_phase = __ldcg(ring + ring_pos(cur, hub.node, Np));
+        if (sums) {
+          if (ORDER) __nanosleep(kSumsSleep);
+          if (!close_step(step)) give_up();
+        }
+        cta_barrier<kThreads>();  // A
+        if (stopped()) {
+          go_on = false;
+          break;
+        }
+        // a timeout here is reported after B (see stopped)
+        if (order && a.early) ok = phases_of(step);
+        if (observe) hub_phase = __ldcg(ring + ring_pos(cur, hub.node, Np));
       }
       cur = (cur + 1 == bsi) ? 0 : cur + 1;
-      cta_barrier();  // B
-      grid_publish_part<R>(wsum, step, nblocks, nsum, cta, lane, s_part);
-      __syncwarp();
-      if (lane == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
-      if (observe && ok && step > 0) hub.observe(hub_phase);
+      cta_barrier<kThreads>();  // B
+      if (!ok) give_up();
+      if (sums) {
+        grid_publish_part<R>(wsum, step, nblocks, nsum, cta, lane, s_part);
+        __syncwarp();
+      }
+      if (order) arrive();
+      if (observe && step > 0) hub.observe(hub_phase);
     }
-    if (!ok) fail();
     // CTA 0 closes the last step
-    if (ok && a.n_steps > 0 && cta == 0) {
-      ok = close_step(a.n_steps) && phases_of(a.n_steps);
-      if (!ok) fail();
-      if (ok && observe) {
+    if (go_on && ok && a.n_steps > 0 && cta == 0) {
+      if (observe) {
+        if (!phases_of(a.n_steps)) give_up();
         hub.observe(__ldcg(ring + ring_pos(cur, hub.node, Np)));
         hub.close(a.n_steps);
       }
-      if (ok && lane == 0) {
-        NetState o = ns;
-        o.g = g;
-        o.r = r;
-        o.cur = cur;
-        o.rbuf = (int)((ns.rbuf + (long long)a.n_steps) % (nd.max_delay + 1));
-        o.t = ns.t + a.n_steps;
-        o.rpos = ns.rpos + a.n_steps;
-        o.ticket = 0u;
-        a.st[me.x] = o;
+      if (sums) {
+        if (!close_step(a.n_steps)) {
+          give_up();
+        } else if (lane == 0) {
+          NetState o = ns;
+          o.g = g;
+          o.r = r;
+          o.cur = cur;
+          o.rbuf = (int)((ns.rbuf + (long long)a.n_steps) % (nd.max_delay + 1));
+          o.t = ns.t + a.n_steps;
+          o.rpos = ns.rpos + a.n_steps;
+          o.ticket = 0u;
+          a.st[me.x] = o;
+        }
       }
     }
   }

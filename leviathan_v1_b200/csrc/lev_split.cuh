@@ -23,6 +23,8 @@
 // one bank.
 #pragma once
 
+#include <type_traits>
+
 #include "lev_kernels.cuh"
 
 namespace lev {
@@ -90,17 +92,24 @@ __device__ __forceinline__ void split_for_entries(const int *sloff, const int *s
 
 // The row's walk (csr_physics_kernel, leviathan_kernel.cu:126-165) over cd /
 // w, the slice's entries in shared memory; gather(word) returns the delayed
-// phase and keep(k, weight) sees the new weight of the row's entry k.  Returns
-// the row's coupling sum in all its lanes.  Entries past the
+// phase and keep(k, weight) sees the new weight of the row's entry k.  `params`
+// is the row's EdgeParams, or a function that returns them, run once while the
+// first chunk's gathers are in flight (it may do the row's predictor there).
+// Returns the row's coupling sum in all its lanes.  Entries past the
 // row's degree enter the sum as 0 * sin(0 - th): a zero, or a NaN in a row
 // whose phase is not finite and whose step sets it to 0 whatever the sum.
-template <int MATH, int LPR, int U, class Gather, class Keep>
+template <int MATH, int LPR, int U, class Params, class Gather, class Keep>
 __device__ __forceinline__ float split_walk_u(const uint32_t *cd, float *w, int len, int deg,
-                                              const SplitLane &sl, float th,
-                                              const EdgeParams &ep, Gather gather, Keep keep) {
+                                              const SplitLane &sl, float th, Params &params,
+                                              Gather gather, Keep keep) {
+  constexpr bool kGiven = std::is_same<Params, const EdgeParams>::value;
+  EdgeParams ep;
+  if constexpr (kGiven) ep = params;
   const unsigned mask = 0xffffffffu;
   const int lq = (sl.l + sl.q) & 31;
   float local_sum = 0.0f;
+  if constexpr (!kGiven)
+    if (len == 0) params();
   for (int kb = 0; kb < len; kb += LPR * U) {  // len: the slice's, warp-uniform
     const int k0 = kb + U * sl.q;
     const int at = 32 * k0 + lq;
@@ -114,6 +123,8 @@ __device__ __forceinline__ float split_walk_u(const uint32_t *cd, float *w, int 
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) dj[u] = (k0 + u < deg) ? gather(p[u]) : 0.0f;
+    if constexpr (!kGiven)
+      if (kb == 0) ep = params();
 #pragma unroll
     for (int u = 0; u < U; ++u) dj[u] -= th;
     float sn[U], cs[U];
@@ -136,26 +147,26 @@ __device__ __forceinline__ float split_walk_u(const uint32_t *cd, float *w, int 
   return local_sum;
 }
 
-template <int MATH, int LPR, class Gather, class Keep>
+template <int MATH, int LPR, class Params, class Gather, class Keep>
 __device__ __forceinline__ float split_walk(const uint32_t *cd, float *w, int len, int deg,
-                                            const SplitLane &sl, float th, const EdgeParams &ep,
+                                            const SplitLane &sl, float th, Params &params,
                                             Gather gather, Keep keep) {
   switch (split_unroll<LPR>(len)) {  // warp-uniform
-    case 1: return split_walk_u<MATH, LPR, 1>(cd, w, len, deg, sl, th, ep, gather, keep);
-    case 2: return split_walk_u<MATH, LPR, 2>(cd, w, len, deg, sl, th, ep, gather, keep);
-    case 3: return split_walk_u<MATH, LPR, 3>(cd, w, len, deg, sl, th, ep, gather, keep);
-    case 4: return split_walk_u<MATH, LPR, 4>(cd, w, len, deg, sl, th, ep, gather, keep);
-    case 5: return split_walk_u<MATH, LPR, 5>(cd, w, len, deg, sl, th, ep, gather, keep);
-    case 6: return split_walk_u<MATH, LPR, 6>(cd, w, len, deg, sl, th, ep, gather, keep);
-    case 7: return split_walk_u<MATH, LPR, 7>(cd, w, len, deg, sl, th, ep, gather, keep);
-    default: return split_walk_u<MATH, LPR, 8>(cd, w, len, deg, sl, th, ep, gather, keep);
+    case 1: return split_walk_u<MATH, LPR, 1>(cd, w, len, deg, sl, th, params, gather, keep);
+    case 2: return split_walk_u<MATH, LPR, 2>(cd, w, len, deg, sl, th, params, gather, keep);
+    case 3: return split_walk_u<MATH, LPR, 3>(cd, w, len, deg, sl, th, params, gather, keep);
+    case 4: return split_walk_u<MATH, LPR, 4>(cd, w, len, deg, sl, th, params, gather, keep);
+    case 5: return split_walk_u<MATH, LPR, 5>(cd, w, len, deg, sl, th, params, gather, keep);
+    case 6: return split_walk_u<MATH, LPR, 6>(cd, w, len, deg, sl, th, params, gather, keep);
+    case 7: return split_walk_u<MATH, LPR, 7>(cd, w, len, deg, sl, th, params, gather, keep);
+    default: return split_walk_u<MATH, LPR, 8>(cd, w, len, deg, sl, th, params, gather, keep);
   }
 }
-template <int MATH, int LPR, class Gather>
+template <int MATH, int LPR, class Params, class Gather>
 __device__ __forceinline__ float split_walk(const uint32_t *cd, float *w, int len, int deg,
-                                            const SplitLane &sl, float th, const EdgeParams &ep,
+                                            const SplitLane &sl, float th, Params &params,
                                             Gather gather) {
-  return split_walk<MATH, LPR>(cd, w, len, deg, sl, th, ep, gather, [](int, float) {});
+  return split_walk<MATH, LPR>(cd, w, len, deg, sl, th, params, gather, [](int, float) {});
 }
 
 // The warp's part of the 32-row tree: rows 16 down to LPR apart; lane 0 holds
