@@ -261,10 +261,12 @@ int lev_set_variant(LevEngine *h, int32_t c, int32_t v);
  * edges, node state and delay ring fit in the shared memory of one
  * thread-block cluster (<= 16 CTAs of <= 1024 rows) is stepped by
  * lev_step_n / lev_step_n_async with one launch per block of steps, delayed
- * phases of other CTAs' nodes read through distributed shared memory, one
- * cluster barrier per step.  Results are bitwise those of the per-step
- * kernel.  Eligibility is decided at creation; lev_set_cluster_mode(h, 0)
- * forces the per-step kernel. */
+ * phases of other CTAs' nodes and the other CTAs' sums exchanged through
+ * distributed shared memory.  Results are bitwise those of the per-step
+ * kernel.  With up to 128 rows per CTA the waits are bounded
+ * (lev_set_grid_wait); a timeout makes lev_step_n / lev_sync return
+ * LEV_ERR_CUDA and disables the path.  Eligibility is decided at creation;
+ * lev_set_cluster_mode(h, 0) forbids the path. */
 int lev_cluster_info(const LevEngine *h, int32_t *eligible, int32_t *enabled,
                      int32_t *ctas, int32_t *rows_per_cta, int64_t *smem_bytes);
 int lev_set_cluster_mode(LevEngine *h, int32_t enabled);
@@ -274,8 +276,8 @@ int lev_set_cluster_mode(LevEngine *h, int32_t enabled);
  * shared memory) can all be resident at once is stepped by lev_step_n /
  * lev_step_n_async with one cooperative launch per block of steps; the delay
  * ring stays in global memory (L2) and the CTAs of a network exchange their
- * sums and arrivals every step.  The waits are bounded; a timeout makes lev_step_n / lev_sync return
- * LEV_ERR_CUDA and disables the path.  Results are bitwise those of the
+ * sums and arrivals every step.  The waits are bounded; a timeout makes
+ * lev_step_n / lev_sync return LEV_ERR_CUDA and disables the path.  Results are bitwise those of the
  * per-step kernel.  The cluster path takes precedence when both are enabled.
  * lev_grid_info: enabled = eligible and allowed (the path step blocks use;
  * 0 after a timeout); rows_per_cta in use; eligible_rows_mask = OR of the
@@ -285,11 +287,11 @@ int lev_grid_info(const LevEngine *h, int32_t *eligible, int32_t *enabled, int32
                   int32_t *rows_per_cta, int64_t *smem_bytes, int32_t *eligible_rows_mask);
 int lev_set_grid_mode(LevEngine *h, int32_t enabled, int32_t rows_per_cta);
 
-/* Bound of the grid-barrier waits of the grid-resident step blocks (no
+/* Bound of the waits of the grid- and cluster-resident step blocks (no
  * reference counterpart).  limit_ns (1 us .. 60 s, default 2 s): longest
  * time one wait may take before the kernel gives up, sets the error flag and
  * returns.  extra_arrivals: 0 in normal use; a positive value makes every
- * wait expect that many more arrivals than the grid makes, so the block's
+ * wait expect that many more arrivals than the CTAs make, so the block's
  * first wait runs out -- for tests of the timeout path, which then neither
  * faults nor hangs the GPU.  After a timeout at the first wait every CTA has
  * done the block's first step into its shared memory and one ring slot that
@@ -305,8 +307,8 @@ int lev_set_grid_wait(LevEngine *h, uint64_t limit_ns, uint32_t extra_arrivals);
  * g(t+1) and so the global r(t+1), in a short node-only launch.  The
  * edge streams then leave HBM once per two steps.  `deep` variants keep two
  * groups of edges in flight per lane.
- * Results are bitwise those of one step per launch.  lev_autotune times the pair variants of each
- * degree class against its best one-step variant and keeps pairs only where
+ * Results are bitwise those of one step per launch.  lev_autotune times the
+ * pair variants of each degree class against its best one-step variant and keeps pairs only where
  * they are faster; pair_variant -1 means one step per launch for that class.
  * lev_step (single steps, and the reference ABI) uses the same pair launches
  * as speculative single steps: the call that starts a pair leaves the state
@@ -390,10 +392,10 @@ int lev_adj_set_reservoir_grads(LevAdjoint *a, const float *dLdy,
                                 float *grad_rb);
 
 /* Grid-resident segments (no reference counterpart): for a single network
- * whose CTAs (64, 128 or 256 rows, four lanes per row) can all be resident
- * at once, each checkpoint segment is one cooperative launch forward (with
- * the recording of the backward recompute) and one backward, with a bounded
- * grid barrier per step; a timeout makes lev_adj_forward / lev_adj_backward
+ * whose CTAs (64, 128 or 256 rows; four, two or one lanes per row) can all be
+ * resident at once, each checkpoint segment is one cooperative launch forward
+ * (with the recording of the backward recompute) and one backward, with
+ * bounded waits for the other CTAs every step; a timeout makes lev_adj_forward / lev_adj_backward
  * return LEV_ERR_CUDA.  Not used with the reservoir readout (ra, rb).  The
  * forward trajectory is bitwise that of the per-step kernels; gradients
  * agree to rounding (sums over a row's edges and over CTAs in another
@@ -589,8 +591,8 @@ int lev_gen_ws(int32_t N, int32_t k, double p, uint64_t seed,
  *                    hub_idx[num_hubs] node indices; S = 2^num_hubs states.
  * lev_attach_hubs    every later step of network `net` of h is observed
  *                    (m = NULL detaches).  While attached, the cluster-
- *                    resident path is not used and lev_hubs_accumulate is
- *                    refused.
+ *                    resident path is used up to 128 rows per CTA only and
+ *                    lev_hubs_accumulate is refused.
  * lev_hubs_accumulate replaces phi_accumulate (:289-298): one observation
  *                    of theta_dev (device pointer; every hub index must be
  *                    inside it) on `stream` (NULL: the monitor's own stream).

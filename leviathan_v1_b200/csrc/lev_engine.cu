@@ -954,8 +954,8 @@ void setup_cluster(LevEngine *h, const std::vector<int> &sl_len) {
     h->cluster_edge_cap = (int)cap;
     h->cluster_smem = smem;
     // up to 128 rows per CTA (N = 2048 on 16 CTAs) the cluster kernel beats the
-    // grid-resident one (N = 1000: 2.0 against 2.5 us per step), above it does
-    // not (N = 4096, k = 32: 8.1 against 2.7); lev_autotune times both
+    // grid-resident one (N = 1000, k = 20: 1.5 against 2.1 us per step), above it does
+    // not (N = 3000, k = 8: 4.4 against 2.1); lev_autotune times both
     h->use_cluster = R <= 128;
     return;
   }

@@ -1,0 +1,322 @@
+"""The step paths that keep a network resident (cluster, grid, adjoint grid
+segments) and the launches around them, at the sizes where their splits change:
+edges of tiles, CTAs and launch rules, ragged and edgeless networks, zero
+delays, blocks longer than one launch (GPU).
+
+Forward results, hub counts and weight conversions are compared with the
+per-step kernels bit for bit.  Gradients are compared at a relative difference
+of 1e-5: between paths only the order of the sums over edges and of the
+float32 scatters differs (some tens of terms of one sign pattern each, so a few
+1e-7 per sum).
+"""
+
+import numpy as np
+import pytest
+import torch
+
+from conftest import has_gpu
+from leviathan_v1_b200 import BatchEngine, HubTransitions, LeviathanEngine, _lib
+from leviathan_v1_b200.adjoint import Adjoint
+from leviathan_v1_b200.graphs import Network, init_state, make_network
+
+pytestmark = pytest.mark.gpu
+
+DT = 0.05
+REL = 1e-5
+
+
+@pytest.fixture(scope="module", autouse=True)
+def _need_gpu():
+    if not has_gpu():
+        pytest.fail("GPU tests need a CUDA device")
+
+
+def _state(e):
+    th_hat, om_hat = e.get_predictor()
+    out = dict(theta=e.get_all_theta(), w=e.get_weights(), thh=th_hat, omh=om_hat)
+    for k in range(e.num_nets):
+        ring, bi = e.get_ring(k)
+        out[f"ring{k}"], out[f"bi{k}"] = ring, np.array(bi)
+        out[f"g{k}"] = np.array(e._get_gain(k))
+        out[f"t{k}"] = np.array(e.step_count(k))
+    return out
+
+
+def _same(a, b, what=""):
+    for k, v in b.items():
+        np.testing.assert_array_equal(a[k], v, err_msg=f"{what}{k}")
+
+
+def _per_step(e):
+    e.set_cluster_mode(False)
+    e.set_grid_mode(False)
+    e.set_pair_mode(False)
+    return e
+
+
+def _from_degrees(deg, max_delay, seed):
+    """Directed network with the given in-degrees, sources drawn at random."""
+    rng = np.random.default_rng(seed)
+    n = len(deg)
+    rp = np.concatenate([[0], np.cumsum(deg)]).astype(np.int32)
+    col = np.concatenate([np.sort(rng.choice(n, d, replace=False)) for d in deg]
+                         + [np.zeros(0, int)]).astype(np.int32)
+    st = init_state(rp, max_delay, seed)
+    return Network(n, max_delay, rp, col, st["delays"], st["weights"], st["theta"],
+                   st["theta_hat"], st["omega"])
+
+
+def _uneven(seed, zero):
+    """Networks of 1 to 2,049 rows: one row, a part of a warp, a tile and one
+    row, without edges, with rows of 0 to 90 entries, and one zero delay or
+    none."""
+    rng = np.random.default_rng(seed)
+    lo = 0 if zero else 1
+    return [_from_degrees(np.zeros(1, int), 3, seed),
+            make_network(33, 4, 0.1, 6, seed=seed + 1, delay_lo=1),
+            make_network(257, 8, 0.1, 20, seed=seed + 2, delay_lo=1),
+            _from_degrees(np.zeros(300, int), 5, seed + 3),
+            _from_degrees(np.where(np.arange(700) % 97 == 0, 90, rng.integers(0, 12, 700)),
+                          17, seed + 4),
+            make_network(2049, 16, 0.1, 9, seed=seed + 5, delay_lo=lo)]
+
+
+@pytest.mark.parametrize("mode,zero", [("reference", False), ("accurate", False),
+                                       ("reference", True)])
+def test_batch_on_the_grid_kernel(mode, zero):
+    nets = [n.as_dict() for n in _uneven(5, zero)]
+    params = [dict(g=0.3 * (i + 1), gain_controller=i % 2) for i in range(len(nets))]
+    ref = _per_step(BatchEngine(nets, params=params, math_mode=mode))
+    want_r = np.concatenate([ref.step_n(DT, 5), ref.step_n(DT, 70)])
+    want = _state(ref)
+    ref.close()
+    e = BatchEngine(nets, params=params, math_mode=mode)
+    rows = e.grid_info()["eligible_rows"]
+    e.close()
+    assert rows
+    for R in rows:
+        e = BatchEngine(nets, params=params, math_mode=mode)
+        e.set_grid_mode(True, R)
+        assert e.grid_info()["enabled"]
+        r = np.concatenate([e.step_n(DT, 5), e.step_n(DT, 70)])
+        np.testing.assert_array_equal(r, want_r, err_msg=f"R={R}")
+        _same(_state(e), want, f"R={R}: ")
+        e.close()
+
+
+# one CTA; two CTAs per SM exactly (148 SMs) and one CTA more, where the exchange
+# goes from two warps to one
+@pytest.mark.parametrize("N,k,R", [(33, 4, 64), (129, 30, 128), (18_944, 8, 64), (18_945, 8, 64),
+                                   (37_888, 4, 128), (37_889, 4, 128)])
+def test_grid_kernel_at_the_edges_of_its_split(N, k, R):
+    net = make_network(N, k, 0.1, 11, seed=N, delay_lo=1)
+    ref = _per_step(LeviathanEngine(*net.engine_args()))
+    want_r = ref.step_n(DT, 40)
+    want = _state(ref)
+    ref.close()
+    e = LeviathanEngine(*net.engine_args())
+    if R not in e.grid_info()["eligible_rows"]:
+        e.close()
+        pytest.skip("these rows per CTA do not fit this device")
+    e.set_cluster_mode(False)
+    e.set_grid_mode(True, R)
+    np.testing.assert_array_equal(e.step_n(DT, 40), want_r)
+    _same(_state(e), want)
+    e.close()
+
+
+@pytest.mark.parametrize("N,R,lo", [(1000, 0, 1), (1000, 0, 0), (5000, 64, 1), (5000, 256, 1),
+                                    (5000, 64, 0), (5000, 256, 0)])
+def test_hubs_on_resident_paths(N, R, lo):
+    """R = 0: the cluster kernel."""
+    net = make_network(N, 12, 0.1, 20, seed=N + R + lo, delay_lo=lo)
+    hubs = [0, N - 1, 31, 32, 255, 256, N // 2]
+    out = []
+    for resident in (False, True):
+        e = LeviathanEngine(*net.engine_args())
+        m = HubTransitions(hubs)
+        m.attach(e)
+        if resident:
+            e.set_cluster_mode(R == 0)
+            e.set_grid_mode(R > 0, R)
+            assert R == 0 or e.grid_info()["enabled"]
+        else:
+            _per_step(e)
+        r = np.concatenate([e.step_n(DT, 37), [e.step(DT)], e.step_n(DT, 1), e.step_n(DT, 90)])
+        out.append((r, *m.read(), e.get_theta()))
+        m.close()
+        e.close()
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
+    assert out[1][4] == 129  # every step observed
+
+
+def test_hubs_of_one_network_of_a_resident_batch():
+    nets = [n.as_dict() for n in _uneven(9, False)]
+    out = []
+    for resident in (False, True):
+        e = BatchEngine(nets)
+        m = HubTransitions([0, 699, 255, 256])
+        m.attach(e, net=4)
+        if resident:
+            e.set_grid_mode(True)
+            assert e.grid_info()["enabled"]
+        else:
+            _per_step(e)
+        out.append((e.step_n(DT, 60), *m.read()))
+        m.close()
+        e.close()
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("lo", [1, 0])
+def test_cluster_wait_timeout_is_reported(lo):
+    """A wait that runs out (20 us, one arrival more than ever comes) ends the
+    launch with an error; the engine goes on with per-step launches from the
+    state before."""
+    net = make_network(1000, 20, 0.1, 30, seed=3, delay_lo=lo)
+    ref = _per_step(LeviathanEngine(*net.engine_args()))
+    want_r = np.concatenate([ref.step_n(DT, 7), ref.step_n(DT, 40)])
+    want = _state(ref)
+    ref.close()
+    e = LeviathanEngine(*net.engine_args())
+    e.set_cluster_mode(True)
+    np.testing.assert_array_equal(e.step_n(DT, 7), want_r[:7])
+    e.set_grid_wait(20_000, extra_arrivals=1)
+    with pytest.raises(_lib.LevError) as exc:
+        e.step_n(DT, 40)
+    assert exc.value.code == _lib.LEV_ERR_CUDA and "timed out" in str(exc.value)
+    e.set_grid_wait()
+    np.testing.assert_array_equal(e.step_n(DT, 40), want_r[7:])
+    _same(_state(e), want)
+    e.close()
+
+
+@pytest.mark.parametrize("N,k,cluster", [(300, 8, True), (3000, 8, False)])
+def test_blocks_longer_than_one_resident_launch(N, k, cluster):
+    """2,100 steps: more than the 2,048 one launch takes."""
+    net = make_network(N, k, 0.1, 12, seed=N, delay_lo=1)
+    ref = LeviathanEngine(*net.engine_args())
+    ref.set_cluster_mode(False)
+    ref.set_grid_mode(False)
+    want_r = ref.step_n(DT, 2100)
+    want = _state(ref)
+    ref.close()
+    e = LeviathanEngine(*net.engine_args())
+    e.set_cluster_mode(cluster)
+    e.set_grid_mode(not cluster)
+    np.testing.assert_array_equal(e.step_n(DT, 2100), want_r)
+    _same(_state(e), want)
+    e.close()
+
+
+def test_engines_of_different_sizes_share_the_kernels():
+    """A smaller engine made later leaves the larger one's launches valid."""
+    nets = [make_network(16_000, 20, 0.1, 30, seed=1, delay_lo=1),
+            make_network(1000, 20, 0.1, 30, seed=2, delay_lo=1),
+            make_network(200, 4, 0.1, 5, seed=3, delay_lo=1)]
+    for cluster in (False, True):
+        es = [LeviathanEngine(*n.engine_args()) for n in nets]
+        for e, n in zip(es, nets):
+            if cluster and not e.cluster_info()["eligible"]:
+                continue
+            e.set_cluster_mode(cluster)
+            ref = _per_step(LeviathanEngine(*n.engine_args()))
+            np.testing.assert_array_equal(e.step_n(DT, 20), ref.step_n(DT, 20))
+            ref.close()
+        for e in es:
+            e.close()
+
+
+# tiles of 256 rows at the limits of the dependent launches: one, 111 | 112,
+# 444 | 445
+@pytest.mark.parametrize("N", [200, 28_416, 28_417, 113_664, 113_665])
+def test_pair_chain_at_the_limits_of_its_launch_rule(N):
+    net = make_network(N, 4, 0.1, 7, seed=N, delay_lo=1)
+    ref = _per_step(LeviathanEngine(*net.engine_args()))
+    want_r = ref.step_n(DT, 21)
+    want = _state(ref)
+    ref.close()
+    e = LeviathanEngine(*net.engine_args())
+    e.set_cluster_mode(False)
+    e.set_grid_mode(False)
+    assert any(c["enabled"] for c in e.pair_info())
+    np.testing.assert_array_equal(e.step_n(DT, 21), want_r)
+    _same(_state(e), want)
+    e.close()
+
+
+@pytest.mark.parametrize("batch", [False, True])
+def test_weights_round_trip(batch):
+    nets = _uneven(13, True) if batch else _uneven(13, True)[4:5]
+    e = BatchEngine([n.as_dict() for n in nets])
+    np.testing.assert_array_equal(e.get_weights(), np.concatenate([n.weights for n in nets]))
+    w = np.random.default_rng(0).random(sum(len(n.weights) for n in nets)).astype(np.float32)
+    e.reset_weights(w)
+    np.testing.assert_array_equal(e.get_weights(), w)
+    e.close()
+
+
+def _rel(a, b):
+    a, b = a.double().cpu().numpy().ravel(), b.double().cpu().numpy().ravel()
+    return np.linalg.norm(a - b) / max(np.linalg.norm(b), 1e-30)
+
+
+# one segment; a last segment of one step; several and a part; 2,200 rows take the
+# split step kernels, 40,000 (over 148 tiles) the one-lane ones
+@pytest.mark.parametrize("N,T,segment", [(2200, 30, 50), (2200, 51, 25), (2200, 60, 25),
+                                         (40_000, 21, 10), (40_000, 24, 10)])
+def test_gradients_from_the_recorded_last_segment(N, T, segment):
+    """The forward pass keeps its last segment's records; a second backward
+    pass, and one on another path than the forward pass, recompute them."""
+    net = make_network(N, 8, 0.1, 9, seed=N + T, delay_lo=1)
+    om, w0 = (torch.tensor(x, device="cuda") for x in (net.omega, net.weights))
+    K = torch.full((1,), 1.5, device="cuda")
+    dr = torch.linspace(-1, 1, T, device="cuda")[:, None].contiguous()
+
+    def run(forward_grid, backward_grid, twice=False):
+        eng = LeviathanEngine(*net.engine_args())
+        adj = Adjoint(eng, segment=segment, max_steps=T)
+        adj.set_grid_mode(forward_grid)
+        r = adj.forward(om, w0, K, T, DT)
+        adj.set_grid_mode(backward_grid)
+        out = [adj.backward(dr)]
+        if twice:
+            out.append(adj.backward(dr))
+        adj.close()
+        eng.close()
+        return r, out
+
+    r_ref, (_, ref) = run(False, False, twice=True)  # recomputed throughout
+    for f, b in [(False, False), (True, True), (True, False), (False, True)]:
+        r, out = run(f, b, twice=f and b)
+        assert torch.equal(r, r_ref)
+        for g in out:
+            for k in ("omega", "w0", "K"):
+                assert _rel(g[k], ref[k]) <= REL, (f, b, k)
+
+
+@pytest.mark.parametrize("N,k,lo", [(65, 4, 1), (2049, 30, 0), (2049, 30, 1)])
+def test_adjoint_grid_segments_at_ragged_sizes(N, k, lo):
+    net = make_network(N, k, 0.1, 6, seed=N + lo, delay_lo=lo)
+    om, w0 = (torch.tensor(x, device="cuda") for x in (net.omega, net.weights))
+    K = torch.full((1,), 1.5, device="cuda")
+    T = 27
+    dr = torch.linspace(-1, 1, T, device="cuda")[:, None].contiguous()
+    eng = LeviathanEngine(*net.engine_args())
+    adj = Adjoint(eng, segment=10, max_steps=T)
+    rows = adj.grid_info()["eligible_rows"]
+    assert rows
+    adj.set_grid_mode(False)
+    r_ref, ref = adj.forward(om, w0, K, T, DT), adj.backward(dr)
+    for R in rows:
+        for paired in (False, True):
+            adj.set_grid_mode(True, R)
+            adj.set_grid_pairing(paired)
+            assert torch.equal(adj.forward(om, w0, K, T, DT), r_ref)
+            g = adj.backward(dr)
+            for name in ("omega", "w0", "K"):
+                assert _rel(g[name], ref[name]) <= REL, (R, paired, name)
+    adj.close()
+    eng.close()
