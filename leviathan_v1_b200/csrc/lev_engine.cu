@@ -242,7 +242,7 @@ struct LevEngine {
   bool grid_R_ok[3] = {false, false, false};  // R = 64, 128, 256
   int grid_cap[3] = {0, 0, 0};                // SELL entries per CTA
   size_t grid_smem_R[3] = {0, 0, 0};
-  bool grid_order[3] = {false, false, false};  // with an order warp
+  int grid_minb[3] = {3, 3, 3};  // CTAs per SM the kernel is compiled for
   int grid_max_tiles = 0;     // tiles of the largest network
   int grid_map_off[3] = {0, 0, 0};            // first entry of each choice in d_gmap
   std::vector<int2> h_gmap;   // batches: (network, CTA) per CTA
@@ -964,16 +964,15 @@ void setup_cluster(LevEngine *h, const std::vector<int> &sl_len) {
 // Grid kernel for R rows per CTA (64, 128, 256).
 using GridFn = void (*)(GridArgs);
 constexpr int kGridRs[3] = {64, 128, 256};
-template <bool ORDER>
+template <int MINB>
 GridFn grid_fn_of(int R, int math_mode) {
   const bool acc = math_mode == LEV_MATH_ACCURATE;
-  if (R == 64) return acc ? grid_kernel<1, 64, ORDER> : grid_kernel<0, 64, ORDER>;
-  return acc ? grid_kernel<1, 128, ORDER> : grid_kernel<0, 128, ORDER>;
+  if (R == 64) return acc ? grid_kernel<1, 64, MINB> : grid_kernel<0, 64, MINB>;
+  if (R == 128) return acc ? grid_kernel<1, 128, MINB> : grid_kernel<0, 128, MINB>;
+  return acc ? grid_kernel<1, 256, MINB> : grid_kernel<0, 256, MINB>;
 }
-GridFn grid_fn(int R, int math_mode, bool order) {
-  if (R == 256)
-    return math_mode == LEV_MATH_ACCURATE ? grid_kernel<1, 256, false> : grid_kernel<0, 256, false>;
-  return order ? grid_fn_of<true>(R, math_mode) : grid_fn_of<false>(R, math_mode);
+GridFn grid_fn(int R, int math_mode, int minb) {
+  return minb == 2 ? grid_fn_of<2>(R, math_mode) : grid_fn_of<3>(R, math_mode);
 }
 inline int grid_r_index(int R) { return R == 64 ? 0 : (R == 128 ? 1 : 2); }
 
@@ -1022,7 +1021,7 @@ int launch_grid(LevEngine *h, float dt, int len) {
   ga.dt = dt;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid_ctas(h, R));
-  cfg.blockDim = dim3(grid_threads(h->grid_order[ri]));
+  cfg.blockDim = dim3(grid_threads(R, h->grid_minb[ri]));
   cfg.dynamicSmemBytes = h->grid_smem_R[ri];
   cfg.stream = h->stream;
   cudaLaunchAttribute attr[1];
@@ -1030,7 +1029,7 @@ int launch_grid(LevEngine *h, float dt, int len) {
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  LEV_TRY_CUDA(cudaLaunchKernelEx(&cfg, grid_fn(R, h->math_mode, h->grid_order[ri]), ga));
+  LEV_TRY_CUDA(cudaLaunchKernelEx(&cfg, grid_fn(R, h->math_mode, h->grid_minb[ri]), ga));
   return LEV_OK;
 }
 
@@ -1071,7 +1070,7 @@ int setup_grid(LevEngine *h, const std::vector<int> &sl_len) {
     for (long long s = 0; s < ns; ++s) sum += sl_len[d.slice_base + s];
     if (ns) mean_len = std::max(mean_len, sum / (double)ns);
   }
-  bool R_set = false;  // the rows-per-CTA choice below is made
+  bool R_set = false, use = false;  // the rows-per-CTA choice below is made; step blocks use it
   for (int ri = 0; ri < 3; ++ri) {
     const int R = kGridRs[ri];
     const long long C = grid_ctas(h, R);
@@ -1091,23 +1090,20 @@ int setup_grid(LevEngine *h, const std::vector<int> &sl_len) {
     const size_t smem = (R < 256 ? sizeof(float2) * 8 * (size_t)h->grid_max_tiles : 0) +
                         sizeof(int) * 2 * (R / 32) + 8 * (size_t)cap;
     if (smem + 1024 > (size_t)max_smem) continue;
-    // With an order warp if every CTA is then resident, else without; with one
-    // lane per row (R = 256) never: us per step with / without at N = 5*10^4,
-    // k = 8 4.50 / 3.27, at N = 7.5*10^4, k = 32 8.75 / 8.16, and for R = 64,
-    // 128 at N = 6,000, k = 20 2.11 / 2.37, at N = 18,900 2.85 / 3.17.
+    // compiled for two CTAs per SM if every CTA is then resident, else for three
     bool ok = false;
-    for (int order = R < 256 ? 1 : 0; order >= 0 && !ok; --order) {
+    for (int minb = 2; minb <= 3 && !ok; ++minb) {
       ok = true;
       for (int m = 0; m < 2 && ok; ++m) {
         const void *fn = reinterpret_cast<const void *>(
-            grid_fn(R, m ? LEV_MATH_ACCURATE : LEV_MATH_REFERENCE, order != 0));
+            grid_fn(R, m ? LEV_MATH_ACCURATE : LEV_MATH_REFERENCE, minb));
         int per_sm = 0;
         ok = allow_smem(fn, smem) &&
-             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, grid_threads(order != 0),
+             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, grid_threads(R, minb),
                                                            smem) == cudaSuccess &&
              (long long)per_sm * sms >= C;
       }
-      h->grid_order[ri] = order != 0;
+      h->grid_minb[ri] = minb;
     }
     cudaGetLastError();  // clear a refused attribute, if any
     if (!ok) continue;
@@ -1118,13 +1114,18 @@ int setup_grid(LevEngine *h, const std::vector<int> &sl_len) {
     // The choice of an engine that has not been tuned: long rows (more than 26
     // entries) want many lanes per row, the smallest R; short ones the smallest
     // R with little more than one CTA per SM, else the largest.  Measured, us
-    // per step at R = 64 / 128 / 256: N = 10^4, k = 20 2.53 / 2.70 / 3.95;
-    // 1.4*10^4 2.83 / 2.68 / 3.89; 2.8*10^4 4.01 / 3.99 / 3.84; k = 32 4.50 /
-    // 4.70 / 6.93; 5*10^4, k = 8 - / 5.19 / 3.30.
+    // per step at R = 64 / 128 / 256: N = 10^4, k = 20 2.43 / 2.61 / 3.81;
+    // 1.4*10^4 2.78 / 2.64 / 4.0; 2.8*10^4 3.98 / 3.59 / 3.78; k = 32 4.49 /
+    // 4.78 / 4.42; 3.78*10^4, k = 32 - / 4.72 / 5.05; 5*10^4, k = 8 - / 5.13 / 3.04.
+    // Three CTAs per SM whose edges leave the gathers less than 60 KB of L1 (of
+    // 256) are no choice: k = 28, N = 8*10^4 (67 KB per CTA) 17.9 against 15.0
+    // for the per-step launches, k = 24, 1.1*10^5 (58 KB) 9.6 against 14.3.
     if (R_set) continue;
     h->grid_R = R;
-    R_set = mean_len > 26.0 || 4 * C <= 5LL * sms;
+    use = h->grid_minb[ri] == 2 || 3 * (smem + 1024) <= 196 * 1024;
+    R_set = use && (mean_len > 26.0 || 4 * C <= 5LL * sms);
   }
+  h->use_grid = use;
   if (!h->grid_ok) return LEV_OK;
   if (h->num_nets > 1) {
     // CTAs of a network side by side, the largest networks first

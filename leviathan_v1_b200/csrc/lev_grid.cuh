@@ -214,9 +214,11 @@ constexpr unsigned kSumsSleep = 400;  // ns, of a sums warp before its first pol
 constexpr int kGridBarPitch = 32;  // arrival counters of two networks share no 128-byte line
 constexpr int kGridThreads = 256 + 32;  // eight warps on rows, one for the other CTAs
 
-// Threads of grid_kernel: with an order warp, two for the other CTAs.
-__host__ __device__ constexpr int grid_threads(bool order_warp) {
-  return order_warp ? 256 + 64 : kGridThreads;
+// grid_kernel for at most `minb` CTAs per SM: two (with an order warp where a
+// row has several lanes) or three.
+__host__ __device__ constexpr bool grid_order_warp(int R, int minb) { return minb == 2 && R < 256; }
+__host__ __device__ constexpr int grid_threads(int R, int minb) {
+  return grid_order_warp(R, minb) ? 256 + 64 : kGridThreads;
 }
 
 // Barrier of a CTA whose warps run different code.
@@ -266,8 +268,12 @@ __device__ __forceinline__ void grid_publish_part(float2 *wsum, int step, int nb
 // for the fence, which only the ring phases need.  The sums warp publishes and
 // collects the sums, the order warp pays the fence, arrives and waits for the
 // others' arrivals.  With R = 256 and in grids of more than two CTAs per SM
-// (ORDER = false) one warp does both, in that order: there the rows' gathers
-// bound the step, and 72 registers keep three CTAs per SM.
+// (MINB = 3, 72 registers) one warp does both, in that order: there the rows'
+// gathers bound the step.  With R = 256 and MINB = 2 a lane has up to twelve
+// entries in flight instead of eight and 96 registers: at 72 the long rows'
+// loads come one after the other.  us per step, MINB = 3 / 2: N = 3,000, k = 32
+// 6.9 / 4.5; 37,800, k = 32 7.1 / 5.1; 5*10^4, k = 8 3.6 / 3.2; 5*10^4, k = 20 5.6 /
+// 5.3; 64 networks of 500 to 2,000 rows, k up to 32 12.0 / 7.0.
 //
 // Order of one step s:
 //   edge warps            | sums warp                 | order warp
@@ -295,11 +301,12 @@ __device__ __forceinline__ void grid_publish_part(float2 *wsum, int step, int nb
 // exchange warp / two: N = 6,000, k = 20 (R = 64) - / 2.37 / 2.11; N = 10^4 (64)
 // 3.5 / 2.62 / 2.46; N = 18,900 (128) - / 3.17 / 2.85; N = 10^5 (256) - / 7.6 /
 // 8.8 (two steps per launch: 13.1).
-template <int MATH, int R, bool ORDER>
-__global__ void __launch_bounds__(grid_threads(ORDER), ORDER ? 2 : 3)
-    grid_kernel(const GridArgs a) {
+template <int MATH, int R, int MINB>
+__global__ void __launch_bounds__(grid_threads(R, MINB), MINB) grid_kernel(const GridArgs a) {
   constexpr int LPR = 256 / R;
-  constexpr int kThreads = grid_threads(ORDER);
+  constexpr bool ORDER = grid_order_warp(R, MINB);
+  constexpr int kThreads = grid_threads(R, MINB);
+  constexpr int kUM = LPR == 1 && MINB == 2 ? 12 : 8;  // entries of a lane in flight
   constexpr int nslices = R / 32;
   constexpr bool kBlocks = R == 256;  // a CTA closes its 256-node block itself
   extern __shared__ __align__(16) unsigned char smem[];
@@ -404,7 +411,8 @@ __global__ void __launch_bounds__(grid_threads(ORDER), ORDER ? 2 : 3)
                                           gather);
       } else {
         const EdgeParams ep = predictor();
-        local_sum = split_walk<MATH, LPR>(s_cd + base, s_w + base, len, deg, sl, th, ep, gather);
+        local_sum =
+            split_walk<MATH, LPR, kUM>(s_cd + base, s_w + base, len, deg, sl, th, ep, gather);
       }
       if (step > 0) {
         cta_barrier<kThreads>();  // A

@@ -48,11 +48,13 @@ __device__ __forceinline__ unsigned long long global_ns() {
 }
 
 // Entries per lane and chunk for slices of `len` entries per row: as few
-// chunks as entries of at most 8 per lane allow, of equal size (an empty
-// entry costs the instructions of a full one).
-template <int LPR>
+// chunks as entries of at most UM per lane allow, of equal size (an empty
+// entry costs the instructions of a full one).  With one lane per row the
+// order in shared memory does not depend on it.
+template <int LPR, int UM = 8>
 __device__ __forceinline__ int split_unroll(int len) {
-  const int chunks = max((len + 8 * LPR - 1) / (8 * LPR), 1);
+  static_assert(UM == 8 || LPR == 1, "");
+  const int chunks = max((len + UM * LPR - 1) / (UM * LPR), 1);
   return max((len + LPR * chunks - 1) / (LPR * chunks), 1);
 }
 
@@ -147,11 +149,11 @@ __device__ __forceinline__ float split_walk_u(const uint32_t *cd, float *w, int 
   return local_sum;
 }
 
-template <int MATH, int LPR, class Params, class Gather, class Keep>
+template <int MATH, int LPR, int UM = 8, class Params, class Gather, class Keep>
 __device__ __forceinline__ float split_walk(const uint32_t *cd, float *w, int len, int deg,
                                             const SplitLane &sl, float th, Params &params,
                                             Gather gather, Keep keep) {
-  switch (split_unroll<LPR>(len)) {  // warp-uniform
+  switch (split_unroll<LPR, UM>(len)) {  // warp-uniform
     case 1: return split_walk_u<MATH, LPR, 1>(cd, w, len, deg, sl, th, params, gather, keep);
     case 2: return split_walk_u<MATH, LPR, 2>(cd, w, len, deg, sl, th, params, gather, keep);
     case 3: return split_walk_u<MATH, LPR, 3>(cd, w, len, deg, sl, th, params, gather, keep);
@@ -159,14 +161,24 @@ __device__ __forceinline__ float split_walk(const uint32_t *cd, float *w, int le
     case 5: return split_walk_u<MATH, LPR, 5>(cd, w, len, deg, sl, th, params, gather, keep);
     case 6: return split_walk_u<MATH, LPR, 6>(cd, w, len, deg, sl, th, params, gather, keep);
     case 7: return split_walk_u<MATH, LPR, 7>(cd, w, len, deg, sl, th, params, gather, keep);
-    default: return split_walk_u<MATH, LPR, 8>(cd, w, len, deg, sl, th, params, gather, keep);
+    case 8: return split_walk_u<MATH, LPR, 8>(cd, w, len, deg, sl, th, params, gather, keep);
   }
+  if constexpr (UM > 8) {
+    static_assert(UM == 12, "");
+    switch (split_unroll<LPR, UM>(len)) {
+      case 9: return split_walk_u<MATH, LPR, 9>(cd, w, len, deg, sl, th, params, gather, keep);
+      case 10: return split_walk_u<MATH, LPR, 10>(cd, w, len, deg, sl, th, params, gather, keep);
+      case 11: return split_walk_u<MATH, LPR, 11>(cd, w, len, deg, sl, th, params, gather, keep);
+    }
+    return split_walk_u<MATH, LPR, 12>(cd, w, len, deg, sl, th, params, gather, keep);
+  }
+  return 0.0f;  // not reached
 }
-template <int MATH, int LPR, class Params, class Gather>
+template <int MATH, int LPR, int UM = 8, class Params, class Gather>
 __device__ __forceinline__ float split_walk(const uint32_t *cd, float *w, int len, int deg,
                                             const SplitLane &sl, float th, Params &params,
                                             Gather gather) {
-  return split_walk<MATH, LPR>(cd, w, len, deg, sl, th, params, gather, [](int, float) {});
+  return split_walk<MATH, LPR, UM>(cd, w, len, deg, sl, th, params, gather, [](int, float) {});
 }
 
 // The warp's part of the 32-row tree: rows 16 down to LPR apart; lane 0 holds

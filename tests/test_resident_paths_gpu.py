@@ -320,3 +320,39 @@ def test_adjoint_grid_segments_at_ragged_sizes(N, k, lo):
                 assert _rel(g[name], ref[name]) <= REL, (R, paired, name)
     adj.close()
     eng.close()
+
+
+@pytest.mark.parametrize("k", [5, 9, 12, 13, 24, 25, 36, 37])
+def test_one_lane_per_row_at_the_edges_of_its_chunks(k):
+    """Rows of k entries and one entry less and more (up to twelve per chunk)."""
+    rng = np.random.default_rng(k)
+    net = _from_degrees(k + rng.integers(-1, 2, 1500), 40, k)
+    ref = _per_step(LeviathanEngine(*net.engine_args()))
+    want_r = ref.step_n(DT, 30)
+    want = _state(ref)
+    ref.close()
+    e = LeviathanEngine(*net.engine_args())
+    e.set_cluster_mode(False)
+    e.set_grid_mode(True, 256)
+    np.testing.assert_array_equal(e.step_n(DT, 30), want_r)
+    _same(_state(e), want)
+    e.close()
+
+
+@pytest.mark.parametrize("N,k,on", [(80_000, 24, True), (80_000, 28, False), (75_000, 28, True)])
+def test_grid_kernel_is_the_default_where_its_gathers_keep_their_cache(N, k, on):
+    """Three CTAs per SM with more than 64 KB of edges each are left to the
+    per-step launches; the path can still be asked for."""
+    net = make_network(N, k, 0.1, 9, seed=k, delay_lo=1)
+    ref = _per_step(LeviathanEngine(*net.engine_args()))
+    want_r = ref.step_n(DT, 12)
+    want = _state(ref)
+    ref.close()
+    e = LeviathanEngine(*net.engine_args())
+    assert e.grid_info()["eligible"] and e.grid_info()["enabled"] == on
+    np.testing.assert_array_equal(e.step_n(DT, 6), want_r[:6])
+    e.set_grid_mode(True)
+    assert e.grid_info()["enabled"]
+    np.testing.assert_array_equal(e.step_n(DT, 6), want_r[6:])
+    _same(_state(e), want)
+    e.close()
