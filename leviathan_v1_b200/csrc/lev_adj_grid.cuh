@@ -23,7 +23,11 @@
 
 namespace lev {
 
-constexpr int kAdjBwdUnroll = 4;  // edges per lane in flight together in the reverse steps
+// Edges per lane in flight together in the reverse steps, for kernels of at most
+// `minb` CTAs per SM: four with 72 registers, six with 96.  T = 200, C = 50,
+// accurate, backward us for four / six: N = 2,000, k = 16 (R = 64) 1,037 / 838;
+// 5,000, k = 20 1,196 / 1,038; 10^4 (R = 128) 1,748 / 1,480.
+__host__ __device__ constexpr int adj_bwd_unroll(int minb) { return minb == 2 ? 6 : 4; }
 
 struct AdjGridFwdArgs {
   const NetDesc *net;  // adjoint copy: bsi = C + max_delay + 2
@@ -76,9 +80,10 @@ struct AdjGridFwdArgs {
 // and arrivals.  The body runs as CTA `cta` of a group of G CTAs (the whole
 // grid, or one half of a paired launch).  Shared memory: sums float2 [sum_cap]
 // (R < 256), sloff / sllen int [R/32], cd uint32 [edge_cap], w float [edge_cap].
-template <int MATH, int R>
+template <int MATH, int R, int MINB>
 __device__ __forceinline__ void adj_grid_fwd_body(const AdjGridFwdArgs &a, const int cta,
                                                   const unsigned G, unsigned char *smem) {
+  constexpr int kUM = grid_walk_max(MATH, R, MINB);
   constexpr int LPR = 256 / R;
   constexpr int nslices = R / 32;
   constexpr bool kBlocks = R == 256;
@@ -201,11 +206,11 @@ __device__ __forceinline__ void adj_grid_fwd_body(const AdjGridFwdArgs &a, const
       float local_sum;
       if (a.w_rec) {
         float *wr = a.w_rec + (long long)step * a.SL + ebase + eoff + sl.l;
-        local_sum = split_walk<MATH, LPR>(s_cd + eoff, s_w + eoff, len, deg, sl, th, ep, gather,
+        local_sum = split_walk<MATH, LPR, kUM>(s_cd + eoff, s_w + eoff, len, deg, sl, th, ep, gather,
                                           [&](int k, float w) { __stcs(wr + 32 * k, w); });
       } else {
         local_sum =
-            split_walk<MATH, LPR>(s_cd + eoff, s_w + eoff, len, deg, sl, th, ep, gather);
+            split_walk<MATH, LPR, kUM>(s_cd + eoff, s_w + eoff, len, deg, sl, th, ep, gather);
       }
       if (step > 0) {
         cta_barrier();  // A
@@ -687,16 +692,16 @@ __device__ __forceinline__ void adj_grid_bwd_body(const AdjGridBwdArgs &a, const
           s_lw[sloff[s] + 32 * k + ((lane + (k & (LPR - 1))) & 31)];
 }
 
-template <int MATH, int R>
-__global__ void __launch_bounds__(kGridThreads, 3) adj_grid_fwd_kernel(const AdjGridFwdArgs a) {
+template <int MATH, int R, int MINB>
+__global__ void __launch_bounds__(kGridThreads, MINB) adj_grid_fwd_kernel(const AdjGridFwdArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
-  adj_grid_fwd_body<MATH, R>(a, blockIdx.x, gridDim.x, smem);
+  adj_grid_fwd_body<MATH, R, MINB>(a, blockIdx.x, gridDim.x, smem);
 }
 
-template <int MATH, int R>
-__global__ void __launch_bounds__(kGridThreads, 3) adj_grid_bwd_kernel(const AdjGridBwdArgs a) {
+template <int MATH, int R, int MINB>
+__global__ void __launch_bounds__(kGridThreads, MINB) adj_grid_bwd_kernel(const AdjGridBwdArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
-  adj_grid_bwd_body<MATH, R, kAdjBwdUnroll>(a, blockIdx.x, gridDim.x, smem);
+  adj_grid_bwd_body<MATH, R, adj_bwd_unroll(MINB)>(a, blockIdx.x, gridDim.x, smem);
 }
 
 // Paired launch of the backward pass: CTAs [0, gf) recompute segment k-1
@@ -704,14 +709,14 @@ __global__ void __launch_bounds__(kGridThreads, 3) adj_grid_bwd_kernel(const Adj
 // other; each group has its own arrival counter and shares the SMs with the
 // other, so the two latency-bound step chains overlap.  Every CTA of both
 // groups is resident at once (cooperative launch).
-template <int MATH, int R>
-__global__ void __launch_bounds__(kGridThreads, 3)
+template <int MATH, int R, int MINB>
+__global__ void __launch_bounds__(kGridThreads, MINB)
     adj_grid_pair_kernel(const AdjGridFwdArgs f, const AdjGridBwdArgs b, const int gf) {
   extern __shared__ __align__(16) unsigned char smem[];
   if ((int)blockIdx.x < gf)
-    adj_grid_fwd_body<MATH, R>(f, blockIdx.x, gf, smem);
+    adj_grid_fwd_body<MATH, R, MINB>(f, blockIdx.x, gf, smem);
   else
-    adj_grid_bwd_body<MATH, R, kAdjBwdUnroll>(b, blockIdx.x - gf, gridDim.x - gf, smem);
+    adj_grid_bwd_body<MATH, R, adj_bwd_unroll(MINB)>(b, blockIdx.x - gf, gridDim.x - gf, smem);
 }
 
 }  // namespace lev

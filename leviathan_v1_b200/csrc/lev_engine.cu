@@ -3353,7 +3353,9 @@ struct LevAdjoint {
   bool gR_ok[3] = {false, false, false};  // R = 64, 128, 256
   int g_cap[3] = {0, 0, 0};
   size_t gf_smem[3] = {0, 0, 0}, gb_smem[3] = {0, 0, 0};
-  bool gp_ok[3] = {false, false, false};  // paired recompute + reverse launch fits
+  // CTAs per SM each kernel is compiled for; gp 0: the paired recompute +
+  // reverse launch does not fit
+  int gf_minb[3] = {0, 0, 0}, gb_minb[3] = {0, 0, 0}, gp_minb[3] = {0, 0, 0};
   bool use_pair = true;
   int g_gpad = 0;
   float2 *g_wsum = nullptr;
@@ -3473,14 +3475,16 @@ int adj_ckpt(LevAdjoint *a, int seg, bool save, cudaStream_t s = nullptr,
 using AdjGridFwdFn = void (*)(AdjGridFwdArgs);
 using AdjGridBwdFn = void (*)(AdjGridBwdArgs);
 using AdjGridPairFn = void (*)(AdjGridFwdArgs, AdjGridBwdArgs, int);
-#define LEV_BY_ROWS(kernel)                                 \
-  const bool acc = math_mode == LEV_MATH_ACCURATE;          \
-  if (R == 64) return acc ? kernel<1, 64> : kernel<0, 64>;  \
-  if (R == 128) return acc ? kernel<1, 128> : kernel<0, 128>; \
-  return acc ? kernel<1, 256> : kernel<0, 256>;
-AdjGridFwdFn adj_grid_fwd_fn(int R, int math_mode) { LEV_BY_ROWS(adj_grid_fwd_kernel) }
-AdjGridPairFn adj_grid_pair_fn(int R, int math_mode) { LEV_BY_ROWS(adj_grid_pair_kernel) }
-AdjGridBwdFn adj_grid_bwd_fn(int R, int math_mode) { LEV_BY_ROWS(adj_grid_bwd_kernel) }
+#define LEV_BY_MATH(kernel, R, MINB) (acc ? kernel<1, R, MINB> : kernel<0, R, MINB>)
+#define LEV_BY_ROWS(kernel)                                                                 \
+  const bool acc = math_mode == LEV_MATH_ACCURATE;                                          \
+  if (R == 64) return minb == 2 ? LEV_BY_MATH(kernel, 64, 2) : LEV_BY_MATH(kernel, 64, 3);  \
+  if (R == 128) return minb == 2 ? LEV_BY_MATH(kernel, 128, 2) : LEV_BY_MATH(kernel, 128, 3); \
+  return minb == 2 ? LEV_BY_MATH(kernel, 256, 2) : LEV_BY_MATH(kernel, 256, 3);
+AdjGridFwdFn adj_grid_fwd_fn(int R, int minb, int math_mode) { LEV_BY_ROWS(adj_grid_fwd_kernel) }
+AdjGridPairFn adj_grid_pair_fn(int R, int minb, int math_mode) { LEV_BY_ROWS(adj_grid_pair_kernel) }
+AdjGridBwdFn adj_grid_bwd_fn(int R, int minb, int math_mode) { LEV_BY_ROWS(adj_grid_bwd_kernel) }
+#undef LEV_BY_MATH
 #undef LEV_BY_ROWS
 
 // Grid-resident segments for a single network: per rows-per-CTA choice, the
@@ -3517,44 +3521,39 @@ int adj_setup_grid(LevAdjoint *a, const std::vector<long long> &sl_off,
                        sizeof(int) * 2 * (R / 32) + 8 * (size_t)cap;
     const size_t bsm = sizeof(int) * 2 * (R / 32) + 16 * (size_t)cap;
     if (std::max(fsm, bsm) + 1024 > (size_t)max_smem) continue;
-    bool ok = true;
-    for (int m = 0; m < 2 && ok; ++m) {
-      const int mm = m ? LEV_MATH_ACCURATE : LEV_MATH_REFERENCE;
-      const void *ff = reinterpret_cast<const void *>(adj_grid_fwd_fn(R, mm));
-      const void *bf = reinterpret_cast<const void *>(adj_grid_bwd_fn(R, mm));
-      int pf = 0, pb = 0;
-      ok = allow_smem(ff, fsm) && allow_smem(bf, bsm) &&
-           cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pf, ff, kGridThreads, fsm) ==
-               cudaSuccess &&
-           cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pb, bf, kGridThreads, bsm) ==
-               cudaSuccess &&
-           (long long)pf * sms >= C && (long long)pb * sms >= C;
-    }
-    cudaGetLastError();
-    if (!ok) continue;
+    // CTAs per SM that the kernel of `pick` has to be compiled for so that n of
+    // its CTAs with `sm` bytes each are resident, 2 or 3, or 0: not even then
+    auto fit = [&](auto pick, size_t sm, long long n) -> int {
+      for (int minb = 2; minb <= 3; ++minb) {
+        bool ok = true;
+        for (int m = 0; m < 2 && ok; ++m) {
+          const void *fn = reinterpret_cast<const void *>(
+              pick(R, minb, m ? LEV_MATH_ACCURATE : LEV_MATH_REFERENCE));
+          int per_sm = 0;
+          ok = allow_smem(fn, sm) &&
+               cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kGridThreads, sm) ==
+                   cudaSuccess &&
+               (long long)per_sm * sms >= n;
+        }
+        cudaGetLastError();  // clear a refused attribute, if any
+        if (ok) return minb;
+      }
+      return 0;
+    };
+    a->gf_minb[ri] = fit(adj_grid_fwd_fn, fsm, C);
+    a->gb_minb[ri] = fit(adj_grid_bwd_fn, bsm, C);
+    if (!a->gf_minb[ri] || !a->gb_minb[ri]) continue;
     // the paired backward launch: both groups resident at once
-    bool pok = true;
-    for (int m = 0; m < 2 && pok; ++m) {
-      const void *pf = reinterpret_cast<const void *>(
-          adj_grid_pair_fn(R, m ? LEV_MATH_ACCURATE : LEV_MATH_REFERENCE));
-      const size_t psm = std::max(fsm, bsm);
-      int per_sm = 0;
-      pok = allow_smem(pf, psm) &&
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pf, kGridThreads, psm) ==
-                cudaSuccess &&
-            (long long)per_sm * sms >= 2LL * C;
-    }
-    cudaGetLastError();
-    a->gp_ok[ri] = pok;
+    a->gp_minb[ri] = fit(adj_grid_pair_fn, std::max(fsm, bsm), 2LL * C);
     a->gR_ok[ri] = true;
     a->g_cap[ri] = (int)cap;
     a->gf_smem[ri] = fsm;
     a->gb_smem[ri] = bsm;
     max_gpad = std::max(max_gpad, gpad);
     // the smallest: the steps wait on instructions, and more lanes per row are
-    // more warps (us per 100 steps forward / backward, k = 20: N = 2*10^4 R = 64
-    // 518 / 1,391, R = 128 587 / 1,439; 5*10^4 R = 128 778 / 2,230, R = 256 918 /
-    // 2,822)
+    // more warps (us per 100 steps forward / backward, k = 20: N = 10^4 R = 64 363 /
+    // 734, R = 128 460 / 740; 2*10^4 R = 64 485 / 1,198, R = 128 552 / 1,098;
+    // 5*10^4 R = 128 745 / 1,980, R = 256 918 / 2,246)
     if (!a->grid_ok) a->grid_R = R;
     a->grid_ok = true;
   }
@@ -3652,7 +3651,7 @@ int adj_grid_launch_fwd(LevAdjoint *a, AdjGridFwdArgs f, int n, cudaStream_t s) 
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  LEV_TRY_CUDA(cudaLaunchKernelEx(&cfg, adj_grid_fwd_fn(R, e->math_mode), f));
+  LEV_TRY_CUDA(cudaLaunchKernelEx(&cfg, adj_grid_fwd_fn(R, a->gf_minb[ri], e->math_mode), f));
   return LEV_OK;
 }
 
@@ -3698,7 +3697,7 @@ int adj_grid_launch_bwd(LevAdjoint *a, AdjGridBwdArgs b, cudaStream_t s) {
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  LEV_TRY_CUDA(cudaLaunchKernelEx(&cfg, adj_grid_bwd_fn(R, e->math_mode), b));
+  LEV_TRY_CUDA(cudaLaunchKernelEx(&cfg, adj_grid_bwd_fn(R, a->gb_minb[ri], e->math_mode), b));
   return LEV_OK;
 }
 
@@ -3723,7 +3722,7 @@ int adj_grid_launch_pair(LevAdjoint *a, AdjGridFwdArgs f, int n, AdjGridBwdArgs 
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  LEV_TRY_CUDA(cudaLaunchKernelEx(&cfg, adj_grid_pair_fn(R, e->math_mode), f, b, C));
+  LEV_TRY_CUDA(cudaLaunchKernelEx(&cfg, adj_grid_pair_fn(R, a->gp_minb[ri], e->math_mode), f, b, C));
   return LEV_OK;
 }
 
@@ -3874,7 +3873,7 @@ int lev_adj_bytes(const LevAdjoint *a, size_t *bytes) {
 // Record set of segment `seg` of a run of `nseg` segments, per path.
 enum { kRecNone = 0, kRecSteps = 1, kRecGrid = 2 };
 static bool adj_paired(const LevAdjoint *a, int nseg) {
-  return a->ring2 != nullptr && a->use_pair && a->gp_ok[grid_r_index(a->grid_R)] && nseg > 1;
+  return a->ring2 != nullptr && a->use_pair && a->gp_minb[grid_r_index(a->grid_R)] > 0 && nseg > 1;
 }
 static int adj_record_set(const LevAdjoint *a, int path, int seg, int nseg) {
   if (path == kRecGrid) return adj_paired(a, nseg) ? (seg & 1) : 0;
@@ -4284,7 +4283,7 @@ int lev_adj_grid_info(const LevAdjoint *a, int32_t *eligible, int32_t *enabled,
   if (rows_per_cta) *rows_per_cta = a->grid_ok ? a->grid_R : 0;
   if (paired)
     *paired = (adj_grid_on(a) && a->use_pair && a->ring2 != nullptr &&
-               a->gp_ok[grid_r_index(a->grid_R)]) ? 1 : 0;
+               a->gp_minb[grid_r_index(a->grid_R)] > 0) ? 1 : 0;
   if (eligible_rows_mask) {
     int m = 0;
     for (int i = 0; i < 3; ++i)

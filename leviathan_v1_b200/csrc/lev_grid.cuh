@@ -217,6 +217,12 @@ constexpr int kGridThreads = 256 + 32;  // eight warps on rows, one for the othe
 // grid_kernel for at most `minb` CTAs per SM: two (with an order warp where a
 // row has several lanes) or three.
 __host__ __device__ constexpr bool grid_order_warp(int R, int minb) { return minb == 2 && R < 256; }
+// Most entries of a lane in flight together: twelve at one lane per row where
+// the registers allow it, but not with the accurate sine and cosine (N = 2*10^4,
+// accurate, R = 256: eight 7.4 us per recorded step, twelve 9.9).
+__host__ __device__ constexpr int grid_walk_max(int math, int R, int minb) {
+  return math == 0 && R == 256 && minb == 2 ? 12 : 8;
+}
 __host__ __device__ constexpr int grid_threads(int R, int minb) {
   return grid_order_warp(R, minb) ? 256 + 64 : kGridThreads;
 }
@@ -306,7 +312,7 @@ __global__ void __launch_bounds__(grid_threads(R, MINB), MINB) grid_kernel(const
   constexpr int LPR = 256 / R;
   constexpr bool ORDER = grid_order_warp(R, MINB);
   constexpr int kThreads = grid_threads(R, MINB);
-  constexpr int kUM = LPR == 1 && MINB == 2 ? 12 : 8;  // entries of a lane in flight
+  constexpr int kUM = grid_walk_max(MATH, R, MINB);
   constexpr int nslices = R / 32;
   constexpr bool kBlocks = R == 256;  // a CTA closes its 256-node block itself
   extern __shared__ __align__(16) unsigned char smem[];

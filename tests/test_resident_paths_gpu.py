@@ -297,14 +297,16 @@ def test_gradients_from_the_recorded_last_segment(N, T, segment):
                 assert _rel(g[k], ref[k]) <= REL, (f, b, k)
 
 
-@pytest.mark.parametrize("N,k,lo", [(65, 4, 1), (2049, 30, 0), (2049, 30, 1)])
-def test_adjoint_grid_segments_at_ragged_sizes(N, k, lo):
+# 18,945 rows: one CTA of 64 rows more than two per SM
+@pytest.mark.parametrize("N,k,lo,mode", [(65, 4, 1, "reference"), (2049, 30, 0, "reference"),
+                                         (2049, 30, 1, "accurate"), (18_945, 4, 1, "reference")])
+def test_adjoint_grid_segments_at_ragged_sizes(N, k, lo, mode):
     net = make_network(N, k, 0.1, 6, seed=N + lo, delay_lo=lo)
     om, w0 = (torch.tensor(x, device="cuda") for x in (net.omega, net.weights))
     K = torch.full((1,), 1.5, device="cuda")
     T = 27
     dr = torch.linspace(-1, 1, T, device="cuda")[:, None].contiguous()
-    eng = LeviathanEngine(*net.engine_args())
+    eng = LeviathanEngine(*net.engine_args(), math_mode=mode)
     adj = Adjoint(eng, segment=10, max_steps=T)
     rows = adj.grid_info()["eligible_rows"]
     assert rows
@@ -322,16 +324,19 @@ def test_adjoint_grid_segments_at_ragged_sizes(N, k, lo):
     eng.close()
 
 
-@pytest.mark.parametrize("k", [5, 9, 12, 13, 24, 25, 36, 37])
-def test_one_lane_per_row_at_the_edges_of_its_chunks(k):
+@pytest.mark.parametrize("k,mode", [(5, "reference"), (9, "reference"), (9, "accurate"),
+                                    (12, "reference"), (13, "reference"), (24, "reference"),
+                                    (25, "accurate"), (25, "reference"), (36, "reference"),
+                                    (37, "reference")])
+def test_one_lane_per_row_at_the_edges_of_its_chunks(k, mode):
     """Rows of k entries and one entry less and more (up to twelve per chunk)."""
     rng = np.random.default_rng(k)
     net = _from_degrees(k + rng.integers(-1, 2, 1500), 40, k)
-    ref = _per_step(LeviathanEngine(*net.engine_args()))
+    ref = _per_step(LeviathanEngine(*net.engine_args(), math_mode=mode))
     want_r = ref.step_n(DT, 30)
     want = _state(ref)
     ref.close()
-    e = LeviathanEngine(*net.engine_args())
+    e = LeviathanEngine(*net.engine_args(), math_mode=mode)
     e.set_cluster_mode(False)
     e.set_grid_mode(True, 256)
     np.testing.assert_array_equal(e.step_n(DT, 30), want_r)
