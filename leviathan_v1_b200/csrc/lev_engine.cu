@@ -1093,6 +1093,7 @@ int setup_grid(LevEngine *h, const std::vector<int> &sl_len) {
     // compiled for two CTAs per SM if every CTA is then resident, else for three
     bool ok = false;
     for (int minb = 2; minb <= 3 && !ok; ++minb) {
+      if (C > (long long)minb * sms) continue;  // (a look at a kernel loads it)
       ok = true;
       for (int m = 0; m < 2 && ok; ++m) {
         const void *fn = reinterpret_cast<const void *>(
@@ -3525,6 +3526,7 @@ int adj_setup_grid(LevAdjoint *a, const std::vector<long long> &sl_off,
     // its CTAs with `sm` bytes each are resident, 2 or 3, or 0: not even then
     auto fit = [&](auto pick, size_t sm, long long n) -> int {
       for (int minb = 2; minb <= 3; ++minb) {
+        if (n > (long long)minb * sms) continue;  // (a look at a kernel loads it)
         bool ok = true;
         for (int m = 0; m < 2 && ok; ++m) {
           const void *fn = reinterpret_cast<const void *>(
