@@ -412,6 +412,13 @@ int lev_adj_set_grid_pairing(LevAdjoint *a, int32_t enabled);
 /* Bound of the adjoint's grid-barrier waits, as lev_set_grid_wait. */
 int lev_adj_set_grid_wait(LevAdjoint *a, uint64_t limit_ns, uint32_t extra_arrivals);
 
+/* The wait of reverse step k (0: the last step of a segment) of the
+ * grid-resident segments: on which of two arrival counters a CTA arrives for
+ * step k, and how many arrivals per CTA that counter has to hold before the CTA
+ * reads adjoint-ring slots in step k.  early: the network has no zero delay.
+ * Host only, no device work: a model of the kernel's order uses it. */
+int lev_adj_reverse_wait(int32_t k, int32_t early, int32_t *counter, int32_t *arrivals);
+
 /* Self-test of the phase wraps (no reference counterpart; checks this
  * library's division-free evaluation of the wraps of
  * leviathan_kernel.cu:105,146,188).  Runs, on the current device, both

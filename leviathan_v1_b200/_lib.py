@@ -136,6 +136,7 @@ PROTOTYPES = {
     "lev_adj_set_grid_mode": (C.c_int, [_P, _i32, _i32]),
     "lev_adj_set_grid_pairing": (C.c_int, [_P, _i32]),
     "lev_adj_set_grid_wait": (C.c_int, [_P, C.c_uint64, C.c_uint32]),
+    "lev_adj_reverse_wait": (C.c_int, [_i32, _i32, C.POINTER(_i32), C.POINTER(_i32)]),
     "lev_set_grid_wait": (C.c_int, [_P, C.c_uint64, C.c_uint32]),
     "lev_selftest_wraps":(C.c_int, [C.POINTER(C.c_uint64), C.POINTER(C.c_uint64)]),
     "lev_step_noalloc":(C.c_int, [_i32, _i32, _i64, _P, _P, _P, _P, _P, _P, _P,

@@ -346,7 +346,7 @@ struct AdjGridBwdArgs {
   float *grad_omega;     // accumulated
   float *lgp;            // [4][gpad] per-CTA lam_g parts, kNoSum at launch
   int gpad;
-  unsigned *bar;         // arrivals, zero at launch
+  unsigned *bar;         // two arrival counters, kGridBarPitch apart, zero at launch
   int *err;
   GridWait wait;  // bound of the barrier waits
   int early;             // no delay is 0: slot s+1 is complete one barrier earlier
@@ -368,6 +368,18 @@ __device__ __forceinline__ void cta_scatter_wait() {
   asm volatile("bar.sync 2, %0;" ::"n"(kGridThreads) : "memory");
 }
 
+// Arrivals of the reverse steps: a CTA arrives for step k, its scatter done, on
+// counter adj_arrival_counter(k); before it reads adjoint-ring slots in step k it
+// waits until that counter holds adj_arrival_wait(k) arrivals per CTA, its
+// own and every other's.  A total can only stand for "everyone" if nobody adds
+// to it again before that wait.  With zero delays step k waits for step k-1 and
+// arrives for k after the wait: one counter.  Without, step k waits for step k-2
+// only, and a fast CTA's arrival for k-1 may come before a slow one's for k-2: the
+// parts of lam_g, which let it go on, are published before the scatter.  So
+// even and odd steps count apart.
+__host__ __device__ constexpr int adj_arrival_counter(int k, int early) { return early ? k & 1 : 0; }
+__host__ __device__ constexpr int adj_arrival_wait(int k, int early) { return early ? k >> 1 : k; }
+
 // One segment's reverse steps.  Most of a step does not depend on the adjoint
 // of the step reversed before: phases, weights, sines and cosines, the row's
 // coupling sum S_i and the |eps| term.  All that comes first and is kept per
@@ -377,8 +389,8 @@ __device__ __forceinline__ void cta_scatter_wait() {
 // the other CTAs runs while the scatter and the next step's first part do.
 //
 // Order of one reverse step k (s = seg_start + n_steps - 1 - k), edge warps | ninth warp:
-//   edges, first part                | wait for the arrivals (scatters) of step
-//                                    | k-2 (k-1 with zero delays)
+//   edges, first part                | wait for everyone's arrival (scatter) of
+//                                    | step k-2 (k-1 with zero delays)
 //   ----------------- barrier D: adjoint slot s+1 is complete -------------------
 //   read and clear slot s+1          | wait for the parts of step k-1; lam_g(s+1)
 //   ----------------- barrier A: lam_g(s+1) -------------------------------------
@@ -640,9 +652,10 @@ __device__ __forceinline__ void adj_grid_bwd_body(const AdjGridBwdArgs &a, const
     for (int k = 0; k < a.n_steps; ++k) {
       const int kk = a.n_steps - 1 - k;
       const float4 tr = a.trace[kk];
-      const int arrived = a.early ? k - 1 : k;  // steps whose scatters slot s+1 waits for
+      unsigned *bar = a.bar + kGridBarPitch * adj_arrival_counter(k, a.early);
+      const unsigned arrived = (unsigned)adj_arrival_wait(k, a.early);
       if (ok && arrived > 0) {
-        ok = lane != 0 || grid_poll(a.bar, (unsigned)arrived * G, a.wait);
+        ok = lane != 0 || grid_poll(bar, arrived * G, a.wait);
         ok = __all_sync(mask, ok);
       }
       cta_barrier_slot();  // D
@@ -669,7 +682,7 @@ __device__ __forceinline__ void adj_grid_bwd_body(const AdjGridBwdArgs &a, const
       __syncwarp();
       cta_scatter_wait();
       if (lane == 0)
-        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.bar) : "memory");
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
     }
     if (!ok) give_up();
     if (ok && a.n_steps > 0 && cta == 0) {

@@ -3563,7 +3563,7 @@ int adj_setup_grid(LevAdjoint *a, const std::vector<long long> &sl_off,
   // arrival counters, published sums and parts: one block, so that a launch
   // clears what it uses with two fills
   a->g_gpad = max_gpad;
-  int rc = adj_alloc(a, &a->g_bar, 2 * kGridBarPitch);
+  int rc = adj_alloc(a, &a->g_bar, 3 * kGridBarPitch);
   if (rc == LEV_OK) rc = adj_alloc(a, &a->g_wsum, 32LL * d.ntiles + 2LL * max_gpad);
   if (rc != LEV_OK) return rc;
   a->g_lgp = reinterpret_cast<float *>(a->g_wsum + 32LL * d.ntiles);
@@ -3626,9 +3626,9 @@ void adj_grid_fill_fwd(LevAdjoint *a, AdjGridFwdArgs &f, int n) {
   f.n_steps = n;
 }
 
-// No arrivals, nothing published.
+// No arrivals (one counter forward, two in reverse), nothing published.
 cudaError_t adj_grid_clear(LevAdjoint *a, cudaStream_t s) {
-  cudaError_t e = cudaMemsetAsync(a->g_bar, 0, sizeof(unsigned) * 2 * kGridBarPitch, s);
+  cudaError_t e = cudaMemsetAsync(a->g_bar, 0, sizeof(unsigned) * 3 * kGridBarPitch, s);
   if (e == cudaSuccess)
     e = cudaMemsetAsync(a->g_wsum, 0xff,
                         sizeof(float2) * (32 * (size_t)a->h_nets[0].ntiles +
@@ -4307,6 +4307,13 @@ int lev_adj_set_grid_wait(LevAdjoint *a, uint64_t limit_ns, uint32_t extra_arriv
 int lev_adj_set_grid_pairing(LevAdjoint *a, int32_t enabled) {
   if (!a) return fail(LEV_ERR_ARG, "null handle");
   a->use_pair = enabled != 0;
+  return LEV_OK;
+}
+
+int lev_adj_reverse_wait(int32_t k, int32_t early, int32_t *counter, int32_t *arrivals) {
+  if (k < 0 || !counter || !arrivals) return fail(LEV_ERR_ARG, "bad argument");
+  *counter = adj_arrival_counter(k, early != 0);
+  *arrivals = adj_arrival_wait(k, early != 0);
   return LEV_OK;
 }
 

@@ -14,9 +14,10 @@ import numpy as np
 import pytest
 import torch
 
+from adjoint64 import simulate as simulate64
 from conftest import has_gpu
 from leviathan_v1_b200 import BatchEngine, HubTransitions, LeviathanEngine, _lib
-from leviathan_v1_b200.adjoint import Adjoint
+from leviathan_v1_b200.adjoint import Adjoint, simulate
 from leviathan_v1_b200.graphs import Network, init_state, make_network
 
 pytestmark = pytest.mark.gpu
@@ -361,3 +362,69 @@ def test_grid_kernel_is_the_default_where_its_gathers_keep_their_cache(N, k, on)
     np.testing.assert_array_equal(e.step_n(DT, 6), want_r[6:])
     _same(_state(e), want)
     e.close()
+
+
+def _long_rows(N, seed):
+    """Rows of 4 to 12 entries, and in some blocks of 256 rows one or two of 100 to
+    280 among them (neighbours, so that a CTA's slices fit its shared memory):
+    CTAs whose scatter takes many times that of the others.  Weights of a long
+    row are scaled to those of a row of eight."""
+    rng = np.random.default_rng(seed)
+    deg = rng.integers(4, 13, N)
+    for b in rng.choice(N // 256, max(1, N // 1500), replace=False):
+        at = 256 * b + 32 * rng.integers(0, 8) + rng.integers(0, 31)
+        deg[at:at + rng.integers(1, 3)] = rng.integers(100, 281)
+    net = _from_degrees(deg, 30, seed)
+    net.weights[:] *= np.repeat(np.minimum(1.0, 8.0 / deg), deg).astype(np.float32)
+    return net
+
+
+# The forward pass is bitwise; a gradient is a sum over 60 steps of sums of up to
+# 280 float32 terms: sqrt(60 * 280) * 6e-8 = 8e-6 of the vector's norm on either
+# side.  dL/dK, one number, cancels to a part of its terms: the bound against float64.
+@pytest.mark.parametrize("N", [700, 6000, 20_000])
+def test_reverse_segments_on_long_rows_among_short_ones(N):
+    net = _long_rows(N, N)
+    T = 60
+    assert net.delays.min() >= 1
+    rng = np.random.default_rng(2)
+    drive = rng.normal(0, 0.5, (T, N)).astype(np.float32)
+    wsel = (rng.normal(size=N) / np.sqrt(N)).astype(np.float32)
+
+    def grads(grid, paired):
+        e = LeviathanEngine(*net.engine_args(), math_mode="accurate")
+        adj = Adjoint(e, segment=20, max_steps=T)
+        adj.set_grid_mode(bool(grid), grid)
+        adj.set_grid_pairing(paired)
+        p = [torch.tensor(v, dtype=torch.float32, device="cuda", requires_grad=True)
+             for v in (net.omega, net.weights, np.array([1.5]), drive)]
+        r, th = simulate(adj, p[0], p[1], p[2], T, DT, drive=p[3], record_theta=True)
+        ((torch.cos(th) @ torch.tensor(wsel, device="cuda")).pow(2).mean()
+         + r[:, 0].mean()).backward()
+        out = [r.detach().cpu().numpy(), th.detach().cpu().numpy()]
+        out += [v.grad.double().cpu().numpy().ravel() for v in p]
+        rows = adj.grid_info()["eligible_rows"]
+        adj.close()
+        e.close()
+        return out, rows
+
+    want, rows = grads(0, False)
+    assert rows
+    for R in rows:
+        for paired in (True, False):
+            got, _ = grads(R, paired)
+            for a, b in zip(got[:2], want[:2]):
+                np.testing.assert_array_equal(a, b)
+            for name, a, b, tol in zip(("omega", "w0", "K", "drive"), got[2:], want[2:],
+                                       (3e-5, 3e-5, 1e-3, 3e-5)):
+                err = np.linalg.norm(a - b) / np.linalg.norm(b)
+                assert err < tol, (R, paired, name, err)
+    if N > 1000:
+        return
+    t64 = [torch.tensor(np.asarray(v, np.float64), requires_grad=True)
+           for v in (net.omega, net.weights, 1.5, drive)]
+    r, th = simulate64(net, t64[0], t64[1], t64[2], T, DT, drive=t64[3], record_theta=True)
+    ((torch.cos(th) @ torch.tensor(wsel.astype(np.float64))).pow(2).mean() + r.mean()).backward()
+    for name, a, v in zip(("omega", "w0", "K", "drive"), want[2:], t64):
+        b = v.grad.numpy().ravel()
+        assert np.linalg.norm(a - b) <= 1e-3 * np.linalg.norm(b), name
