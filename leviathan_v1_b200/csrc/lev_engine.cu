@@ -89,10 +89,10 @@ constexpr int kNumVariants = sizeof(kVariants) / sizeof(kVariants[0]);
 // launch, reduce included; 1M: N = 10^6, k = 32; 1M8: N = 10^6, k = 8; 100k:
 // N = 10^5, k = 20; sweep: 128 networks, 29 M edges):
 //          (8,3,0) (6,3,1) (6,3,0) (4,4,1) (4,4,0) (8,2,1) (12,2,0)
-//   1M       257     264     270     309     302     289     265
-//   1M8      133     126     126     125     124     179     137
-//   100k    27.5    28.0    25.9    28.5    25.9    29.5    27.5
-//   sweep    262     265     261     270     265     319     287
+//   1M       260     288     264     326     296     287     260
+//   1M8      127     137     123     132     121     162     135
+//   100k    28.1    30.0    28.0    29.2    27.8    30.2    29.4
+//   sweep    247     265     245     267     248     300     273
 // Long rows want many entries in flight per lane, short rows and networks of
 // less than one wave more resident CTAs.
 struct PairVariant {

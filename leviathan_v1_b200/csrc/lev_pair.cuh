@@ -166,7 +166,7 @@ __device__ __forceinline__ int nxt_slot(int cur, int bsi) {
 template <int MATH, int U, int SECOND, int DEEP>
 __device__ __forceinline__ float row_walk(const uint32_t *__restrict__ cdp,
                                           float *wp, float *wo, int len, int deg,
-                                          const float *__restrict__ ring, int base,
+                                          const float *ring, int base,
                                           int bsi, int Np, float th, float my_eps,
                                           float dt, const NetDesc &nd) {
   const EdgeParams ep = {dt, nd.eta, nd.lam, __fmaf_rn(-nd.gamma, my_eps, 1.0f),
@@ -191,9 +191,9 @@ __device__ __forceinline__ float row_walk(const uint32_t *__restrict__ cdp,
     for (int u = 0; u < U; ++u) {
       const float *src = ring + ring_pos_word(p[u], base, bsi, Np);
       if (SECOND)
-        g[u] = (k0 + u < deg) ? ld_ring(src) : 0.0f;
+        g[u] = (k0 + u < deg) ? ld_ring_dependent(src) : 0.0f;
       else
-        g[u] = ld_ring(src);
+        g[u] = ld_ring_dependent(src);
     }
   };
   auto compute = [&](int k0, float (&g)[U], const float (&wv)[U]) {

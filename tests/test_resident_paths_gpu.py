@@ -428,3 +428,22 @@ def test_reverse_segments_on_long_rows_among_short_ones(N):
     for name, a, v in zip(("omega", "w0", "K", "drive"), want[2:], t64):
         b = v.grad.numpy().ravel()
         assert np.linalg.norm(a - b) <= 1e-3 * np.linalg.norm(b), name
+
+
+@pytest.mark.parametrize("N", [120_000, 200_000, 600_000])
+def test_long_pair_chains_with_dependent_launches(N):
+    """More than one wave of pair CTAs: blocks issued directly, recorded and
+    replayed, and single steps between, bitwise as single step launches."""
+    net = make_network(N, 32, 0.1, 64, seed=N, delay_lo=1)
+    ref = _per_step(LeviathanEngine(*net.engine_args()))
+    want_r = ref.step_n(DT, 331)
+    want = _state(ref)
+    ref.close()
+    e = LeviathanEngine(*net.engine_args())
+    e.set_grid_mode(False)
+    r = [e.step_n(DT, 100), e.step_n(DT, 100)]
+    r += [[e.step(DT)] for _ in range(31)]
+    r += [e.step_n(DT, 100)]
+    np.testing.assert_array_equal(np.concatenate(r).astype(np.float32), want_r)
+    _same(_state(e), want)
+    e.close()
