@@ -337,14 +337,14 @@ struct AdjGridBwdArgs {
   const float *win;      // reservoir drive (xin[s]); grad_win accumulated; or null
   const float *xin;
   float *grad_win;
-  float *lam_th;
+  double *lam_th;
   float *lam_thh;
   float *lam_omh;
   float *lam_w;          // SELL
   float *adj_ring;
-  float *lam_g;          // [1]: in lam_g(seg_end), out lam_g(seg_start)
+  double *lam_g;         // [1]: in lam_g(seg_end), out lam_g(seg_start)
   float *grad_omega;     // accumulated
-  float *lgp;            // [4][gpad] per-CTA lam_g parts, kNoSum at launch
+  double *lgp;           // [4][gpad] per-CTA lam_g parts, kNoPart at launch
   int gpad;
   unsigned *bar;         // two arrival counters, kGridBarPitch apart, zero at launch
   int *err;
@@ -356,6 +356,13 @@ struct AdjGridBwdArgs {
   int edge_cap;
   float dt;
 };
+
+// A part of lam_g that has not been published yet: a NaN pattern that no
+// published part has.
+constexpr unsigned long long kNoPart = ~0ull;
+__device__ __forceinline__ void st_relaxed_gpu(double *p, unsigned long long v) {
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
 
 // Barriers of the reverse body (cta_barrier is number 1).
 __device__ __forceinline__ void cta_barrier_slot() {
@@ -411,7 +418,7 @@ __device__ __forceinline__ void adj_grid_bwd_body(const AdjGridBwdArgs &a, const
                                                   const unsigned G, unsigned char *smem) {
   constexpr int LPR = 256 / R;
   constexpr int nslices = R / 32;
-  __shared__ float s_red[8];
+  __shared__ double s_red[8];
   __shared__ float s_lg;
   __shared__ int s_ok;
 
@@ -453,7 +460,8 @@ __device__ __forceinline__ void adj_grid_bwd_body(const AdjGridBwdArgs &a, const
       s_lw[at] = a.lam_w[ebase + sloff[s] + 32 * k + lane];
     }
   int deg = 0;
-  float lt = 0.0f, lthh = 0.0f, lomh = 0.0f, go = 0.0f;  // alike in the row's lanes
+  double lt = 0.0;  // lam_th; alike in the row's lanes
+  float lthh = 0.0f, lomh = 0.0f, go = 0.0f;
   if (live) {
     lt = a.lam_th[gi];
     lthh = a.lam_thh[gi];
@@ -487,7 +495,7 @@ __device__ __forceinline__ void adj_grid_bwd_body(const AdjGridBwdArgs &a, const
     const int at0 = eoff + ((sl.l + sl.q) & 31);
     float th1 = 0.0f;  // theta(s+1): theta(s) of the step reversed before
     if (live) th1 = H[(long long)(a.n_steps + nd.max_delay) * Np + row];
-    float lamg = a.lam_g[0];  // lam_g(s+1)
+    float lamg = (float)a.lam_g[0];  // lam_g(s+1)
     for (int k = 0; k < a.n_steps; ++k) {
       const long long s = a.seg_start + a.n_steps - 1 - k;
       const int kk = (int)(s - a.seg_start);
@@ -560,14 +568,14 @@ __device__ __forceinline__ void adj_grid_bwd_body(const AdjGridBwdArgs &a, const
       }
       // ---- (A) adjoint of theta(s+1), complete; (B) integrate --------------------
       const float lam_r = dldr + lamg * dgdr;
-      float lt1 = 0.0f;
       if (live) {
         const float Cm = tr.z * invN, Sm = tr.w * invN, r1 = tr.y;
-        lt1 = lt + arv;
-        if (r1 > 0.0f) lt1 += lam_r * (Sm * cs1 - Cm * sn1) * invN / r1;
-        if (a.dLdth) lt1 += extra;
+        lt += arv;
+        if (r1 > 0.0f) lt += lam_r * (Sm * cs1 - Cm * sn1) * invN / r1;
+        if (a.dLdth) lt += extra;
       }
-      float part = sl.q == 0 ? lt1 * dt * S_i : 0.0f;
+      const float lt1 = (float)lt;  // lam_th'
+      double part = sl.q == 0 ? (double)lt1 * dt * S_i : 0.0;
 #pragma unroll
       for (int off = 16; off > 0; off /= 2) part += __shfl_down_sync(mask, part, off);
       if (lane == 0) s_red[warp] = part;
@@ -601,7 +609,7 @@ __device__ __forceinline__ void adj_grid_bwd_body(const AdjGridBwdArgs &a, const
         const float leps = -lt1 * dt * nd.alpha - dt * eta * gamma * labs * sgn +
                            lomh * nd.kappa_w * dt;
         const float ldiff = leps * cosf(diff);
-        lt = lt1 + lsum + ldiff;
+        lt += lsum + ldiff;
         const float lthh1 = lthh;
         lthh = lthh1 - ldiff;
         lomh = lomh + lthh1 * dt;
@@ -610,35 +618,36 @@ __device__ __forceinline__ void adj_grid_bwd_body(const AdjGridBwdArgs &a, const
       cta_scatter_done();
     }
   } else {
-    float lamg = a.lam_g[0], dgdg_prev = 1.0f;
+    double lamg = a.lam_g[0];
+    float dgdg_prev = 1.0f;
     // lam_g(s+1) from lam_g(s+2) and the parts of reverse step `k`
     auto fold_parts = [&](int k) -> bool {
-      const float *buf = a.lgp + (k & 3) * gpad;
+      const double *buf = a.lgp + (k & 3) * gpad;
       const unsigned long long t0 = global_ns();
-      float sum = 0.0f;
+      double sum = 0.0;
       constexpr int K = 4;
       for (int c0 = 0; c0 < (int)G; c0 += 32 * K) {
-        unsigned v[K];
+        unsigned long long v[K];
         for (;;) {
           bool ready = a.wait.extra == 0;
 #pragma unroll
           for (int j = 0; j < K; ++j) {
-            v[j] = 0u;
+            v[j] = 0ull;
             if (c0 + 32 * j + lane < (int)G)
-              asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];"
-                           : "=r"(v[j]) : "l"(buf + c0 + 32 * j + lane) : "memory");
-            ready = ready && v[j] != kNoSum;
+              asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];"
+                           : "=l"(v[j]) : "l"(buf + c0 + 32 * j + lane) : "memory");
+            ready = ready && v[j] != kNoPart;
           }
           if (__all_sync(mask, ready)) break;
           if (__any_sync(mask, global_ns() - t0 > a.wait.ns)) return false;
         }
 #pragma unroll
-        for (int j = 0; j < K; ++j) sum += __uint_as_float(v[j]);
+        for (int j = 0; j < K; ++j) sum += __longlong_as_double((long long)v[j]);
       }
 #pragma unroll
       for (int off = 16; off > 0; off /= 2) sum += __shfl_down_sync(mask, sum, off);
       lamg = lamg * dgdg_prev + __shfl_sync(mask, sum, 0);
-      if (lane == 0) s_lg = lamg;
+      if (lane == 0) s_lg = (float)lamg;
       return true;
     };
     auto give_up = [&]() {
@@ -668,16 +677,14 @@ __device__ __forceinline__ void adj_grid_bwd_body(const AdjGridBwdArgs &a, const
       float dgdr;
       controller(tr, &dgdr, &dgdg_prev);
       cta_barrier();  // B
-      float part = lane < 8 ? s_red[lane] : 0.0f;
+      double part = lane < 8 ? s_red[lane] : 0.0;
 #pragma unroll
       for (int off = 4; off > 0; off /= 2) part += __shfl_down_sync(mask, part, off);
       if (lane == 0) {
-        unsigned v = __float_as_uint(part);
-        if (v == kNoSum) v = 0x7fffffffu;
-        asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(a.lgp + (k & 3) * gpad + cta),
-                     "r"(v) : "memory");
-        asm volatile("st.relaxed.gpu.global.u32 [%0], %1;"
-                     ::"l"(a.lgp + ((k + 2) & 3) * gpad + cta), "r"(kNoSum) : "memory");
+        unsigned long long v = (unsigned long long)__double_as_longlong(part);
+        if (v == kNoPart) v = kNoPart >> 1;  // another NaN
+        st_relaxed_gpu(a.lgp + (k & 3) * gpad + cta, v);
+        st_relaxed_gpu(a.lgp + ((k + 2) & 3) * gpad + cta, kNoPart);
       }
       __syncwarp();
       cta_scatter_wait();

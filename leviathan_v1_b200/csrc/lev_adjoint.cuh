@@ -30,6 +30,11 @@
 //   prep: lam_eps -> lam_diff = lam_eps cos(diff);  lam_th(s) += lam_diff;
 //     lam_thh(s) = lam_thh(s+1) - lam_diff;  lam_omh(s) = lam_omh(s+1) + dt lam_thh(s+1)
 //   lam_g(s)   = lam_g(s+1) dg(s+1)/dg(s) + sum_i lam_th'_i dt S_i
+// lam_th and lam_g are carried from step to step in float64 (one value per node,
+// one per network): the terms of lam_g cancel to a small part of their size (N =
+// 2,000, k = 12: to 1/30), and carried in float32 dL/dK followed the roundings
+// that the order of the scatters sets off: 2.2e-6 of its value from run to run, 1.0e-6
+// now (grid-resident 0.7e-6), for 1 % of a reverse step's time.
 // The wraps have derivative 1; a clamped weight or gain passes nothing;
 // |eps| has derivative sign(eps).  The adjoint ring has max_delay+3 slots: the
 // slot finalised by a reverse step (time s+1) is not one that the same step
@@ -482,15 +487,15 @@ struct AdjBwdArgs {
   const float4 *trace; // per network (g_s, r_{s+1}, sum cos, sum sin)
   const float *dLdr;   // per network dL/dr(s+1), or null
   const float *dLdth;  // [total nodes] dL/dtheta(s+1), or null
-  float *lam_th;       // current-phase adjoint: in time s+1, out time s
+  double *lam_th;      // current-phase adjoint: in time s+1, out time s
   float *lam_thh;
   float *lam_omh;
   float *lam_w;        // SELL
   float *adj_ring;
-  float *lam_g;        // per network: in lam_g(s+1), out lam_g(s)
+  double *lam_g;       // per network: in lam_g(s+1), out lam_g(s)
   float *grad_omega;   // accumulated
   float *grad_drive;   // [total nodes] for step s, or null
-  float2 *partials;    // per tile (lam_g partial, unused)
+  double *partials;    // lam_g partial per tile
   unsigned *tickets;   // per network
   // reservoir terms (see AdjFwdArgs); all may be null
   const float *win;
@@ -515,7 +520,7 @@ __device__ __forceinline__ int pos_mod(long long x, int m) {
 // per SM the register budget is sized for.
 template <int MATH, int U, int MINB>
 __global__ void __launch_bounds__(kTile, MINB) adj_bwd_kernel(const AdjBwdArgs a) {
-  __shared__ float s_red[32];
+  __shared__ double s_red[32];
   __shared__ int s_last;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int2 tile = a.tiles[blockIdx.x];
@@ -542,30 +547,32 @@ __global__ void __launch_bounds__(kTile, MINB) adj_bwd_kernel(const AdjBwdArgs a
     dgdr = free ? -dt * nd.beta : 0.0f;
     dgdg = free ? 1.0f - dt * nd.mu : 0.0f;
   }
-  const float lam_g1 = a.lam_g[tile.x];
-  const float lam_r = (a.dLdr ? a.dLdr[tile.x] : 0.0f) + lam_g1 * dgdr;
+  const double lam_g1 = a.lam_g[tile.x];
+  const float lam_r = (a.dLdr ? a.dLdr[tile.x] : 0.0f) + (float)lam_g1 * dgdr;
   const float invN = 1.0f / (float)N;
   const float Cm = tr.z * invN, Sm = tr.w * invN;
 
-  float lg_part = 0.0f;
+  double lg_part = 0.0;
   float lt1 = 0.0f, th = 0.0f, eps = 0.0f, diff = 0.0f, lam_S = 0.0f;
   int deg = 0;
   if (live) {
     // (A) adjoint of theta(s+1), complete
     const float th1 = H[(long long)(hs + 1) * Np + row];
     float* slot_next = AR + (long long)as_next * Np + row;
-    lt1 = a.lam_th[gi] + *slot_next;
+    double ltd = a.lam_th[gi] + *slot_next;
     *slot_next = 0.0f;
     float sn, cs;
     sincosf(th1, &sn, &cs);
-    if (r1 > 0.0f) lt1 += lam_r * (Sm * cs - Cm * sn) * invN / r1;
-    if (a.dLdth) lt1 += a.dLdth[gi];
+    if (r1 > 0.0f) ltd += lam_r * (Sm * cs - Cm * sn) * invN / r1;
+    if (a.dLdth) ltd += a.dLdth[gi];
     if (a.dLdy) {  // readout y = sum ra cos theta + rb sin theta
       const float gy = a.dLdy[tile.x];
-      lt1 += gy * (a.rb[gi] * cs - a.ra[gi] * sn);
+      ltd += gy * (a.rb[gi] * cs - a.ra[gi] * sn);
       a.grad_ra[gi] += gy * cs;
       a.grad_rb[gi] += gy * sn;
     }
+    a.lam_th[gi] = ltd;  // read back below: no registers held over the walk
+    lt1 = (float)ltd;
     // (B) integrate
     lam_S = lt1 * dt * g_s;
     a.grad_omega[gi] += lt1 * dt;
@@ -582,7 +589,7 @@ __global__ void __launch_bounds__(kTile, MINB) adj_bwd_kernel(const AdjBwdArgs a
                          nd.w_min, nd.w_max};
   const float decay = 1.0f - dt * nd.lam;
   const float hq = dt * nd.eta * ep.hebb;
-  float S_i = 0.0f, lth = lt1, labs = 0.0f;
+  float S_i = 0.0f, lsum = 0.0f, labs = 0.0f;
   const int slice_row0 = row0 + 32 * warp;
   if (slice_row0 < N) {
     const long long s = nd.slice_base + (slice_row0 >> 5);
@@ -622,7 +629,7 @@ __global__ void __launch_bounds__(kTile, MINB) adj_bwd_kernel(const AdjBwdArgs a
         if (k0 + u < deg) {
           S_i += w * sn[u];
           labs += m * cs[u];
-          lth -= lD;
+          lsum -= lD;
           a.lam_w[base + 32 * (k0 + u)] = m * decay + lam_S * sn[u];
           const unsigned s0 = (unsigned)(as_s - (int)(p[u] & 255u));
           atomicAdd(AR + (min(s0, s0 + (unsigned)bsa) * (unsigned)Np + (p[u] >> 8)), lD);
@@ -637,11 +644,10 @@ __global__ void __launch_bounds__(kTile, MINB) adj_bwd_kernel(const AdjBwdArgs a
     const float lthh1 = a.lam_thh[gi], lomh1 = a.lam_omh[gi];
     const float leps = -lt1 * dt * nd.alpha + labs * sgn + lomh1 * nd.kappa_w * dt;
     const float ldiff = leps * cosf(diff);
-    lth += ldiff;
-    a.lam_th[gi] = lth;
+    a.lam_th[gi] += lsum + ldiff;
     a.lam_thh[gi] = lthh1 - ldiff;
     a.lam_omh[gi] = lomh1 + lthh1 * dt;
-    lg_part = lt1 * dt * S_i;
+    lg_part = (double)lt1 * dt * S_i;
   }
   // (E) lam_g(s) = lam_g(s+1) dg/dg + sum_i lam_th'_i dt S_i
   const unsigned mask = 0xffffffffu;
@@ -650,11 +656,11 @@ __global__ void __launch_bounds__(kTile, MINB) adj_bwd_kernel(const AdjBwdArgs a
   if (lane == 0) s_red[warp] = lg_part;
   __syncthreads();
   if (warp == 0) {
-    lg_part = (lane < kTile / 32) ? s_red[lane] : 0.0f;
+    lg_part = (lane < kTile / 32) ? s_red[lane] : 0.0;
 #pragma unroll
     for (int off = 16; off > 0; off /= 2) lg_part += __shfl_down_sync(mask, lg_part, off);
     if (lane == 0) {
-      a.partials[nd.part_off + row0 / kTile] = make_float2(lg_part, 0.0f);
+      a.partials[nd.part_off + row0 / kTile] = lg_part;
       __threadfence();
       const unsigned prev = atomicAdd(a.tickets + tile.x, 1u);
       s_last = (prev == (unsigned)(nd.ntiles - 1));
@@ -664,9 +670,9 @@ __global__ void __launch_bounds__(kTile, MINB) adj_bwd_kernel(const AdjBwdArgs a
   if (!s_last) return;
   __threadfence();
   if (warp == 0) {
-    float sum = 0.0f;
-    const float2 *part = a.partials + nd.part_off;
-    for (int k = lane; k < nd.ntiles; k += 32) sum += __ldcg(part + k).x;
+    double sum = 0.0;
+    const double *part = a.partials + nd.part_off;
+    for (int k = lane; k < nd.ntiles; k += 32) sum += __ldcg(part + k);
 #pragma unroll
     for (int off = 16; off > 0; off /= 2) sum += __shfl_down_sync(mask, sum, off);
     if (lane == 0) {
@@ -687,7 +693,7 @@ __global__ void __launch_bounds__(kTile, MINB) adj_bwd_kernel(const AdjBwdArgs a
 template <int MATH, int LPR, int U>
 __global__ void __launch_bounds__(kTile, 4) adj_bwd_split_kernel(const AdjBwdArgs a) {
   constexpr int RPC = kTile / LPR;  // rows per CTA
-  __shared__ float s_red[32];
+  __shared__ double s_red[32];
   __shared__ int s_last;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int sub = blockIdx.x % LPR;
@@ -716,12 +722,13 @@ __global__ void __launch_bounds__(kTile, 4) adj_bwd_split_kernel(const AdjBwdArg
     dgdr = free ? -dt * nd.beta : 0.0f;
     dgdg = free ? 1.0f - dt * nd.mu : 0.0f;
   }
-  const float lam_g1 = a.lam_g[tile.x];
-  const float lam_r = (a.dLdr ? a.dLdr[tile.x] : 0.0f) + lam_g1 * dgdr;
+  const double lam_g1 = a.lam_g[tile.x];
+  const float lam_r = (a.dLdr ? a.dLdr[tile.x] : 0.0f) + (float)lam_g1 * dgdr;
   const float invN = 1.0f / (float)N;
   const float Cm = tr.z * invN, Sm = tr.w * invN;
 
-  float lg_part = 0.0f;
+  double lg_part = 0.0;
+  double ltd = 0.0;  // lam_th', on the row's first lane
   float lt1 = 0.0f, th = 0.0f, eps = 0.0f, diff = 0.0f;
   int deg = 0;
   if (live) {
@@ -734,18 +741,19 @@ __global__ void __launch_bounds__(kTile, 4) adj_bwd_split_kernel(const AdjBwdArg
       // (A) adjoint of theta(s+1), complete; (B) integrate
       const float th1 = H[(long long)(hs + 1) * Np + row];
       float *slot_next = AR + (long long)as_next * Np + row;
-      lt1 = a.lam_th[gi] + *slot_next;
+      ltd = a.lam_th[gi] + *slot_next;
       *slot_next = 0.0f;
       float sn, cs;
       sincosf(th1, &sn, &cs);
-      if (r1 > 0.0f) lt1 += lam_r * (Sm * cs - Cm * sn) * invN / r1;
-      if (a.dLdth) lt1 += a.dLdth[gi];
+      if (r1 > 0.0f) ltd += lam_r * (Sm * cs - Cm * sn) * invN / r1;
+      if (a.dLdth) ltd += a.dLdth[gi];
       if (a.dLdy) {
         const float gy = a.dLdy[tile.x];
-        lt1 += gy * (a.rb[gi] * cs - a.ra[gi] * sn);
+        ltd += gy * (a.rb[gi] * cs - a.ra[gi] * sn);
         a.grad_ra[gi] += gy * cs;
         a.grad_rb[gi] += gy * sn;
       }
+      lt1 = (float)ltd;
       a.grad_omega[gi] += lt1 * dt;
       if (a.grad_drive) a.grad_drive[gi] = lt1 * dt;
       if (a.grad_win) a.grad_win[gi] += lt1 * dt * a.xin[tile.x];
@@ -817,10 +825,10 @@ __global__ void __launch_bounds__(kTile, 4) adj_bwd_split_kernel(const AdjBwdArg
     const float lthh1 = a.lam_thh[gi], lomh1 = a.lam_omh[gi];
     const float leps = -lt1 * dt * nd.alpha + labs * sgn + lomh1 * nd.kappa_w * dt;
     const float ldiff = leps * cosf(diff);
-    a.lam_th[gi] = lt1 + lsum + ldiff;
+    a.lam_th[gi] = ltd + (lsum + ldiff);
     a.lam_thh[gi] = lthh1 - ldiff;
     a.lam_omh[gi] = lomh1 + lthh1 * dt;
-    lg_part = lt1 * dt * S_i;
+    lg_part = (double)lt1 * dt * S_i;
   }
   // (E) lam_g(s) = lam_g(s+1) dg/dg + sum_i lam_th'_i dt S_i
 #pragma unroll
@@ -829,12 +837,11 @@ __global__ void __launch_bounds__(kTile, 4) adj_bwd_split_kernel(const AdjBwdArg
   __syncthreads();
   const int nparts = nd.ntiles * LPR;
   if (warp == 0) {
-    lg_part = (lane < kTile / 32) ? s_red[lane] : 0.0f;
+    lg_part = (lane < kTile / 32) ? s_red[lane] : 0.0;
 #pragma unroll
     for (int off = 16; off > 0; off /= 2) lg_part += __shfl_down_sync(mask, lg_part, off);
     if (lane == 0) {
-      a.partials[(long long)nd.part_off * LPR + (row0 / kTile) * LPR + sub] =
-          make_float2(lg_part, 0.0f);
+      a.partials[(long long)nd.part_off * LPR + (row0 / kTile) * LPR + sub] = lg_part;
       __threadfence();
       const unsigned prev = atomicAdd(a.tickets + tile.x, 1u);
       s_last = (prev == (unsigned)(nparts - 1));
@@ -844,9 +851,9 @@ __global__ void __launch_bounds__(kTile, 4) adj_bwd_split_kernel(const AdjBwdArg
   if (!s_last) return;
   __threadfence();
   if (warp == 0) {
-    float sum = 0.0f;
-    const float2 *part = a.partials + (long long)nd.part_off * LPR;
-    for (int k = lane; k < nparts; k += 32) sum += __ldcg(part + k).x;
+    double sum = 0.0;
+    const double *part = a.partials + (long long)nd.part_off * LPR;
+    for (int k = lane; k < nparts; k += 32) sum += __ldcg(part + k);
 #pragma unroll
     for (int off = 16; off > 0; off /= 2) sum += __shfl_down_sync(mask, sum, off);
     if (lane == 0) {
@@ -890,7 +897,7 @@ __global__ void adj_ring_ckpt_kernel(int mode, const NetDesc *__restrict__ nets,
 // Final adjoint of theta(0): current part plus every adjoint-ring slot (reads
 // of times <= 0 all read theta(0), the value every slot starts with).
 __global__ void adj_finalize_kernel(const NetDesc *nets, int num_nets,
-                                    const float *lam_th, const float *adj_ring,
+                                    const double *lam_th, const float *adj_ring,
                                     float *grad_theta0) {
   const int n = blockIdx.y;
   if (n >= num_nets) return;
@@ -898,9 +905,9 @@ __global__ void adj_finalize_kernel(const NetDesc *nets, int num_nets,
   const int bsa = adj_slots(nd.max_delay);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nd.N;
        i += gridDim.x * blockDim.x) {
-    float v = lam_th[nd.node_off + i];
+    double v = lam_th[nd.node_off + i];
     for (int s = 0; s < bsa; ++s) v += adj_ring[nd.aux_off + (long long)s * nd.Np + i];
-    grad_theta0[nd.node_off + i] = v;
+    grad_theta0[nd.node_off + i] = (float)v;
   }
 }
 
@@ -908,6 +915,11 @@ __global__ void add_kernel(float *dst, const float *src, long long n) {
   for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n;
        k += (long long)gridDim.x * blockDim.x)
     dst[k] += src[k];
+}
+
+// dL/dK of every network: lam_g of the run's first step.
+__global__ void lam_g_kernel(float *grad_K, const double *lam_g, int num_nets) {
+  for (int n = threadIdx.x; n < num_nets; n += blockDim.x) grad_K[n] = (float)lam_g[n];
 }
 
 }  // namespace lev

@@ -3311,7 +3311,8 @@ struct LevAdjoint {
   float *theta0 = nullptr, *theta_hat0 = nullptr;
   float *theta = nullptr, *theta_hat = nullptr, *omega = nullptr,
         *omega_hat = nullptr, *w = nullptr, *ring = nullptr;
-  float2 *partials = nullptr, *bpart = nullptr;
+  float2 *partials = nullptr;
+  double *bpart = nullptr;
   unsigned *tickets = nullptr;
   float *ck_theta = nullptr, *ck_thh = nullptr, *ck_omh = nullptr,
         *ck_w = nullptr, *ck_ring = nullptr, *ck_g = nullptr;
@@ -3329,9 +3330,10 @@ struct LevAdjoint {
   cudaStream_t rstream = nullptr;
   cudaEvent_t ev_rec[2] = {nullptr, nullptr}, ev_rev[2] = {nullptr, nullptr},
               ev_start = nullptr;
-  float *lam_th = nullptr, *lam_thh = nullptr, *lam_omh = nullptr,
-        *lam_w = nullptr, *adj_ring = nullptr, *lam_g = nullptr,
+  float *lam_thh = nullptr, *lam_omh = nullptr,
+        *lam_w = nullptr, *adj_ring = nullptr,
         *grad_omega_acc = nullptr, *grad_theta0 = nullptr;
+  double *lam_th = nullptr, *lam_g = nullptr;
   std::vector<void *> allocs;
   size_t bytes = 0;
   int last_T = 0;
@@ -3360,7 +3362,7 @@ struct LevAdjoint {
   bool use_pair = true;
   int g_gpad = 0;
   float2 *g_wsum = nullptr;
-  float *g_lgp = nullptr;
+  double *g_lgp = nullptr;
   unsigned *g_bar = nullptr;
   int *h_gerr = nullptr, *d_gerr = nullptr;
   GridWait grid_wait = {kGridWaitNs, 0u, 0u};  // bound of the barrier waits
@@ -3564,9 +3566,9 @@ int adj_setup_grid(LevAdjoint *a, const std::vector<long long> &sl_off,
   // clears what it uses with two fills
   a->g_gpad = max_gpad;
   int rc = adj_alloc(a, &a->g_bar, 3 * kGridBarPitch);
-  if (rc == LEV_OK) rc = adj_alloc(a, &a->g_wsum, 32LL * d.ntiles + 2LL * max_gpad);
+  if (rc == LEV_OK) rc = adj_alloc(a, &a->g_wsum, 32LL * d.ntiles + 4LL * max_gpad);
   if (rc != LEV_OK) return rc;
-  a->g_lgp = reinterpret_cast<float *>(a->g_wsum + 32LL * d.ntiles);
+  a->g_lgp = reinterpret_cast<double *>(a->g_wsum + 32LL * d.ntiles);
   a->h_gerr = reinterpret_cast<int *>(mapped_alloc(1));
   if (!a->h_gerr) return fail(LEV_ERR_NOMEM, "mapped host memory: allocation failed");
   *a->h_gerr = 0;
@@ -3632,7 +3634,7 @@ cudaError_t adj_grid_clear(LevAdjoint *a, cudaStream_t s) {
   if (e == cudaSuccess)
     e = cudaMemsetAsync(a->g_wsum, 0xff,
                         sizeof(float2) * (32 * (size_t)a->h_nets[0].ntiles +
-                                          2 * (size_t)a->g_gpad), s);
+                                          4 * (size_t)a->g_gpad), s);
   return e;
 }
 
@@ -4032,13 +4034,13 @@ int lev_adj_backward(LevAdjoint *a, const float *dLdr, const float *dLdtheta,
   const float dt = a->last_dt;
   const size_t nb = sizeof(float) * a->TN;
   const size_t wb = sizeof(float) * std::max<long long>(a->SL, 1);
-  LEV_TRY_CUDA(cudaMemsetAsync(a->lam_th, 0, nb, s));
+  LEV_TRY_CUDA(cudaMemsetAsync(a->lam_th, 0, 2 * nb, s));
   LEV_TRY_CUDA(cudaMemsetAsync(a->lam_thh, 0, nb, s));
   LEV_TRY_CUDA(cudaMemsetAsync(a->lam_omh, 0, nb, s));
   LEV_TRY_CUDA(cudaMemsetAsync(a->grad_omega_acc, 0, nb, s));
   LEV_TRY_CUDA(cudaMemsetAsync(a->lam_w, 0, wb, s));
   LEV_TRY_CUDA(cudaMemsetAsync(a->adj_ring, 0, sizeof(float) * std::max<long long>(a->aux_floats, 1), s));
-  LEV_TRY_CUDA(cudaMemsetAsync(a->lam_g, 0, sizeof(float) * a->NN, s));
+  LEV_TRY_CUDA(cudaMemsetAsync(a->lam_g, 0, sizeof(double) * a->NN, s));
   LEV_TRY_CUDA(cudaMemsetAsync(a->tickets, 0, sizeof(unsigned) * a->NN, s));
   if (a->res_gwin) LEV_TRY_CUDA(cudaMemsetAsync(a->res_gwin, 0, nb, s));
   if (a->res_gra) LEV_TRY_CUDA(cudaMemsetAsync(a->res_gra, 0, nb, s));
@@ -4269,9 +4271,7 @@ int lev_adj_backward(LevAdjoint *a, const float *dLdr, const float *dLdtheta,
   if (grad_w0_csr)
     sell_weights_kernel<<<e->total_tiles, kTile, 0, s>>>(
         1, e->d_nets, e->d_tiles, e->d_row_ptr, e->d_sl_off, e->d_sl_len, grad_w0_csr, a->lam_w);
-  if (grad_K)
-    LEV_TRY_CUDA(cudaMemcpyAsync(grad_K, a->lam_g, sizeof(float) * a->NN,
-                                 cudaMemcpyDeviceToDevice, s));
+  if (grad_K) lam_g_kernel<<<1, 128, 0, s>>>(grad_K, a->lam_g, a->NN);
   LEV_TRY_CUDA(cudaGetLastError());
   LEV_TRY_CUDA(cudaStreamSynchronize(s));
   return adj_grid_check(a);
