@@ -2721,6 +2721,11 @@ int lev_autotune(LevEngine *h, float dt, int32_t trial_steps,
     return fail(LEV_ERR_NOMEM, "autotune: no room for a state snapshot");
   }
   int rc = snapshot_copy(h, snap, true);
+  // the trials are no steps of the simulation: an attached monitor does not see
+  // them (recorded blocks name the monitor)
+  LevHubs *const hubs = h->hubs;
+  h->hubs = nullptr;
+  clear_graphs(h);
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (rc == LEV_OK && (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess))
     rc = fail(LEV_ERR_CUDA, "autotune: event creation failed");
@@ -2851,7 +2856,7 @@ int lev_autotune(LevEngine *h, float dt, int32_t trial_steps,
         if (h->classes[c].ntiles > 0) h->classes[c].pair_variant = best_v >= 0 ? best_v : own[c];
     }
   }
-  // small and mid-sized single networks: per-step graph replay, the
+  // small and mid-sized networks and batches: per-step graph replay, the
   // cluster-resident kernel or the grid-resident kernel (each rows-per-CTA
   // choice), whichever is fastest
   if (rc == LEV_OK && (h->cluster_ok || h->grid_ok)) {
@@ -2860,7 +2865,7 @@ int lev_autotune(LevEngine *h, float dt, int32_t trial_steps,
     float best_t = -1.0f;
     int best_m = 0;
     for (int m = 0; m < 5 && rc == LEV_OK; ++m) {
-      if (m == 1 && !h->cluster_ok) continue;
+      if (m == 1 && (!h->cluster_ok || (hubs && h->cluster_R > 128))) continue;
       if (m >= 2 && !h->grid_R_ok[m - 2]) continue;
       h->use_cluster = (m == 1);
       h->use_grid = (m >= 2);
@@ -2892,6 +2897,7 @@ int lev_autotune(LevEngine *h, float dt, int32_t trial_steps,
   else snapshot_copy(h, snap, false);
   snap.release();
   clear_graphs(h);
+  h->hubs = hubs;
   return rc;
 }
 

@@ -154,3 +154,35 @@ def test_batch_engine_observes_one_network():
     m.close()
     be.close()
     e.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("Ns", [(1000,), (3000,), (600, 1500)])
+def test_autotune_is_not_observed(Ns):
+    """The trials of autotune are undone in the state, so an attached monitor
+    must not count them: as the same steps without autotune."""
+    from leviathan_v1_b200 import BatchEngine, HubTransitions, LeviathanEngine
+    from leviathan_v1_b200.graphs import make_network
+
+    nets = [make_network(n, 8, 0.1, 20, seed=n, delay_lo=1) for n in Ns]
+    out = []
+    for tune in (False, True):
+        e = (LeviathanEngine(*nets[0].engine_args()) if len(nets) == 1
+             else BatchEngine([n.as_dict() for n in nets]))
+        m = HubTransitions([0, Ns[0] - 1, 255, 256])
+        m.attach(e)
+        for _ in range(3):  # issued directly, recorded, replayed
+            e.step_n(0.05, 32)
+        if tune:
+            before = m.read()
+            e.autotune(0.05, 32)
+            for a, b in zip(m.read(), before):
+                np.testing.assert_array_equal(a, b)
+        e.step_n(0.05, 40)
+        e.step(0.05)
+        out.append(m.read())  # right after a single step
+        m.close()
+        e.close()
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
+    assert out[0][3] == 3 * 32 + 41
