@@ -155,7 +155,11 @@ int lev_net_shape(const LevEngine *h, int32_t net, int32_t *N, int64_t *E,
  * (leviathan_kernel.cu:391-438): predictor, delayed gather + coupling +
  * Hebbian update, integration + ring write, order parameter r, gain
  * controller.  r_out[num_nets] receives r of theta(t+1) per network
- * (may be NULL).  Synchronous, like the reference.  When every degree class
+ * (may be NULL).  Returns when r has arrived, a few microseconds before the
+ * last stores of the step (state words, hub counts) are through: every call of
+ * this library is ordered after them, and so is work on the engine's stream
+ * (lev_get_stream); for other streams lev_sync comes between.  An error of the
+ * device that shows after r is reported by a later call.  When every degree class
  * takes two steps per launch, a call that starts a pair also computes the
  * next step up to its integrate into shadow buffers (the engine state is
  * exactly that after this step); the next call, with the same dt and no

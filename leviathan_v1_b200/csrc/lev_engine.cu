@@ -1977,13 +1977,9 @@ static int wait_r(LevEngine *h) {
   return LEV_OK;
 }
 
-int lev_step(LevEngine *h, float dt, float *r_out) {
-  if (!h) return fail(LEV_ERR_ARG, "null handle");
-  if (h->part) return fail(LEV_ERR_STATE, "partition engine: step with lev_part_step_begin / lev_part_step_end");
-  if (!std::isfinite(dt)) return fail(LEV_ERR_ARG, "dt is not finite");
-  DeviceScope ds(h->device);
+// The launches of one single step; on an error some may be under way.
+static int launch_single(LevEngine *h, float dt) {
   StepArgs a = make_args(h, dt, nullptr, 0, h->d_rmap);
-  mark_r(h);
   int rc = LEV_OK;
   uint32_t dbits;
   std::memcpy(&dbits, &dt, 4);
@@ -2040,11 +2036,24 @@ int lev_step(LevEngine *h, float dt, float *r_out) {
       h->spec_dt = dbits;
     }
   } else {
-    rc = launch_step(h, a);
-    if (rc != LEV_OK) return rc;
+    return launch_step(h, a);
   }
-  rc = wait_r(h);
-  if (rc != LEV_OK) return rc;
+  return LEV_OK;
+}
+
+int lev_step(LevEngine *h, float dt, float *r_out) {
+  if (!h) return fail(LEV_ERR_ARG, "null handle");
+  if (h->part) return fail(LEV_ERR_STATE, "partition engine: step with lev_part_step_begin / lev_part_step_end");
+  if (!std::isfinite(dt)) return fail(LEV_ERR_ARG, "dt is not finite");
+  DeviceScope ds(h->device);
+  mark_r(h);
+  int rc = launch_single(h, dt);
+  if (rc == LEV_OK) rc = wait_r(h);
+  if (rc != LEV_OK) {
+    // an r that is still to come must not be taken for the next step's
+    cudaStreamSynchronize(h->stream);
+    return rc;
+  }
   if (r_out) {
     const volatile float *src = h->h_rmap;
     for (int n = 0; n < h->num_nets; ++n) r_out[n] = src[n];

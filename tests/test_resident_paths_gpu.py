@@ -447,3 +447,29 @@ def test_long_pair_chains_with_dependent_launches(N):
     np.testing.assert_array_equal(np.concatenate(r).astype(np.float32), want_r)
     _same(_state(e), want)
     e.close()
+
+
+@pytest.mark.parametrize("batch", [False, True])
+def test_calls_right_after_a_single_step(batch):
+    """step() returns when r has arrived; what is called next is ordered after
+    the step all the same: hub counts, state, a new adjoint, close."""
+    nets = [make_network(n, 8, 0.1, 20, seed=n, delay_lo=1) for n in (700, 1500)]
+    for i in range(20):
+        def make():
+            return (BatchEngine([n.as_dict() for n in nets]) if batch
+                    else LeviathanEngine(*nets[i % 2].engine_args()))
+        ref = _per_step(make())
+        want_r = ref.step_n(DT, 1 + i % 3)[-1]
+        want = _state(ref)
+        ref.close()
+        e = make()
+        m = HubTransitions([0, 31, 256])
+        m.attach(e)
+        for _ in range(1 + i % 3):
+            r = e.step(DT)
+        assert m.read()[3] == 1 + i % 3
+        np.testing.assert_array_equal(np.float32(r), want_r)
+        _same(_state(e), want)
+        e.step(DT)
+        e.close()
+        m.close()
