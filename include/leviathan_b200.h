@@ -284,7 +284,7 @@ int lev_set_cluster_mode(LevEngine *h, int32_t enabled);
  * lev_step_n / lev_sync return LEV_ERR_CUDA and disables the path.  Results are bitwise those of the
  * per-step kernel.  The cluster path takes precedence when both are enabled.
  * lev_grid_info: enabled = eligible and allowed (the path step blocks use;
- * 0 after a timeout); rows_per_cta in use; eligible_rows_mask = OR of the
+ * 0 after a timeout); ctas of one launch, over all networks; rows_per_cta in use; eligible_rows_mask = OR of the
  * eligible rows-per-CTA values.  lev_set_grid_mode: enabled 0 forces the
  * per-step kernel; rows_per_cta 0 keeps the current choice. */
 int lev_grid_info(const LevEngine *h, int32_t *eligible, int32_t *enabled, int32_t *ctas,

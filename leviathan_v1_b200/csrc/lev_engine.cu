@@ -2484,7 +2484,7 @@ int lev_grid_info(const LevEngine *h, int32_t *eligible, int32_t *enabled, int32
   const int ri = grid_r_index(R);
   if (eligible) *eligible = h->grid_ok ? 1 : 0;
   if (enabled) *enabled = (h->grid_ok && h->use_grid) ? 1 : 0;  // in use by step blocks
-  if (ctas) *ctas = (h->grid_ok && R > 0) ? (h->h_nets[0].N + R - 1) / R : 0;
+  if (ctas) *ctas = (h->grid_ok && R > 0) ? (int32_t)grid_ctas(h, R) : 0;
   if (rows_per_cta) *rows_per_cta = h->grid_ok ? R : 0;
   if (smem_bytes) *smem_bytes = h->grid_ok ? (int64_t)h->grid_smem_R[ri] : 0;
   if (eligible_rows_mask) {

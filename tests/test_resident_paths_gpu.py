@@ -473,3 +473,14 @@ def test_calls_right_after_a_single_step(batch):
         e.step(DT)
         e.close()
         m.close()
+
+
+def test_grid_info_counts_the_ctas_of_every_network():
+    sizes = (700, 64, 1500, 1)
+    e = BatchEngine([make_network(n, 4, 0.1, 6, seed=n, delay_lo=1).as_dict() if n > 1
+                     else _from_degrees(np.zeros(1, int), 3, 1).as_dict() for n in sizes])
+    for R in e.grid_info()["eligible_rows"]:
+        e.set_grid_mode(True, R)
+        info = e.grid_info()
+        assert info["rows_per_cta"] == R and info["ctas"] == sum(-(-n // R) for n in sizes)
+    e.close()
