@@ -1652,11 +1652,21 @@ int create_impl(LevEngine **out, int num_nets, const int32_t *Ns,
         len_sum += h->classes[c].mean_len * h->classes[c].ntiles;
       const int pv = default_pair_variant(h->total_tiles, len_sum / std::max(h->total_tiles, 1));
       std::lock_guard<std::mutex> lk(g_tune_mu);
+      // a class without one goes with the largest that has: with one variant
+      // for all the classes run merged
+      int common = pv, common_tiles = 0;
+      for (int c = 0; c < kNumClasses; ++c) {
+        const TileClass &tc = h->classes[c];
+        auto ip = g_pair_cache.find(tune_key(tc, c));
+        if (ip == g_pair_cache.end() || ip->second < 0 || tc.ntiles <= common_tiles) continue;
+        common = ip->second;
+        common_tiles = tc.ntiles;
+      }
       for (int c = 0; c < kNumClasses; ++c) {
         auto it = g_tune_cache.find(tune_key(h->classes[c], c));
         h->classes[c].variant = (it != g_tune_cache.end()) ? it->second : 0;
         auto ip = g_pair_cache.find(tune_key(h->classes[c], c));
-        h->classes[c].pair_variant = (ip != g_pair_cache.end()) ? ip->second : pv;
+        h->classes[c].pair_variant = (ip != g_pair_cache.end()) ? ip->second : common;
       }
     }
 
@@ -2739,6 +2749,7 @@ int lev_autotune(LevEngine *h, float dt, int32_t trial_steps,
   if (rc == LEV_OK && (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess))
     rc = fail(LEV_ERR_CUDA, "autotune: event creation failed");
   StepArgs a = make_args(h, dt, nullptr, 0, nullptr);
+  float pair_ms[kNumClasses][kNumPairVariants] = {};
   for (int c = 0; c < kNumClasses && rc == LEV_OK; ++c) {
     TileClass &tc = h->classes[c];
     if (tc.ntiles == 0) {
@@ -2805,6 +2816,7 @@ int lev_autotune(LevEngine *h, float dt, int32_t trial_steps,
         float ms = 0.0f;
         cudaEventElapsedTime(&ms, e0, e1);
         ms /= 2.0f * pairs;
+        pair_ms[c][v] = ms;
         if (best_pv < 0 || ms < best_p) {
           best_p = ms;
           best_pv = v;
@@ -2813,56 +2825,60 @@ int lev_autotune(LevEngine *h, float dt, int32_t trial_steps,
       tc.pair_ms = best_p;
       tc.pair_variant = (best_pv >= 0 && best_p < best) ? best_pv : -1;
     }
-    std::lock_guard<std::mutex> lk(g_tune_mu);
-    g_tune_cache[tune_key(tc, c)] = best_v;
-    if (h->pair_ok) g_pair_cache[tune_key(tc, c)] = tc.pair_variant;
   }
-  // classes that chose different pair variants run as one chain of launches
-  // each; with one variant for all they run merged (merged_pairs).  Time both
-  // and keep the faster.
+  // Classes that chose different pair variants run as one chain of launches
+  // each, side by side; with one variant for all they run merged (merged_pairs).
+  // Both are timed as the blocks of steps run them.
   {
     TileClass merged;
     int busy = 0;
-    bool pairs = rc == LEV_OK && h->pair_ok;
-    float apart = 0.0f;
-    int own[kNumClasses];
+    bool pairs = rc == LEV_OK && pairs_all(h);
+    int best[kNumClasses];
     for (int c = 0; c < kNumClasses; ++c) {
-      own[c] = h->classes[c].pair_variant;
-      if (h->classes[c].ntiles == 0) continue;
-      ++busy;
-      pairs = pairs && own[c] >= 0;
-      apart += h->classes[c].pair_ms;
+      best[c] = h->classes[c].pair_variant;
+      busy += h->classes[c].ntiles > 0;
     }
     if (pairs && busy > 1 && !merged_pairs(h, &merged)) {
-      int best_v = -1;
-      for (int v = 0; v < kNumPairVariants && rc == LEV_OK; ++v) {
-        bool used = false;  // the choice of some class
+      const bool cluster = h->use_cluster, grid = h->use_grid;
+      h->use_cluster = h->use_grid = false;
+      const int n = 2 * std::max(trial_steps, 16);
+      float best_t = -1.0f;
+      int own[kNumClasses];
+      std::copy(best, best + kNumClasses, own);
+      for (int v = -1; v < kNumPairVariants && rc == LEV_OK; ++v) {  // -1: the classes' own
+        bool used = v < 0;  // the choice of some class
         for (int c = 0; c < kNumClasses; ++c)
           used = used || (h->classes[c].ntiles > 0 && own[c] == v);
         if (!used) continue;
-        for (int c = 0; c < kNumClasses; ++c) h->classes[c].pair_variant = v;
-        merged_pairs(h, &merged);
-        float ms = 0.0f;
-        for (int round = 0; round < 2 && rc == LEV_OK; ++round) {  // warm-up, timed
+        for (int c = 0; c < kNumClasses; ++c)
+          if (h->classes[c].ntiles > 0) h->classes[c].pair_variant = v < 0 ? own[c] : v;
+        clear_graphs(h);
+        float t = 0.0f;
+        for (int round = 0; round < 3 && rc == LEV_OK; ++round) {  // issued, recorded, replayed
           cudaEventRecord(e0, h->stream);
-          for (int i = 0; i < 2 * trial_steps && rc == LEV_OK; ++i) {
-            a.reverse = i & 1;
-            rc = launch_pair_tc(h, merged, a, i & 1);
-          }
+          rc = enqueue_steps(h, dt, n, nullptr);
           cudaEventRecord(e1, h->stream);
-          if (rc == LEV_OK && cudaEventSynchronize(e1) != cudaSuccess)
+          if (rc == LEV_OK && (cudaEventSynchronize(e1) != cudaSuccess ||
+                               cudaEventElapsedTime(&t, e0, e1) != cudaSuccess))
             rc = fail(LEV_ERR_CUDA, "autotune: merged trial failed");
         }
-        if (rc != LEV_OK) break;
-        cudaEventElapsedTime(&ms, e0, e1);
-        ms /= 2.0f * trial_steps;
-        if (ms < apart) {
-          apart = ms;
-          best_v = v;
+        if (rc == LEV_OK && (best_t < 0.0f || t < best_t)) {
+          best_t = t;
+          for (int c = 0; c < kNumClasses; ++c) best[c] = h->classes[c].pair_variant;
         }
       }
-      for (int c = 0; c < kNumClasses; ++c)
-        if (h->classes[c].ntiles > 0) h->classes[c].pair_variant = best_v >= 0 ? best_v : own[c];
+      h->use_cluster = cluster;
+      h->use_grid = grid;
+    }
+    std::lock_guard<std::mutex> lk(g_tune_mu);
+    for (int c = 0; c < kNumClasses; ++c) {
+      TileClass &tc = h->classes[c];
+      if (tc.ntiles == 0) continue;
+      tc.pair_variant = best[c];
+      if (best[c] >= 0) tc.pair_ms = pair_ms[c][best[c]];
+      if (rc != LEV_OK) continue;
+      g_tune_cache[tune_key(tc, c)] = tc.variant;
+      if (h->pair_ok) g_pair_cache[tune_key(tc, c)] = tc.pair_variant;
     }
   }
   // small and mid-sized networks and batches: per-step graph replay, the

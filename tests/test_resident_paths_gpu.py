@@ -484,3 +484,34 @@ def test_grid_info_counts_the_ctas_of_every_network():
         info = e.grid_info()
         assert info["rows_per_cta"] == R and info["ctas"] == sum(-(-n // R) for n in sizes)
     e.close()
+
+
+def test_tuned_choices_reach_later_engines_together():
+    """What autotune settled on, one pair variant for all classes or one per class,
+    is what a later engine of the same networks starts with; networks of a class
+    that was never tuned go with the tuned ones."""
+    ring = [make_network(n, k, 0.1, 30, seed=n, delay_lo=1).as_dict()
+            for n, k in ((90_000, 6), (61_000, 16), (70_000, 40))]
+
+    e = BatchEngine(ring[:2])
+    e.autotune(DT, 8)
+    tuned = {c["cls"]: c for c in e.pair_info() if c["step_ms"] > 0.0}  # classes with networks
+    assert len(tuned) == 2
+    assert all(c["pair_ms"] > 0.0 for c in tuned.values())
+    e.close()
+    e = BatchEngine(ring[:2])
+    for c in e.pair_info():
+        if c["cls"] in tuned:
+            assert c["pair_variant"] == tuned[c["cls"]]["pair_variant"]
+    e.close()
+    e = BatchEngine(ring)
+    if all(c["pair_variant"] >= 0 for c in tuned.values()):
+        assert ({c["pair_variant"] for c in e.pair_info()}
+                <= {c["pair_variant"] for c in tuned.values()})
+    want_r = None
+    for per_step in (False, True):  # ... and the mixture runs as any other
+        b = _per_step(BatchEngine(ring)) if per_step else e
+        r = b.step_n(DT, 12)
+        want_r = r if want_r is None else want_r
+        np.testing.assert_array_equal(r, want_r)
+        b.close()
