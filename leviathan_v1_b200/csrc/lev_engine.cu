@@ -896,6 +896,32 @@ bool allow_smem(const void *fn, size_t bytes) {
   return true;
 }
 
+// How many CTAs of a kernel, of `threads` threads and `smem` bytes of dynamic
+// shared memory each, one SM holds; 0 if it refuses them.  The first look at a
+// kernel loads it (0.1 to 0.3 ms), so the answers are kept for the process.
+int ctas_per_sm(const void *fn, int threads, size_t smem) {
+  static std::mutex mu;
+  static std::map<std::tuple<int, const void *, int, size_t>, int> known;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+  const auto key = std::make_tuple(dev, fn, threads, smem);
+  {
+    std::lock_guard<std::mutex> lk(mu);
+    auto it = known.find(key);
+    if (it != known.end()) return it->second;
+  }
+  int n = 0;
+  if (!allow_smem(fn, smem) ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, threads, smem) != cudaSuccess) {
+    cudaGetLastError();  // clear a refused attribute
+    n = 0;
+  }
+  std::lock_guard<std::mutex> lk(mu);
+  if (known.size() >= 4096) known.clear();
+  known[key] = n;
+  return n;
+}
+
 // Small single networks: choose rows per CTA and check that the cluster
 // kernel can run (shared memory, cluster size, occupancy).
 void setup_cluster(LevEngine *h, const std::vector<int> &sl_len) {
@@ -1098,15 +1124,10 @@ int setup_grid(LevEngine *h, const std::vector<int> &sl_len) {
       for (int m = 0; m < 2 && ok; ++m) {
         const void *fn = reinterpret_cast<const void *>(
             grid_fn(R, m ? LEV_MATH_ACCURATE : LEV_MATH_REFERENCE, minb));
-        int per_sm = 0;
-        ok = allow_smem(fn, smem) &&
-             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, grid_threads(R, minb),
-                                                           smem) == cudaSuccess &&
-             (long long)per_sm * sms >= C;
+        ok = (long long)ctas_per_sm(fn, grid_threads(R, minb), smem) * sms >= C;
       }
       h->grid_minb[ri] = minb;
     }
-    cudaGetLastError();  // clear a refused attribute, if any
     if (!ok) continue;
     h->grid_R_ok[ri] = true;
     h->grid_cap[ri] = (int)cap;
@@ -3329,6 +3350,15 @@ __global__ void adj_state_kernel(int mode, const NetDesc *nets, NetState *st,
 
 }  // namespace lev
 
+// Which grid-resident adjoint kernels of one rows-per-CTA choice and math mode
+// can have all their CTAs resident: the CTAs per SM each is compiled for, 2 or
+// 3, or 0.  pair: the paired recompute + reverse launch.
+struct AdjFit {
+  bool looked = false;
+  int fwd = 0, bwd = 0, pair = 0;
+  bool ok() const { return fwd > 0 && bwd > 0; }
+};
+
 struct LevAdjoint {
   LevEngine *e = nullptr;
   int C = 50, Tmax = 0, nseg = 0;
@@ -3365,6 +3395,7 @@ struct LevAdjoint {
         *lam_w = nullptr, *adj_ring = nullptr,
         *grad_omega_acc = nullptr, *grad_theta0 = nullptr;
   double *lam_th = nullptr, *lam_g = nullptr;
+  std::vector<std::pair<void **, size_t>> wanted;  // see adj_commit
   std::vector<void *> allocs;
   size_t bytes = 0;
   int last_T = 0;
@@ -3384,12 +3415,12 @@ struct LevAdjoint {
   bool grid_ok = false;
   bool use_grid = true;
   int grid_R = 0;
-  bool gR_ok[3] = {false, false, false};  // R = 64, 128, 256
+  int sms = 0;
+  // per rows-per-CTA choice (64, 128, 256): SELL entries per CTA and shared
+  // memory, 0 where it cannot fit, and per math mode what fits
   int g_cap[3] = {0, 0, 0};
   size_t gf_smem[3] = {0, 0, 0}, gb_smem[3] = {0, 0, 0};
-  // CTAs per SM each kernel is compiled for; gp 0: the paired recompute +
-  // reverse launch does not fit
-  int gf_minb[3] = {0, 0, 0}, gb_minb[3] = {0, 0, 0}, gp_minb[3] = {0, 0, 0};
+  mutable AdjFit g_fit[2][3];
   bool use_pair = true;
   int g_gpad = 0;
   float2 *g_wsum = nullptr;
@@ -3401,17 +3432,32 @@ struct LevAdjoint {
 
 namespace {
 
+// Device arrays of an adjoint are asked for one by one (adj_alloc) and come out
+// of one driver allocation (adj_commit): thirty of them, each mapping and
+// unmapping blocks of its own, were most of a creation (N = 1,000 1.57 ms and
+// N = 10^4 3.9 then, 0.85 both now).
 template <typename T>
-int adj_alloc(LevAdjoint *a, T **p, long long count) {
-  size_t b = std::max<long long>(count, 1) * sizeof(T);
-  cudaError_t e = cudaMalloc(reinterpret_cast<void **>(p), b);
+void adj_alloc(LevAdjoint *a, T **p, long long count) {
+  a->wanted.emplace_back(reinterpret_cast<void **>(p), std::max<long long>(count, 1) * sizeof(T));
+}
+
+int adj_commit(LevAdjoint *a) {
+  size_t total = 0;
+  for (const auto &w : a->wanted) total += (w.second + 255) / 256 * 256;
+  char *base = nullptr;
+  cudaError_t e = cudaMalloc(reinterpret_cast<void **>(&base), total);
   if (e != cudaSuccess) {
-    *p = nullptr;
-    return fail(LEV_ERR_NOMEM, "adjoint: cudaMalloc of " + std::to_string(b) +
+    cudaGetLastError();
+    return fail(LEV_ERR_NOMEM, "adjoint: cudaMalloc of " + std::to_string(total) +
                                    " bytes failed: " + cudaGetErrorString(e));
   }
-  a->allocs.push_back(*p);
-  a->bytes += b;
+  a->allocs.push_back(base);
+  for (const auto &w : a->wanted) {
+    *w.first = base;
+    base += (w.second + 255) / 256 * 256;
+    a->bytes += w.second;
+  }
+  a->wanted.clear();
   return LEV_OK;
 }
 
@@ -3521,19 +3567,47 @@ AdjGridBwdFn adj_grid_bwd_fn(int R, int minb, int math_mode) { LEV_BY_ROWS(adj_g
 #undef LEV_BY_MATH
 #undef LEV_BY_ROWS
 
-// Grid-resident segments for a single network: per rows-per-CTA choice, the
-// shared memory of both kernels and whether every CTA can be resident at once.
-int adj_setup_grid(LevAdjoint *a, const std::vector<long long> &sl_off,
-                   const std::vector<int> &sl_len) {
+// What fits of rows-per-CTA choice `ri` in the engine's math mode.  A look at a
+// kernel loads it, and there are 36: a choice is looked at when it is first
+// needed (N = 10^4, the first adjoint of a process: 6.0 ms with a look at all of
+// them at creation, 4.6 with a look at the default).
+const AdjFit &adj_fit(const LevAdjoint *a, int ri) {
+  const int mm = a->e->math_mode;
+  AdjFit &f = a->g_fit[mm == LEV_MATH_ACCURATE ? 1 : 0][ri];
+  if (f.looked) return f;
+  f.looked = true;
+  if (a->gf_smem[ri] == 0) return f;
+  const int R = kGridRs[ri];
+  const long long C = (a->h_nets[0].N + R - 1) / R;
+  auto fit = [&](auto pick, size_t smem, long long n) -> int {
+    for (int minb = 2; minb <= 3; ++minb) {
+      if (n > (long long)minb * a->sms) continue;
+      const void *fn = reinterpret_cast<const void *>(pick(R, minb, mm));
+      if ((long long)ctas_per_sm(fn, kGridThreads, smem) * a->sms >= n) return minb;
+    }
+    return 0;
+  };
+  f.fwd = fit(adj_grid_fwd_fn, a->gf_smem[ri], C);
+  if (f.fwd) f.bwd = fit(adj_grid_bwd_fn, a->gb_smem[ri], C);
+  // the paired backward launch: both groups resident at once
+  if (f.bwd && a->nseg > 1)
+    f.pair = fit(adj_grid_pair_fn, std::max(a->gf_smem[ri], a->gb_smem[ri]), 2LL * C);
+  return f;
+}
+
+// Grid-resident segments for a single network: per rows-per-CTA choice the
+// shared memory of both kernels, and the smallest choice whose CTAs can all be
+// resident at once.
+int adj_setup_grid(LevAdjoint *a, const std::vector<int> &sl_len) {
   a->grid_ok = false;
   if (a->NN != 1) return LEV_OK;
   const NetDesc &d = a->h_nets[0];
-  int dev = 0, max_smem = 0, coop = 0, sms = 0;
+  int dev = 0, max_smem = 0, coop = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) !=
           cudaSuccess ||
       cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+      cudaDeviceGetAttribute(&a->sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
     cudaGetLastError();
     return LEV_OK;
   }
@@ -3542,8 +3616,7 @@ int adj_setup_grid(LevAdjoint *a, const std::vector<long long> &sl_off,
   for (int ri = 0; ri < 3; ++ri) {
     const int R = kGridRs[ri];
     const int C = (d.N + R - 1) / R;
-    if (C < 2) continue;
-    const int gpad = (C + 3) & ~3;
+    if (C < 2 || C > 3LL * a->sms) continue;
     long long cap = 0;
     for (int c = 0; c < C; ++c) {
       long long e = 0;
@@ -3555,51 +3628,24 @@ int adj_setup_grid(LevAdjoint *a, const std::vector<long long> &sl_off,
                        sizeof(int) * 2 * (R / 32) + 8 * (size_t)cap;
     const size_t bsm = sizeof(int) * 2 * (R / 32) + 16 * (size_t)cap;
     if (std::max(fsm, bsm) + 1024 > (size_t)max_smem) continue;
-    // CTAs per SM that the kernel of `pick` has to be compiled for so that n of
-    // its CTAs with `sm` bytes each are resident, 2 or 3, or 0: not even then
-    auto fit = [&](auto pick, size_t sm, long long n) -> int {
-      for (int minb = 2; minb <= 3; ++minb) {
-        if (n > (long long)minb * sms) continue;  // (a look at a kernel loads it)
-        bool ok = true;
-        for (int m = 0; m < 2 && ok; ++m) {
-          const void *fn = reinterpret_cast<const void *>(
-              pick(R, minb, m ? LEV_MATH_ACCURATE : LEV_MATH_REFERENCE));
-          int per_sm = 0;
-          ok = allow_smem(fn, sm) &&
-               cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kGridThreads, sm) ==
-                   cudaSuccess &&
-               (long long)per_sm * sms >= n;
-        }
-        cudaGetLastError();  // clear a refused attribute, if any
-        if (ok) return minb;
-      }
-      return 0;
-    };
-    a->gf_minb[ri] = fit(adj_grid_fwd_fn, fsm, C);
-    a->gb_minb[ri] = fit(adj_grid_bwd_fn, bsm, C);
-    if (!a->gf_minb[ri] || !a->gb_minb[ri]) continue;
-    // the paired backward launch: both groups resident at once
-    a->gp_minb[ri] = fit(adj_grid_pair_fn, std::max(fsm, bsm), 2LL * C);
-    a->gR_ok[ri] = true;
     a->g_cap[ri] = (int)cap;
     a->gf_smem[ri] = fsm;
     a->gb_smem[ri] = bsm;
-    max_gpad = std::max(max_gpad, gpad);
+    max_gpad = std::max(max_gpad, (C + 3) & ~3);
     // the smallest: the steps wait on instructions, and more lanes per row are
     // more warps (us per 100 steps forward / backward, k = 20: N = 10^4 R = 64 363 /
     // 734, R = 128 460 / 740; 2*10^4 R = 64 485 / 1,198, R = 128 552 / 1,098;
     // 5*10^4 R = 128 745 / 1,980, R = 256 918 / 2,246)
-    if (!a->grid_ok) a->grid_R = R;
+    if (a->grid_ok || !adj_fit(a, ri).ok()) continue;
+    a->grid_R = R;
     a->grid_ok = true;
   }
   if (!a->grid_ok) return LEV_OK;
   // arrival counters, published sums and parts: one block, so that a launch
   // clears what it uses with two fills
   a->g_gpad = max_gpad;
-  int rc = adj_alloc(a, &a->g_bar, 3 * kGridBarPitch);
-  if (rc == LEV_OK) rc = adj_alloc(a, &a->g_wsum, 32LL * d.ntiles + 4LL * max_gpad);
-  if (rc != LEV_OK) return rc;
-  a->g_lgp = reinterpret_cast<double *>(a->g_wsum + 32LL * d.ntiles);
+  adj_alloc(a, &a->g_bar, 3 * kGridBarPitch);
+  adj_alloc(a, &a->g_wsum, 32LL * d.ntiles + 4LL * max_gpad);
   a->h_gerr = reinterpret_cast<int *>(mapped_alloc(1));
   if (!a->h_gerr) return fail(LEV_ERR_NOMEM, "mapped host memory: allocation failed");
   *a->h_gerr = 0;
@@ -3619,8 +3665,10 @@ void adj_grid_ckpt_args(LevAdjoint *a, int seg, int mode, AdjGridFwdArgs &g) {
   g.ck_g = a->ck_g + (size_t)seg * a->NN;
 }
 
+inline const AdjFit &adj_fit(const LevAdjoint *a) { return adj_fit(a, grid_r_index(a->grid_R)); }
+
 inline bool adj_grid_on(const LevAdjoint *a) {
-  return a->grid_ok && a->use_grid && a->res_ra == nullptr;
+  return a->grid_ok && a->use_grid && a->res_ra == nullptr && adj_fit(a).ok();
 }
 
 int adj_grid_check(LevAdjoint *a) {
@@ -3686,7 +3734,7 @@ int adj_grid_launch_fwd(LevAdjoint *a, AdjGridFwdArgs f, int n, cudaStream_t s) 
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  LEV_TRY_CUDA(cudaLaunchKernelEx(&cfg, adj_grid_fwd_fn(R, a->gf_minb[ri], e->math_mode), f));
+  LEV_TRY_CUDA(cudaLaunchKernelEx(&cfg, adj_grid_fwd_fn(R, adj_fit(a).fwd, e->math_mode), f));
   return LEV_OK;
 }
 
@@ -3732,7 +3780,7 @@ int adj_grid_launch_bwd(LevAdjoint *a, AdjGridBwdArgs b, cudaStream_t s) {
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  LEV_TRY_CUDA(cudaLaunchKernelEx(&cfg, adj_grid_bwd_fn(R, a->gb_minb[ri], e->math_mode), b));
+  LEV_TRY_CUDA(cudaLaunchKernelEx(&cfg, adj_grid_bwd_fn(R, adj_fit(a).bwd, e->math_mode), b));
   return LEV_OK;
 }
 
@@ -3757,7 +3805,7 @@ int adj_grid_launch_pair(LevAdjoint *a, AdjGridFwdArgs f, int n, AdjGridBwdArgs 
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  LEV_TRY_CUDA(cudaLaunchKernelEx(&cfg, adj_grid_pair_fn(R, a->gp_minb[ri], e->math_mode), f, b, C));
+  LEV_TRY_CUDA(cudaLaunchKernelEx(&cfg, adj_grid_pair_fn(R, adj_fit(a).pair, e->math_mode), f, b, C));
   return LEV_OK;
 }
 
@@ -3800,8 +3848,7 @@ int lev_adj_create(LevAdjoint **out, LevEngine *e, int32_t segment,
   const long long TN = a->TN, SL = a->SL, NN = a->NN;
   const long long S = a->nseg, C = a->C;
   int rc = LEV_OK;
-#define A(ptr, n) \
-  if (rc == LEV_OK) rc = adj_alloc(a, &(ptr), (n));
+#define A(ptr, n) adj_alloc(a, &(ptr), (n))
   A(a->d_nets, NN);
   A(a->d_st, NN);
   A(a->d_ck_off, NN);
@@ -3828,6 +3875,16 @@ int lev_adj_create(LevAdjoint **out, LevEngine *e, int32_t segment,
   A(a->lam_g, NN);
   A(a->grad_omega_acc, TN);
   A(a->grad_theta0, TN);
+  if (NN == 1) {
+    std::vector<int> h_len(e->num_slices);
+    if (cudaMemcpy(h_len.data(), e->d_sl_len, sizeof(int) * e->num_slices,
+                   cudaMemcpyDeviceToHost) != cudaSuccess)
+      rc = fail(LEV_ERR_CUDA, "adjoint: reading the SELL slice table failed");
+    else
+      rc = adj_setup_grid(a, h_len);
+  }
+  if (rc == LEV_OK) rc = adj_commit(a);
+  if (a->g_wsum) a->g_lgp = reinterpret_cast<double *>(a->g_wsum + 32LL * a->h_nets[0].ntiles);
   if (rc == LEV_OK && S > 1) {
     // optional second record set; without it the backward pass runs the
     // recompute and the reverse steps of each segment one after the other
@@ -3841,6 +3898,7 @@ int lev_adj_create(LevAdjoint **out, LevEngine *e, int32_t segment,
       if (dj_rec) A(a->dj_hist2, C * SL);
       A(a->thh_hist2, C * TN);
       A(a->trace2, C * NN);
+      rc = adj_commit(a);
       if (rc == LEV_OK &&
           (cudaStreamCreateWithFlags(&a->rstream, cudaStreamNonBlocking) != cudaSuccess ||
            cudaEventCreateWithFlags(&a->ev_rec[0], cudaEventDisableTiming) != cudaSuccess ||
@@ -3852,17 +3910,6 @@ int lev_adj_create(LevAdjoint **out, LevEngine *e, int32_t segment,
     }
   }
 #undef A
-  if (rc == LEV_OK && NN == 1) {
-    std::vector<long long> h_off(e->num_slices);
-    std::vector<int> h_len(e->num_slices);
-    if (cudaMemcpy(h_off.data(), e->d_sl_off, sizeof(long long) * e->num_slices,
-                   cudaMemcpyDeviceToHost) != cudaSuccess ||
-        cudaMemcpy(h_len.data(), e->d_sl_len, sizeof(int) * e->num_slices,
-                   cudaMemcpyDeviceToHost) != cudaSuccess)
-      rc = fail(LEV_ERR_CUDA, "adjoint: reading the SELL slice table failed");
-    else
-      rc = adj_setup_grid(a, h_off, h_len);
-  }
   if (rc != LEV_OK) {
     std::string msg = g_last_error;
     adj_free(a);
@@ -3908,7 +3955,7 @@ int lev_adj_bytes(const LevAdjoint *a, size_t *bytes) {
 // Record set of segment `seg` of a run of `nseg` segments, per path.
 enum { kRecNone = 0, kRecSteps = 1, kRecGrid = 2 };
 static bool adj_paired(const LevAdjoint *a, int nseg) {
-  return a->ring2 != nullptr && a->use_pair && a->gp_minb[grid_r_index(a->grid_R)] > 0 && nseg > 1;
+  return a->ring2 != nullptr && a->use_pair && adj_fit(a).pair > 0 && nseg > 1;
 }
 static int adj_record_set(const LevAdjoint *a, int path, int seg, int nseg) {
   if (path == kRecGrid) return adj_paired(a, nseg) ? (seg & 1) : 0;
@@ -4311,16 +4358,17 @@ int lev_adj_backward(LevAdjoint *a, const float *dLdr, const float *dLdtheta,
 int lev_adj_grid_info(const LevAdjoint *a, int32_t *eligible, int32_t *enabled,
                       int32_t *rows_per_cta, int32_t *eligible_rows_mask, int32_t *paired) {
   if (!a) return fail(LEV_ERR_ARG, "null handle");
+  DeviceScope ds(a->e->device);
   if (eligible) *eligible = a->grid_ok ? 1 : 0;
   if (enabled) *enabled = adj_grid_on(a) ? 1 : 0;
   if (rows_per_cta) *rows_per_cta = a->grid_ok ? a->grid_R : 0;
   if (paired)
     *paired = (adj_grid_on(a) && a->use_pair && a->ring2 != nullptr &&
-               a->gp_minb[grid_r_index(a->grid_R)] > 0) ? 1 : 0;
+               adj_fit(a).pair > 0) ? 1 : 0;
   if (eligible_rows_mask) {
     int m = 0;
     for (int i = 0; i < 3; ++i)
-      if (a->gR_ok[i]) m |= kGridRs[i];
+      if (adj_fit(a, i).ok()) m |= kGridRs[i];
     *eligible_rows_mask = m;
   }
   return LEV_OK;
@@ -4353,7 +4401,8 @@ int lev_adj_set_grid_mode(LevAdjoint *a, int32_t enabled, int32_t rows_per_cta) 
   if (rows_per_cta != 0) {
     if (rows_per_cta != 64 && rows_per_cta != 128 && rows_per_cta != 256)
       return fail(LEV_ERR_ARG, "rows_per_cta must be 0, 64, 128 or 256");
-    if (!a->gR_ok[grid_r_index(rows_per_cta)])
+    DeviceScope ds(a->e->device);
+    if (!adj_fit(a, grid_r_index(rows_per_cta)).ok())
       return fail(LEV_ERR_ARG, "rows_per_cta not eligible for this adjoint");
     a->grid_R = rows_per_cta;
   }

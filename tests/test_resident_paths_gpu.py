@@ -515,3 +515,30 @@ def test_tuned_choices_reach_later_engines_together():
         want_r = r if want_r is None else want_r
         np.testing.assert_array_equal(r, want_r)
         b.close()
+
+
+@pytest.mark.parametrize("R", [64, 128, 256])
+def test_adjoint_after_a_change_of_math_mode(R):
+    """What fits of the grid-resident adjoint kernels is looked at per math mode
+    when it is first needed."""
+    net = make_network(3000, 10, 0.1, 20, seed=8, delay_lo=1)
+    T, out = 50, []
+    for mode, then in (("accurate", None), ("reference", "accurate")):
+        e = LeviathanEngine(*net.engine_args(), math_mode=mode)
+        adj = Adjoint(e, segment=20, max_steps=T)
+        if then:
+            e.set_math_mode(then)
+        adj.set_grid_mode(True, R)
+        info = adj.grid_info()
+        assert info["enabled"] and info["rows_per_cta"] == R and info["paired"]
+        assert R in info["eligible_rows"]
+        p = [torch.tensor(v, dtype=torch.float32, device="cuda")
+             for v in (net.omega, net.weights, np.array([1.5]))]
+        r = adj.forward(*p, T, DT)
+        g = adj.backward(torch.ones_like(r))
+        out.append([r.cpu().numpy()] + [g[k].cpu().numpy() for k in ("omega", "w0")])
+        adj.close()
+        e.close()
+    np.testing.assert_array_equal(out[0][0], out[1][0])
+    for a, b in zip(out[0][1:], out[1][1:]):
+        assert np.linalg.norm(a - b) < REL * np.linalg.norm(b)
