@@ -410,10 +410,16 @@ __host__ __device__ constexpr int adj_arrival_wait(int k, int early) { return ea
 // last are those of step s+2, two reversed before.  Its clearing at step k is
 // ordered by arrival k, which barrier D of step k+2 waits for, and the slot's
 // next scatter comes from that step at the earliest (adj_slots).  Buffers of
-// the parts as in grid_kernel.  Shared memory: sloff / sllen int [R/32], cd uint32 [edge_cap],
-// lw float [edge_cap] (lam_w; within a step c * lam_w(s+1)), sa float2
-// [edge_cap] (sin, w cos).
-template <int MATH, int R, int U>
+// the parts as in grid_kernel.  Shared memory: sa float2 [edge_cap] (sin, w cos),
+// cd uint32 [edge_cap], lw float [edge_cap] (lam_w; within a step c *
+// lam_w(s+1)), sloff / sllen int [R/32].
+//
+// KEEP = false, for rows too long for 16 bytes per entry: no sa.  The edges are
+// walked once, between A and B, scatter included; the exchange then waits for
+// the walk, which is most of a step of such rows.  Backward us of 200 steps, per
+// step launches / here: N = 30,000, k = 60 6,930 / 5,520; 15,000, k = 120 8,050 /
+// 5,510; 9,000, k = 230 12,090 / 6,660; 4,000, k = 300 14,440 / 7,790.
+template <int MATH, int R, int U, bool KEEP>
 __device__ __forceinline__ void adj_grid_bwd_body(const AdjGridBwdArgs &a, const int cta,
                                                   const unsigned G, unsigned char *smem) {
   constexpr int LPR = 256 / R;
@@ -437,7 +443,7 @@ __device__ __forceinline__ void adj_grid_bwd_body(const AdjGridBwdArgs &a, const
   float *AR = a.adj_ring + nd.aux_off;
 
   float2 *s_sa = reinterpret_cast<float2 *>(smem);
-  uint32_t *s_cd = reinterpret_cast<uint32_t *>(s_sa + a.edge_cap);
+  uint32_t *s_cd = reinterpret_cast<uint32_t *>(s_sa + (KEEP ? a.edge_cap : 0));
   float *s_lw = reinterpret_cast<float *>(s_cd + a.edge_cap);
   int *sloff = reinterpret_cast<int *>(s_lw + a.edge_cap);
   int *sllen = sloff + nslices;
@@ -516,43 +522,48 @@ __device__ __forceinline__ void adj_grid_bwd_body(const AdjGridBwdArgs &a, const
       const EdgeParams ep = {dt, eta, lam, __fmaf_rn(-gamma, fabsf(eps), 1.0f), w_min, w_max};
       const float *w_s = a.w_hist + (long long)kk * a.SL + ebase + eoff + sl.l;
       float S_i = 0.0f, labs = 0.0f;
-      for (int kb = 0; kb < len; kb += LPR * U) {
-        uint32_t p[U];
-        float wv[U], dj[U];
+      // the row's entries: each(entry, word, c * lam_w(s+1), sin, w cos)
+      auto walk = [&](auto each) {
+        for (int kb = 0; kb < len; kb += LPR * U) {
+          uint32_t p[U];
+          float wv[U], dj[U];
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-          const int e = kb + LPR * u + sl.q;
-          const bool in = e < deg;
-          p[u] = in ? s_cd[at0 + 32 * e] : 0u;
-          wv[u] = in ? __ldcs(w_s + 32 * e) : 0.0f;
-        }
+          for (int u = 0; u < U; ++u) {
+            const int e = kb + LPR * u + sl.q;
+            const bool in = e < deg;
+            p[u] = in ? s_cd[at0 + 32 * e] : 0u;
+            wv[u] = in ? __ldcs(w_s + 32 * e) : 0.0f;
+          }
 #pragma unroll
-        for (int u = 0; u < U; ++u)
-          dj[u] = (kb + LPR * u + sl.q < deg)
-                      ? __ldg(H + ((unsigned)(hs - (int)(p[u] & 255u)) * (unsigned)Np + (p[u] >> 8))) - th
-                      : 0.0f;
-        float sn[U], cs[U];
-        wrap_sincos_group<MATH>(dj, sn, cs);
+          for (int u = 0; u < U; ++u)
+            dj[u] = (kb + LPR * u + sl.q < deg)
+                        ? __ldg(H + ((unsigned)(hs - (int)(p[u] & 255u)) * (unsigned)Np + (p[u] >> 8))) - th
+                        : 0.0f;
+          float sn[U], cs[U];
+          wrap_sincos_group<MATH>(dj, sn, cs);
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-          const int e = kb + LPR * u + sl.q;
-          const float w = wv[u];
-          S_i += w * sn[u];
-          const float w_pre = edge_weight_free(ep, cs[u], w);
-          const float lw = (e < deg) ? s_lw[at0 + 32 * e] : 0.0f;
-          const float m = (w_pre >= w_min && w_pre <= w_max) ? lw : 0.0f;
-          labs += m * cs[u];
-          if (e < deg) {
-            s_lw[at0 + 32 * e] = m;
-            s_sa[at0 + 32 * e] = make_float2(sn[u], w * cs[u]);
+          for (int u = 0; u < U; ++u) {
+            const int e = kb + LPR * u + sl.q;
+            const float w = wv[u];
+            S_i += w * sn[u];
+            const float w_pre = edge_weight_free(ep, cs[u], w);
+            const float lw = (e < deg) ? s_lw[at0 + 32 * e] : 0.0f;
+            const float m = (w_pre >= w_min && w_pre <= w_max) ? lw : 0.0f;
+            labs += m * cs[u];
+            if (e < deg) each(e, p[u], m, sn[u], w * cs[u]);
           }
         }
-      }
 #pragma unroll
-      for (int off = 1; off < LPR; off *= 2) {
-        S_i += __shfl_xor_sync(mask, S_i, off);
-        labs += __shfl_xor_sync(mask, labs, off);
-      }
+        for (int off = 1; off < LPR; off *= 2) {
+          S_i += __shfl_xor_sync(mask, S_i, off);
+          labs += __shfl_xor_sync(mask, labs, off);
+        }
+      };
+      if constexpr (KEEP)
+        walk([&](int e, uint32_t, float m, float sn, float wcs) {
+          s_lw[at0 + 32 * e] = m;
+          s_sa[at0 + 32 * e] = make_float2(sn, wcs);
+        });
       cta_barrier_slot();  // D
       float arv = 0.0f;
       if (live) arv = __ldcg(AR + (long long)as_next * Np + row);
@@ -575,25 +586,29 @@ __device__ __forceinline__ void adj_grid_bwd_body(const AdjGridBwdArgs &a, const
         if (a.dLdth) lt += extra;
       }
       const float lt1 = (float)lt;  // lam_th'
+      float lsum = 0.0f;
+      auto scatter = [&](int e, uint32_t p, float m, float sn, float wcs) {
+        const float lam_S = lt1 * dt * tr.x;
+        const float hq = dt * eta * ep.hebb;
+        s_lw[at0 + 32 * e] = m * decay + lam_S * sn;
+        const float lD = lam_S * wcs - m * hq * sn;
+        const unsigned s0 = (unsigned)(as_s - (int)(p & 255u));
+        atomicAdd(AR + (min(s0, s0 + (unsigned)bsa) * (unsigned)Np + (p >> 8)), lD);
+        lsum -= lD;
+      };
+      if constexpr (!KEEP) walk(scatter);
       double part = sl.q == 0 ? (double)lt1 * dt * S_i : 0.0;
 #pragma unroll
       for (int off = 16; off > 0; off /= 2) part += __shfl_down_sync(mask, part, off);
       if (lane == 0) s_red[warp] = part;
       cta_barrier();  // B
       // ---- scatter ------------------------------------------------------------------
-      const float lam_S = lt1 * dt * tr.x;
-      const float hq = dt * eta * ep.hebb;
-      float lsum = 0.0f;
+      if constexpr (KEEP) {
 #pragma unroll 4
-      for (int e = sl.q; e < deg; e += LPR) {
-        const uint32_t p = s_cd[at0 + 32 * e];
-        const float m = s_lw[at0 + 32 * e];
-        const float2 sa = s_sa[at0 + 32 * e];
-        s_lw[at0 + 32 * e] = m * decay + lam_S * sa.x;
-        const float lD = lam_S * sa.y - m * hq * sa.x;
-        const unsigned s0 = (unsigned)(as_s - (int)(p & 255u));
-        atomicAdd(AR + (min(s0, s0 + (unsigned)bsa) * (unsigned)Np + (p >> 8)), lD);
-        lsum -= lD;
+        for (int e = sl.q; e < deg; e += LPR) {
+          const float2 sa = s_sa[at0 + 32 * e];
+          scatter(e, s_cd[at0 + 32 * e], s_lw[at0 + 32 * e], sa.x, sa.y);
+        }
       }
 #pragma unroll
       for (int off = 1; off < LPR; off *= 2) lsum += __shfl_xor_sync(mask, lsum, off);
@@ -718,10 +733,10 @@ __global__ void __launch_bounds__(kGridThreads, MINB) adj_grid_fwd_kernel(const 
   adj_grid_fwd_body<MATH, R, MINB>(a, blockIdx.x, gridDim.x, smem);
 }
 
-template <int MATH, int R, int MINB>
+template <int MATH, int R, int MINB, bool KEEP>
 __global__ void __launch_bounds__(kGridThreads, MINB) adj_grid_bwd_kernel(const AdjGridBwdArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
-  adj_grid_bwd_body<MATH, R, adj_bwd_unroll(MINB)>(a, blockIdx.x, gridDim.x, smem);
+  adj_grid_bwd_body<MATH, R, adj_bwd_unroll(MINB), KEEP>(a, blockIdx.x, gridDim.x, smem);
 }
 
 // Paired launch of the backward pass: CTAs [0, gf) recompute segment k-1
@@ -736,7 +751,7 @@ __global__ void __launch_bounds__(kGridThreads, MINB)
   if ((int)blockIdx.x < gf)
     adj_grid_fwd_body<MATH, R, MINB>(f, blockIdx.x, gf, smem);
   else
-    adj_grid_bwd_body<MATH, R, adj_bwd_unroll(MINB)>(b, blockIdx.x - gf, gridDim.x - gf, smem);
+    adj_grid_bwd_body<MATH, R, adj_bwd_unroll(MINB), true>(b, blockIdx.x - gf, gridDim.x - gf, smem);
 }
 
 }  // namespace lev

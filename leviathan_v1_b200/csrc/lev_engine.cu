@@ -3356,6 +3356,7 @@ __global__ void adj_state_kernel(int mode, const NetDesc *nets, NetState *st,
 struct AdjFit {
   bool looked = false;
   int fwd = 0, bwd = 0, pair = 0;
+  bool small = false;  // bwd: the kernel that keeps 8 bytes per entry
   bool ok() const { return fwd > 0 && bwd > 0; }
 };
 
@@ -3419,7 +3420,7 @@ struct LevAdjoint {
   // per rows-per-CTA choice (64, 128, 256): SELL entries per CTA and shared
   // memory, 0 where it cannot fit, and per math mode what fits
   int g_cap[3] = {0, 0, 0};
-  size_t gf_smem[3] = {0, 0, 0}, gb_smem[3] = {0, 0, 0};
+  size_t gf_smem[3] = {0, 0, 0}, gb_smem[3] = {0, 0, 0}, gb_small[3] = {0, 0, 0};
   mutable AdjFit g_fit[2][3];
   bool use_pair = true;
   int g_gpad = 0;
@@ -3555,16 +3556,26 @@ int adj_ckpt(LevAdjoint *a, int seg, bool save, cudaStream_t s = nullptr,
 using AdjGridFwdFn = void (*)(AdjGridFwdArgs);
 using AdjGridBwdFn = void (*)(AdjGridBwdArgs);
 using AdjGridPairFn = void (*)(AdjGridFwdArgs, AdjGridBwdArgs, int);
-#define LEV_BY_MATH(kernel, R, MINB) (acc ? kernel<1, R, MINB> : kernel<0, R, MINB>)
-#define LEV_BY_ROWS(kernel)                                                                 \
-  const bool acc = math_mode == LEV_MATH_ACCURATE;                                          \
-  if (R == 64) return minb == 2 ? LEV_BY_MATH(kernel, 64, 2) : LEV_BY_MATH(kernel, 64, 3);  \
-  if (R == 128) return minb == 2 ? LEV_BY_MATH(kernel, 128, 2) : LEV_BY_MATH(kernel, 128, 3); \
-  return minb == 2 ? LEV_BY_MATH(kernel, 256, 2) : LEV_BY_MATH(kernel, 256, 3);
+#define LEV_BY_MATH(kernel, ...) (acc ? kernel<1, __VA_ARGS__> : kernel<0, __VA_ARGS__>)
+#define LEV_BY_MINB(kernel, R, ...)                              \
+  (minb == 2 ? LEV_BY_MATH(kernel, R, 2 __VA_OPT__(, ) __VA_ARGS__) \
+             : LEV_BY_MATH(kernel, R, 3 __VA_OPT__(, ) __VA_ARGS__))
+#define LEV_BY_ROWS(kernel, ...)                                 \
+  const bool acc = math_mode == LEV_MATH_ACCURATE;               \
+  if (R == 64) return LEV_BY_MINB(kernel, 64, __VA_ARGS__);      \
+  if (R == 128) return LEV_BY_MINB(kernel, 128, __VA_ARGS__);    \
+  return LEV_BY_MINB(kernel, 256, __VA_ARGS__);
 AdjGridFwdFn adj_grid_fwd_fn(int R, int minb, int math_mode) { LEV_BY_ROWS(adj_grid_fwd_kernel) }
 AdjGridPairFn adj_grid_pair_fn(int R, int minb, int math_mode) { LEV_BY_ROWS(adj_grid_pair_kernel) }
-AdjGridBwdFn adj_grid_bwd_fn(int R, int minb, int math_mode) { LEV_BY_ROWS(adj_grid_bwd_kernel) }
+AdjGridBwdFn adj_grid_bwd_fn(int R, int minb, int math_mode) {
+  LEV_BY_ROWS(adj_grid_bwd_kernel, true)
+}
+// ... with 8 bytes of shared memory per entry instead of 16
+AdjGridBwdFn adj_grid_bwd_small_fn(int R, int minb, int math_mode) {
+  LEV_BY_ROWS(adj_grid_bwd_kernel, false)
+}
 #undef LEV_BY_MATH
+#undef LEV_BY_MINB
 #undef LEV_BY_ROWS
 
 // What fits of rows-per-CTA choice `ri` in the engine's math mode.  A look at a
@@ -3588,9 +3599,13 @@ const AdjFit &adj_fit(const LevAdjoint *a, int ri) {
     return 0;
   };
   f.fwd = fit(adj_grid_fwd_fn, a->gf_smem[ri], C);
-  if (f.fwd) f.bwd = fit(adj_grid_bwd_fn, a->gb_smem[ri], C);
+  if (f.fwd) {
+    f.bwd = fit(adj_grid_bwd_fn, a->gb_smem[ri], C);
+    f.small = !f.bwd;
+    if (f.small) f.bwd = fit(adj_grid_bwd_small_fn, a->gb_small[ri], C);
+  }
   // the paired backward launch: both groups resident at once
-  if (f.bwd && a->nseg > 1)
+  if (f.bwd && !f.small && a->nseg > 1)
     f.pair = fit(adj_grid_pair_fn, std::max(a->gf_smem[ri], a->gb_smem[ri]), 2LL * C);
   return f;
 }
@@ -3626,11 +3641,11 @@ int adj_setup_grid(LevAdjoint *a, const std::vector<int> &sl_len) {
     }
     const size_t fsm = (R < 256 ? sizeof(float2) * 8 * (size_t)d.ntiles : 0) +
                        sizeof(int) * 2 * (R / 32) + 8 * (size_t)cap;
-    const size_t bsm = sizeof(int) * 2 * (R / 32) + 16 * (size_t)cap;
-    if (std::max(fsm, bsm) + 1024 > (size_t)max_smem) continue;
+    if (fsm + 1024 > (size_t)max_smem) continue;
     a->g_cap[ri] = (int)cap;
     a->gf_smem[ri] = fsm;
-    a->gb_smem[ri] = bsm;
+    a->gb_smem[ri] = sizeof(int) * 2 * (R / 32) + 16 * (size_t)cap;
+    a->gb_small[ri] = sizeof(int) * 2 * (R / 32) + 8 * (size_t)cap;
     max_gpad = std::max(max_gpad, (C + 3) & ~3);
     // the smallest: the steps wait on instructions, and more lanes per row are
     // more warps (us per 100 steps forward / backward, k = 20: N = 10^4 R = 64 363 /
@@ -3773,14 +3788,16 @@ int adj_grid_launch_bwd(LevAdjoint *a, AdjGridBwdArgs b, cudaStream_t s) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((a->h_nets[0].N + R - 1) / R);
   cfg.blockDim = dim3(kGridThreads);
-  cfg.dynamicSmemBytes = a->gb_smem[ri];
+  const AdjFit &fit = adj_fit(a);
+  cfg.dynamicSmemBytes = fit.small ? a->gb_small[ri] : a->gb_smem[ri];
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  LEV_TRY_CUDA(cudaLaunchKernelEx(&cfg, adj_grid_bwd_fn(R, adj_fit(a).bwd, e->math_mode), b));
+  LEV_TRY_CUDA(cudaLaunchKernelEx(&cfg, fit.small ? adj_grid_bwd_small_fn(R, fit.bwd, e->math_mode)
+                                                  : adj_grid_bwd_fn(R, fit.bwd, e->math_mode), b));
   return LEV_OK;
 }
 

@@ -542,3 +542,32 @@ def test_adjoint_after_a_change_of_math_mode(R):
     np.testing.assert_array_equal(out[0][0], out[1][0])
     for a, b in zip(out[0][1:], out[1][1:]):
         assert np.linalg.norm(a - b) < REL * np.linalg.norm(b)
+
+
+# rows too long for 16 bytes of shared memory per entry at R rows per CTA, up to
+# two CTAs per SM and three; bounds as for the long rows above
+@pytest.mark.parametrize("N,k,R,lo,mode", [(2000, 400, 64, 1, "accurate"),
+                                           (2000, 200, 128, 1, "reference"),
+                                           (2001, 100, 256, 1, "accurate"),
+                                           (2001, 100, 256, 0, "reference"),
+                                           (19_500, 80, 64, 1, "reference")])
+def test_reverse_segments_of_rows_that_fill_the_shared_memory(N, k, R, lo, mode):
+    net = make_network(N, k, 0.1, 25, seed=N + k, delay_lo=lo)
+    net.weights[:] *= np.float32(8.0 / k)
+    T, out = 45, []
+    for grid in (0, R):
+        e = LeviathanEngine(*net.engine_args(), math_mode=mode)
+        adj = Adjoint(e, segment=20, max_steps=T)
+        assert R in adj.grid_info()["eligible_rows"]
+        adj.set_grid_mode(bool(grid), grid)
+        p = [torch.tensor(v, dtype=torch.float32, device="cuda")
+             for v in (net.omega, net.weights, np.array([1.5]))]
+        r, th = adj.forward(*p, T, DT, record_theta=True)
+        g = adj.backward(torch.ones_like(r), torch.sin(th) / N)
+        out.append([v.cpu().numpy() for v in (r, th, g["omega"], g["w0"])])
+        adj.close()
+        e.close()
+    for a, b in zip(out[1][:2], out[0][:2]):
+        np.testing.assert_array_equal(a, b)
+    for a, b in zip(out[1][2:], out[0][2:]):
+        assert np.linalg.norm(a - b) < 3e-5 * np.linalg.norm(b)
