@@ -926,7 +926,7 @@ int ctas_per_sm(const void *fn, int threads, size_t smem) {
 // kernel can run (shared memory, cluster size, occupancy).
 void setup_cluster(LevEngine *h, const std::vector<int> &sl_len) {
   h->cluster_ok = false;
-  if (h->num_nets != 1) return;
+  if (h->num_nets != 1 || h->part) return;
   const NetDesc &d = h->h_nets[0];
   int dev = 0, max_smem = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return;
@@ -1420,8 +1420,9 @@ int create_impl(LevEngine **out, int num_nets, const int32_t *Ns,
                 const int32_t *col_cat, const uint8_t *d_cat,
                 const float *w_cat, const float *th_cat,
                 const float *thh_cat, const float *om_cat,
-                const LevParams *params, int math_mode, int n_ext = 0,
+                const LevParams *params, int math_mode, bool part = false, int n_ext = 0,
                 const float *theta_ext = nullptr) {
+  // part: the engine of a partition, stepped by the host.
   // n_ext > 0 (one network only): ring columns N .. N + n_ext - 1 hold the
   // phases of halo nodes of a partition (lev_part.cuh), initially theta_ext;
   // col_idx may then address them
@@ -1471,6 +1472,7 @@ int create_impl(LevEngine **out, int num_nets, const int32_t *Ns,
   const auto t_start = std::chrono::steady_clock::now();
   double t_mark = 0.0;
   LevEngine *h = new LevEngine();
+  h->part = part;
   auto lap = [&]() {
     const double t = ms_since(t_start), d = t - t_mark;
     t_mark = t;
@@ -4498,11 +4500,10 @@ int lev_part_create(LevEngine **out, int32_t N, int32_t n_halo, int32_t max_dela
   // a halo column that no edge reads is allowed (its phases are just kept)
   LevEngine *h = nullptr;
   int rc = create_impl(&h, 1, &N, &max_delay, row_ptr, col_idx, delays, weights,
-                       theta, theta_hat, omega, params, math_mode, n_halo,
+                       theta, theta_hat, omega, params, math_mode, true, n_halo,
                        theta_halo);
   if (rc != LEV_OK) return rc;
   DeviceScope ds(h->device);
-  h->part = true;
   h->part_halo = n_halo;
   h->part_N_global = N_global;
   h->part_tile_off = tile_off_global;
@@ -4510,9 +4511,7 @@ int lev_part_create(LevEngine **out, int32_t N, int32_t n_halo, int32_t max_dela
   // steps driven by the host (lev_part_step_*, lev_part_pair_*) with the
   // whole-network reduction on gathered partials: none of the block paths;
   // pair_ok (no zero delay) stays as creation found it
-  h->cluster_ok = false;
   h->use_cluster = false;
-  h->grid_ok = false;
   h->use_grid = false;
   h->h_nets[0].dist = 1;
   h->h_nets[0].part_off = tile_off_global;

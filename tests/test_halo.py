@@ -15,6 +15,7 @@ wait on each other inside kernels (the host orders every exchange), so this
 runs safely on one GPU.
 """
 
+import ctypes as C
 import os
 import socket
 import threading
@@ -270,3 +271,32 @@ def test_cuda_partitions_equal_single_engine(world, math_mode, pairs):
     if errs:
         raise errs[0]
     _check_equal(res, ref, world)
+
+
+@pytest.mark.gpu
+def test_partition_engine_holds_nothing_for_blocks_of_steps():
+    """A partition is stepped by the host: no resident path is set up for it,
+    and it has none of their arrays (sums, counters, long r history)."""
+    if not has_gpu():
+        pytest.fail("needs a CUDA device")
+    from leviathan_v1_b200 import LeviathanEngine, _lib
+    from leviathan_v1_b200.halo import CudaPartition
+
+    net = make_network(5000, 8, 0.1, 10, seed=3)
+    eng = LeviathanEngine(*net.engine_args())
+    assert eng.grid_info()["eligible"]
+    whole = eng.get_vram_usage()
+    eng.close()
+    p = PartitionedEngine(0, 1, *net.engine_args(), exchange=ThreadExchange(1).bind(0),
+                          plan=PartitionPlan(net.row_ptr, net.col_idx, 1), core=CudaPartition)
+    lib = _lib.load()
+    b = C.c_size_t()
+    assert lib.lev_get_vram_usage(p.core.h, C.byref(b)) == 0
+    el = [C.c_int32() for _ in range(5)]
+    sm = C.c_int64()
+    assert lib.lev_grid_info(p.core.h, *[C.byref(v) for v in el[:4]], C.byref(sm),
+                             C.byref(el[4])) == 0
+    assert el[0].value == 0
+    # 1,792 rows of r history and 32 sums of 8 bytes per 256-node block
+    assert whole - b.value >= 4 * (2048 - 256) + 32 * 8 * 20
+    p.close()
