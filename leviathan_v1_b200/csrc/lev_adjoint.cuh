@@ -864,33 +864,27 @@ __global__ void __launch_bounds__(kTile, 4) adj_bwd_split_kernel(const AdjBwdArg
 }
 
 // Checkpoint of the ring window of every network (one block row per 256-row
-// tile): mode 0 saves theta(t-m), m = 0..max_delay, from the ring (slot (cur -
-// m) mod bsi) into ck[m][N] (per network at ck_off); mode 1 writes it back as
-// theta(t-m) -> slot max_delay - m of an unwrapped segment ring; mode 2 does
-// both, from `ring` through ck into `seg`.
-__global__ void adj_ring_ckpt_kernel(int mode, const NetDesc *__restrict__ nets,
+// tile): save theta(t-m), m = 0..max_delay, from the ring (slot (cur - m) mod
+// bsi) into ck[m][N] (per network at ck_off), or restore it as theta(t-m) ->
+// slot max_delay - m of an unwrapped segment ring.
+__global__ void adj_ring_ckpt_kernel(bool restore, const NetDesc *__restrict__ nets,
                                      const int2 *__restrict__ tiles,
                                      const NetState *__restrict__ st, float *__restrict__ ring,
-                                     float *__restrict__ seg, float *__restrict__ ck,
-                                     const long long *__restrict__ ck_off) {
+                                     float *__restrict__ ck, const long long *__restrict__ ck_off) {
   const int2 tile = tiles[blockIdx.x];
   const NetDesc &nd = nets[tile.x];
   const int row = tile.y + threadIdx.x;
   if (row >= nd.N) return;
   const int cur = st[tile.x].cur;
   float *c = ck + ck_off[tile.x] + row;
-  const long long at = nd.ring_off + row;
+  float *at = ring + nd.ring_off + row;
   for (int m = blockIdx.y; m <= nd.max_delay; m += gridDim.y) {
-    float x;
-    if (mode == 1) {
-      x = c[(long long)m * nd.N];
-    } else {
-      int slot = cur - m;
-      slot += (slot < 0) ? nd.bsi : 0;
-      x = ring[at + (long long)slot * nd.Np];
-      c[(long long)m * nd.N] = x;
-    }
-    if (mode != 0) seg[at + (long long)(nd.max_delay - m) * nd.Np] = x;
+    int slot = restore ? nd.max_delay - m : cur - m;
+    slot += (slot < 0) ? nd.bsi : 0;
+    if (restore)
+      at[(long long)slot * nd.Np] = c[(long long)m * nd.N];
+    else
+      c[(long long)m * nd.N] = at[(long long)slot * nd.Np];
   }
 }
 

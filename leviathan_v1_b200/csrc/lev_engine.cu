@@ -3518,16 +3518,15 @@ int adj_launch_fwd(LevAdjoint *a, const AdjFwdArgs &f, cudaStream_t s = nullptr)
   return LEV_OK;
 }
 
-// The ring part of checkpoint `seg` (modes of adj_ring_ckpt_kernel).
-void adj_ring_ckpt(LevAdjoint *a, int seg, int mode, float *ring, float *segment,
-                   cudaStream_t s) {
+// The ring part of checkpoint `seg`, saved from or restored into `ring`.
+void adj_ring_ckpt(LevAdjoint *a, int seg, bool restore, float *ring, cudaStream_t s) {
   LevEngine *e = a->e;
   int md = 0;
   for (const NetDesc &d : a->h_nets) md = std::max(md, d.max_delay);
   // few tiles: the slots are spread over blocks as well
   const int by = std::max(1, std::min(md + 1, 148 * 8 / std::max(e->total_tiles, 1)));
   adj_ring_ckpt_kernel<<<dim3(e->total_tiles, by), kTile, 0, s>>>(
-      mode, a->d_nets, e->d_tiles, a->d_st, ring, segment,
+      restore, a->d_nets, e->d_tiles, a->d_st, ring,
       a->ck_ring + (size_t)seg * a->ckr_floats, a->d_ck_off);
 }
 
@@ -3548,7 +3547,7 @@ int adj_ckpt(LevAdjoint *a, int seg, bool save, cudaStream_t s = nullptr,
   LEV_TRY_CUDA(cp(a->ck_omh + (size_t)seg * a->TN, a->omega_hat, nb));
   LEV_TRY_CUDA(cp(a->ck_w + (size_t)seg * a->SL, a->w,
                   sizeof(float) * std::max<long long>(a->SL, 1)));
-  adj_ring_ckpt(a, seg, save ? 0 : 1, save ? ring : nullptr, save ? nullptr : ring, s);
+  adj_ring_ckpt(a, seg, !save, ring, s);
   adj_state_kernel<<<1, 128, 0, s>>>(save ? 1 : 2, a->d_nets, a->d_st,
                                      a->ck_g + (size_t)seg * a->NN, nullptr, a->NN);
   LEV_TRY_CUDA(cudaGetLastError());
@@ -4077,7 +4076,7 @@ int lev_adj_forward(LevAdjoint *a, float dt, int32_t T, const float *omega,
     if (t == last0) {
       // from here on in the record set: the ring window unwrapped, as after a
       // restore
-      adj_ring_ckpt(a, nseg - 1, 1, nullptr, rec_ring, s);
+      adj_ring_ckpt(a, nseg - 1, true, rec_ring, s);
       adj_state_kernel<<<1, 128, 0, s>>>(2, a->d_nets, a->d_st,
                                          a->ck_g + (size_t)(nseg - 1) * a->NN, nullptr, a->NN);
       LEV_TRY_CUDA(cudaMemcpyAsync(rec_w, a->w,
