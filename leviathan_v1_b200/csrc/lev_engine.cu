@@ -111,10 +111,10 @@ constexpr int kNumPairVariants = sizeof(kPairVariants) / sizeof(kPairVariants[0]
 
 // Pair variant of an engine that has not been tuned, by its tiles and mean
 // slice length, one for all its classes so that they run merged: up to one
-// wave of (4,4,0) -- 592 tiles -- or short rows, (4,4,0); up to 26 entries per
-// row (6,3,0); above, (8,3,0).  The lines follow the table above.
-inline int default_pair_variant(int ntiles, double mean_slice_len) {
-  if (ntiles <= 592 || mean_slice_len <= 14.0) return 4;
+// wave of (4,4,0) -- 592 tiles on 148 SMs -- or short rows, (4,4,0); up to 26
+// entries per row (6,3,0); above, (8,3,0).  The lines follow the table above.
+inline int default_pair_variant(int ntiles, double mean_slice_len, int sms) {
+  if (ntiles <= 4 * sms || mean_slice_len <= 14.0) return 4;
   return mean_slice_len <= 26.0 ? 2 : 0;
 }
 
@@ -159,6 +159,7 @@ struct LevHubs;
 
 struct LevEngine {
   int device = 0;
+  int sms = 0;  // of the device
   cudaStream_t stream = nullptr;
   int num_nets = 0;
   long long total_nodes = 0;
@@ -587,14 +588,30 @@ bool pairs_active(const LevEngine *h) {
   return false;
 }
 
+// Whether a pair chain of `ntiles` tiles is launched dependently (launch_after).
+// Always for a single step, which waits for each of its two or three launches: us
+// per call, without / with, k = 20: N = 1,000 21.1 / 18.6, 4.5*10^4 23.9 / 21.0,
+// 1.145*10^5 27.4 / 24.9, 5*10^5 65.3 / 61.7; k = 8 and 32 alike.  In a block, from
+// one wave of the pair kernel on, `minb` CTAs per SM, the next launch is set up
+// while the last CTAs run; up to 0.9 tiles per SM it has SMs of its own, and the
+// launches are most of the step.  Between, the launches that wait hold SMs that the
+// pair kernel needs: mostly slower.  us per step, without / with:
+//   tiles           133         143         235         313         446         508         606
+//   k = 8   (4,4)  7.4/ 6.8    7.7/ 8.4    8.6/ 9.2    9.1/ 9.4   10.3/10.7   10.6/10.6   12.1/11.0
+//           (8,3)  7.5/ 6.8    7.7/ 8.6    8.9/ 8.8    9.6/ 9.1   11.2/10.0   11.7/10.6   13.0/11.6
+//   k = 20  (4,4)  9.1/ 8.5    9.5/10.6   10.8/13.8   12.3/13.7   14.2/15.1   14.9/14.8   17.2/16.5
+//           (8,3)  8.5/ 7.9    8.9/10.4   10.6/11.2   12.1/11.5   13.8/12.9   14.5/13.8   16.3/16.1
+//   k = 32  (4,4) 10.7/10.1   10.7/12.6   12.9/17.6   15.3/17.9   18.6/19.5   19.0/19.1   22.5/22.6
+//           (8,3)  9.7/ 9.1    9.8/12.4   12.6/14.3   15.3/14.6   18.3/17.4   18.7/18.1   21.5/21.0
+// Far above the gain is small: k = 32, N = 2*10^5 26.4/25.9, 5*10^5 63.6/62.5, 10^6
+// 128.0/127.6.
+inline bool dependent_chain(int ntiles, int minb, int sms, bool single) {
+  return single || 10 * ntiles <= 9 * sms || ntiles > minb * sms;
+}
+
 // Launch by programmatic dependent launch (see wait_dependency) when `early`: the
 // next kernel of the chain is set up and its CTAs read what does not change
-// while this one drains.  With more than one wave of pair CTAs (444 tiles) that
-// is faster (us per step, without / with: N = 10^6 133.1 / 131.3, 5*10^5 68.0 /
-// 66.4, 2*10^5 18.8 / 17.7, 1.2*10^5 20.8 / 20.7), and so it is where launches
-// are most of the step (10^4 9.4 / 8.6, 2.8*10^4 9.7 / 8.2); between, the whole
-// chain comes to wait on the SMs beside the first kernel (1.1*10^5 13.0 / 15.0,
-// 6*10^4 10.9 / 13.8).
+// while this one drains.
 cudaError_t launch_after(const void *fn, int blocks, int threads, void **args, bool early,
                          cudaStream_t s) {
   cudaLaunchConfig_t cfg = {};
@@ -617,7 +634,9 @@ int launch_pair_tc(LevEngine *h, const TileClass &tc, StepArgs a, int phase,
   if (!s) s = h->stream;
   a.tiles = h->d_tiles + tc.tile_off;
   const int mode = (h->math_mode == LEV_MATH_ACCURATE) ? 1 : 0;
-  const bool early = tc.ntiles > 444 || tc.ntiles <= 111;
+  const bool early = tc.pair_variant >= 0 &&
+                     dependent_chain(tc.ntiles, kPairVariants[tc.pair_variant].MINB, h->sms,
+                                     a.r_host != nullptr);
   if (tc.pair_variant < 0 || phase == 0) {
     const void *fn =
         tc.pair_variant < 0
@@ -1078,12 +1097,12 @@ int setup_wait_flag(LevEngine *h) {
 int setup_grid(LevEngine *h, const std::vector<int> &sl_len) {
   h->grid_ok = false;
   if (h->part) return LEV_OK;
-  int dev = 0, max_smem = 0, coop = 0, sms = 0;
+  const int sms = h->sms;
+  int dev = 0, max_smem = 0, coop = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) !=
           cudaSuccess ||
-      cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+      cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess) {
     cudaGetLastError();
     return LEV_OK;
   }
@@ -1483,6 +1502,8 @@ int create_impl(LevEngine **out, int num_nets, const int32_t *Ns,
   h->h_nets.resize(num_nets);
   h->net_E.resize(num_nets);
   cudaError_t ce = cudaGetDevice(&h->device);
+  if (ce == cudaSuccess)
+    ce = cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, h->device);
   if (ce != cudaSuccess) {
     delete h;
     return fail(LEV_ERR_CUDA, std::string("no CUDA device: ") + cudaGetErrorString(ce));
@@ -1673,7 +1694,8 @@ int create_impl(LevEngine **out, int num_nets, const int32_t *Ns,
       double len_sum = 0.0;
       for (int c = 0; c < kNumClasses; ++c)
         len_sum += h->classes[c].mean_len * h->classes[c].ntiles;
-      const int pv = default_pair_variant(h->total_tiles, len_sum / std::max(h->total_tiles, 1));
+      const int pv = default_pair_variant(h->total_tiles, len_sum / std::max(h->total_tiles, 1),
+                                          h->sms);
       std::lock_guard<std::mutex> lk(g_tune_mu);
       // a class without one goes with the largest that has: with one variant
       // for all the classes run merged
@@ -3418,7 +3440,6 @@ struct LevAdjoint {
   bool grid_ok = false;
   bool use_grid = true;
   int grid_R = 0;
-  int sms = 0;
   // per rows-per-CTA choice (64, 128, 256): SELL entries per CTA and shared
   // memory, 0 where it cannot fit, and per math mode what fits
   int g_cap[3] = {0, 0, 0};
@@ -3593,9 +3614,9 @@ const AdjFit &adj_fit(const LevAdjoint *a, int ri) {
   const long long C = (a->h_nets[0].N + R - 1) / R;
   auto fit = [&](auto pick, size_t smem, long long n) -> int {
     for (int minb = 2; minb <= 3; ++minb) {
-      if (n > (long long)minb * a->sms) continue;
+      if (n > (long long)minb * a->e->sms) continue;
       const void *fn = reinterpret_cast<const void *>(pick(R, minb, mm));
-      if ((long long)ctas_per_sm(fn, kGridThreads, smem) * a->sms >= n) return minb;
+      if ((long long)ctas_per_sm(fn, kGridThreads, smem) * a->e->sms >= n) return minb;
     }
     return 0;
   };
@@ -3622,8 +3643,7 @@ int adj_setup_grid(LevAdjoint *a, const std::vector<int> &sl_len) {
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) !=
           cudaSuccess ||
-      cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&a->sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+      cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess) {
     cudaGetLastError();
     return LEV_OK;
   }
@@ -3632,7 +3652,7 @@ int adj_setup_grid(LevAdjoint *a, const std::vector<int> &sl_len) {
   for (int ri = 0; ri < 3; ++ri) {
     const int R = kGridRs[ri];
     const int C = (d.N + R - 1) / R;
-    if (C < 2 || C > 3LL * a->sms) continue;
+    if (C < 2 || C > 3LL * a->e->sms) continue;
     long long cap = 0;
     for (int c = 0; c < C; ++c) {
       long long e = 0;

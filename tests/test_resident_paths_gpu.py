@@ -571,3 +571,27 @@ def test_reverse_segments_of_rows_that_fill_the_shared_memory(N, k, R, lo, mode)
         np.testing.assert_array_equal(a, b)
     for a, b in zip(out[1][2:], out[0][2:]):
         assert np.linalg.norm(a - b) < 3e-5 * np.linalg.norm(b)
+
+
+# tiles of 256 rows at the limits of the dependent launches on 148 SMs: 133 | 134,
+# and one wave of each kind of pair variant (two, three, four CTAs per SM)
+@pytest.mark.parametrize("tiles,variants", [(133, (4, 0)), (134, (4, 0)), (296, (6,)), (297, (6,)),
+                                            (444, (4, 0)), (445, (4, 0)), (592, (4,)),
+                                            (593, (4,))])
+def test_pair_chain_at_the_waves_of_its_variants(tiles, variants):
+    N = 256 * tiles - 3
+    net = make_network(N, 4, 0.1, 7, seed=N, delay_lo=1)
+    ref = _per_step(LeviathanEngine(*net.engine_args()))
+    want_r = ref.step_n(DT, 21)
+    want = _state(ref)
+    ref.close()
+    for v in variants:
+        e = LeviathanEngine(*net.engine_args())
+        e.set_cluster_mode(False)
+        e.set_grid_mode(False)
+        for c in range(3):
+            e.set_pair_variant(c, v)
+        r = [e.step_n(DT, 6), e.step_n(DT, 6), e.step_n(DT, 6), [e.step(DT) for _ in range(3)]]
+        np.testing.assert_array_equal(np.concatenate(r).astype(np.float32), want_r)
+        _same(_state(e), want)
+        e.close()
