@@ -3632,9 +3632,33 @@ const AdjFit &adj_fit(const LevAdjoint *a, int ri) {
   return f;
 }
 
+// Whether 128 rows per CTA are tried before 64 (adj_setup_grid).  More lanes per row
+// are more warps, and the steps wait on instructions: where both have the paired
+// backward launch, 64.  From 14,209 rows on 64 has it no more and 128 has, up to
+// 28,416, which is more for short rows and less for the accurate sine and cosine
+// until 64 needs three CTAs per SM too (18,945).  us of 200 steps forward + backward
+// at R = 64 / 128, reference and accurate:
+//   N        k = 8       k = 16      k = 20      k = 24      k = 32
+//   10^4     1,518/1,492             1,972/2,055             2,525/2,747
+//   16,000   1,861/1,644             2,311/2,277             2,879/3,017
+//   18,000   2,100/1,781 2,292/2,132 2,502/2,394 2,659/2,607 2,951/3,037
+//   24,000   2,459/2,087             3,229/2,982             4,002/4,636
+//   28,000   2,581/2,170 3,201/2,712 3,339/3,043 3,487/3,332 4,137/4,359
+//   16,000   2,007/1,820             2,512/2,673 2,917/3,172 3,309/3,716
+//   18,000   2,219/2,048 2,484/2,557 2,689/2,902 2,920/3,269 3,389/3,970
+//   24,000   2,569/2,395             3,556/3,456 3,924/4,055 4,622/5,309
+//   28,000   2,672/2,501 3,482/3,127 3,647/3,540 3,900/4,081 4,921/5,235
+bool adj_prefers_128(const LevAdjoint *a, double mean_len) {
+  const long long N = a->h_nets[0].N, sms = a->e->sms;
+  const long long C64 = (N + 63) / 64, C128 = (N + 127) / 128;
+  return a->nseg > 1 && mean_len <= 26.0 && 2 * C64 > 3 * sms && 2 * C128 <= 3 * sms &&
+         (a->e->math_mode != LEV_MATH_ACCURATE || C64 > 2 * sms) && adj_fit(a, 1).pair > 0;
+}
+
 // Grid-resident segments for a single network: per rows-per-CTA choice the
-// shared memory of both kernels, and the smallest choice whose CTAs can all be
-// resident at once.
+// shared memory of both kernels, and of the choices whose CTAs can all be
+// resident at once the smallest, or 128 (adj_prefers_128).  5*10^4 rows, k = 20, us
+// of 100 steps forward / backward: R = 128 745 / 1,980, R = 256 918 / 2,246.
 int adj_setup_grid(LevAdjoint *a, const std::vector<int> &sl_len) {
   a->grid_ok = false;
   if (a->NN != 1) return LEV_OK;
@@ -3668,12 +3692,13 @@ int adj_setup_grid(LevAdjoint *a, const std::vector<int> &sl_len) {
     a->gb_smem[ri] = sizeof(int) * 2 * (R / 32) + 16 * (size_t)cap;
     a->gb_small[ri] = sizeof(int) * 2 * (R / 32) + 8 * (size_t)cap;
     max_gpad = std::max(max_gpad, (C + 3) & ~3);
-    // the smallest: the steps wait on instructions, and more lanes per row are
-    // more warps (us per 100 steps forward / backward, k = 20: N = 10^4 R = 64 363 /
-    // 734, R = 128 460 / 740; 2*10^4 R = 64 485 / 1,198, R = 128 552 / 1,098;
-    // 5*10^4 R = 128 745 / 1,980, R = 256 918 / 2,246)
-    if (a->grid_ok || !adj_fit(a, ri).ok()) continue;
-    a->grid_R = R;
+  }
+  double sum_len = 0.0;
+  for (int l : sl_len) sum_len += l;
+  const int first = adj_prefers_128(a, sum_len / std::max<size_t>(sl_len.size(), 1)) ? 1 : 0;
+  for (int ri = first; ri < 3 && !a->grid_ok; ++ri) {
+    if (!adj_fit(a, ri).ok()) continue;
+    a->grid_R = kGridRs[ri];
     a->grid_ok = true;
   }
   if (!a->grid_ok) return LEV_OK;

@@ -595,3 +595,35 @@ def test_pair_chain_at_the_waves_of_its_variants(tiles, variants):
         np.testing.assert_array_equal(np.concatenate(r).astype(np.float32), want_r)
         _same(_state(e), want)
         e.close()
+
+
+# rows per CTA of an adjoint by default on 148 SMs: 14,208 rows are the last that have the paired
+# backward launch at 64, 28,416 at 128; 18,944 are two CTAs of 64 per SM
+@pytest.mark.parametrize("N,k,mode,segment,R,paired",
+                         [(14_208, 8, "reference", 10, 64, True),
+                          (14_209, 8, "reference", 10, 128, True),
+                          (14_209, 8, "reference", 20, 64, False),
+                          (14_209, 28, "reference", 10, 64, False),
+                          (18_944, 8, "accurate", 10, 64, False),
+                          (18_945, 8, "accurate", 10, 128, True),
+                          (28_416, 8, "reference", 10, 128, True),
+                          (28_417, 8, "reference", 10, 128, False)])
+def test_adjoint_rows_per_cta(N, k, mode, segment, R, paired):
+    net = make_network(N, k, 0.1, 6, seed=N, delay_lo=1)
+    T, out = 20, []
+    for grid in (True, False):
+        e = LeviathanEngine(*net.engine_args(), math_mode=mode)
+        adj = Adjoint(e, segment=segment, max_steps=T)
+        info = adj.grid_info()
+        assert info["enabled"] and (info["rows_per_cta"], info["paired"]) == (R, paired)
+        adj.set_grid_mode(grid)
+        p = [torch.tensor(v, dtype=torch.float32, device="cuda")
+             for v in (net.omega, net.weights, np.array([1.5]))]
+        r = adj.forward(*p, T, DT)
+        g = adj.backward(torch.ones_like(r))
+        out.append([r.cpu().numpy()] + [g[k].cpu().numpy() for k in ("omega", "w0")])
+        adj.close()
+        e.close()
+    np.testing.assert_array_equal(out[0][0], out[1][0])
+    for a, b in zip(out[0][1:], out[1][1:]):
+        assert np.linalg.norm(a - b) < REL * np.linalg.norm(b)
