@@ -627,3 +627,38 @@ def test_adjoint_rows_per_cta(N, k, mode, segment, R, paired):
     np.testing.assert_array_equal(out[0][0], out[1][0])
     for a, b in zip(out[0][1:], out[1][1:]):
         assert np.linalg.norm(a - b) < REL * np.linalg.norm(b)
+
+
+# 20,000 rows: up to three CTAs per SM; a drive win_i x(t) without a readout
+@pytest.mark.parametrize("lo,mode", [(1, "reference"), (0, "accurate")])
+def test_grid_segments_with_a_lone_reservoir_drive(lo, mode):
+    N, T = 20_000, 45
+    net = make_network(N, 6, 0.1, 9, seed=lo, delay_lo=lo)
+    rng = np.random.default_rng(5)
+    win = torch.tensor(rng.normal(size=N).astype(np.float32), device="cuda")
+    x = torch.tensor(rng.normal(size=(T, 1)).astype(np.float32), device="cuda")
+    e = LeviathanEngine(*net.engine_args(), math_mode=mode)
+    adj = Adjoint(e, segment=20, max_steps=T)
+    p = [torch.tensor(v, dtype=torch.float32, device="cuda")
+         for v in (net.omega, net.weights, np.array([1.5]))]
+    g_win = torch.empty(N, device="cuda")
+    _lib.check(adj.lib.lev_adj_set_reservoir(adj._h, win.data_ptr(), x.data_ptr(), None, None, None))
+    _lib.check(adj.lib.lev_adj_set_reservoir_grads(adj._h, None, g_win.data_ptr(), None, None))
+    out = {}
+    for R in [0] + adj.grid_info()["eligible_rows"]:
+        for paired in (True, False) if R else (False,):
+            adj.set_grid_mode(bool(R), R)
+            adj.set_grid_pairing(paired)
+            assert adj.grid_info()["enabled"] == bool(R)
+            r, th = adj.forward(*p, T, DT, record_theta=True)
+            g = adj.backward(torch.ones_like(r), torch.sin(th) / N)
+            out[R, paired] = [r, th, g["omega"], g["w0"], g_win.clone()]
+    adj.close()
+    e.close()
+    want = out.pop((0, False))
+    assert len(out) >= 4
+    for key, got in out.items():
+        for a, b in zip(got[:2], want[:2]):
+            assert torch.equal(a, b), key
+        for a, b in zip(got[2:], want[2:]):
+            assert _rel(a, b) <= REL, key
