@@ -337,7 +337,7 @@ struct AdjGridBwdArgs {
   const float *win;      // reservoir drive (xin[s]); grad_win accumulated; or null
   const float *xin;
   float *grad_win;
-  double *lam_th;
+  SplitArray lam_th;
   float *lam_thh;
   float *lam_omh;
   float *lam_w;          // SELL
@@ -469,7 +469,7 @@ __device__ __forceinline__ void adj_grid_bwd_body(const AdjGridBwdArgs &a, const
   double lt = 0.0;  // lam_th; alike in the row's lanes
   float lthh = 0.0f, lomh = 0.0f, go = 0.0f;
   if (live) {
-    lt = a.lam_th[gi];
+    lt = a.lam_th.get(gi).value();
     lthh = a.lam_thh[gi];
     lomh = a.lam_omh[gi];
     go = a.grad_omega[gi];
@@ -716,7 +716,7 @@ __device__ __forceinline__ void adj_grid_bwd_body(const AdjGridBwdArgs &a, const
   __syncthreads();
   if (*reinterpret_cast<volatile int *>(&s_ok) == 0) return;
   if (live && sl.q == 0) {
-    a.lam_th[gi] = lt;
+    a.lam_th.put(gi, SplitFloat::of(lt));
     a.lam_thh[gi] = lthh;
     a.lam_omh[gi] = lomh;
     a.grad_omega[gi] = go;

@@ -30,11 +30,12 @@
 //   prep: lam_eps -> lam_diff = lam_eps cos(diff);  lam_th(s) += lam_diff;
 //     lam_thh(s) = lam_thh(s+1) - lam_diff;  lam_omh(s) = lam_omh(s+1) + dt lam_thh(s+1)
 //   lam_g(s)   = lam_g(s+1) dg(s+1)/dg(s) + sum_i lam_th'_i dt S_i
-// lam_th and lam_g are carried from step to step in float64 (one value per node,
-// one per network): the terms of lam_g cancel to a small part of their size (N =
-// 2,000, k = 12: to 1/30), and carried in float32 dL/dK followed the roundings
-// that the order of the scatters sets off: 2.2e-6 of its value from run to run, 1.0e-6
-// now (grid-resident 0.7e-6), for 1 % of a reverse step's time.
+// lam_th and lam_g are carried from step to step in more than float32, lam_th (one
+// value per node) as a sum of two floats (SplitArray), lam_g (one per network) in
+// float64: the terms of lam_g cancel to a small part of their size (N = 2,000, k =
+// 12: to 1/30), and carried in float32 dL/dK followed the roundings that the order
+// of the scatters sets off: 2.2e-6 of its value from run to run, 1.0e-6 now
+// (grid-resident 0.7e-6).
 // The wraps have derivative 1; a clamped weight or gain passes nothing;
 // |eps| has derivative sign(eps).  The adjoint ring has max_delay+3 slots: the
 // slot finalised by a reverse step (time s+1) is not one that the same step
@@ -473,6 +474,40 @@ __global__ void __launch_bounds__(4 * kTile, 1) adj_fwd_split_kernel(const AdjFw
   }
 }
 
+// A value of about 48 bits as the sum of two floats, high = RN(high + low).  add:
+// the exact error of a float addition (Knuth's two-sum) goes to the low part; an
+// infinite or NaN sum has none.
+struct SplitFloat {
+  float high, low;
+  static __device__ __forceinline__ SplitFloat of(double x) {
+    const float h = (float)x;
+    return {h, isfinite(h) ? (float)(x - h) : 0.0f};
+  }
+  __device__ __forceinline__ double value() const { return (double)high + low; }
+  __device__ __forceinline__ void add(float x) {
+    const float t = __fadd_rn(high, x), b = __fsub_rn(t, high);
+    const float err = __fadd_rn(__fsub_rn(high, __fsub_rn(t, b)), __fsub_rn(x, b));
+    const float l = __fadd_rn(low, err);
+    high = __fadd_rn(t, l);
+    low = __fsub_rn(l, __fsub_rn(high, t));
+    if (!isfinite(t)) {
+      high = t;
+      low = 0.0f;
+    }
+  }
+};
+// Such values in two arrays.  A reverse step of 16 networks of 20,000 rows takes 111.7
+// us; with one array of eight-byte values 121, with the arrays loaded after the
+// readout's terms 124.5, with plain floats 111.3.
+struct SplitArray {
+  float *high, *low;
+  __device__ __forceinline__ SplitFloat get(long long i) const { return {high[i], low[i]}; }
+  __device__ __forceinline__ void put(long long i, SplitFloat x) const {
+    high[i] = x.high;
+    low[i] = x.low;
+  }
+};
+
 struct AdjBwdArgs {
   const NetDesc *nets;  // adjoint copies (ring_off: history ring, aux_off: adjoint ring)
   const int2 *tiles;
@@ -487,7 +522,7 @@ struct AdjBwdArgs {
   const float4 *trace; // per network (g_s, r_{s+1}, sum cos, sum sin)
   const float *dLdr;   // per network dL/dr(s+1), or null
   const float *dLdth;  // [total nodes] dL/dtheta(s+1), or null
-  double *lam_th;      // current-phase adjoint: in time s+1, out time s
+  SplitArray lam_th;   // current-phase adjoint: in time s+1, out time s
   float *lam_thh;
   float *lam_omh;
   float *lam_w;        // SELL
@@ -553,26 +588,28 @@ __global__ void __launch_bounds__(kTile, MINB) adj_bwd_kernel(const AdjBwdArgs a
   const float Cm = tr.z * invN, Sm = tr.w * invN;
 
   double lg_part = 0.0;
+  SplitFloat lt = {0.0f, 0.0f};  // lam_th'
   float lt1 = 0.0f, th = 0.0f, eps = 0.0f, diff = 0.0f, lam_S = 0.0f;
   int deg = 0;
   if (live) {
     // (A) adjoint of theta(s+1), complete
     const float th1 = H[(long long)(hs + 1) * Np + row];
     float* slot_next = AR + (long long)as_next * Np + row;
-    double ltd = a.lam_th[gi] + *slot_next;
+    lt = a.lam_th.get(gi);  // with the other loads, before the first store
+    float add = *slot_next;
     *slot_next = 0.0f;
     float sn, cs;
     sincosf(th1, &sn, &cs);
-    if (r1 > 0.0f) ltd += lam_r * (Sm * cs - Cm * sn) * invN / r1;
-    if (a.dLdth) ltd += a.dLdth[gi];
+    if (r1 > 0.0f) add += lam_r * (Sm * cs - Cm * sn) * invN / r1;
+    if (a.dLdth) add += a.dLdth[gi];
     if (a.dLdy) {  // readout y = sum ra cos theta + rb sin theta
       const float gy = a.dLdy[tile.x];
-      ltd += gy * (a.rb[gi] * cs - a.ra[gi] * sn);
+      add += gy * (a.rb[gi] * cs - a.ra[gi] * sn);
       a.grad_ra[gi] += gy * cs;
       a.grad_rb[gi] += gy * sn;
     }
-    a.lam_th[gi] = ltd;  // read back below: no registers held over the walk
-    lt1 = (float)ltd;
+    lt.add(add);
+    lt1 = lt.high;
     // (B) integrate
     lam_S = lt1 * dt * g_s;
     a.grad_omega[gi] += lt1 * dt;
@@ -644,7 +681,8 @@ __global__ void __launch_bounds__(kTile, MINB) adj_bwd_kernel(const AdjBwdArgs a
     const float lthh1 = a.lam_thh[gi], lomh1 = a.lam_omh[gi];
     const float leps = -lt1 * dt * nd.alpha + labs * sgn + lomh1 * nd.kappa_w * dt;
     const float ldiff = leps * cosf(diff);
-    a.lam_th[gi] += lsum + ldiff;
+    lt.add(lsum + ldiff);
+    a.lam_th.put(gi, lt);
     a.lam_thh[gi] = lthh1 - ldiff;
     a.lam_omh[gi] = lomh1 + lthh1 * dt;
     lg_part = (double)lt1 * dt * S_i;
@@ -741,7 +779,7 @@ __global__ void __launch_bounds__(kTile, 4) adj_bwd_split_kernel(const AdjBwdArg
       // (A) adjoint of theta(s+1), complete; (B) integrate
       const float th1 = H[(long long)(hs + 1) * Np + row];
       float *slot_next = AR + (long long)as_next * Np + row;
-      ltd = a.lam_th[gi] + *slot_next;
+      ltd = a.lam_th.get(gi).value() + *slot_next;
       *slot_next = 0.0f;
       float sn, cs;
       sincosf(th1, &sn, &cs);
@@ -825,7 +863,7 @@ __global__ void __launch_bounds__(kTile, 4) adj_bwd_split_kernel(const AdjBwdArg
     const float lthh1 = a.lam_thh[gi], lomh1 = a.lam_omh[gi];
     const float leps = -lt1 * dt * nd.alpha + labs * sgn + lomh1 * nd.kappa_w * dt;
     const float ldiff = leps * cosf(diff);
-    a.lam_th[gi] = ltd + (lsum + ldiff);
+    a.lam_th.put(gi, SplitFloat::of(ltd + (lsum + ldiff)));
     a.lam_thh[gi] = lthh1 - ldiff;
     a.lam_omh[gi] = lomh1 + lthh1 * dt;
     lg_part = (double)lt1 * dt * S_i;
@@ -891,7 +929,7 @@ __global__ void adj_ring_ckpt_kernel(bool restore, const NetDesc *__restrict__ n
 // Final adjoint of theta(0): current part plus every adjoint-ring slot (reads
 // of times <= 0 all read theta(0), the value every slot starts with).
 __global__ void adj_finalize_kernel(const NetDesc *nets, int num_nets,
-                                    const double *lam_th, const float *adj_ring,
+                                    const SplitArray lam_th, const float *adj_ring,
                                     float *grad_theta0) {
   const int n = blockIdx.y;
   if (n >= num_nets) return;
@@ -899,7 +937,7 @@ __global__ void adj_finalize_kernel(const NetDesc *nets, int num_nets,
   const int bsa = adj_slots(nd.max_delay);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nd.N;
        i += gridDim.x * blockDim.x) {
-    double v = lam_th[nd.node_off + i];
+    double v = lam_th.get(nd.node_off + i).value();
     for (int s = 0; s < bsa; ++s) v += adj_ring[nd.aux_off + (long long)s * nd.Np + i];
     grad_theta0[nd.node_off + i] = (float)v;
   }

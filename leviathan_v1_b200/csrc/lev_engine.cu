@@ -3419,7 +3419,8 @@ struct LevAdjoint {
   float *lam_thh = nullptr, *lam_omh = nullptr,
         *lam_w = nullptr, *adj_ring = nullptr,
         *grad_omega_acc = nullptr, *grad_theta0 = nullptr;
-  double *lam_th = nullptr, *lam_g = nullptr;
+  float *lam_th = nullptr;  // [2][TN], see SplitArray
+  double *lam_g = nullptr;
   std::vector<std::pair<void **, size_t>> wanted;  // see adj_commit
   std::vector<void *> allocs;
   size_t bytes = 0;
@@ -3538,6 +3539,8 @@ int adj_launch_fwd(LevAdjoint *a, const AdjFwdArgs &f, cudaStream_t s = nullptr)
   LEV_TRY_CUDA(cudaGetLastError());
   return LEV_OK;
 }
+
+inline SplitArray adj_lam_th(const LevAdjoint *a) { return {a->lam_th, a->lam_th + a->TN}; }
 
 // The ring part of checkpoint `seg`, saved from or restored into `ring`.
 void adj_ring_ckpt(LevAdjoint *a, int seg, bool restore, float *ring, cudaStream_t s) {
@@ -3808,7 +3811,7 @@ void adj_grid_fill_bwd(LevAdjoint *a, AdjGridBwdArgs &b) {
   b.sl_off = e->d_sl_off;
   b.sl_len = e->d_sl_len;
   b.sl_cd = e->d_sl_cd;
-  b.lam_th = a->lam_th;
+  b.lam_th = adj_lam_th(a);
   b.lam_thh = a->lam_thh;
   b.lam_omh = a->lam_omh;
   b.lam_w = a->lam_w;
@@ -3932,7 +3935,7 @@ int lev_adj_create(LevAdjoint **out, LevEngine *e, int32_t segment,
   A(a->trace, C * NN);
   const bool dj_rec = e->total_tiles > 148;  // adj_fwd_kernel / adj_bwd_kernel
   if (dj_rec) A(a->dj_hist, C * SL);
-  A(a->lam_th, TN); A(a->lam_thh, TN); A(a->lam_omh, TN);
+  A(a->lam_th, 2 * TN); A(a->lam_thh, TN); A(a->lam_omh, TN);
   A(a->lam_w, SL);
   A(a->adj_ring, a->aux_floats);
   A(a->lam_g, NN);
@@ -4336,7 +4339,7 @@ int lev_adj_backward(LevAdjoint *a, const float *dLdr, const float *dLdtheta,
     b.sl_len = e->d_sl_len;
     b.sl_cd = e->d_sl_cd;
     b.H = rings[buf];
-    b.lam_th = a->lam_th;
+    b.lam_th = adj_lam_th(a);
     b.lam_thh = a->lam_thh;
     b.lam_omh = a->lam_omh;
     b.lam_w = a->lam_w;
@@ -4402,7 +4405,7 @@ int lev_adj_backward(LevAdjoint *a, const float *dLdr, const float *dLdtheta,
   }  // per-step launches
   // gradients
   dim3 grid(64, a->NN);
-  adj_finalize_kernel<<<grid, 256, 0, s>>>(a->d_nets, a->NN, a->lam_th, a->adj_ring,
+  adj_finalize_kernel<<<grid, 256, 0, s>>>(a->d_nets, a->NN, adj_lam_th(a), a->adj_ring,
                                            a->grad_theta0);
   if (grad_omega) {
     // omega enters directly and through omega_hat(0) = omega
