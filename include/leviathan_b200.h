@@ -407,7 +407,7 @@ int lev_adj_set_reservoir_grads(LevAdjoint *a, const float *dLdy,
  * rows_per_cta 0 keeps the current choice.  When a second segment record set
  * fits and both CTA groups fit on the device at once, the backward pass
  * recomputes segment k-1 and reverses segment k in ONE paired launch (two
- * CTA groups, one barrier counter each); *paired tells whether it does;
+ * CTA groups with counters of their own); *paired tells whether it does;
  * lev_adj_set_grid_pairing(a, 0) makes the two separate launches again. */
 int lev_adj_grid_info(const LevAdjoint *a, int32_t *eligible, int32_t *enabled,
                       int32_t *rows_per_cta, int32_t *eligible_rows_mask, int32_t *paired);

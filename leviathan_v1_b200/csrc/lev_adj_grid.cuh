@@ -741,7 +741,7 @@ __global__ void __launch_bounds__(kGridThreads, MINB) adj_grid_bwd_kernel(const 
 
 // Paired launch of the backward pass: CTAs [0, gf) recompute segment k-1
 // into one record set while CTAs [gf, grid) reverse segment k from the
-// other; each group has its own arrival counter and shares the SMs with the
+// other; each group has its own arrival counters and shares the SMs with the
 // other, so the two latency-bound step chains overlap.  Every CTA of both
 // groups is resident at once (cooperative launch).
 template <int MATH, int R, int MINB>

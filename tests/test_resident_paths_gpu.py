@@ -7,7 +7,8 @@ Forward results, hub counts and weight conversions are compared with the
 per-step kernels bit for bit.  Gradients are compared at a relative difference
 of 1e-5: between paths only the order of the sums over edges and of the
 float32 scatters differs (some tens of terms of one sign pattern each, so a few
-1e-7 per sum).
+1e-7 per sum; dL/dK, a sum over nodes and steps that cancels, has differed by
+5.7e-6 in 60,000 pairs of runs).
 """
 
 import numpy as np
