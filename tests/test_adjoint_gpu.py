@@ -226,3 +226,38 @@ def test_gain_gradient_does_not_follow_the_scatter_order(grid):
     adj.close()
     eng.close()
     assert np.std(out) < 1.5e-6 * abs(np.mean(out)), np.std(out) / abs(np.mean(out))
+
+
+# 2 tiles each: 160 and 900 tiles, the two kinds of reverse kernel with one lane per row
+@pytest.mark.parametrize("copies,mode", [(80, "reference"), (80, "accurate"),
+                                         (450, "reference"), (450, "accurate")])
+def test_large_batches_equal_separate_networks(copies, mode):
+    """The sums over a row's edges and the scatters come in another order than
+    with four lanes per row: a few 1e-7 of a gradient's norm."""
+    kinds = [make_network(300 + 50 * s, 6 + 2 * s, 0.1, 15, seed=s, delay_lo=s % 2) for s in range(3)]
+    T = 60
+    dr = torch.linspace(-1, 1, T, device="cuda")[:, None]
+
+    def grads(eng, nets):
+        adj = Adjoint(eng, segment=25, max_steps=T)
+        adj.set_grid_mode(False)
+        om, w0 = (torch.tensor(np.concatenate([getattr(n, k) for n in nets]), device="cuda")
+                  for k in ("omega", "weights"))
+        K = torch.full((len(nets),), 1.5, device="cuda")
+        r, th = adj.forward(om, w0, K, T, DT, record_theta=True)
+        g = adj.backward(dr.expand(T, len(nets)).contiguous(), torch.sin(th) / 300)
+        adj.close()
+        eng.close()
+        return r.cpu().numpy(), {k: g[k].cpu().numpy() for k in ("omega", "w0", "K")}
+
+    want = [grads(LeviathanEngine(*n.engine_args(), math_mode=mode), [n]) for n in kinds]
+    nets = [kinds[i % 3] for i in range(copies)]
+    r, g = grads(BatchEngine([n.as_dict() for n in nets], math_mode=mode), nets)
+    at = at_w = 0
+    for i, n in enumerate(nets):
+        r1, g1 = want[i % 3]
+        np.testing.assert_array_equal(r[:, i], r1[:, 0])
+        assert _rel(g["omega"][at:at + n.N], g1["omega"]) < 1e-5
+        assert _rel(g["w0"][at_w:at_w + n.E], g1["w0"]) < 1e-5
+        assert abs(g["K"][i] - g1["K"][0]) < 1e-5 * abs(g1["K"][0])
+        at, at_w = at + n.N, at_w + n.E
